@@ -6,9 +6,8 @@
 //    :246-270) divides by min(k, count - 1) and falls back to the search
 //    radius for isolated points;
 //  * global mean / std (:43-55): the reference sums sequentially in float,
-//    so one lane per frame adds the values in input order (a parallel tree
-//    sum would round differently and move the threshold), fed through
-//    shared memory by its warp;
+//    and a sum in another order would round differently and move the
+//    threshold; k_sor_stats reproduces those roundings in parallel;
 //  * keep mean <= mu + alpha * sigma and copy kept points out in input order
 //    (flag scan + scatter).
 #include "internal.cuh"
@@ -46,79 +45,236 @@ __global__ void k_sor_mean(const u64 *pairs, int kk, const int32_t *counts, size
   }
 }
 
-// One warp per frame: lanes stage 1024 consecutive values in shared memory
-// (coalesced), then lane 0 adds them in input order -- the same sequence of
-// roundings as the reference's loop, without one global load per add.
-constexpr int ST_CHUNK = 1024;
-// One block of two warps per frame: warp 1 stages the next chunk of means
-// in shared memory while lane 0 of warp 0 adds up the current one in input
-// order (the reference's sequential float sums), four values per load.
-__global__ __launch_bounds__(64) void k_sor_stats_warp(const float *__restrict__ mean,
-                                                       const int64_t *offs, int n_frames,
-                                                       float alpha, float *thresh) {
-  __shared__ __align__(16) float buf[2][ST_CHUNK];
-  __shared__ float s_mu;
+// The reference's sequential float sums, added in parallel. While the running
+// sum A stays in one binade [2^e, 2^(e+1)) it is an integer S times its unit
+// u = 2^(e-23), and adding v >= 0, v = (q + r) u, moves S by an integer: q
+// (r < 1/2), q + 1 (r > 1/2), or, on a tie, to the even neighbour. Without
+// ties the moves do not depend on S: they are summed (exactly, as floats
+// below 2^24 u) by a block scan. With a tie among them every value becomes a
+// pair of increments (S even, S odd), which compose associatively, and the
+// scan runs over the pairs. Either way S after every value has exactly the
+// roundings of the loop. The thread in whose run S first reaches 2^24 (the
+// next binade) adds its own values one by one in float, and the rest of the
+// chunk is scanned again from there: about log2(n) times over the whole sum,
+// so the chunks start at 512 values and double up to 8192.
+//   Bound by one SM's issue and the scans' latency (a block per frame): 89,343
+// values 544 us with one lane adding in order (a dependent add per value),
+// 123 us here; 256 frames of 11 M values 379 and 182 us.
+constexpr int ST_TH = 512, ST_IT = 16, ST_CHUNK = ST_TH * ST_IT;
+constexpr u32 ST_TOP = 1u << 24, ST_CAP = 1u << 30;
+
+struct Incr {  // increments of S when it is even / odd, capped at ST_CAP
+  u32 a, b;
+};
+__device__ __forceinline__ Incr incr_then(const Incr &f, const Incr &g) {
+  const u32 x = f.a + ((f.a & 1) ? g.b : g.a);
+  const u32 y = f.b + ((f.b & 1) ? g.a : g.b);  // odd S: parity flips with f.b
+  return Incr{x < ST_CAP ? x : ST_CAP, y < ST_CAP ? y : ST_CAP};
+}
+// exponent field and 24-bit significand of a float >= 0: v = m * 2^(e - 150)
+// (denormals share the smallest normal exponent)
+__device__ __forceinline__ int st_exp(float v) { return max((int)(__float_as_uint(v) >> 23), 1); }
+__device__ __forceinline__ u32 st_sig(float v) {
+  const u32 b = __float_as_uint(v);
+  return (b & 0x7FFFFFu) | (b >= 0x800000u ? 0x800000u : 0u);
+}
+// the increments of S by v, S in units of 2^(ex - 150)
+__device__ __forceinline__ Incr incr_of(float v, int ex) {
+  const u32 m = st_sig(v);
+  const int s = ex - st_exp(v);  // low bits of v below the unit
+  if (s <= 0) {
+    const u32 q = s >= -6 ? m << -s : (m ? ST_CAP : 0u);
+    return Incr{q, q};
+  }
+  if (s > 25) return Incr{0, 0};
+  const u32 q = m >> s, r = m & ((1u << s) - 1u), half = 1u << (s - 1);
+  if (r != half) {
+    const u32 i = q + (r > half ? 1u : 0u);
+    return Incr{i, i};
+  }
+  return Incr{q + (q & 1), q + ((q & 1) ^ 1)};
+}
+
+__global__ __launch_bounds__(ST_TH) void k_sor_stats(const float *__restrict__ mean,
+                                                     const int64_t *offs, int n_frames,
+                                                     float alpha, float *thresh) {
+  __shared__ float buf[ST_CHUNK + ST_CHUNK / ST_IT];  // a gap per run: no bank conflicts
+  __shared__ Incr warp_tot[ST_TH / 32];
+  __shared__ float warp_sum[ST_TH / 32];
+  __shared__ float s_acc;
+  __shared__ int s_next;
   const int f = blockIdx.x;
   if (f >= n_frames) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int64_t a = offs[f], b = offs[f + 1];
-  const int64_t n = b - a;
+  const int64_t a = offs[f], n = offs[f + 1] - a;
   if (n <= 0) {
     if (tid == 0) thresh[f] = 0.0f;
     return;
   }
-  const int nch = (int)((n + ST_CHUNK - 1) / ST_CHUNK);
-  auto stage = [&](int c) {
-    const int64_t base = a + (int64_t)c * ST_CHUNK;
-    const int m = (int)((b - base) < ST_CHUNK ? (b - base) : ST_CHUNK);
-    float *dst = buf[c & 1];
-    for (int j = lane; j < m; j += 32) dst[j] = __ldg(&mean[base + j]);
-  };
-  float acc = 0.0f;
+  mean += a;
+  float mu = 0.0f;
   for (int pass = 0; pass < 2; ++pass) {
-    const float mu = pass ? s_mu : 0.0f;
-    if (warp == 1) stage(0);
-    __syncthreads();
-    for (int c = 0; c < nch; ++c) {
-      if (warp == 1 && c + 1 < nch) stage(c + 1);
-      if (tid == 0) {
-        const int m = (int)((n - (int64_t)c * ST_CHUNK) < ST_CHUNK ? (n - (int64_t)c * ST_CHUNK)
-                                                                   : ST_CHUNK);
-        const float *src = buf[c & 1];
-        const float4 *src4 = reinterpret_cast<const float4 *>(src);
-        int t = 0;
-        for (; t + 4 <= m; t += 4) {
-          const float4 v = src4[t >> 2];
-          if (pass == 0) {
-            acc = fadd(acc, v.x); acc = fadd(acc, v.y); acc = fadd(acc, v.z); acc = fadd(acc, v.w);
-          } else {
-            float d = fsub(v.x, mu); acc = fadd(acc, fmul(d, d));
-            d = fsub(v.y, mu); acc = fadd(acc, fmul(d, d));
-            d = fsub(v.z, mu); acc = fadd(acc, fmul(d, d));
-            d = fsub(v.w, mu); acc = fadd(acc, fmul(d, d));
+    float acc = 0.0f;
+    float nxt[ST_IT];
+    auto chunk_at = [&](int64_t base) {
+      const int64_t len = base < 512 ? 512 : (base < ST_CHUNK ? base : ST_CHUNK);
+      return (int)(n - base < len ? n - base : len);
+    };
+    auto fetch = [&](int64_t base) {
+      const int m = base < n ? chunk_at(base) : 0;
+#pragma unroll
+      for (int j = 0; j < ST_IT; ++j) {
+        const int i = j * ST_TH + tid;
+        nxt[j] = i < m ? __ldg(&mean[base + i]) : mu;
+      }
+    };
+    fetch(0);
+    for (int64_t base = 0; base < n;) {
+      const int m = chunk_at(base);
+      bool odd = false;  // a value the increments cannot express
+#pragma unroll
+      for (int j = 0; j < ST_IT; ++j) {
+        const int i = j * ST_TH + tid;
+        if (j * ST_TH >= m) break;  // (uniform) rows past the chunk's end
+        float v = nxt[j];
+        if (pass == 1) {
+          v = fsub(v, mu);
+          v = fmul(v, v);
+        }
+        odd = odd || !(v >= 0.0f && v < INFINITY);
+        buf[i + i / ST_IT] = v;
+      }
+      odd = __syncthreads_or(odd) || !(acc < INFINITY);
+      base += m;
+      if (odd) {  // (infinities, NaN, negative values): one lane, in order
+        if (tid == 0) {
+          float s = acc;
+          for (int i = 0; i < m; ++i) s = fadd(s, buf[i + i / ST_IT]);
+          s_acc = s;
+        }
+        fetch(base);
+        __syncthreads();
+        acc = s_acc;
+        continue;
+      }
+      const int runs = (m + ST_IT - 1) / ST_IT;  // threads with values
+      float v[ST_IT];
+#pragma unroll
+      for (int j = 0; j < ST_IT; ++j) v[j] = tid < runs ? buf[tid * (ST_IT + 1) + j] : 0.0f;
+      fetch(base);
+      int from = 0;  // threads before it are added already
+      while (from < runs) {
+        const int ex = st_exp(acc);
+        const bool mine = tid >= from && tid < runs;
+        // moves without ties: rounded to units by adding and taking away
+        // 1.5 * 2^23 u, which needs v < 2^22 u
+        const float magic = __uint_as_float(((u32)ex << 23) | 0x400000u);
+        const float top = __uint_as_float((u32)(ex + 1) << 23);  // 2^24 u (inf past the last)
+        const float half = ex > 30 ? __uint_as_float((u32)(ex - 24) << 23) : 0.0f;  // u / 2
+        const float most = __uint_as_float((u32)(ex - 1) << 23);  // 2^22 u
+        float sum = 0.0f;
+        bool hard = ex <= 30;
+        if (mine) {
+#pragma unroll
+          for (int j = 0; j < ST_IT; ++j) {
+            const float q = fsub(fadd(v[j], magic), magic);
+            hard = hard || fabsf(fsub(v[j], q)) == half || !(v[j] < most);
+            sum = fadd(sum, q);
           }
         }
-        for (; t < m; ++t) {
-          if (pass == 0) {
-            acc = fadd(acc, src[t]);
-          } else {
-            const float d = fsub(src[t], mu);
-            acc = fadd(acc, fmul(d, d));
+        float incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const float p = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl = fadd(p, incl);
+        }
+        if (lane == 31) warp_sum[warp] = incl;
+        hard = __syncthreads_or(hard);
+        float pre_acc, end_acc, all_acc;  // the sum before and after this run, and at the end
+        if (!hard) {
+          float before = 0.0f, total = 0.0f;
+#pragma unroll
+          for (int w = 0; w < ST_TH / 32; ++w) {
+            if (w == warp) before = total;
+            total = fadd(total, warp_sum[w]);
           }
+          float pre = __shfl_up_sync(0xffffffffu, incl, 1);
+          pre = fadd(before, lane == 0 ? 0.0f : pre);
+          pre_acc = fadd(acc, pre);
+          end_acc = fadd(acc, fadd(before, incl));
+          all_acc = fadd(acc, total);
+        } else {
+          const u32 s0 = st_sig(acc);
+          auto to_float = [&](u32 t) {  // below 2^24: in acc's binade; else past it
+            return t >= ST_TOP ? top
+                               : __uint_as_float(t >= 0x800000u ? ((u32)ex << 23) | (t & 0x7FFFFFu)
+                                                                : t);
+          };
+          Incr run{0, 0};
+          if (mine) {
+            Incr t[ST_IT];
+#pragma unroll
+            for (int j = 0; j < ST_IT; ++j) t[j] = incr_of(v[j], ex);
+#pragma unroll
+            for (int w = 1; w < ST_IT; w <<= 1)  // pairwise, in order: a short chain
+#pragma unroll
+              for (int j = 0; j < ST_IT; j += 2 * w) t[j] = incr_then(t[j], t[j + w]);
+            run = t[0];
+          }
+          Incr upto = run;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            Incr p;
+            p.a = __shfl_up_sync(0xffffffffu, upto.a, o);
+            p.b = __shfl_up_sync(0xffffffffu, upto.b, o);
+            if (lane >= o) upto = incr_then(p, upto);
+          }
+          if (lane == 31) warp_tot[warp] = upto;
+          __syncthreads();
+          Incr before{0, 0}, total{0, 0};
+#pragma unroll
+          for (int w = 0; w < ST_TH / 32; ++w) {
+            if (w == warp) before = total;
+            total = incr_then(total, warp_tot[w]);
+          }
+          Incr pre;  // everything before this thread's run
+          pre.a = __shfl_up_sync(0xffffffffu, upto.a, 1);
+          pre.b = __shfl_up_sync(0xffffffffu, upto.b, 1);
+          if (lane == 0) pre = Incr{0, 0};
+          pre = incr_then(before, pre);
+          const Incr end = incr_then(pre, run);
+          const bool p0 = s0 & 1;
+          pre_acc = to_float(s0 + (p0 ? pre.b : pre.a));
+          end_acc = to_float(s0 + (p0 ? end.b : end.a));
+          all_acc = to_float(s0 + (p0 ? total.b : total.a));
+        }
+        if (all_acc < top) {
+          acc = all_acc;
+          break;
+        }
+        if (mine && pre_acc < top && !(end_acc < top)) {  // one thread
+          float s = pre_acc;
+#pragma unroll
+          for (int j = 0; j < ST_IT; ++j) s = fadd(s, v[j]);
+          s_acc = s;
+          s_next = tid + 1;
+        }
+        __syncthreads();
+        acc = s_acc;
+        from = s_next;
+        if (!(acc < INFINITY)) {  // overflow: every later sum is infinite too
+          acc = INFINITY;
+          break;
         }
       }
-      __syncthreads();
+      __syncthreads();  // buf and the warps' totals are refilled
     }
-    if (tid == 0) {
-      if (pass == 0) {
-        s_mu = fdiv(acc, (float)n);
-        acc = 0.0f;
-      } else {
-        const float sd = __fsqrt_rn(fdiv(acc, (float)n));
-        thresh[f] = fadd(s_mu, fmul(alpha, sd));
-      }
+    if (pass == 0) {
+      mu = fdiv(acc, (float)n);
+    } else if (tid == 0) {
+      const float sd = __fsqrt_rn(fdiv(acc, (float)n));
+      thresh[f] = fadd(mu, fmul(alpha, sd));
     }
-    __syncthreads();
   }
 }
 
@@ -193,8 +349,8 @@ void sor_filter_frames(rvp_context *ctx, const float *x, const float *y, const f
   p += al((size_t)(n_frames + 1) * 4);
   void *scan_tmp = p;
   cudaStream_t st = ctx->stream;
-  k_sor_stats_warp<<<(unsigned)(n_frames > 0 ? n_frames : 1), 64, 0, st>>>(mean, offs, n_frames,
-                                                                         alpha, thresh);
+  k_sor_stats<<<(unsigned)(n_frames > 0 ? n_frames : 1), ST_TH, 0, st>>>(mean, offs, n_frames,
+                                                                       alpha, thresh);
   RVP_LAUNCH_CHECK(ctx);
   k_sor_keep<<<grid_for(n_max, 256, ctx->num_sms * 16), 256, 0, st>>>(mean, offs, n_frames, n_max,
                                                                      n_dev, thresh, keep, flags);
