@@ -27,3 +27,15 @@ def test_sor_statistics_sum_in_order(gpu_ctx, restatement, n, cloud):
     out2, mean2, keep2 = restatement.sor_exact(c, 3, 0.5)
     assert np.array_equal(bits(mean), bits(mean2))
     assert np.array_equal(keep, keep2) and np.array_equal(bits(out), bits(out2))
+
+
+# the voxel grid sorts its keys: up to 148 x 4096 of them in one cooperative
+# kernel (512 threads, up to eight keys each), more in tiles of 4096
+@pytest.mark.parametrize("n", [1, 31, 513, 4097, 75_777, 606_208, 606_209, 2_424_833])
+def test_sorted_voxels(gpu_ctx, restatement, n):
+    from rvpoint_b200.api import voxel_grid_downsamp_rvv_v2
+    rng = np.random.default_rng(n)
+    c = D.Cloud.from_xyz(rng.uniform(-40, 40, (n, 3)) * [1.0, 0.5, 0.02])
+    out, keys = voxel_grid_downsamp_rvv_v2(c, 0.25, return_keys=True)
+    out2, keys2 = restatement.voxel_grid(c, 0.25)
+    assert np.array_equal(keys, keys2) and np.array_equal(bits(out), bits(out2))
