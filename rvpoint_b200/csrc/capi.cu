@@ -91,7 +91,9 @@ struct rvp_hash {
   float cell = 0.0f;
   long long p1 = 73856093LL, p2 = 19349663LL;
   rvp::Grid grid;
-  bool has_cloud = false, built = false;
+  rvp::KnnTree tree;  // k nearest: built by the first search that needs it
+  rvp::TreeView tree_view{};
+  bool has_cloud = false, built = false, tree_built = false;
   int collision = 0;
 };
 
@@ -174,18 +176,17 @@ __global__ void k_unpack(const u64 *pairs, size_t total, int32_t *idx, float *d2
 }
 
 // fixed-stride rows (nq x K, counts[q] valid) -> CSR rows
-__global__ void k_rows_to_csr(const u64 *pairs, int K, const int32_t *counts, const u64 *offs,
-                              size_t nq, int cut, int32_t *idx, float *d2) {
+__global__ void k_rows_to_csr(const int32_t *row_idx, const float *row_d2, int K,
+                              const int32_t *counts, const u64 *offs, size_t nq, int32_t *idx,
+                              float *d2) {
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < nq * (size_t)K;
        t += (size_t)gridDim.x * blockDim.x) {
     const size_t q = t / K;
     const int j = (int)(t % K);
-    const int c = min(counts[q], cut);
-    if (j >= c) continue;
-    const u64 k = pairs[t];
+    if (j >= counts[q]) continue;
     const u64 o = offs[q] + j;
-    idx[o] = (int32_t)(u32)(k & 0x7FFFFFFFull);
-    d2[o] = __uint_as_float((u32)(k >> 32));
+    idx[o] = row_idx[t];
+    d2[o] = row_d2[t];
   }
 }
 
@@ -215,115 +216,41 @@ __global__ void k_i32_to_u32(const int32_t *in, size_t n, u32 *out) {
     out[i] = (u32)max(in[i], 0);
 }
 
-__global__ void k_fill_rows(const u64 *pairs, int K, const int32_t *counts, size_t nq,
-                            int32_t *idx, float *d2) {
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < nq * (size_t)K;
-       t += (size_t)gridDim.x * blockDim.x) {
-    const size_t q = t / K;
-    const int j = (int)(t % K);
-    if (j < counts[q]) {
-      const u64 k = pairs[t];
-      if (idx) idx[t] = (int32_t)(u32)(k & 0x7FFFFFFFull);
-      if (d2) d2[t] = __uint_as_float((u32)(k >> 32));
-    } else {
-      if (idx) idx[t] = -1;
-      if (d2) d2[t] = INFINITY;
-    }
-  }
+// one scratch tree per context, kept across calls so its buffers are reused
+rvp::KnnTree &ctx_tree(rvp_context *ctx) {
+  if (!ctx->tree) ctx->tree = new rvp::KnnTree();
+  return *ctx->tree;
 }
 
-__global__ void k_bbox_simple(const float *x, const float *y, const float *z, size_t n,
-                              float *bb) {
-  float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const float v[3] = {x[i], y[i], z[i]};
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      mn[a] = fminf(mn[a], v[a]);
-      mx[a] = fmaxf(mx[a], v[a]);
-    }
-  }
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    for (int o = 16; o; o >>= 1) {
-      mn[a] = fminf(mn[a], __shfl_xor_sync(0xffffffffu, mn[a], o));
-      mx[a] = fmaxf(mx[a], __shfl_xor_sync(0xffffffffu, mx[a], o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-      rvp::atomic_min_f(&bb[a], mn[a]);
-      rvp::atomic_max_f(&bb[3 + a], mx[a]);
-    }
-  }
+// the k nearest of every point of a device cloud
+void knn_cloud(rvp_context *ctx, const float *x, const float *y, const float *z, size_t n, int K,
+               int mode, const rvp::TreeOut &o) {
+  rvp::KnnTree &w = ctx_tree(ctx);
+  const rvp::TreeView t = rvp::tree_build(ctx, w, x, y, z, n);
+  rvp::tree_knn(ctx, t, rvp::tree_queries(ctx, w, t, x, y, z, x, y, z, n), K, 0.0f, mode, o);
 }
 
-// ---------------------------------------------------------------------------
-// kNN over a device cloud with an automatically chosen cell: build on a
-// volume-based guess, measure the k-th neighbour distance of a sample of
-// queries, rebuild with cell = median k-th distance (the 27-cell ring then
-// usually certifies the answer).
-// ---------------------------------------------------------------------------
-float auto_cell(rvp_context *ctx, rvp::Grid &g, const float *x, const float *y, const float *z,
-                size_t n, const int64_t *offs_dev, int K) {
-  float *bb = static_cast<float *>(scratch(ctx, 20, 64));
-  float init[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
-  RVP_CUDA_TRY(cudaMemcpyAsync(bb, init, 24, cudaMemcpyHostToDevice, ctx->stream));
-  k_bbox_simple<<<rvp::grid_for(n, 256, ctx->num_sms * 4), 256, 0, ctx->stream>>>(x, y, z, n, bb);
-  RVP_LAUNCH_CHECK(ctx);
-  float h[6];
-  RVP_CUDA_TRY(cudaMemcpyAsync(h, bb, 24, cudaMemcpyDeviceToHost, ctx->stream));
-  sync(ctx);
-  double ext[3];
-  for (int a = 0; a < 3; ++a) ext[a] = std::max(1e-6, (double)h[3 + a] - (double)h[a]);
-  const double V = ext[0] * ext[1] * ext[2];
-  double c0 = cbrt(V * (double)K / (double)std::max<size_t>(n, 1));
-  const double emax = std::max(ext[0], std::max(ext[1], ext[2]));
-  c0 = std::min(c0, emax);
-  if (!(c0 > 0)) c0 = 1.0;
-  const size_t S = std::min<size_t>(n, 1024);
-  if (S < 8) return (float)c0;
-  rvp::grid_build(ctx, g, x, y, z, offs_dev, 1, n, (float)c0, rvp::KEY_DENSE, 0, 0, nullptr);
-  // sample queries: every (n/S)-th point
-  float *sq = static_cast<float *>(scratch(ctx, 21, 3 * S * 4));
-  {  // every (n/S)-th point as a query, by strided device copies
-    const size_t stride = n / S;
-    RVP_CUDA_TRY(cudaMemcpy2DAsync(sq, 4, x, stride * 4, 4, S, cudaMemcpyDeviceToDevice, ctx->stream));
-    RVP_CUDA_TRY(cudaMemcpy2DAsync(sq + S, 4, y, stride * 4, 4, S, cudaMemcpyDeviceToDevice, ctx->stream));
-    RVP_CUDA_TRY(cudaMemcpy2DAsync(sq + 2 * S, 4, z, stride * 4, 4, S, cudaMemcpyDeviceToDevice, ctx->stream));
+// the same among a hash's points
+void knn_hash(rvp_hash *h, const float *qx, const float *qy, const float *qz, size_t nq, int K,
+              float radius, int mode, const rvp::TreeOut &o) {
+  const float *x = h->x.as<float>(), *y = h->y.as<float>(), *z = h->z.as<float>();
+  if (!h->tree_built) {
+    h->tree_view = rvp::tree_build(h->ctx, h->tree, x, y, z, h->n);
+    h->tree_built = true;
   }
-  u64 *pairs = static_cast<u64 *>(scratch(ctx, 22, S * K * 8));
-  int32_t *cnt = static_cast<int32_t *>(scratch(ctx, 23, S * 4));
-  rvp::QuerySet qs{sq, sq + S, sq + 2 * S, S, nullptr, nullptr, nullptr};
-  rvp::grid_knn(ctx, g.view(rvp::KEY_DENSE, 0, 0), qs, K, 0.0f, pairs, cnt, 1, 256);
-  std::vector<u64> hp(S * K);
-  std::vector<int32_t> hc(S);
-  RVP_CUDA_TRY(cudaMemcpyAsync(hp.data(), pairs, S * K * 8, cudaMemcpyDeviceToHost, ctx->stream));
-  RVP_CUDA_TRY(cudaMemcpyAsync(hc.data(), cnt, S * 4, cudaMemcpyDeviceToHost, ctx->stream));
-  sync(ctx);
-  std::vector<float> kd;
-  for (size_t s = 0; s < S; ++s)
-    if (hc[s] == K) {
-      u32 b = (u32)(hp[s * K + K - 1] >> 32);
-      float d2;
-      memcpy(&d2, &b, 4);
-      kd.push_back(sqrtf(d2));
-    }
-  if (kd.empty()) return (float)c0;
-  std::nth_element(kd.begin(), kd.begin() + kd.size() / 2, kd.end());
-  double c = kd[kd.size() / 2];
-  c = std::max(c, c0 / 64.0);
-  c = std::min(c, c0);
-  if (!(c > 0)) c = c0;
-  return (float)c;
-}
-
-void knn_cloud(rvp_context *ctx, rvp::Grid &g, const float *x, const float *y, const float *z,
-               size_t n, int K, u64 *pairs, int32_t *counts) {
-  int64_t *offs = single_frame_offsets(ctx, 19, n);
-  const float cell = auto_cell(ctx, g, x, y, z, n, offs, K);
-  rvp::grid_build(ctx, g, x, y, z, offs, 1, n, cell, rvp::KEY_DENSE, 0, 0, nullptr);
-  rvp::QuerySet qs{x, y, z, n, nullptr, nullptr, nullptr};
-  rvp::grid_knn(ctx, g.view(rvp::KEY_DENSE, 0, 0), qs, K, 0.0f, pairs, counts, 1, 256);
+  // (32-bit query numbers in the kernels: a billion at a time)
+  constexpr size_t kMost = (size_t)1 << 30;
+  for (size_t a = 0; a < nq; a += kMost) {
+    const size_t m = std::min(kMost, nq - a);
+    rvp::TreeOut p = o;
+    if (p.mean) p.mean += a;
+    if (p.idx) p.idx += a * K;
+    if (p.d2) p.d2 += a * K;
+    if (p.counts) p.counts += a;
+    const rvp::TreeQueries q = rvp::tree_queries(h->ctx, h->tree, h->tree_view, x, y, z, qx + a,
+                                                 qy + a, qz + a, m);
+    rvp::tree_knn(h->ctx, h->tree_view, q, K, radius, mode, p);
+  }
 }
 
 // one scratch grid per context, kept across calls so its buffers are reused
@@ -388,6 +315,10 @@ rvp_status rvp_context_destroy(rvp_context *ctx) {
     ctx->grid->release();
     delete ctx->grid;
   }
+  if (ctx->tree) {
+    ctx->tree->release();
+    delete ctx->tree;
+  }
   if (ctx->vwork) {
     ctx->vwork->release();
     delete ctx->vwork;
@@ -429,6 +360,7 @@ rvp_status rvp_hash_destroy(rvp_hash *h) {
   cudaStreamSynchronize(h->ctx->stream);
   h->x.release(); h->y.release(); h->z.release(); h->offs.release();
   h->grid.release();
+  h->tree.release();
   delete h;
   return RVP_OK;
 }
@@ -454,6 +386,7 @@ rvp_status rvp_hash_set_input_cloud(rvp_hash *h, const float *x, const float *y,
     // leaves the hash without one, not with the previous cloud's size)
     h->has_cloud = false;
     h->built = false;
+    h->tree_built = false;
     h->n = 0;
     h->x.reserve(n * 4 + 16); h->y.reserve(n * 4 + 16); h->z.reserve(n * 4 + 16);
     h->offs.reserve(16);
@@ -526,9 +459,11 @@ rvp_status rvp_hash_radius_search(rvp_hash *h, const float *qx, const float *qy,
     void *scan_tmp = scratch(ctx, 4, rvp::scan_temp_bytes(nq + 1));
     if (max_nn > 0 && max_nn <= 64 && !refwin) {
       const int K = max_nn;
-      u64 *pairs = static_cast<u64 *>(scratch(ctx, 5, nq * (size_t)K * 8));
-      int32_t *cnt = static_cast<int32_t *>(scratch(ctx, 6, nq * 4));
-      rvp::grid_knn(ctx, gv, qs, K, radius, pairs, cnt, 1, 256);
+      rvp::TreeOut o;
+      o.idx = static_cast<int32_t *>(scratch(ctx, 5, nq * (size_t)K * 8));
+      o.d2 = reinterpret_cast<float *>(o.idx + nq * (size_t)K);
+      int32_t *cnt = o.counts = static_cast<int32_t *>(scratch(ctx, 6, nq * 4));
+      knn_hash(h, dqx, dqy, dqz, nq, K, radius, rvp::TREE_PAIRS, o);
       u32 *ucnt = static_cast<u32 *>(scratch(ctx, 7, nq * 4));
       k_i32_to_u32<<<rvp::grid_for(nq, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(cnt, nq, ucnt);
       RVP_LAUNCH_CHECK(ctx);
@@ -544,7 +479,7 @@ rvp_status rvp_hash_radius_search(rvp_hash *h, const float *qx, const float *qy,
       int32_t *di = out_dev(ctx, 8, indices, tot, mem);
       float *dd = out_dev(ctx, 9, dists, tot, mem);
       k_rows_to_csr<<<rvp::grid_for(nq * K, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
-          pairs, K, cnt, offs_d, nq, K, di, dd);
+          o.idx, o.d2, K, cnt, offs_d, nq, di, dd);
       RVP_LAUNCH_CHECK(ctx);
       out_copy(ctx, offsets, reinterpret_cast<int64_t *>(offs_d), nq + 1, mem);
       out_copy(ctx, indices, di, tot, mem);
@@ -627,14 +562,11 @@ rvp_status rvp_hash_knn(rvp_hash *h, const float *qx, const float *qy, const flo
     const float *dqx = in_dev(ctx, 1, qx, nq, mem);
     const float *dqy = in_dev(ctx, 2, qy, nq, mem);
     const float *dqz = in_dev(ctx, 3, qz, nq, mem);
-    rvp::QuerySet qs{dqx, dqy, dqz, nq, nullptr, nullptr, nullptr};
-    u64 *pairs = static_cast<u64 *>(scratch(ctx, 5, nq * (size_t)k * 8));
-    int32_t *cnt = dc ? dc : static_cast<int32_t *>(scratch(ctx, 7, nq * 4));
-    rvp::grid_knn(ctx, h->grid.view(rvp::KEY_REF_HASH, h->p1, h->p2), qs, k, radius, pairs, cnt,
-                  1, 256);
-    k_fill_rows<<<rvp::grid_for(nq * k, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
-        pairs, k, cnt, nq, di, dd);
-    RVP_LAUNCH_CHECK(ctx);
+    rvp::TreeOut o;
+    o.idx = di;
+    o.d2 = dd;
+    o.counts = dc;
+    knn_hash(h, dqx, dqy, dqz, nq, k, radius, rvp::TREE_PAIRS, o);
     out_copy(ctx, counts, dc, nq, mem);
     out_copy(ctx, indices, di, nq * (size_t)k, mem);
     out_copy(ctx, dists, dd, nq * (size_t)k, mem);
@@ -686,14 +618,15 @@ rvp_status rvp_voxel_grid(rvp_context *ctx, const float *x, const float *y, cons
 // ===========================================================================
 // SOR
 // ===========================================================================
-static void sor_common(rvp_context *ctx, const float *dx, const float *dy, const float *dz,
-                       size_t n, const u64 *pairs, int kk, const int32_t *cnt, bool radius_mode,
-                       float fallback, float alpha, int mem, float *out_aos, size_t *out_count,
-                       float *mean_dists, uint8_t *keep) {
+static float *sor_mean_buffer(rvp_context *ctx, float *mean_dists, size_t n, int mem) {
   float *mean = out_dev(ctx, 12, mean_dists, n, mem);
-  if (!mean) mean = static_cast<float *>(scratch(ctx, 12, n * 4));
+  return mean ? mean : static_cast<float *>(scratch(ctx, 12, n * 4));
+}
+
+static void sor_common(rvp_context *ctx, const float *dx, const float *dy, const float *dz,
+                       size_t n, float *mean, float alpha, int mem, float *out_aos,
+                       size_t *out_count, float *mean_dists, uint8_t *keep) {
   uint8_t *dkeep = out_dev(ctx, 13, keep, n, mem);
-  rvp::sor_mean_from_knn(ctx, pairs, kk, cnt, n, nullptr, mean, fallback, radius_mode);
   int64_t *offs = single_frame_offsets(ctx, 14, n);
   float *dout = out_dev(ctx, 15, out_aos, 3 * n, mem);
   int64_t *so = static_cast<int64_t *>(scratch(ctx, 16, 64));
@@ -727,12 +660,10 @@ rvp_status rvp_sor(rvp_context *ctx, const float *x, const float *y, const float
     const float *dx = in_dev(ctx, 1, x, n, mem);
     const float *dy = in_dev(ctx, 2, y, n, mem);
     const float *dz = in_dev(ctx, 3, z, n, mem);
-    const int kk = k + 1;
-    u64 *pairs = static_cast<u64 *>(scratch(ctx, 9, n * (size_t)kk * 8));
-    int32_t *cnt = static_cast<int32_t *>(scratch(ctx, 10, n * 4));
-    knn_cloud(ctx, ctx_grid(ctx), dx, dy, dz, n, kk, pairs, cnt);
-    sor_common(ctx, dx, dy, dz, n, pairs, kk, cnt, false, 0.0f, alpha, mem, out_aos, out_count,
-               mean_dists, keep);
+    rvp::TreeOut o;
+    o.mean = sor_mean_buffer(ctx, mean_dists, n, mem);
+    knn_cloud(ctx, dx, dy, dz, n, k + 1, rvp::TREE_MEAN, o);
+    sor_common(ctx, dx, dy, dz, n, o.mean, alpha, mem, out_aos, out_count, mean_dists, keep);
   });
 }
 
@@ -751,15 +682,13 @@ rvp_status rvp_sor_spatial_hash(rvp_hash *h, int k, float alpha, float search_ra
     RVP_REQUIRE(k >= 1 && k + 1 <= 64, "k must be in [1, 63]");
     RVP_REQUIRE(h->collision == 0, "sor_spatial_hash needs a collision-free hash");
     set_device(ctx);
-    const int kk = k + 1;
-    u64 *pairs = static_cast<u64 *>(scratch(ctx, 9, n * (size_t)kk * 8));
-    int32_t *cnt = static_cast<int32_t *>(scratch(ctx, 10, n * 4));
     const float *dx = h->x.as<float>(), *dy = h->y.as<float>(), *dz = h->z.as<float>();
-    rvp::QuerySet qs{dx, dy, dz, n, nullptr, nullptr, nullptr};
-    rvp::grid_knn(ctx, h->grid.view(rvp::KEY_REF_HASH, h->p1, h->p2), qs, kk, search_radius,
-                  pairs, cnt, 1, 256);
-    sor_common(ctx, dx, dy, dz, n, pairs, kk, cnt, true, search_radius, alpha, mem, out_aos,
-               out_count, mean_dists, keep);
+    rvp::TreeOut o;
+    o.mean = sor_mean_buffer(ctx, mean_dists, n, mem);
+    o.radius_mode = true;
+    o.fallback = search_radius;
+    knn_hash(h, dx, dy, dz, n, k + 1, search_radius, rvp::TREE_MEAN, o);
+    sor_common(ctx, dx, dy, dz, n, o.mean, alpha, mem, out_aos, out_count, mean_dists, keep);
   });
 }
 
@@ -813,14 +742,17 @@ rvp_status rvp_normals_knn(rvp_context *ctx, const float *x, const float *y, con
     const float *dx = in_dev(ctx, 1, x, n, mem);
     const float *dy = in_dev(ctx, 2, y, n, mem);
     const float *dz = in_dev(ctx, 3, z, n, mem);
-    const int kk = k + 1;
-    u64 *pairs = static_cast<u64 *>(scratch(ctx, 9, n * (size_t)kk * 8));
-    int32_t *cnt = static_cast<int32_t *>(scratch(ctx, 10, n * 4));
-    knn_cloud(ctx, ctx_grid(ctx), dx, dy, dz, n, kk, pairs, cnt);
     float *dnx = out_dev(ctx, 12, nx, n, mem), *dny = out_dev(ctx, 13, ny, n, mem),
           *dnz = out_dev(ctx, 14, nz, n, mem);
-    rvp::normals_from_lists(ctx, dx, dy, dz, pairs, nullptr, cnt, kk, n, nullptr, true,
-                            eigen_iters, vp_x, vp_y, vp_z, dx, dy, dz, dnx, dny, dnz);
+    rvp::TreeOut o;
+    o.nx = dnx;
+    o.ny = dny;
+    o.nz = dnz;
+    o.iters = eigen_iters;
+    o.vpx = vp_x;
+    o.vpy = vp_y;
+    o.vpz = vp_z;
+    knn_cloud(ctx, dx, dy, dz, n, k + 1, rvp::TREE_NORMALS, o);
     out_copy(ctx, nx, dnx, n, mem);
     out_copy(ctx, ny, dny, n, mem);
     out_copy(ctx, nz, dnz, n, mem);
@@ -842,16 +774,21 @@ rvp_status rvp_normals_knn_precise(rvp_context *ctx, const float *x, const float
     const float *dx = in_dev(ctx, 1, x, n, mem);
     const float *dy = in_dev(ctx, 2, y, n, mem);
     const float *dz = in_dev(ctx, 3, z, n, mem);
-    const int kk = k + 1;
-    u64 *pairs = static_cast<u64 *>(scratch(ctx, 9, n * (size_t)kk * 8));
-    int32_t *cnt = static_cast<int32_t *>(scratch(ctx, 10, n * 4));
-    knn_cloud(ctx, ctx_grid(ctx), dx, dy, dz, n, kk, pairs, cnt);
     float *dnx = out_dev(ctx, 12, nx, n, mem), *dny = out_dev(ctx, 13, ny, n, mem),
           *dnz = out_dev(ctx, 14, nz, n, mem);
     float *dc = out_dev(ctx, 15, cond, n, mem);
     uint8_t *du = out_dev(ctx, 16, used_fp64, n, mem);
-    rvp::normals_precise(ctx, dx, dy, dz, pairs, kk, n, vp_x, vp_y, vp_z, cond_fp64, dnx, dny,
-                         dnz, dc, du);
+    rvp::TreeOut o;
+    o.nx = dnx;
+    o.ny = dny;
+    o.nz = dnz;
+    o.vpx = vp_x;
+    o.vpy = vp_y;
+    o.vpz = vp_z;
+    o.cond_fp64 = cond_fp64;
+    o.cond = dc;
+    o.used64 = du;
+    knn_cloud(ctx, dx, dy, dz, n, k + 1, rvp::TREE_PRECISE, o);
     out_copy(ctx, nx, dnx, n, mem);
     out_copy(ctx, ny, dny, n, mem);
     out_copy(ctx, nz, dnz, n, mem);

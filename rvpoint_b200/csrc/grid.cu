@@ -400,6 +400,13 @@ GridView Grid::view(int mode, long long p1, long long p2) const {
   return v;
 }
 
+void cloud_bbox(rvp_context *ctx, const float *x, const float *y, const float *z, size_t n,
+                float *bb) {
+  k_bbox<<<grid_for(n, 256, ctx->num_sms * kBoxBlocks), 256, 0, ctx->stream>>>(
+      x, y, z, nullptr, 1, n, nullptr, bb);
+  RVP_LAUNCH_CHECK(ctx);
+}
+
 void grid_build(rvp_context *ctx, Grid &g, const float *x, const float *y, const float *z,
                 const int64_t *offs, int n_frames, size_t n_points, float cell, int mode,
                 long long p1, long long p2, const u64 *n_dev_opt, int base_level,

@@ -69,6 +69,7 @@ struct HostBuf {  // pinned
 
 struct Grid;
 struct VoxelWork;
+struct KnnTree;
 }  // namespace rvp
 
 struct rvp_context {
@@ -80,7 +81,8 @@ struct rvp_context {
   // scratch owned by one-shot entry points (grow-only, reused across calls)
   rvp::DevBuf scratch[32];  // 0-23 one-shot entry points, 24-27 batched RANSAC
   rvp::HostBuf pinned[4];
-  rvp::Grid *grid = nullptr;        // grid reused by one-shot kNN entry points
+  rvp::Grid *grid = nullptr;        // grid of the clustering entry point
+  rvp::KnnTree *tree = nullptr;     // tree reused by one-shot kNN entry points
   rvp::VoxelWork *vwork = nullptr;  // voxel scratch of rvp_voxel_grid
 };
 
@@ -361,6 +363,62 @@ bool grid_knn_tau(rvp_context *ctx, const GridView &g, int k, int mode, const Ti
                   u32 *stats = nullptr);
 
 // ---------------------------------------------------------------------------
+// box tree of one cloud (knn_tree.cu): exact k nearest, k <= 64
+// ---------------------------------------------------------------------------
+constexpr int kTreeLevels = 4;
+struct TreeView {  // what the search reads
+  float4 *pts;                // {x, y, z, index} in tree order
+  u32 *pos_of;                // tree position of each point
+  const u64 *keys;            // sorted keys
+  const float *bb;            // the cloud's box
+  float *box[kTreeLevels];    // per level: lo x, y, z, hi x, y, z (stride each)
+  u32 stride[kTreeLevels];
+  u32 count[kTreeLevels];     // nodes per level (level 0: leaves of 32 points)
+  u32 n;
+};
+struct TreeQueries {
+  const float4 *q = nullptr;     // {x, y, z, index} in key order
+  const u64 *keys = nullptr;     // their sorted keys
+  const u64 *n_sort = nullptr;   // null, or 0 there: the queries are the cloud
+  u32 n = 0;
+};
+// TREE_MEAN: SOR's mean distance; TREE_PAIRS: rows of k indices and squared
+// distances (-1 and infinity past the found) and counts; TREE_NORMALS /
+// TREE_PRECISE: normals of the k nearest (k <= n)
+enum TreeMode { TREE_MEAN = 0, TREE_PAIRS = 1, TREE_NORMALS = 2, TREE_PRECISE = 3 };
+struct TreeOut {  // by query index; null pointers are skipped
+  float *mean = nullptr;
+  bool radius_mode = false;
+  float fallback = 0.0f;
+  int32_t *idx = nullptr;
+  float *d2 = nullptr;
+  int32_t *counts = nullptr;
+  float *nx = nullptr, *ny = nullptr, *nz = nullptr;
+  int iters = 0;
+  float vpx = 0.0f, vpy = 0.0f, vpz = 0.0f;
+  double cond_fp64 = 0.0;
+  float *cond = nullptr;
+  uint8_t *used64 = nullptr;
+};
+struct KnnTree {
+  DevBuf keys, vals, sort, pts, pos, boxes, misc, qkeys, qvals, qpts;
+  void release();
+};
+TreeView tree_build(rvp_context *ctx, KnnTree &w, const float *x, const float *y, const float *z,
+                    size_t n);
+// the queries in tree order; the cloud itself (by pointer, or by value, found
+// out on the device) is in it already
+TreeQueries tree_queries(rvp_context *ctx, KnnTree &w, const TreeView &t, const float *x,
+                         const float *y, const float *z, const float *qx, const float *qy,
+                         const float *qz, size_t nq);
+// radius > 0: neighbours with d2 <= radius * radius only
+void tree_knn(rvp_context *ctx, const TreeView &t, const TreeQueries &q, int k, float radius,
+              int mode, const TreeOut &o);
+// bounds of a cloud, folded into bb (min x, y, z, max x, y, z)
+void cloud_bbox(rvp_context *ctx, const float *x, const float *y, const float *z, size_t n,
+                float *bb);
+
+// ---------------------------------------------------------------------------
 // voxel grid (voxel.cu)
 // ---------------------------------------------------------------------------
 struct VoxelWork {
@@ -380,10 +438,6 @@ void voxel_grid_run(rvp_context *ctx, VoxelWork &w, const float *x,
 // ---------------------------------------------------------------------------
 // SOR (sor.cu)
 // ---------------------------------------------------------------------------
-// mean distance from sorted kNN lists (k+1 incl. self)
-void sor_mean_from_knn(rvp_context *ctx, const u64 *pairs, int kk,
-                       const int32_t *counts, size_t n_max, const u64 *n_dev,
-                       float *mean, float fallback_radius, bool radius_mode);
 // per-frame sequential statistics, keep mask and ordered AoS copy-out
 void sor_filter_frames(rvp_context *ctx, const float *x, const float *y,
                        const float *z, const float *mean,
@@ -410,11 +464,6 @@ void normals_from_lists(rvp_context *ctx, const float *x, const float *y,
                         const float *qx, const float *qy, const float *qz,
                         float *nx, float *ny, float *nz, const u32 *order = nullptr,
                         const u64 *out_pos = nullptr);
-void normals_precise(rvp_context *ctx, const float *x, const float *y,
-                     const float *z, const u64 *pairs, int kk, size_t n,
-                     float vpx, float vpy, float vpz, double cond_fp64,
-                     float *nx, float *ny, float *nz, float *cond,
-                     uint8_t *used_fp64);
 
 // ---------------------------------------------------------------------------
 // RANSAC (ransac.cu)

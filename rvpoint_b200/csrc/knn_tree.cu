@@ -1,0 +1,679 @@
+// Exact k nearest neighbours in one cloud (k <= 64) over a 32-wide box tree.
+//
+// Build: the points sorted by the Morton code of their quantised position
+// (32 bits, one power-of-two cell for all axes), every 32 consecutive points
+// a leaf with its bounding box, every 32 leaves a node, and so on, four levels
+// in all. No cell size is chosen and nothing depends on the
+// density: a leaf is small where the points are dense.
+//
+// Search: one warp answers 32 queries that lie close together (the points of
+// a leaf, or 32 consecutive queries of a sorted query set). The lanes test
+// the boxes of 32 children at once against the box of the queries and go down
+// into those nearer than the largest K-th distance so far, nearest first; a
+// leaf's points are staged in shared memory and every lane tests all of them
+// against its own query. What passes waits in a buffer per lane and goes
+// through a sorted list of distances (registers) when a buffer fills, so the
+// insertions of the lanes run side by side. With the K-th distance known, a
+// second walk collects the points within it and each goes to its rank.
+//
+// Pruning needs no slack: every operation of the distance (subtract, square,
+// add) is monotone under rounding, so the distance to a box computed with the
+// same operations is never above the computed distance to a point inside it.
+// Equal distances are ordered by index: a query whose list holds equal ones
+// is answered again by the whole warp on packed (distance, index) keys.
+//
+// Bound by issue (box tests, distance tests and list insertions). The grid
+// search it replaces for single clouds ran one warp per query on cells sized
+// from a sample of queries: 105k LiDAR points, k 16, 3818 us; a 2M-point map,
+// k 33, 14,225 us.
+#include <math.h>
+
+#include <algorithm>
+#include <type_traits>
+
+#include "grid_device.cuh"
+#include "internal.cuh"
+#include "normals_device.cuh"
+
+namespace rvp {
+using namespace gd;
+
+namespace {
+inline size_t al(size_t b) { return (b + 255) & ~(size_t)255; }
+
+constexpr int kTreeKeyBits = 32;
+
+// ---------------------------------------------------------------------------
+// build
+// ---------------------------------------------------------------------------
+struct TreeFrame {  // the quantisation of the cloud's box
+  float lo[3];
+  float inv;    // cells per unit (a power of two)
+  int bits[3];  // of each axis, kTreeKeyBits together at most
+};
+
+__global__ void k_tree_init(float *bb) {
+  if (threadIdx.x < 3) bb[threadIdx.x] = INFINITY;
+  else if (threadIdx.x < 6) bb[threadIdx.x] = -INFINITY;
+}
+
+// the finest power-of-two cell whose codes fit the key
+__device__ void tree_frame(const float *bb, TreeFrame &F) {
+  float ext[3], emax = 0.0f;
+  for (int a = 0; a < 3; ++a) {
+    const float lo = bb[a], hi = bb[3 + a];
+    F.lo[a] = lo < INFINITY && lo > -INFINITY ? lo : 0.0f;
+    float e = fsub(hi, lo);
+    e = e > 0.0f ? fminf(e, 1e30f) : 0.0f;  // (NaN and empty axes: one cell)
+    ext[a] = e;
+    emax = fmaxf(emax, e);
+  }
+  int k = emax > 0.0f ? ilogbf(emax) - kTreeKeyBits : -60;
+  k = max(k, -100);
+  for (;; ++k) {
+    int sum = 0;
+    for (int a = 0; a < 3; ++a) {
+      const float q = ldexpf(ext[a], -k);  // cells along the axis
+      F.bits[a] = q < 1.0f ? 0 : ilogbf(q) + 1;
+      sum += F.bits[a];
+    }
+    if (sum <= kTreeKeyBits) break;
+  }
+  F.inv = ldexpf(1.0f, -k);
+}
+
+__device__ __forceinline__ u32 tree_key(const TreeFrame &F, float x, float y, float z) {
+  const float v[3] = {x, y, z};
+  u32 q[3];
+  int top = 0;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const float t = fmul(fsub(v[a], F.lo[a]), F.inv);
+    const u32 last = F.bits[a] >= 32 ? 0xFFFFFFFFu : (1u << F.bits[a]) - 1u;
+    q[a] = t > 0.0f ? (t < 4.0e9f ? min((u32)t, last) : last) : 0u;
+    top = max(top, F.bits[a]);
+  }
+  u32 key = 0;
+  for (int b = top - 1; b >= 0; --b) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+      if (b < F.bits[a]) key = (key << 1) | ((q[a] >> b) & 1u);
+  }
+  return key;
+}
+
+__global__ __launch_bounds__(256) void k_tree_keys(const float *__restrict__ x,
+                                                   const float *__restrict__ y,
+                                                   const float *__restrict__ z, size_t n_max,
+                                                   const u64 *n_dev, const float *bb, u64 *keys,
+                                                   u32 *vals) {
+  __shared__ TreeFrame F;
+  const size_t n = n_dev ? *n_dev : n_max;
+  if (threadIdx.x == 0) tree_frame(bb, F);
+  __syncthreads();
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x) {
+    keys[i] = tree_key(F, x[i], y[i], z[i]);
+    vals[i] = (u32)i;
+  }
+}
+
+// box reduction over a warp; lane 0 writes node `c` of a level
+__device__ __forceinline__ void box_out(float (&m)[6], float *box, u32 stride, u32 c) {
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      const float t = __shfl_xor_sync(0xffffffffu, m[k], o);
+      m[k] = k < 3 ? fminf(m[k], t) : fmaxf(m[k], t);
+    }
+  }
+  if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) box[(size_t)k * stride + c] = m[k];
+  }
+}
+
+// one warp per leaf: its records in tree order and its box
+__global__ __launch_bounds__(256) void k_tree_leaves(const float *__restrict__ x,
+                                                     const float *__restrict__ y,
+                                                     const float *__restrict__ z,
+                                                     const u32 *__restrict__ vals, u32 n,
+                                                     float4 *pts, u32 *pos_of, float *box,
+                                                     u32 stride) {
+  const u32 c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, i = c * 32 + (threadIdx.x & 31);
+  if (c * 32 >= n) return;
+  float m[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  if (i < n) {
+    const u32 v = vals[i];
+    const float p[3] = {x[v], y[v], z[v]};
+    pts[i] = make_float4(p[0], p[1], p[2], __uint_as_float(v));
+    pos_of[v] = i;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      m[a] = fminf(m[a], p[a]);
+      m[3 + a] = fmaxf(m[3 + a], p[a]);
+    }
+  }
+  box_out(m, box, stride, c);
+}
+
+// one warp per node of the next level: the box of up to 32 children
+__device__ __forceinline__ void parent_box(const float *kid, u32 kid_stride, u32 kids, float *box,
+                                           u32 stride, u32 c) {
+  const u32 i = c * 32 + (threadIdx.x & 31);
+  float m[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  if (i < kids) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) m[k] = kid[(size_t)k * kid_stride + i];
+  }
+  box_out(m, box, stride, c);
+}
+
+__global__ __launch_bounds__(256) void k_tree_parents(TreeView t, int level) {
+  const u32 c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (c >= t.count[level]) return;
+  parent_box(t.box[level - 1], t.stride[level - 1], t.count[level - 1], t.box[level],
+             t.stride[level], c);
+}
+
+// the levels from `level` on, by one block
+__global__ __launch_bounds__(1024) void k_tree_top(TreeView t, int level) {
+  for (; level < kTreeLevels; ++level) {
+    for (u32 c = threadIdx.x >> 5; c < t.count[level]; c += 32)
+      parent_box(t.box[level - 1], t.stride[level - 1], t.count[level - 1], t.box[level],
+                 t.stride[level], c);
+    __syncthreads();
+  }
+}
+
+// 0 in *n_sort if the queries are the cloud itself, value by value, else nq:
+// the sort of the queries then has nothing to do
+__global__ void k_tree_same(const float *qx, const float *qy, const float *qz, const float *x,
+                            const float *y, const float *z, size_t n, u64 *n_sort) {
+  bool differs = false;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x)
+    differs = differs || __float_as_uint(qx[i]) != __float_as_uint(x[i]) ||
+              __float_as_uint(qy[i]) != __float_as_uint(y[i]) ||
+              __float_as_uint(qz[i]) != __float_as_uint(z[i]);
+  if (__any_sync(0xffffffffu, differs) && (threadIdx.x & 31) == 0) *n_sort = n;
+}
+__global__ void k_tree_count(u64 *n_sort, u64 v) { *n_sort = v; }
+
+__global__ void k_tree_queries(const float *__restrict__ x, const float *__restrict__ y,
+                               const float *__restrict__ z, const u32 *__restrict__ vals,
+                               const u64 *n_sort, float4 *q) {
+  const size_t n = *n_sort;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x) {
+    const u32 v = vals[i];
+    q[i] = make_float4(x[v], y[v], z[v], __uint_as_float(v));
+  }
+}
+
+// ---------------------------------------------------------------------------
+// search
+// ---------------------------------------------------------------------------
+// the squared distance between two boxes (a point is a box), with the
+// operations of dist2
+__device__ __forceinline__ float box_gap(float alo, float ahi, float blo, float bhi) {
+  return fmaxf(fmaxf(fsub(blo, ahi), fsub(alo, bhi)), 0.0f);
+}
+struct Box {
+  float lo[3], hi[3];
+};
+__device__ __forceinline__ float box_d2(const Box &q, const float *box, u32 stride, u32 c) {
+  float g[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+    g[a] = box_gap(q.lo[a], q.hi[a], __ldg(&box[(size_t)a * stride + c]),
+                   __ldg(&box[(size_t)(3 + a) * stride + c]));
+  return fadd(fadd(fmul(g[0], g[0]), fmul(g[1], g[1])), fmul(g[2], g[2]));
+}
+
+// Walks every leaf within limit() of the box q, nearest child first. All
+// lanes take part; limit() is uniform and may shrink on the way.
+template <int LV, class Limit, class Leaf>
+__device__ __forceinline__ void tree_walk(const TreeView &t, const Box &q, u32 first, Limit &limit,
+                                          Leaf &leaf) {
+  const int lane = threadIdx.x & 31;
+  const u32 c = first + lane;
+  const float lb = c < t.count[LV] ? box_d2(q, t.box[LV], t.stride[LV], c) : 0.0f;
+  bool open = c < t.count[LV] && lb <= limit();
+  while (true) {
+    // (the low bits of the distance give way to the lane)
+    const u32 key = open ? (__float_as_uint(lb) & ~31u) | lane : 0xFFFFFFFFu;
+    const u32 best = __reduce_min_sync(0xffffffffu, key);
+    if (best == 0xFFFFFFFFu) break;
+    const int s = best & 31;
+    if (lane == s) open = false;
+    if (__uint_as_float(best & ~31u) > limit()) break;  // and so are all that are left
+    if (__shfl_sync(0xffffffffu, lb, s) > limit()) continue;
+    if constexpr (LV == 0) leaf(first + s);
+    else tree_walk<LV - 1>(t, q, (first + s) * 32, limit, leaf);
+  }
+}
+// (at most 32 nodes are left at the top up to 33.5M points; more than that go
+// 32 at a time)
+template <class Limit, class Leaf>
+__device__ __forceinline__ void tree_walk_all(const TreeView &t, const Box &q, Limit &limit,
+                                              Leaf &leaf) {
+  for (u32 f = 0; f < t.count[kTreeLevels - 1]; f += 32)
+    tree_walk<kTreeLevels - 1>(t, q, f, limit, leaf);
+}
+
+constexpr int kTreeBuf = 64;   // buffered distances per lane; flushed above 32
+constexpr int kTreeExtra = 3;  // collected points past K (equal distances)
+
+template <int KCAP, int MODE>
+constexpr size_t tree_smem() {
+  size_t buf = (size_t)kTreeBuf * 32 * 4;
+  const size_t pairs = (size_t)(KCAP + kTreeExtra) * 32 * 8;
+  if (MODE != TREE_MEAN && pairs > buf) buf = pairs;
+  const size_t sorted = MODE == TREE_NORMALS || MODE == TREE_PRECISE ? (size_t)KCAP * 32 * 4 : 0;
+  return 32 * 16 + buf + sorted;
+}
+
+// one warp (block) per packet of 32 queries; KCAP >= K
+template <int KCAP, int MODE>
+__global__ __launch_bounds__(32, KCAP > 33 ? 12 : 16) void k_knn_tree(TreeView t, TreeQueries qs,
+                                                                      int K, float bound,
+                                                                      TreeOut o) {
+  extern __shared__ __align__(16) unsigned char tree_sm[];
+  float4 *stage = reinterpret_cast<float4 *>(tree_sm);
+  float(*fbuf)[32] = reinterpret_cast<float(*)[32]>(tree_sm + 512);
+  uint2(*pbuf)[32] = reinterpret_cast<uint2(*)[32]>(tree_sm + 512);
+  constexpr int PCAP = KCAP + kTreeExtra;
+  constexpr size_t kBuf = tree_smem<KCAP, TREE_PAIRS>() - 512;
+  u32(*sorted)[32] = reinterpret_cast<u32(*)[32]>(tree_sm + 512 + kBuf);
+  const int lane = threadIdx.x;
+  const u32 packet = blockIdx.x;
+  // the cloud's own points (leaf `packet`), or 32 of the sorted queries
+  const bool self = qs.n_sort == nullptr || *qs.n_sort == 0;
+  const float4 *src = self ? t.pts : qs.q;
+  const u32 qi = packet * 32 + lane;
+  const bool active = qi < qs.n;
+  const float4 q = src[active ? qi : packet * 32];
+  const u32 qidx = __float_as_uint(q.w);
+  u32 start = packet;
+  if (!self) {  // the leaf where a query of the middle would lie
+    const u64 mid = qs.keys[min(packet * 32 + 16, qs.n - 1)];
+    u32 lo = 0, hi = t.n - 1;
+    while (lo < hi) {
+      const u32 m = (lo + hi) >> 1;
+      if (t.keys[m] < mid) lo = m + 1; else hi = m;
+    }
+    start = lo / 32;
+  }
+  Box pk;  // the box of the packet
+  {
+    const float v[3] = {q.x, q.y, q.z};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      float l = v[a], h = v[a];
+#pragma unroll
+      for (int s = 16; s; s >>= 1) {
+        l = fminf(l, __shfl_xor_sync(0xffffffffu, l, s));
+        h = fmaxf(h, __shfl_xor_sync(0xffffffffu, h, s));
+      }
+      pk.lo[a] = l;
+      pk.hi[a] = h;
+    }
+  }
+  const Box own{{q.x, q.y, q.z}, {q.x, q.y, q.z}};
+
+  // ---- the sorted distances: slots 0 .. pad - 1 hold -1 and never move
+  const int pad = KCAP - K;
+  float L[KCAP];
+#pragma unroll
+  for (int j = 0; j < KCAP; ++j) L[j] = j < pad ? -1.0f : INFINITY;
+  float thr = INFINITY;
+  int cnt = 0;
+  float pmax = 0.0f;
+  auto update_pmax = [&]() {
+    const float lim = active ? fminf(thr, bound) : -1.0f;
+    pmax = __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(lim)));
+  };
+  update_pmax();
+  auto flush = [&]() {
+    const int most = __reduce_max_sync(0xffffffffu, cnt);
+    for (int i = 0; i < most; ++i) {
+      const float key = i < cnt ? fbuf[i][lane] : INFINITY;
+      if (__any_sync(0xffffffffu, key < L[KCAP - 1])) {
+#pragma unroll
+        for (int j = KCAP - 1; j > 0; --j) L[j] = fmaxf(L[j - 1], fminf(L[j], key));
+        L[0] = fminf(L[0], key);
+      }
+    }
+    cnt = 0;
+    thr = L[KCAP - 1];
+    update_pmax();
+  };
+  // leaf l staged; false if no lane has a point within lim of it
+  auto stage_leaf = [&](u32 l, bool need) {
+    if (!__any_sync(0xffffffffu, need)) return false;
+    const u32 i = l * 32 + lane;
+    const float4 p = i < t.n ? __ldg(&t.pts[i]) : make_float4(INFINITY, INFINITY, INFINITY, 0.0f);
+    __syncwarp();
+    stage[lane] = p;
+    __syncwarp();
+    return true;
+  };
+  auto scan_leaf = [&](u32 l) {
+    const float lb = box_d2(own, t.box[0], t.stride[0], l);
+    const bool need = active && lb <= bound && lb < thr;
+    if (!stage_leaf(l, need)) return;
+    if (need) {
+#pragma unroll 8
+      for (int c = 0; c < 32; ++c) {
+        const float4 p = stage[c];
+        const float d = dist2(p.x, p.y, p.z, q.x, q.y, q.z);
+        if (d < thr && d <= bound) fbuf[cnt++][lane] = d;
+      }
+    }
+    if (__any_sync(0xffffffffu, cnt > kTreeBuf - 32)) flush();
+  };
+  // the leaves around the packet's place first: they set the limits
+  const u32 s0 = start > 0 ? start - 1 : 0, s1 = min(start + 1, t.count[0] - 1);
+  scan_leaf(start);
+  flush();
+  for (u32 l = s0; l <= s1; ++l)
+    if (l != start) scan_leaf(l);
+  flush();
+  {
+    auto limit = [&]() { return pmax; };
+    auto leaf = [&](u32 l) {
+      if (l < s0 || l > s1) scan_leaf(l);
+    };
+    tree_walk_all(t, pk, limit, leaf);
+    flush();
+  }
+
+  if constexpr (MODE == TREE_MEAN) {
+    // sor_sc's mean (statistical_outlier_removal.cpp:36-40): ascending sum of
+    // sqrtf(d2_j), j = 1 .. k, over k (over those found within a radius:
+    // :246-270, the radius itself for a point without neighbours)
+    // (without a radius K points are there, some infinitely far perhaps)
+    int found = 0;
+    float sum = 0.0f;
+#pragma unroll
+    for (int j = 0; j < KCAP; ++j) {
+      if (j >= pad && (!o.radius_mode || L[j] < INFINITY)) {
+        if (found) sum = fadd(sum, __fsqrt_rn(L[j]));
+        ++found;
+      }
+    }
+    if (active) {
+      float m = found > 1 ? fdiv(sum, (float)(found - 1)) : 0.0f;
+      if (o.radius_mode && found <= 1) m = o.fallback;
+      const float none = dist2(q.x, q.y, q.z, q.x, q.y, q.z);  // NaN without a position
+      o.mean[qidx] = none == 0.0f ? m : none;
+    }
+    return;
+  } else {
+    // ---- second walk: the points within the K-th distance
+    const float tau = active ? fminf(thr, bound) : -1.0f;
+    int want = 0;
+    bool tied = false;
+#pragma unroll
+    for (int j = 0; j < KCAP; ++j) {
+      if (j >= pad && L[j] < INFINITY) ++want;
+      if (j > pad && L[j] < INFINITY && L[j] == L[j - (j > 0)]) tied = true;
+    }
+    cnt = 0;
+    pmax = __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(tau)));
+    {
+      auto limit = [&]() { return pmax; };
+      auto leaf = [&](u32 l) {
+        const float lb = box_d2(own, t.box[0], t.stride[0], l);
+        const bool need = lb <= tau;
+        if (!stage_leaf(l, need)) return;
+        if (need) {
+          const int m = (int)min(32u, t.n - l * 32);
+#pragma unroll 4
+          for (int c = 0; c < m; ++c) {
+            const float4 p = stage[c];
+            const float d = dist2(p.x, p.y, p.z, q.x, q.y, q.z);
+            if (d <= tau) {
+              if (cnt < PCAP) pbuf[cnt][lane] = make_uint2(__float_as_uint(d), l * 32 + c);
+              ++cnt;
+            }
+          }
+        }
+      };
+      tree_walk_all(t, pk, limit, leaf);
+    }
+    __syncwarp();
+    const bool exact = active && cnt == want && !tied;
+    // each to its rank among the sorted distances
+    if (exact) {
+      for (int i = 0; i < want; ++i) {
+        const uint2 b = pbuf[i][lane];
+        const float d = __uint_as_float(b.x);
+        int r = -pad;
+#pragma unroll
+        for (int j = 0; j < KCAP; ++j) r += L[j] < d ? 1 : 0;
+        if constexpr (MODE == TREE_PAIRS) {
+          const size_t at = (size_t)qidx * K + r;
+          if (o.idx) o.idx[at] = (int32_t)__float_as_uint(__ldg(&t.pts[b.y]).w);
+          if (o.d2) o.d2[at] = d;
+        } else {
+          sorted[r][lane] = b.y;
+        }
+      }
+    }
+    int have = want;
+    // equal distances: the whole warp on (distance, index) keys, one query
+    // at a time
+    unsigned again = __ballot_sync(0xffffffffu, active && !exact);
+    while (again) {
+      const int s = __ffs(again) - 1;
+      again &= again - 1;
+      const float sx = __shfl_sync(0xffffffffu, q.x, s), sy = __shfl_sync(0xffffffffu, q.y, s),
+                  sz = __shfl_sync(0xffffffffu, q.z, s);
+      const u32 sidx = __shfl_sync(0xffffffffu, qidx, s);
+      WarpList<(KCAP > 32 ? 2 : 1)> W;
+      W.init();
+      u64 key_thr = W.get(K - 1);
+      u32 found = 0;
+      const Box one{{sx, sy, sz}, {sx, sy, sz}};
+      auto limit = [&]() {
+        return key_thr == ~0ull ? bound : fminf(nbr_d2(key_thr), bound);
+      };
+      auto leaf = [&](u32 l) {
+        const u32 i = l * 32 + lane;
+        u64 key = ~0ull;
+        if (i < t.n) {
+          const float4 p = __ldg(&t.pts[i]);
+          const float d = dist2(p.x, p.y, p.z, sx, sy, sz);
+          if (d <= bound) key = pack_nbr(d, (int)__float_as_uint(p.w));
+        }
+        found += __popc(__ballot_sync(0xffffffffu, key != ~0ull));
+        unsigned m = __ballot_sync(0xffffffffu, key < key_thr);
+        while (m) {
+          const int b = __ffs(m) - 1;
+          m &= m - 1;
+          const u64 k = __shfl_sync(0xffffffffu, key, b);
+          if (k < key_thr) {
+            W.insert(k);
+            key_thr = W.get(K - 1);
+          }
+        }
+      };
+      tree_walk_all(t, one, limit, leaf);
+      const int got = min((int)found, K);
+      if (lane == s) have = got;
+#pragma unroll
+      for (int p = 0; p < (KCAP > 32 ? 2 : 1); ++p) {
+        const int j = p * 32 + lane;
+        if (j < got) {
+          if constexpr (MODE == TREE_PAIRS) {
+            const size_t at = (size_t)sidx * K + j;
+            if (o.idx) o.idx[at] = nbr_idx(W.e[p]);
+            if (o.d2) o.d2[at] = nbr_d2(W.e[p]);
+          } else {
+            sorted[j][s] = t.pos_of[nbr_idx(W.e[p])];
+          }
+        }
+      }
+    }
+    if constexpr (MODE == TREE_PAIRS) {
+      if (active) {
+        for (int j = have; j < K; ++j) {
+          if (o.idx) o.idx[(size_t)qidx * K + j] = -1;
+          if (o.d2) o.d2[(size_t)qidx * K + j] = INFINITY;
+        }
+        if (o.counts) o.counts[qidx] = have;
+      }
+    } else {
+      __syncwarp();
+      if (!active) return;
+      auto nbr = [&](int j) { return __ldg(&t.pts[sorted[j][lane]]); };
+      if constexpr (MODE == TREE_NORMALS) {
+        float nx = 0.0f, ny = 0.0f, nz = 0.0f;
+        if (have >= 3)
+          nd::normal_from_points(nbr, have, true, o.iters, q.x, q.y, q.z, o.vpx, o.vpy, o.vpz, nx,
+                                 ny, nz);
+        o.nx[qidx] = nx;
+        o.ny[qidx] = ny;
+        o.nz[qidx] = nz;
+      } else {
+        float nx, ny, nz, cond;
+        bool wide;
+        nd::precise_normal(nbr, have, q.x, q.y, q.z, o.vpx, o.vpy, o.vpz, o.cond_fp64, nx, ny, nz,
+                           cond, wide);
+        o.nx[qidx] = nx;
+        o.ny[qidx] = ny;
+        o.nz[qidx] = nz;
+        if (o.cond) o.cond[qidx] = cond;
+        if (o.used64) o.used64[qidx] = wide ? 1 : 0;
+      }
+    }
+  }
+}
+
+template <int KCAP, int MODE>
+void launch_tree(rvp_context *ctx, const TreeView &t, const TreeQueries &q, int K, float bound,
+                 const TreeOut &o) {
+  constexpr size_t smem = tree_smem<KCAP, MODE>();
+  static_assert(smem <= 48 * 1024, "no opt-in to larger shared memory here");
+  k_knn_tree<KCAP, MODE><<<(q.n + 31) / 32, 32, smem, ctx->stream>>>(t, q, K, bound, o);
+  RVP_LAUNCH_CHECK(ctx);
+}
+
+template <int MODE>
+void launch_tree_k(rvp_context *ctx, const TreeView &t, const TreeQueries &q, int K, float bound,
+                   const TreeOut &o) {
+  if (K <= 9) launch_tree<9, MODE>(ctx, t, q, K, bound, o);
+  else if (K <= 17) launch_tree<17, MODE>(ctx, t, q, K, bound, o);
+  else if (K <= 25) launch_tree<25, MODE>(ctx, t, q, K, bound, o);
+  else if (K <= 33) launch_tree<33, MODE>(ctx, t, q, K, bound, o);
+  else launch_tree<64, MODE>(ctx, t, q, K, bound, o);
+}
+}  // namespace
+
+void KnnTree::release() {
+  keys.release(); vals.release(); sort.release(); pts.release(); pos.release(); boxes.release();
+  misc.release(); qkeys.release(); qvals.release(); qpts.release();
+}
+
+TreeView tree_build(rvp_context *ctx, KnnTree &w, const float *x, const float *y, const float *z,
+                    size_t n) {
+  w.keys.reserve(n * 8);
+  w.vals.reserve(n * 4);
+  w.sort.reserve(sort_temp_bytes(n));
+  w.pts.reserve(n * 16);
+  w.pos.reserve(n * 4);
+  w.misc.reserve(256);
+  TreeView t{};
+  t.n = (u32)n;
+  size_t total = 0;
+  u32 c = (u32)((n + 31) / 32);
+  for (int l = 0; l < kTreeLevels; ++l, c = (c + 31) / 32) {
+    t.count[l] = c;
+    t.stride[l] = (c + 31) & ~31u;
+    total += (size_t)t.stride[l] * 6 * 4;
+  }
+  w.boxes.reserve(total);
+  float *b = w.boxes.as<float>();
+  for (int l = 0; l < kTreeLevels; ++l) {
+    t.box[l] = b;
+    b += (size_t)t.stride[l] * 6;
+  }
+  t.pts = w.pts.as<float4>();
+  t.pos_of = w.pos.as<u32>();
+  t.keys = w.keys.as<u64>();
+  t.bb = w.misc.as<float>();
+  cudaStream_t st = ctx->stream;
+  const int sms = ctx->num_sms;
+  k_tree_init<<<1, 32, 0, st>>>(w.misc.as<float>());
+  RVP_LAUNCH_CHECK(ctx);
+  cloud_bbox(ctx, x, y, z, n, w.misc.as<float>());
+  k_tree_keys<<<grid_for(n, 256, sms * 8), 256, 0, st>>>(x, y, z, n, nullptr, t.bb,
+                                                         w.keys.as<u64>(), w.vals.as<u32>());
+  RVP_LAUNCH_CHECK(ctx);
+  SortTemp tmp;
+  sort_temp_carve(tmp, w.sort.ptr, n);
+  radix_sort_pairs(ctx, w.keys.as<u64>(), w.vals.as<u32>(), n, nullptr, tmp);
+  k_tree_leaves<<<(unsigned)((t.count[0] + 7) / 8), 256, 0, st>>>(
+      x, y, z, w.vals.as<u32>(), t.n, w.pts.as<float4>(), w.pos.as<u32>(), t.box[0], t.stride[0]);
+  RVP_LAUNCH_CHECK(ctx);
+  int level = 1;
+  if (t.count[1] > 32) {  // past one block's reach
+    k_tree_parents<<<(t.count[1] + 7) / 8, 256, 0, st>>>(t, 1);
+    RVP_LAUNCH_CHECK(ctx);
+    level = 2;
+  }
+  k_tree_top<<<1, 1024, 0, st>>>(t, level);
+  RVP_LAUNCH_CHECK(ctx);
+  return t;
+}
+
+TreeQueries tree_queries(rvp_context *ctx, KnnTree &w, const TreeView &t, const float *x,
+                         const float *y, const float *z, const float *qx, const float *qy,
+                         const float *qz, size_t nq) {
+  TreeQueries q{};
+  q.n = (u32)nq;
+  if (qx == x && qy == y && qz == z && nq == t.n) return q;
+  w.qkeys.reserve(nq * 8);
+  w.qvals.reserve(nq * 4);
+  w.qpts.reserve(nq * 16);
+  w.sort.reserve(sort_temp_bytes(std::max<size_t>(nq, t.n)));
+  u64 *n_sort = w.misc.as<u64>() + 4;
+  cudaStream_t st = ctx->stream;
+  const unsigned gb = grid_for(nq, 256, ctx->num_sms * 8);
+  k_tree_count<<<1, 1, 0, st>>>(n_sort, nq == t.n ? 0 : (u64)nq);
+  RVP_LAUNCH_CHECK(ctx);
+  if (nq == t.n) {
+    k_tree_same<<<gb, 256, 0, st>>>(qx, qy, qz, x, y, z, nq, n_sort);
+    RVP_LAUNCH_CHECK(ctx);
+  }
+  k_tree_keys<<<gb, 256, 0, st>>>(qx, qy, qz, nq, n_sort, t.bb, w.qkeys.as<u64>(),
+                                  w.qvals.as<u32>());
+  RVP_LAUNCH_CHECK(ctx);
+  SortTemp tmp;
+  sort_temp_carve(tmp, w.sort.ptr, nq);
+  radix_sort_pairs(ctx, w.qkeys.as<u64>(), w.qvals.as<u32>(), nq, n_sort, tmp);
+  k_tree_queries<<<gb, 256, 0, st>>>(qx, qy, qz, w.qvals.as<u32>(), n_sort, w.qpts.as<float4>());
+  RVP_LAUNCH_CHECK(ctx);
+  q.q = w.qpts.as<float4>();
+  q.keys = w.qkeys.as<u64>();
+  q.n_sort = n_sort;
+  return q;
+}
+
+void tree_knn(rvp_context *ctx, const TreeView &t, const TreeQueries &q, int k, float radius,
+              int mode, const TreeOut &o) {
+  // the radius search's bound: d2 <= radius * radius in float
+  volatile float r = radius;
+  const float bound = radius > 0.0f ? r * r : INFINITY;
+  switch (mode) {
+    case TREE_MEAN: launch_tree_k<TREE_MEAN>(ctx, t, q, k, bound, o); break;
+    case TREE_PAIRS: launch_tree_k<TREE_PAIRS>(ctx, t, q, k, bound, o); break;
+    case TREE_NORMALS: launch_tree_k<TREE_NORMALS>(ctx, t, q, k, bound, o); break;
+    default: launch_tree_k<TREE_PRECISE>(ctx, t, q, k, bound, o);
+  }
+}
+
+}  // namespace rvp

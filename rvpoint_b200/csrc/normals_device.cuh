@@ -192,3 +192,176 @@ __device__ __forceinline__ void normal_from_keys(const float *__restrict__ x,
 }
 }  // namespace nd
 }  // namespace rvp
+
+namespace rvp {
+namespace nd {
+// normal_from_list over points: nbr(t) is the t-th neighbour's record
+template <class Nbr>
+__device__ __forceinline__ void normal_from_points(Nbr nbr, int m, bool div_centroid, int iters,
+                                                   float qx, float qy, float qz, float vpx,
+                                                   float vpy, float vpz, float &nx, float &ny,
+                                                   float &nz) {
+  float cx = 0.0f, cy = 0.0f, cz = 0.0f;
+  for (int t = 0; t < m; ++t) {
+    const float4 p = nbr(t);
+    cx = fadd(cx, p.x);
+    cy = fadd(cy, p.y);
+    cz = fadd(cz, p.z);
+  }
+  if (div_centroid) {
+    const float fm = (float)m;
+    cx = fdiv(cx, fm);
+    cy = fdiv(cy, fm);
+    cz = fdiv(cz, fm);
+  } else {
+    const float inv_n = fdiv(1.0f, (float)m);
+    cx = fmul(cx, inv_n);
+    cy = fmul(cy, inv_n);
+    cz = fmul(cz, inv_n);
+  }
+  float c00 = 0, c01 = 0, c02 = 0, c11 = 0, c12 = 0, c22 = 0;
+  for (int t = 0; t < m; ++t) {
+    const float4 p = nbr(t);
+    const float dx = fsub(p.x, cx), dy = fsub(p.y, cy), dz = fsub(p.z, cz);
+    c00 = fadd(c00, fmul(dx, dx));
+    c01 = fadd(c01, fmul(dx, dy));
+    c02 = fadd(c02, fmul(dx, dz));
+    c11 = fadd(c11, fmul(dy, dy));
+    c12 = fadd(c12, fmul(dy, dz));
+    c22 = fadd(c22, fmul(dz, dz));
+  }
+  float A[3][3] = {{c00, c01, c02}, {c01, c11, c12}, {c02, c12, c22}};
+  eigen_smallest_ref(A, iters, nx, ny, nz);
+  flip_ref(qx, qy, qz, vpx, vpy, vpz, nx, ny, nz);
+}
+
+// ---------------------------------------------------------------------------
+// precision path: covariance accumulated in FP32 about the query point
+// (differences of nearby points are exact) with compensated (Kahan) sums,
+// converged cyclic Jacobi in FP32, and the eigen-solve redone in FP64 only
+// when lambda_max / lambda_min exceeds a threshold.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void kahan_add(float &s, float &c, float v) {
+  const float y = fsub(v, c);
+  const float t = fadd(s, y);
+  c = fsub(fsub(t, s), y);
+  s = t;
+}
+
+template <class T>
+__device__ void jacobi_sym3(T A[3][3], T V[3][3], int sweeps) {
+  for (int i = 0; i < 3; ++i)
+    for (int j = 0; j < 3; ++j) V[i][j] = (i == j) ? T(1) : T(0);
+  for (int sw = 0; sw < sweeps; ++sw) {
+    const T off = A[0][1] * A[0][1] + A[0][2] * A[0][2] + A[1][2] * A[1][2];
+    const T dia = A[0][0] * A[0][0] + A[1][1] * A[1][1] + A[2][2] * A[2][2];
+    if (!(off > (sizeof(T) == 4 ? T(1e-14) : T(1e-30)) * dia)) break;
+#pragma unroll
+    for (int pq = 0; pq < 3; ++pq) {
+      const int p = pq == 2 ? 1 : 0;
+      const int q = pq == 0 ? 1 : 2;
+      if (A[p][q] == T(0)) continue;
+      const T theta = (A[q][q] - A[p][p]) / (T(2) * A[p][q]);
+      const T t = (theta >= T(0) ? T(1) : T(-1)) / (fabs(theta) + sqrt(theta * theta + T(1)));
+      const T c = T(1) / sqrt(t * t + T(1)), s = t * c;
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        const T arp = A[r][p], arq = A[r][q];
+        A[r][p] = c * arp - s * arq;
+        A[r][q] = s * arp + c * arq;
+      }
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        const T apr = A[p][r], aqr = A[q][r];
+        A[p][r] = c * apr - s * aqr;
+        A[q][r] = s * apr + c * aqr;
+      }
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        const T vrp = V[r][p], vrq = V[r][q];
+        V[r][p] = c * vrp - s * vrq;
+        V[r][q] = s * vrp + c * vrq;
+      }
+    }
+  }
+}
+
+// column of the smallest / largest diagonal entry (first of equals)
+template <class T>
+__device__ __forceinline__ int smallest_diag(const T (&A)[3][3]) {
+  int m = 0;
+  T d = A[0][0];
+  if (A[1][1] < d) { m = 1; d = A[1][1]; }
+  if (A[2][2] < d) m = 2;
+  return m;
+}
+template <class T>
+__device__ __forceinline__ T pick3(int m, T a, T b, T c) {
+  return m == 0 ? a : (m == 1 ? b : c);
+}
+
+template <class Nbr>
+__device__ __forceinline__ void precise_normal(Nbr nbr, int kk, float qx, float qy, float qz,
+                                               float vpx, float vpy, float vpz, double cond_fp64,
+                                               float &nx, float &ny, float &nz, float &cond,
+                                               bool &wide) {
+  // shifted, compensated centroid of (p - q)
+  float sx = 0, sy = 0, sz = 0, ex = 0, ey = 0, ez = 0;
+  for (int t = 0; t < kk; ++t) {
+    const float4 p = nbr(t);
+    kahan_add(sx, ex, fsub(p.x, qx));
+    kahan_add(sy, ey, fsub(p.y, qy));
+    kahan_add(sz, ez, fsub(p.z, qz));
+  }
+  const float inv = fdiv(1.0f, (float)kk);
+  const float cx = fmul(sx, inv), cy = fmul(sy, inv), cz = fmul(sz, inv);
+  float s[6] = {0, 0, 0, 0, 0, 0}, e[6] = {0, 0, 0, 0, 0, 0};
+  for (int t = 0; t < kk; ++t) {
+    const float4 p = nbr(t);
+    const float dx = fsub(fsub(p.x, qx), cx);
+    const float dy = fsub(fsub(p.y, qy), cy);
+    const float dz = fsub(fsub(p.z, qz), cz);
+    kahan_add(s[0], e[0], fmul(dx, dx));
+    kahan_add(s[1], e[1], fmul(dx, dy));
+    kahan_add(s[2], e[2], fmul(dx, dz));
+    kahan_add(s[3], e[3], fmul(dy, dy));
+    kahan_add(s[4], e[4], fmul(dy, dz));
+    kahan_add(s[5], e[5], fmul(dz, dz));
+  }
+  float A[3][3] = {{s[0], s[1], s[2]}, {s[1], s[3], s[4]}, {s[2], s[4], s[5]}};
+  float V[3][3];
+  jacobi_sym3<float>(A, V, 8);
+  const int mi = smallest_diag(A);
+  const float lo = fabsf(pick3(mi, A[0][0], A[1][1], A[2][2]));
+  const float hi = fabsf(A[2][2] > fmaxf(A[0][0], A[1][1])
+                             ? A[2][2] : (A[1][1] > A[0][0] ? A[1][1] : A[0][0]));
+  const double cnd = lo > 0.0f ? (double)hi / (double)lo : 1e300;
+  double ax, ay, az;
+  wide = cnd > cond_fp64;
+  if (wide) {
+    // fold the compensation terms back in
+    const double d00 = (double)s[0] - e[0], d01 = (double)s[1] - e[1], d02 = (double)s[2] - e[2],
+                 d11 = (double)s[3] - e[3], d12 = (double)s[4] - e[4], d22 = (double)s[5] - e[5];
+    double D[3][3] = {{d00, d01, d02}, {d01, d11, d12}, {d02, d12, d22}};
+    double W[3][3];
+    jacobi_sym3<double>(D, W, 32);
+    const int m2 = smallest_diag(D);
+    ax = pick3(m2, W[0][0], W[0][1], W[0][2]);
+    ay = pick3(m2, W[1][0], W[1][1], W[1][2]);
+    az = pick3(m2, W[2][0], W[2][1], W[2][2]);
+  } else {
+    ax = pick3(mi, V[0][0], V[0][1], V[0][2]);
+    ay = pick3(mi, V[1][0], V[1][1], V[1][2]);
+    az = pick3(mi, V[2][0], V[2][1], V[2][2]);
+  }
+  const double nr = sqrt(ax * ax + ay * ay + az * az);
+  ax /= nr; ay /= nr; az /= nr;
+  const double dot = ((double)vpx - qx) * ax + ((double)vpy - qy) * ay + ((double)vpz - qz) * az;
+  if (dot < 0) { ax = -ax; ay = -ay; az = -az; }
+  nx = (float)ax;
+  ny = (float)ay;
+  nz = (float)az;
+  cond = (float)cnd;
+}
+}  // namespace nd
+}  // namespace rvp

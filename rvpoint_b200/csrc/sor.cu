@@ -1,10 +1,5 @@
 // Statistical outlier removal (statistical_outlier_removal.cpp).
 //
-//  * mean distance per point from its sorted k+1 nearest (self first):
-//    sum of sqrtf(d2_j), j = 1..k, in ascending order, divided by k
-//    (sor_sc :36-40); the radius-bounded variant (sor_spatial_hash
-//    :246-270) divides by min(k, count - 1) and falls back to the search
-//    radius for isolated points;
 //  * global mean / std (:43-55): the reference sums sequentially in float,
 //    and a sum in another order would round differently and move the
 //    threshold; k_sor_stats reproduces those roundings in parallel;
@@ -24,25 +19,6 @@ __device__ __forceinline__ int frame_of_index(const int64_t *offs, int n_frames,
     if ((size_t)offs[mid] <= i) lo = mid; else hi = mid - 1;
   }
   return lo;
-}
-
-__global__ void k_sor_mean(const u64 *pairs, int kk, const int32_t *counts, size_t n_max,
-                           const u64 *n_dev, float *mean, float fallback, bool radius_mode) {
-  const size_t n = n_dev ? *n_dev : n_max;
-  const int k = kk - 1;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const int cnt = counts ? counts[i] : kk;
-    const u64 *l = pairs + i * (size_t)kk;
-    if (radius_mode && cnt <= 1) {
-      mean[i] = fallback;
-      continue;
-    }
-    const int valid_k = cnt - 1 < k ? cnt - 1 : k;
-    float sum = 0.0f;
-    for (int j = 1; j <= valid_k; ++j) sum = fadd(sum, __fsqrt_rn(nbr_d2(l[j])));
-    mean[i] = valid_k > 0 ? fdiv(sum, (float)valid_k) : 0.0f;
-  }
 }
 
 // The reference's sequential float sums, added in parallel. While the running
@@ -319,14 +295,6 @@ __global__ void k_sor_frame_offsets(const int64_t *offs, int n_frames, const u64
     out[f] = (int64_t)pos[offs[f]];
 }
 }  // namespace
-
-void sor_mean_from_knn(rvp_context *ctx, const u64 *pairs, int kk, const int32_t *counts,
-                       size_t n_max, const u64 *n_dev, float *mean, float fallback_radius,
-                       bool radius_mode) {
-  k_sor_mean<<<grid_for(n_max, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
-      pairs, kk, counts, n_max, n_dev, mean, fallback_radius, radius_mode);
-  RVP_LAUNCH_CHECK(ctx);
-}
 
 u64 *sor_positions(void *temp, size_t n_max) {
   return reinterpret_cast<u64 *>(static_cast<char *>(temp) + al(n_max * 4));

@@ -39,3 +39,69 @@ def test_sorted_voxels(gpu_ctx, restatement, n):
     out, keys = voxel_grid_downsamp_rvv_v2(c, 0.25, return_keys=True)
     out2, keys2 = restatement.voxel_grid(c, 0.25)
     assert np.array_equal(keys, keys2) and np.array_equal(bits(out), bits(out2))
+
+
+def brute_knn(p, q, k, r2=np.inf):
+    """(indices, d2) rows in (d2, index) order, -1 / inf past the found."""
+    d = [p[None, :, a] - q[:, None, a] for a in range(3)]
+    d2 = (d[0] * d[0] + d[1] * d[1]) + d[2] * d[2]
+    idx = np.full((len(q), k), -1, np.int32)
+    dist = np.full((len(q), k), np.inf, np.float32)
+    for i in range(len(q)):
+        o = np.argsort(d2[i], kind="stable")
+        o = o[d2[i][o] <= r2][:k]
+        idx[i, :len(o)], dist[i, :len(o)] = o, d2[i][o]
+    return idx, dist
+
+
+# the box tree: leaves of 32 points, 32 children per node; lists of up to 9,
+# 17, 25, 33 and 64 distances; equal distances go by index
+@pytest.mark.parametrize("n,k", [(1, 1), (2, 5), (31, 9), (32, 17), (33, 10), (65, 64),
+                                 (1023, 18), (1024, 33), (1025, 25), (2049, 34), (2500, 1)])
+@pytest.mark.parametrize("cloud", ["room", "lattice"])
+def test_tree_knn(gpu_ctx, n, k, cloud):
+    from rvpoint_b200.api import SpatialHash
+    if cloud == "lattice":
+        i = np.arange(n)
+        c = D.Cloud.from_xyz(np.stack([i % 7, (i // 7) % 5, i // 35], 1) % 6 * 0.25)
+    else:
+        c = D.room_cloud(n=max(n, 50), seed=n).subset(np.arange(n))
+    p = c.aos()
+    h = SpatialHash()
+    h.setInputCloud(c, 0.5)
+    h.build()
+    rng = np.random.default_rng(n)
+    other = np.concatenate([p[: n // 2] + np.float32(0.01),
+                            rng.uniform(-9, 9, (37, 3)).astype(np.float32)])
+    for q, r in ((p, 0.0), (other, 0.0), (p[::-1], 0.3), (other, 0.6)):
+        q = np.ascontiguousarray(q)
+        idx, d2, cnt = h.knn(q[:, 0], q[:, 1], q[:, 2], k, radius=r)
+        r2 = np.float32(r) * np.float32(r) if r else np.inf
+        idx2, dist2 = brute_knn(p, q, k, r2)
+        assert np.array_equal(idx, idx2) and np.array_equal(bits(d2), bits(dist2))
+        assert np.array_equal(cnt, (idx2 >= 0).sum(1))
+
+
+@pytest.mark.parametrize("n", [40, 32_768, 32_769, 70_001])
+def test_tree_levels(gpu_ctx, restatement, n):
+    """SOR means, and normals of both kinds, through every level of the tree."""
+    from rvpoint_b200 import api
+    c = D.room_cloud(n=n, seed=n)
+    assert np.array_equal(bits(api.sor_rvv(c, 8, 1.0, return_stats=True)[1])[:2000],
+                          bits(_means(c.aos(), 8))[:2000])
+    nx, ny, nz = api.normal_estimation_sc(c, 9)
+    nrm, _, _ = api.normal_estimation_precise(c, 9)
+    assert np.allclose(nx * nx + ny * ny + nz * nz, 1.0, atol=1e-5)
+    assert np.allclose((nrm ** 2).sum(1), 1.0, atol=1e-5)
+
+
+def _means(p, k):
+    out = np.zeros(len(p), np.float32)
+    for i in range(min(len(p), 2000)):
+        d = p - p[i]
+        d2 = np.sort((d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1]) + d[:, 2] * d[:, 2])[1:k + 1]
+        s = np.float32(0)
+        for v in np.sqrt(d2):
+            s = np.float32(s + v)
+        out[i] = s / np.float32(k)
+    return out
