@@ -380,6 +380,8 @@ struct TreeQueries {
   const float4 *q = nullptr;     // {x, y, z, index} in key order
   const u64 *keys = nullptr;     // their sorted keys
   const u64 *n_sort = nullptr;   // null, or 0 there: the queries are the cloud
+  u32 *hard_count = nullptr;     // queries left for the warp-per-query kernel
+  u32 *hard = nullptr;           // (their places in q, or in the tree)
   u32 n = 0;
 };
 // TREE_MEAN: SOR's mean distance; TREE_PAIRS: rows of k indices and squared
@@ -401,7 +403,7 @@ struct TreeOut {  // by query index; null pointers are skipped
   uint8_t *used64 = nullptr;
 };
 struct KnnTree {
-  DevBuf keys, vals, sort, pts, pos, boxes, misc, qkeys, qvals, qpts;
+  DevBuf keys, vals, sort, pts, pos, boxes, misc, qkeys, qvals, qpts, hard;
   void release();
 };
 TreeView tree_build(rvp_context *ctx, KnnTree &w, const float *x, const float *y, const float *z,

@@ -11,21 +11,24 @@
 // the boxes of 32 children at once against the box of the queries and go down
 // into those nearer than the largest K-th distance so far, nearest first; a
 // leaf's points are staged in shared memory and every lane tests all of them
-// against its own query. What passes waits in a buffer per lane and goes
-// through a sorted list of distances (registers) when a buffer fills, so the
-// insertions of the lanes run side by side. With the K-th distance known, a
-// second walk collects the points within it and each goes to its rank.
+// against its own query. What passes waits in a buffer per lane (distance and
+// position) and goes through a sorted list of distances (registers) when a
+// buffer fills, so the insertions of the lanes run side by side; the buffer
+// keeps what is within the K-th distance, and at the end each goes to its
+// rank. Queries that do not fit this (far from their packet, equal distances)
+// are listed and answered one per warp by a second kernel.
 //
 // Pruning needs no slack: every operation of the distance (subtract, square,
 // add) is monotone under rounding, so the distance to a box computed with the
 // same operations is never above the computed distance to a point inside it.
-// Equal distances are ordered by index: a query whose list holds equal ones
-// is answered again by the whole warp on packed (distance, index) keys.
+// Equal distances are ordered by index: the second kernel works on packed
+// (distance, index) keys.
 //
 // Bound by issue (box tests, distance tests and list insertions). The grid
 // search it replaces for single clouds ran one warp per query on cells sized
 // from a sample of queries: 105k LiDAR points, k 16, 3818 us; a 2M-point map,
 // k 33, 14,225 us.
+#include <float.h>
 #include <math.h>
 
 #include <algorithm>
@@ -263,30 +266,84 @@ __device__ __forceinline__ void tree_walk_all(const TreeView &t, const Box &q, L
     tree_walk<kTreeLevels - 1>(t, q, f, limit, leaf);
 }
 
-constexpr int kTreeBuf = 64;   // buffered distances per lane; flushed above 32
-constexpr int kTreeExtra = 3;  // collected points past K (equal distances)
+constexpr int kTreeExtra = 3;  // rows past K for equal distances
+// a query joins its packet's walk if its limit (a squared distance) is within
+// this factor of the median one
+constexpr float kLoner = 16.0f;
+// leaves a packet tests before it gives up. Packets test 19 to 41 leaves on
+// average (k 16 to 32); one that spans a jump of the Morton order has every
+// leaf of a large box to test, up to 2 ms, with no other work left to hide it
+constexpr int kLeafBudget = 128;
 
+// per lane and row: a distance (the mean needs no more) or a distance and a
+// tree position; a flush leaves at most KCAP + kTreeExtra rows (distances
+// only: none), a leaf adds up to 32
+template <int KCAP, int MODE>
+constexpr int tree_rows() {
+  return MODE == TREE_MEAN ? 64 : KCAP + kTreeExtra + 32;
+}
 template <int KCAP, int MODE>
 constexpr size_t tree_smem() {
-  size_t buf = (size_t)kTreeBuf * 32 * 4;
-  const size_t pairs = (size_t)(KCAP + kTreeExtra) * 32 * 8;
-  if (MODE != TREE_MEAN && pairs > buf) buf = pairs;
-  const size_t sorted = MODE == TREE_NORMALS || MODE == TREE_PRECISE ? (size_t)KCAP * 32 * 4 : 0;
-  return 32 * 16 + buf + sorted;
+  return 32 * 16 + (size_t)tree_rows<KCAP, MODE>() * 32 * (MODE == TREE_MEAN ? 4 : 8);
+}
+
+// the leaf where a query of this key would lie
+__device__ __forceinline__ u32 leaf_of_key(const TreeView &t, u64 key) {
+  u32 lo = 0, hi = t.n - 1;
+  while (lo < hi) {
+    const u32 m = (lo + hi) >> 1;
+    if (t.keys[m] < key) lo = m + 1; else hi = m;
+  }
+  return lo / 32;
+}
+
+// sor_sc's mean (statistical_outlier_removal.cpp:36-40): the ascending sum of
+// sqrtf(d2_j), j = 1 .. k, over k; within a radius over those found, and the
+// radius itself for a point without neighbours (:246-270)
+__device__ __forceinline__ void tree_mean_out(float sum, int have, const float4 &q, u32 qidx,
+                                              const TreeOut &o) {
+  float m = have > 1 ? fdiv(sum, (float)(have - 1)) : 0.0f;
+  if (o.radius_mode && have <= 1) m = o.fallback;
+  const float none = dist2(q.x, q.y, q.z, q.x, q.y, q.z);  // NaN without a position
+  o.mean[qidx] = none == 0.0f ? m : none;
+}
+
+// the normal of a query from its sorted neighbours nbr(0 .. have - 1)
+template <int MODE, class Nbr>
+__device__ __forceinline__ void tree_normal_out(Nbr nbr, int have, const float4 &q, u32 qidx,
+                                                const TreeOut &o) {
+  float nx = 0.0f, ny = 0.0f, nz = 0.0f;
+  if constexpr (MODE == TREE_NORMALS) {
+    if (have >= 3)
+      nd::normal_from_points(nbr, have, true, o.iters, q.x, q.y, q.z, o.vpx, o.vpy, o.vpz, nx, ny,
+                             nz);
+  } else {
+    float cond;
+    bool wide;
+    nd::precise_normal(nbr, have, q.x, q.y, q.z, o.vpx, o.vpy, o.vpz, o.cond_fp64, nx, ny, nz,
+                       cond, wide);
+    if (o.cond) o.cond[qidx] = cond;
+    if (o.used64) o.used64[qidx] = wide ? 1 : 0;
+  }
+  o.nx[qidx] = nx;
+  o.ny[qidx] = ny;
+  o.nz[qidx] = nz;
 }
 
 // one warp (block) per packet of 32 queries; KCAP >= K
 template <int KCAP, int MODE>
-__global__ __launch_bounds__(32, KCAP > 33 ? 12 : 16) void k_knn_tree(TreeView t, TreeQueries qs,
-                                                                      int K, float bound,
-                                                                      TreeOut o) {
+__global__ __launch_bounds__(32, KCAP > 33 ? 8 : 16) void k_knn_tree(TreeView t, TreeQueries qs,
+                                                                     int K, float bound,
+                                                                     TreeOut o) {
   extern __shared__ __align__(16) unsigned char tree_sm[];
+  constexpr bool MEAN = MODE == TREE_MEAN;
+  constexpr int ROWS = tree_rows<KCAP, MODE>();
   float4 *stage = reinterpret_cast<float4 *>(tree_sm);
   float(*fbuf)[32] = reinterpret_cast<float(*)[32]>(tree_sm + 512);
   uint2(*pbuf)[32] = reinterpret_cast<uint2(*)[32]>(tree_sm + 512);
-  constexpr int PCAP = KCAP + kTreeExtra;
-  constexpr size_t kBuf = tree_smem<KCAP, TREE_PAIRS>() - 512;
-  u32(*sorted)[32] = reinterpret_cast<u32(*)[32]>(tree_sm + 512 + kBuf);
+  // the sorted positions, over the 32 rows that only a leaf's hits use
+  u32(*sorted)[32] = reinterpret_cast<u32(*)[32]>(tree_sm + 512 + (size_t)(KCAP + kTreeExtra) * 256);
+  static_assert(KCAP <= 64, "sorted positions fit the rows of a leaf");
   const int lane = threadIdx.x;
   const u32 packet = blockIdx.x;
   // the cloud's own points (leaf `packet`), or 32 of the sorted queries
@@ -297,21 +354,112 @@ __global__ __launch_bounds__(32, KCAP > 33 ? 12 : 16) void k_knn_tree(TreeView t
   const float4 q = src[active ? qi : packet * 32];
   const u32 qidx = __float_as_uint(q.w);
   u32 start = packet;
-  if (!self) {  // the leaf where a query of the middle would lie
-    const u64 mid = qs.keys[min(packet * 32 + 16, qs.n - 1)];
-    u32 lo = 0, hi = t.n - 1;
-    while (lo < hi) {
-      const u32 m = (lo + hi) >> 1;
-      if (t.keys[m] < mid) lo = m + 1; else hi = m;
+  if (!self) start = leaf_of_key(t, qs.keys[min(packet * 32 + 16, qs.n - 1)]);
+  const Box own{{q.x, q.y, q.z}, {q.x, q.y, q.z}};
+
+  // ---- the sorted distances: slots 0 .. pad - 1 hold -1 and never move
+  const int pad = KCAP - K;
+  float L[KCAP];
+#pragma unroll
+  for (int j = 0; j < KCAP; ++j) L[j] = j < pad ? -1.0f : INFINITY;
+  bool mine = active;  // answered with the packet
+  int cnt = 0, done = 0;  // buffered rows, and those already in the list
+  float lim = -1.0f, pmax = -1.0f;  // what the buffer takes: d2 <= lim; its largest
+  auto limits = [&]() {
+    lim = mine ? fminf(fminf(L[KCAP - 1], bound), FLT_MAX) : -1.0f;
+    pmax = __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(lim)));
+  };
+  limits();
+  auto flush = [&]() {
+    const int most = __reduce_max_sync(0xffffffffu, cnt - done);
+    for (int i = 0; i < most; ++i) {
+      float key = INFINITY;
+      if (done + i < cnt)
+        key = MEAN ? fbuf[done + i][lane] : __uint_as_float(pbuf[done + i][lane].x);
+      if (__any_sync(0xffffffffu, key < L[KCAP - 1])) {
+#pragma unroll
+        for (int j = KCAP - 1; j > 0; --j) L[j] = fmaxf(L[j - 1], fminf(L[j], key));
+        L[0] = fminf(L[0], key);
+      }
     }
-    start = lo / 32;
+    if constexpr (MEAN) {
+      cnt = 0;
+    } else {  // keep what is within the K-th distance
+      const float top = L[KCAP - 1];
+      int m = 0;
+      for (int i = 0; i < cnt; ++i) {
+        const uint2 b = pbuf[i][lane];
+        if (__uint_as_float(b.x) <= top) pbuf[m++][lane] = b;
+      }
+      cnt = m;
+      if (m > KCAP + kTreeExtra) {  // too many equal ones: not with the packet
+        mine = false;
+        cnt = 0;
+      }
+      done = cnt;
+    }
+    __syncwarp();
+    limits();
+  };
+  int budget = kLeafBudget;
+  auto scan_leaf = [&](u32 l) {
+    if (--budget < 0) {  // (uniform) nothing is left open: the walk ends
+      mine = false;
+      pmax = -1.0f;
+      return;
+    }
+    const u32 i = l * 32 + lane;
+    const float4 mate =
+        i < t.n ? __ldg(&t.pts[i]) : make_float4(INFINITY, INFINITY, INFINITY, 0.0f);
+    const float at = box_d2(own, t.box[0], t.stride[0], l) <= lim ? lim : -1.0f;
+    if (!__any_sync(0xffffffffu, at >= 0.0f)) return;
+    __syncwarp();
+    stage[lane] = mate;
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < 32; c += 4) {
+      float d[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float4 p = stage[c + u];
+        d[u] = dist2(p.x, p.y, p.z, q.x, q.y, q.z);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (d[u] <= at) {
+          if constexpr (MEAN) fbuf[cnt][lane] = d[u];
+          else pbuf[cnt][lane] = make_uint2(__float_as_uint(d[u]), l * 32 + c + u);
+          ++cnt;
+        }
+      }
+    }
+    if (__any_sync(0xffffffffu, cnt > ROWS - 32)) flush();
+  };
+  // the leaves around the packet's place first: they set the limits
+  const u32 s0 = start > 0 ? start - 1 : 0, s1 = min(start + 1, t.count[0] - 1);
+  for (u32 l = s0; l <= s1; ++l) scan_leaf(l);
+  flush();
+  {  // A query whose limit is far above the others' (four times the median
+     // radius) would take the packet through all the leaves around it: such
+     // loners are answered by the whole warp, one by one.
+    int rank = 0;
+    for (int s = 0; s < 32; ++s) {
+      const float other = __shfl_sync(0xffffffffu, mine ? lim : INFINITY, s);
+      rank += other < lim || (other == lim && s < lane) ? 1 : 0;
+    }
+    const unsigned mid = __ballot_sync(0xffffffffu, mine && rank == 16);
+    if (mid) {
+      const float ref = __shfl_sync(0xffffffffu, lim, __ffs(mid) - 1);
+      mine = mine && lim <= kLoner * ref;
+      limits();
+    }
   }
   Box pk;  // the box of the packet
   {
     const float v[3] = {q.x, q.y, q.z};
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      float l = v[a], h = v[a];
+      float l = mine ? v[a] : INFINITY, h = mine ? v[a] : -INFINITY;
 #pragma unroll
       for (int s = 16; s; s >>= 1) {
         l = fminf(l, __shfl_xor_sync(0xffffffffu, l, s));
@@ -321,66 +469,6 @@ __global__ __launch_bounds__(32, KCAP > 33 ? 12 : 16) void k_knn_tree(TreeView t
       pk.hi[a] = h;
     }
   }
-  const Box own{{q.x, q.y, q.z}, {q.x, q.y, q.z}};
-
-  // ---- the sorted distances: slots 0 .. pad - 1 hold -1 and never move
-  const int pad = KCAP - K;
-  float L[KCAP];
-#pragma unroll
-  for (int j = 0; j < KCAP; ++j) L[j] = j < pad ? -1.0f : INFINITY;
-  float thr = INFINITY;
-  int cnt = 0;
-  float pmax = 0.0f;
-  auto update_pmax = [&]() {
-    const float lim = active ? fminf(thr, bound) : -1.0f;
-    pmax = __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(lim)));
-  };
-  update_pmax();
-  auto flush = [&]() {
-    const int most = __reduce_max_sync(0xffffffffu, cnt);
-    for (int i = 0; i < most; ++i) {
-      const float key = i < cnt ? fbuf[i][lane] : INFINITY;
-      if (__any_sync(0xffffffffu, key < L[KCAP - 1])) {
-#pragma unroll
-        for (int j = KCAP - 1; j > 0; --j) L[j] = fmaxf(L[j - 1], fminf(L[j], key));
-        L[0] = fminf(L[0], key);
-      }
-    }
-    cnt = 0;
-    thr = L[KCAP - 1];
-    update_pmax();
-  };
-  // leaf l staged; false if no lane has a point within lim of it
-  auto stage_leaf = [&](u32 l, bool need) {
-    if (!__any_sync(0xffffffffu, need)) return false;
-    const u32 i = l * 32 + lane;
-    const float4 p = i < t.n ? __ldg(&t.pts[i]) : make_float4(INFINITY, INFINITY, INFINITY, 0.0f);
-    __syncwarp();
-    stage[lane] = p;
-    __syncwarp();
-    return true;
-  };
-  auto scan_leaf = [&](u32 l) {
-    const float lb = box_d2(own, t.box[0], t.stride[0], l);
-    const bool need = active && lb <= bound && lb < thr;
-    if (!stage_leaf(l, need)) return;
-    if (need) {
-#pragma unroll 8
-      for (int c = 0; c < 32; ++c) {
-        const float4 p = stage[c];
-        const float d = dist2(p.x, p.y, p.z, q.x, q.y, q.z);
-        if (d < thr && d <= bound) fbuf[cnt++][lane] = d;
-      }
-    }
-    if (__any_sync(0xffffffffu, cnt > kTreeBuf - 32)) flush();
-  };
-  // the leaves around the packet's place first: they set the limits
-  const u32 s0 = start > 0 ? start - 1 : 0, s1 = min(start + 1, t.count[0] - 1);
-  scan_leaf(start);
-  flush();
-  for (u32 l = s0; l <= s1; ++l)
-    if (l != start) scan_leaf(l);
-  flush();
   {
     auto limit = [&]() { return pmax; };
     auto leaf = [&](u32 l) {
@@ -390,65 +478,34 @@ __global__ __launch_bounds__(32, KCAP > 33 ? 12 : 16) void k_knn_tree(TreeView t
     flush();
   }
 
-  if constexpr (MODE == TREE_MEAN) {
-    // sor_sc's mean (statistical_outlier_removal.cpp:36-40): ascending sum of
-    // sqrtf(d2_j), j = 1 .. k, over k (over those found within a radius:
-    // :246-270, the radius itself for a point without neighbours)
+  // ---- results of the packet
+  bool exact = mine;
+  int have = 0;
+  if constexpr (MEAN) {
     // (without a radius K points are there, some infinitely far perhaps)
-    int found = 0;
     float sum = 0.0f;
 #pragma unroll
     for (int j = 0; j < KCAP; ++j) {
       if (j >= pad && (!o.radius_mode || L[j] < INFINITY)) {
-        if (found) sum = fadd(sum, __fsqrt_rn(L[j]));
-        ++found;
+        if (have) sum = fadd(sum, __fsqrt_rn(L[j]));
+        ++have;
       }
     }
-    if (active) {
-      float m = found > 1 ? fdiv(sum, (float)(found - 1)) : 0.0f;
-      if (o.radius_mode && found <= 1) m = o.fallback;
-      const float none = dist2(q.x, q.y, q.z, q.x, q.y, q.z);  // NaN without a position
-      o.mean[qidx] = none == 0.0f ? m : none;
-    }
-    return;
+    if (exact) tree_mean_out(sum, have, q, qidx, o);
   } else {
-    // ---- second walk: the points within the K-th distance
-    const float tau = active ? fminf(thr, bound) : -1.0f;
-    int want = 0;
     bool tied = false;
 #pragma unroll
     for (int j = 0; j < KCAP; ++j) {
-      if (j >= pad && L[j] < INFINITY) ++want;
+      if (j >= pad && L[j] < INFINITY) ++have;
       if (j > pad && L[j] < INFINITY && L[j] == L[j - (j > 0)]) tied = true;
     }
-    cnt = 0;
-    pmax = __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(tau)));
-    {
-      auto limit = [&]() { return pmax; };
-      auto leaf = [&](u32 l) {
-        const float lb = box_d2(own, t.box[0], t.stride[0], l);
-        const bool need = lb <= tau;
-        if (!stage_leaf(l, need)) return;
-        if (need) {
-          const int m = (int)min(32u, t.n - l * 32);
-#pragma unroll 4
-          for (int c = 0; c < m; ++c) {
-            const float4 p = stage[c];
-            const float d = dist2(p.x, p.y, p.z, q.x, q.y, q.z);
-            if (d <= tau) {
-              if (cnt < PCAP) pbuf[cnt][lane] = make_uint2(__float_as_uint(d), l * 32 + c);
-              ++cnt;
-            }
-          }
-        }
-      };
-      tree_walk_all(t, pk, limit, leaf);
-    }
-    __syncwarp();
-    const bool exact = active && cnt == want && !tied;
+    // exactly these points are within the K-th distance, no two equal (and
+    // what is missing is not there: points infinitely far would be)
+    exact = mine && cnt == have && !tied &&
+            (have == K || bound < INFINITY || (u32)have == t.n);
     // each to its rank among the sorted distances
     if (exact) {
-      for (int i = 0; i < want; ++i) {
+      for (int i = 0; i < have; ++i) {
         const uint2 b = pbuf[i][lane];
         const float d = __uint_as_float(b.x);
         int r = -pad;
@@ -463,91 +520,109 @@ __global__ __launch_bounds__(32, KCAP > 33 ? 12 : 16) void k_knn_tree(TreeView t
         }
       }
     }
-    int have = want;
-    // equal distances: the whole warp on (distance, index) keys, one query
-    // at a time
-    unsigned again = __ballot_sync(0xffffffffu, active && !exact);
-    while (again) {
-      const int s = __ffs(again) - 1;
-      again &= again - 1;
-      const float sx = __shfl_sync(0xffffffffu, q.x, s), sy = __shfl_sync(0xffffffffu, q.y, s),
-                  sz = __shfl_sync(0xffffffffu, q.z, s);
-      const u32 sidx = __shfl_sync(0xffffffffu, qidx, s);
-      WarpList<(KCAP > 32 ? 2 : 1)> W;
-      W.init();
-      u64 key_thr = W.get(K - 1);
-      u32 found = 0;
-      const Box one{{sx, sy, sz}, {sx, sy, sz}};
-      auto limit = [&]() {
-        return key_thr == ~0ull ? bound : fminf(nbr_d2(key_thr), bound);
-      };
-      auto leaf = [&](u32 l) {
-        const u32 i = l * 32 + lane;
-        u64 key = ~0ull;
-        if (i < t.n) {
-          const float4 p = __ldg(&t.pts[i]);
-          const float d = dist2(p.x, p.y, p.z, sx, sy, sz);
-          if (d <= bound) key = pack_nbr(d, (int)__float_as_uint(p.w));
-        }
-        found += __popc(__ballot_sync(0xffffffffu, key != ~0ull));
-        unsigned m = __ballot_sync(0xffffffffu, key < key_thr);
-        while (m) {
-          const int b = __ffs(m) - 1;
-          m &= m - 1;
-          const u64 k = __shfl_sync(0xffffffffu, key, b);
-          if (k < key_thr) {
-            W.insert(k);
-            key_thr = W.get(K - 1);
-          }
-        }
-      };
-      tree_walk_all(t, one, limit, leaf);
-      const int got = min((int)found, K);
-      if (lane == s) have = got;
-#pragma unroll
-      for (int p = 0; p < (KCAP > 32 ? 2 : 1); ++p) {
-        const int j = p * 32 + lane;
-        if (j < got) {
-          if constexpr (MODE == TREE_PAIRS) {
-            const size_t at = (size_t)sidx * K + j;
-            if (o.idx) o.idx[at] = nbr_idx(W.e[p]);
-            if (o.d2) o.d2[at] = nbr_d2(W.e[p]);
-          } else {
-            sorted[j][s] = t.pos_of[nbr_idx(W.e[p])];
-          }
-        }
-      }
+  }
+  // the others are listed for the second kernel
+  const unsigned again = __ballot_sync(0xffffffffu, active && !exact);
+  if (again) {
+    u32 at = 0;
+    if (lane == 0) at = atomicAdd(qs.hard_count, (u32)__popc(again));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (active && !exact) qs.hard[at + __popc(again & ((1u << lane) - 1))] = qi;
+  }
+  if (!exact) return;
+  if constexpr (MODE == TREE_PAIRS) {
+    for (int j = have; j < K; ++j) {
+      if (o.idx) o.idx[(size_t)qidx * K + j] = -1;
+      if (o.d2) o.d2[(size_t)qidx * K + j] = INFINITY;
     }
-    if constexpr (MODE == TREE_PAIRS) {
-      if (active) {
-        for (int j = have; j < K; ++j) {
-          if (o.idx) o.idx[(size_t)qidx * K + j] = -1;
-          if (o.d2) o.d2[(size_t)qidx * K + j] = INFINITY;
-        }
-        if (o.counts) o.counts[qidx] = have;
+    if (o.counts) o.counts[qidx] = have;
+  } else if constexpr (!MEAN) {
+    tree_normal_out<MODE>([&](int j) { return __ldg(&t.pts[sorted[j][lane]]); }, have, q, qidx, o);
+  }
+}
+// one warp per listed query, lanes over a leaf's points, a list of packed
+// (distance, index) keys over the lanes
+template <int P, int MODE>
+__global__ __launch_bounds__(128) void k_knn_tree_hard(TreeView t, TreeQueries qs, int K,
+                                                       float bound, TreeOut o) {
+  __shared__ u32 sorted[4][32 * P];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const u32 n = *qs.hard_count;
+  const bool self = qs.n_sort == nullptr || *qs.n_sort == 0;
+  for (u32 w = blockIdx.x * 4 + wib; w < n; w += gridDim.x * 4) {
+    const u32 qi = qs.hard[w];
+    const float4 q = self ? t.pts[qi] : qs.q[qi];
+    const u32 qidx = __float_as_uint(q.w);
+    u32 start = qi / 32;
+    if (!self) start = leaf_of_key(t, qs.keys[qi]);
+    WarpList<P> W;
+    W.init();
+    u64 key_thr = ~0ull;
+    u32 found = 0;
+    const Box own{{q.x, q.y, q.z}, {q.x, q.y, q.z}};
+    auto limit = [&]() {
+      return key_thr == ~0ull ? bound : fminf(nbr_d2(key_thr), bound);
+    };
+    auto scan = [&](u32 l) {
+      const u32 i = l * 32 + lane;
+      u64 key = ~0ull;
+      if (i < t.n) {
+        const float4 p = __ldg(&t.pts[i]);
+        const float d = dist2(p.x, p.y, p.z, q.x, q.y, q.z);
+        if (d <= bound) key = pack_nbr(d, (int)__float_as_uint(p.w));
       }
+      found += __popc(__ballot_sync(0xffffffffu, key != ~0ull));
+      unsigned m = __ballot_sync(0xffffffffu, key < key_thr);
+      if constexpr (P == 1) {
+        if (__popc(m) > 4) {  // many at once: one merge instead of serial inserts
+          W.merge_lanes((m >> lane) & 1u ? key : ~0ull);
+          key_thr = W.get(K - 1);
+          m = 0;
+        }
+      }
+      while (m) {
+        const int b = __ffs(m) - 1;
+        m &= m - 1;
+        const u64 k = __shfl_sync(0xffffffffu, key, b);
+        if (k < key_thr) {
+          W.insert(k);
+          key_thr = W.get(K - 1);
+        }
+      }
+    };
+    const u32 s0 = start > 0 ? start - 1 : 0, s1 = min(start + 1, t.count[0] - 1);
+    for (u32 l = s0; l <= s1; ++l) scan(l);
+    auto leaf = [&](u32 l) {
+      if (l < s0 || l > s1) scan(l);
+    };
+    tree_walk_all(t, own, limit, leaf);
+    const int have = min((int)found, K);
+    if constexpr (MODE == TREE_MEAN) {
+      float sum = 0.0f;
+      for (int j = 1; j < have; ++j) sum = fadd(sum, __fsqrt_rn(nbr_d2(W.get(j))));
+      if (lane == 0) tree_mean_out(sum, have, q, qidx, o);
     } else {
-      __syncwarp();
-      if (!active) return;
-      auto nbr = [&](int j) { return __ldg(&t.pts[sorted[j][lane]]); };
-      if constexpr (MODE == TREE_NORMALS) {
-        float nx = 0.0f, ny = 0.0f, nz = 0.0f;
-        if (have >= 3)
-          nd::normal_from_points(nbr, have, true, o.iters, q.x, q.y, q.z, o.vpx, o.vpy, o.vpz, nx,
-                                 ny, nz);
-        o.nx[qidx] = nx;
-        o.ny[qidx] = ny;
-        o.nz[qidx] = nz;
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        const int j = p * 32 + lane;
+        if constexpr (MODE == TREE_PAIRS) {
+          if (j < K) {
+            const size_t at = (size_t)qidx * K + j;
+            if (o.idx) o.idx[at] = j < have ? nbr_idx(W.e[p]) : -1;
+            if (o.d2) o.d2[at] = j < have ? nbr_d2(W.e[p]) : INFINITY;
+          }
+        } else {
+          if (j < have) sorted[wib][j] = t.pos_of[nbr_idx(W.e[p])];
+        }
+      }
+      if constexpr (MODE == TREE_PAIRS) {
+        if (lane == 0 && o.counts) o.counts[qidx] = have;
       } else {
-        float nx, ny, nz, cond;
-        bool wide;
-        nd::precise_normal(nbr, have, q.x, q.y, q.z, o.vpx, o.vpy, o.vpz, o.cond_fp64, nx, ny, nz,
-                           cond, wide);
-        o.nx[qidx] = nx;
-        o.ny[qidx] = ny;
-        o.nz[qidx] = nz;
-        if (o.cond) o.cond[qidx] = cond;
-        if (o.used64) o.used64[qidx] = wide ? 1 : 0;
+        __syncwarp();
+        if (lane == 0)
+          tree_normal_out<MODE>([&](int j) { return __ldg(&t.pts[sorted[wib][j]]); }, have, q,
+                                qidx, o);
+        __syncwarp();
       }
     }
   }
@@ -559,6 +634,9 @@ void launch_tree(rvp_context *ctx, const TreeView &t, const TreeQueries &q, int 
   constexpr size_t smem = tree_smem<KCAP, MODE>();
   static_assert(smem <= 48 * 1024, "no opt-in to larger shared memory here");
   k_knn_tree<KCAP, MODE><<<(q.n + 31) / 32, 32, smem, ctx->stream>>>(t, q, K, bound, o);
+  RVP_LAUNCH_CHECK(ctx);
+  k_knn_tree_hard<(KCAP > 32 ? 2 : 1), MODE>
+      <<<grid_for(q.n, 4, ctx->num_sms * 8), 128, 0, ctx->stream>>>(t, q, K, bound, o);
   RVP_LAUNCH_CHECK(ctx);
 }
 
@@ -575,7 +653,7 @@ void launch_tree_k(rvp_context *ctx, const TreeView &t, const TreeQueries &q, in
 
 void KnnTree::release() {
   keys.release(); vals.release(); sort.release(); pts.release(); pos.release(); boxes.release();
-  misc.release(); qkeys.release(); qvals.release(); qpts.release();
+  misc.release(); qkeys.release(); qvals.release(); qpts.release(); hard.release();
 }
 
 TreeView tree_build(rvp_context *ctx, KnnTree &w, const float *x, const float *y, const float *z,
@@ -635,6 +713,10 @@ TreeQueries tree_queries(rvp_context *ctx, KnnTree &w, const TreeView &t, const 
                          const float *qz, size_t nq) {
   TreeQueries q{};
   q.n = (u32)nq;
+  w.hard.reserve(nq * 4 + 256);
+  q.hard_count = w.hard.as<u32>();
+  q.hard = q.hard_count + 64;
+  RVP_CUDA_TRY(cudaMemsetAsync(q.hard_count, 0, 4, ctx->stream));
   if (qx == x && qy == y && qz == z && nq == t.n) return q;
   w.qkeys.reserve(nq * 8);
   w.qvals.reserve(nq * 4);
