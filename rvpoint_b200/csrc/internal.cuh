@@ -383,6 +383,7 @@ struct TreeQueries {
   u32 *hard_count = nullptr;     // queries left for the warp-per-query kernel
   u32 *hard = nullptr;           // (their places in q, or in the tree)
   u32 n = 0;
+  u64 minus_zero = 0x8000000080000000ull;  // two of them
 };
 // TREE_MEAN: SOR's mean distance; TREE_PAIRS: rows of k indices and squared
 // distances (-1 and infinity past the found) and counts; TREE_NORMALS /

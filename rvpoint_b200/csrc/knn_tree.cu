@@ -11,12 +11,12 @@
 // the boxes of 32 children at once against the box of the queries and go down
 // into those nearer than the largest K-th distance so far, nearest first; a
 // leaf's points are staged in shared memory and every lane tests all of them
-// against its own query. What passes waits in a buffer per lane (distance and
-// position) and goes through a sorted list of distances (registers) when a
-// buffer fills, so the insertions of the lanes run side by side; the buffer
-// keeps what is within the K-th distance, and at the end each goes to its
-// rank. Queries that do not fit this (far from their packet, equal distances)
-// are listed and answered one per warp by a second kernel.
+// against its own query. The distances that pass wait in a buffer per lane;
+// when one fills, every lane sorts its own in registers and merges them into
+// its sorted list, all lanes in step. With the K-th distance known, the leaves
+// scanned are gone over again, the points within it collected and each put at
+// its rank. Queries that do not fit this (far from their packet, equal
+// distances) are listed and answered one per warp by a second kernel.
 //
 // Pruning needs no slack: every operation of the distance (subtract, square,
 // add) is monotone under rounding, so the distance to a box computed with the
@@ -24,10 +24,11 @@
 // Equal distances are ordered by index: the second kernel works on packed
 // (distance, index) keys.
 //
-// Bound by issue (box tests, distance tests and list insertions). The grid
-// search it replaces for single clouds ran one warp per query on cells sized
-// from a sample of queries: 105k LiDAR points, k 16, 3818 us; a 2M-point map,
-// k 33, 14,225 us.
+// Bound by issue (distance tests, list networks, box tests); small clouds by
+// the latency of one packet. The grid search it replaces for single clouds ran
+// one warp per query on cells sized from a sample of queries: 105k LiDAR
+// points, k 16: 3818 us, now 171 us; 89k room points, mean of 30: 863 and
+// 254 us; normals of a 2M-point map, k 32: 15.9 ms and 4.0 ms.
 #include <float.h>
 #include <math.h>
 
@@ -218,6 +219,31 @@ __global__ void k_tree_queries(const float *__restrict__ x, const float *__restr
 // ---------------------------------------------------------------------------
 // search
 // ---------------------------------------------------------------------------
+// two single-precision operations at once, each rounded by itself
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+  u64 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+// (a product as fma(a, b, -0): mul.rn.f32x2 is contracted with the add that
+// follows, one rounding for both; the zero comes from a kernel argument, so it
+// is no constant to the compiler)
+__device__ __forceinline__ u64 mul2(u64 a, u64 b, u64 minus_zero) {
+  u64 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(minus_zero));
+  return d;
+}
+__device__ __forceinline__ u64 pack2(float a, float b) {
+  return (u64)__float_as_uint(a) | ((u64)__float_as_uint(b) << 32);
+}
+__device__ __forceinline__ float half2f(u64 v, int i) { return __uint_as_float((u32)(v >> (32 * i))); }
+// dist2 of two points: p + (-q) is p - q
+__device__ __forceinline__ u64 dist2x2(u64 px, u64 py, u64 pz, u64 nqx, u64 nqy, u64 nqz,
+                                        u64 mz) {
+  const u64 dx = add2(px, nqx), dy = add2(py, nqy), dz = add2(pz, nqz);
+  return add2(add2(mul2(dx, dx, mz), mul2(dy, dy, mz)), mul2(dz, dz, mz));
+}
+
 // the squared distance between two boxes (a point is a box), with the
 // operations of dist2
 __device__ __forceinline__ float box_gap(float alo, float ahi, float blo, float bhi) {
@@ -266,7 +292,77 @@ __device__ __forceinline__ void tree_walk_all(const TreeView &t, const Box &q, L
     tree_walk<kTreeLevels - 1>(t, q, f, limit, leaf);
 }
 
-constexpr int kTreeExtra = 3;  // rows past K for equal distances
+// The same walk leaf by leaf, for a caller whose leaf code is too long to be
+// inlined more than once (it would not fit the instruction cache).
+template <class T>
+__device__ __forceinline__ T by_level(const T (&v)[kTreeLevels], int l) {
+  static_assert(kTreeLevels == 4, "four levels");
+  return l < 2 ? (l == 0 ? v[0] : v[1]) : (l == 2 ? v[2] : v[3]);  // (stays in registers)
+}
+template <class T>
+__device__ __forceinline__ void set_level(T (&v)[kTreeLevels], int l, T x) {
+#pragma unroll
+  for (int i = 0; i < kTreeLevels; ++i) v[i] = i == l ? x : v[i];
+}
+
+struct TreeWalk {
+  float lb[kTreeLevels];   // per level: the lane's child's distance
+  u32 open[kTreeLevels];   // children left (a mask, uniform)
+  u32 first[kTreeLevels];  // their numbers start here
+  int level;               // where the walk stands
+  u32 top;                 // next group of top nodes
+  __device__ __forceinline__ void begin() {
+    level = kTreeLevels;
+    top = 0;
+#pragma unroll
+    for (int l = 0; l < kTreeLevels; ++l) {
+      lb[l] = 0.0f;
+      open[l] = first[l] = 0;
+    }
+  }
+  // the next leaf within `limit` of q; false at the end
+  __device__ __forceinline__ bool next(const TreeView &t, const Box &q, float limit, u32 &leaf) {
+    const int lane = threadIdx.x & 31;
+    while (true) {
+      u32 f = top;
+      int to = kTreeLevels - 1;
+      if (level == kTreeLevels) {
+        if (top >= t.count[kTreeLevels - 1]) return false;
+        top += 32;
+      } else {
+        const u32 mask = by_level(open, level);
+        const float v = by_level(lb, level);
+        // (the low bits of the distance give way to the lane)
+        const u32 best = __reduce_min_sync(
+            0xffffffffu,
+            (mask >> lane) & 1u ? (__float_as_uint(v) & ~31u) | lane : 0xFFFFFFFFu);
+        if (best == 0xFFFFFFFFu || __uint_as_float(best & ~31u) > limit) {  // none near enough
+          ++level;
+          continue;
+        }
+        const int s = best & 31;
+        set_level(open, level, mask & ~(1u << s));
+        if (__shfl_sync(0xffffffffu, v, s) > limit) continue;
+        f = by_level(first, level) + s;
+        if (level == 0) {
+          leaf = f;
+          return true;
+        }
+        f *= 32;
+        to = level - 1;
+      }
+      const u32 c = f + lane, n = by_level(t.count, to);
+      const float d = c < n ? box_d2(q, by_level(t.box, to), by_level(t.stride, to), c) : 0.0f;
+      set_level(lb, to, d);
+      set_level(open, to, __ballot_sync(0xffffffffu, c < n && d <= limit));
+      set_level(first, to, f);
+      level = to;
+    }
+  }
+};
+
+constexpr int kTreeBuf = 64;   // buffered distances per lane, flushed above 32
+constexpr int kTreeExtra = 3;  // collected points past the list, for equal distances
 // a query joins its packet's walk if its limit (a squared distance) is within
 // this factor of the median one
 constexpr float kLoner = 16.0f;
@@ -275,16 +371,55 @@ constexpr float kLoner = 16.0f;
 // leaf of a large box to test, up to 2 ms, with no other work left to hide it
 constexpr int kLeafBudget = 128;
 
-// per lane and row: a distance (the mean needs no more) or a distance and a
-// tree position; a flush leaves at most KCAP + kTreeExtra rows (distances
-// only: none), a leaf adds up to 32
+// shared memory of a packet: the staged leaf, the leaves scanned, the buffered
+// distances and later (in the same place) the collected points, and the
+// positions in order where a normal follows
+constexpr int kTreeLeaves = (kLeafBudget + 3 + 3) & ~3;
 template <int KCAP, int MODE>
-constexpr int tree_rows() {
-  return MODE == TREE_MEAN ? 64 : KCAP + kTreeExtra + 32;
+constexpr size_t tree_buffer() {
+  constexpr size_t dist = (size_t)kTreeBuf * 32 * 4;
+  constexpr size_t near = (size_t)(KCAP + kTreeExtra) * 32 * 8;
+  return MODE != TREE_MEAN && near > dist ? near : dist;
 }
 template <int KCAP, int MODE>
 constexpr size_t tree_smem() {
-  return 32 * 16 + (size_t)tree_rows<KCAP, MODE>() * 32 * (MODE == TREE_MEAN ? 4 : 8);
+  return 3 * 32 * 4 + kTreeLeaves * 4 + tree_buffer<KCAP, MODE>() +
+         (MODE == TREE_NORMALS || MODE == TREE_PRECISE ? (size_t)(KCAP + 1) * 32 * 4 : 0);
+}
+
+// Compare-exchange networks over registers. They are straight code: batches of
+// 32 took fewer steps than 16, but the kernel then waited for instructions
+// (4.7 of 9 cycles per issue).
+__device__ __forceinline__ void order2(float &a, float &b) {
+  const float l = fminf(a, b), h = fmaxf(a, b);
+  a = l;
+  b = h;
+}
+template <int N>
+__device__ __forceinline__ void bitonic_merge(float (&v)[N]) {
+#pragma unroll
+  for (int j = N / 2; j > 0; j >>= 1) {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if ((i ^ j) > i) order2(v[i], v[i ^ j]);
+  }
+}
+template <int N>
+__device__ __forceinline__ void bitonic_sort(float (&v)[N]) {
+#pragma unroll
+  for (int k = 2; k <= N; k <<= 1) {
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) {
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        const int l = i ^ j;
+        if (l > i) {
+          if ((i & k) == 0) order2(v[i], v[l]);
+          else order2(v[l], v[i]);
+        }
+      }
+    }
+  }
 }
 
 // the leaf where a query of this key would lie
@@ -330,20 +465,22 @@ __device__ __forceinline__ void tree_normal_out(Nbr nbr, int have, const float4 
   o.nz[qidx] = nz;
 }
 
-// one warp (block) per packet of 32 queries; KCAP >= K
+// One warp (block) per packet of 32 queries. The list holds the K nearest, or
+// for the cloud's own points the K - 1 nearest others (the point itself, at
+// distance 0, is the first of its row); KCAP is at least that, a power of two.
 template <int KCAP, int MODE>
-__global__ __launch_bounds__(32, KCAP > 33 ? 8 : 16) void k_knn_tree(TreeView t, TreeQueries qs,
-                                                                     int K, float bound,
-                                                                     TreeOut o) {
+__global__ __launch_bounds__(32, KCAP > 32 ? 10 : 16) void k_knn_tree(TreeView t, TreeQueries qs, int K,
+                                                     float bound, TreeOut o) {
   extern __shared__ __align__(16) unsigned char tree_sm[];
   constexpr bool MEAN = MODE == TREE_MEAN;
-  constexpr int ROWS = tree_rows<KCAP, MODE>();
-  float4 *stage = reinterpret_cast<float4 *>(tree_sm);
-  float(*fbuf)[32] = reinterpret_cast<float(*)[32]>(tree_sm + 512);
-  uint2(*pbuf)[32] = reinterpret_cast<uint2(*)[32]>(tree_sm + 512);
-  // the sorted positions, over the 32 rows that only a leaf's hits use
-  u32(*sorted)[32] = reinterpret_cast<u32(*)[32]>(tree_sm + 512 + (size_t)(KCAP + kTreeExtra) * 256);
-  static_assert(KCAP <= 64, "sorted positions fit the rows of a leaf");
+  constexpr int PCAP = KCAP + kTreeExtra;
+  constexpr int BATCH = KCAP < 16 ? KCAP : 16;  // distances sorted at once
+  float(*stage)[32] = reinterpret_cast<float(*)[32]>(tree_sm);  // x, y, z
+  u32 *leaves = reinterpret_cast<u32 *>(tree_sm + 384);
+  unsigned char *buf = tree_sm + 384 + kTreeLeaves * 4;
+  float(*fbuf)[32] = reinterpret_cast<float(*)[32]>(buf);
+  uint2(*pbuf)[32] = reinterpret_cast<uint2(*)[32]>(buf);
+  u32(*sorted)[32] = reinterpret_cast<u32(*)[32]>(buf + tree_buffer<KCAP, MODE>());
   const int lane = threadIdx.x;
   const u32 packet = blockIdx.x;
   // the cloud's own points (leaf `packet`), or 32 of the sorted queries
@@ -358,12 +495,13 @@ __global__ __launch_bounds__(32, KCAP > 33 ? 8 : 16) void k_knn_tree(TreeView t,
   const Box own{{q.x, q.y, q.z}, {q.x, q.y, q.z}};
 
   // ---- the sorted distances: slots 0 .. pad - 1 hold -1 and never move
-  const int pad = KCAP - K;
+  const bool drop = self && K > 1;  // the point itself is not in the list
+  const int KL = drop ? K - 1 : K, pad = KCAP - KL;
   float L[KCAP];
 #pragma unroll
   for (int j = 0; j < KCAP; ++j) L[j] = j < pad ? -1.0f : INFINITY;
   bool mine = active;  // answered with the packet
-  int cnt = 0, done = 0;  // buffered rows, and those already in the list
+  int cnt = 0;         // buffered distances
   float lim = -1.0f, pmax = -1.0f;  // what the buffer takes: d2 <= lim; its largest
   auto limits = [&]() {
     lim = mine ? fminf(fminf(L[KCAP - 1], bound), FLT_MAX) : -1.0f;
@@ -371,81 +509,98 @@ __global__ __launch_bounds__(32, KCAP > 33 ? 8 : 16) void k_knn_tree(TreeView t,
   };
   limits();
   auto flush = [&]() {
-    const int most = __reduce_max_sync(0xffffffffu, cnt - done);
-    for (int i = 0; i < most; ++i) {
-      float key = INFINITY;
-      if (done + i < cnt)
-        key = MEAN ? fbuf[done + i][lane] : __uint_as_float(pbuf[done + i][lane].x);
-      if (__any_sync(0xffffffffu, key < L[KCAP - 1])) {
+    const int most = __reduce_max_sync(0xffffffffu, cnt);
+    int i = 0;
+    // a sorted batch merged at once; the last few one by one
+    for (; i + BATCH / 4 < most; i += BATCH) {
+      float S[BATCH];
 #pragma unroll
-        for (int j = KCAP - 1; j > 0; --j) L[j] = fmaxf(L[j - 1], fminf(L[j], key));
-        L[0] = fminf(L[0], key);
-      }
+      for (int j = 0; j < BATCH; ++j) S[j] = i + j < cnt ? fbuf[i + j][lane] : INFINITY;
+      bitonic_sort<BATCH>(S);
+#pragma unroll
+      for (int j = 0; j < BATCH; ++j)
+        L[KCAP - BATCH + j] = fminf(L[KCAP - BATCH + j], S[BATCH - 1 - j]);
+      bitonic_merge<KCAP>(L);
     }
-    if constexpr (MEAN) {
-      cnt = 0;
-    } else {  // keep what is within the K-th distance
-      const float top = L[KCAP - 1];
-      int m = 0;
-      for (int i = 0; i < cnt; ++i) {
-        const uint2 b = pbuf[i][lane];
-        if (__uint_as_float(b.x) <= top) pbuf[m++][lane] = b;
-      }
-      cnt = m;
-      if (m > KCAP + kTreeExtra) {  // too many equal ones: not with the packet
-        mine = false;
-        cnt = 0;
-      }
-      done = cnt;
+    for (; i < most; ++i) {
+      const float key = i < cnt ? fbuf[i][lane] : INFINITY;
+#pragma unroll
+      for (int j = KCAP - 1; j > 0; --j) L[j] = fmaxf(L[j - 1], fminf(L[j], key));
+      L[0] = fminf(L[0], key);
     }
-    __syncwarp();
+    cnt = 0;
     limits();
   };
-  int budget = kLeafBudget;
+  int scanned = 0, budget = kLeafBudget;
+  auto stage_leaf = [&](u32 l, float at, const float4 &mate) {
+    if (!__any_sync(0xffffffffu, at >= 0.0f)) return false;
+    __syncwarp();
+    stage[0][lane] = mate.x;
+    stage[1][lane] = mate.y;
+    stage[2][lane] = mate.z;
+    __syncwarp();
+    return true;
+  };
+  const u64 nqx = pack2(-q.x, -q.x), nqy = pack2(-q.y, -q.y), nqz = pack2(-q.z, -q.z);
+  // hit(c, d2) for the staged points c within `at`, except `skip`
+  auto test_staged = [&](float at, int skip, auto &&hit) {
+#pragma unroll 2
+    for (int c = 0; c < 32; c += 4) {
+      const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(&stage[0][c]);
+      const ulonglong2 y = *reinterpret_cast<const ulonglong2 *>(&stage[1][c]);
+      const ulonglong2 z = *reinterpret_cast<const ulonglong2 *>(&stage[2][c]);
+      const u64 a = dist2x2(x.x, y.x, z.x, nqx, nqy, nqz, qs.minus_zero);
+      const u64 b = dist2x2(x.y, y.y, z.y, nqx, nqy, nqz, qs.minus_zero);
+      const float d[4] = {half2f(a, 0), half2f(a, 1), half2f(b, 0), half2f(b, 1)};
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (d[u] <= at && c + u != skip) hit(c + u, d[u]);
+    }
+  };
+  auto mate_of = [&](u32 l) {  // the lane's point of leaf l
+    const u32 i = l * 32 + lane;
+    return i < t.n ? __ldg(&t.pts[i]) : make_float4(INFINITY, INFINITY, INFINITY, 0.0f);
+  };
   auto scan_leaf = [&](u32 l) {
     if (--budget < 0) {  // (uniform) nothing is left open: the walk ends
       mine = false;
       pmax = -1.0f;
       return;
     }
-    const u32 i = l * 32 + lane;
-    const float4 mate =
-        i < t.n ? __ldg(&t.pts[i]) : make_float4(INFINITY, INFINITY, INFINITY, 0.0f);
+    const float4 mate = mate_of(l);
     const float at = box_d2(own, t.box[0], t.stride[0], l) <= lim ? lim : -1.0f;
-    if (!__any_sync(0xffffffffu, at >= 0.0f)) return;
-    __syncwarp();
-    stage[lane] = mate;
-    __syncwarp();
-#pragma unroll
-    for (int c = 0; c < 32; c += 4) {
-      float d[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const float4 p = stage[c + u];
-        d[u] = dist2(p.x, p.y, p.z, q.x, q.y, q.z);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (d[u] <= at) {
-          if constexpr (MEAN) fbuf[cnt][lane] = d[u];
-          else pbuf[cnt][lane] = make_uint2(__float_as_uint(d[u]), l * 32 + c + u);
-          ++cnt;
-        }
-      }
-    }
-    if (__any_sync(0xffffffffu, cnt > ROWS - 32)) flush();
+    if (!stage_leaf(l, at, mate)) return;
+    leaves[scanned++] = l;
+    const int skip = drop && l == packet ? lane : -1;  // the point itself
+    float *to = &fbuf[cnt][lane];
+    test_staged(at, skip, [&](int, float d) {
+      *to = d;
+      to += 32;
+    });
+    cnt = (int)(to - &fbuf[0][lane]) >> 5;
   };
-  // the leaves around the packet's place first: they set the limits
+  // the leaves around the packet's place first (they set the limits), then
+  // the walk
   const u32 s0 = start > 0 ? start - 1 : 0, s1 = min(start + 1, t.count[0] - 1);
-  for (u32 l = s0; l <= s1; ++l) scan_leaf(l);
-  flush();
-  {  // A query whose limit is far above the others' (four times the median
-     // radius) would take the packet through all the leaves around it: such
-     // loners are answered by the whole warp, one by one.
+  const int near = (int)(s1 - s0) + 1;
+  Box pk{};  // the box of the packet
+  TreeWalk walk;
+  walk.begin();
+  for (int step = 0;; ++step) {
+    bool more = true;
+    u32 l = step == 0 ? start : (step == 1 && s0 < start ? s0 : s1);
+    if (step >= near) more = walk.next(t, pk, pmax, l);
+    if (more && (step < near || l < s0 || l > s1)) scan_leaf(l);
+    if (!more || step == 0 || step == near - 1 || __any_sync(0xffffffffu, cnt > kTreeBuf - 32))
+      flush();
+    if (!more) break;
+    if (step != near - 1) continue;
+    // A query whose limit is far above the others' (four times the median
+    // radius) would take the packet through all the leaves around it
     int rank = 0;
-    for (int s = 0; s < 32; ++s) {
-      const float other = __shfl_sync(0xffffffffu, mine ? lim : INFINITY, s);
-      rank += other < lim || (other == lim && s < lane) ? 1 : 0;
+    for (int i = 0; i < 32; ++i) {
+      const float other = __shfl_sync(0xffffffffu, mine ? lim : INFINITY, i);
+      rank += other < lim || (other == lim && i < lane) ? 1 : 0;
     }
     const unsigned mid = __ballot_sync(0xffffffffu, mine && rank == 16);
     if (mid) {
@@ -453,62 +608,75 @@ __global__ __launch_bounds__(32, KCAP > 33 ? 8 : 16) void k_knn_tree(TreeView t,
       mine = mine && lim <= kLoner * ref;
       limits();
     }
-  }
-  Box pk;  // the box of the packet
-  {
     const float v[3] = {q.x, q.y, q.z};
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      float l = mine ? v[a] : INFINITY, h = mine ? v[a] : -INFINITY;
+      float lo = mine ? v[a] : INFINITY, hi = mine ? v[a] : -INFINITY;
 #pragma unroll
-      for (int s = 16; s; s >>= 1) {
-        l = fminf(l, __shfl_xor_sync(0xffffffffu, l, s));
-        h = fmaxf(h, __shfl_xor_sync(0xffffffffu, h, s));
+      for (int i = 16; i; i >>= 1) {
+        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, i));
+        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, i));
       }
-      pk.lo[a] = l;
-      pk.hi[a] = h;
+      pk.lo[a] = lo;
+      pk.hi[a] = hi;
     }
-  }
-  {
-    auto limit = [&]() { return pmax; };
-    auto leaf = [&](u32 l) {
-      if (l < s0 || l > s1) scan_leaf(l);
-    };
-    tree_walk_all(t, pk, limit, leaf);
-    flush();
   }
 
   // ---- results of the packet
   bool exact = mine;
-  int have = 0;
+  int have = 0;  // distances in the list
   if constexpr (MEAN) {
-    // (without a radius K points are there, some infinitely far perhaps)
+    // (without a radius they are all there, some infinitely far perhaps)
     float sum = 0.0f;
+    bool first = !drop;  // the nearest of all does not count
 #pragma unroll
     for (int j = 0; j < KCAP; ++j) {
       if (j >= pad && (!o.radius_mode || L[j] < INFINITY)) {
-        if (have) sum = fadd(sum, __fsqrt_rn(L[j]));
+        if (!first) sum = fadd(sum, __fsqrt_rn(L[j]));
+        first = false;
         ++have;
       }
     }
-    if (exact) tree_mean_out(sum, have, q, qidx, o);
+    if (exact) tree_mean_out(sum, have + (drop ? 1 : 0), q, qidx, o);
   } else {
     bool tied = false;
 #pragma unroll
     for (int j = 0; j < KCAP; ++j) {
       if (j >= pad && L[j] < INFINITY) ++have;
       if (j > pad && L[j] < INFINITY && L[j] == L[j - (j > 0)]) tied = true;
+      if (drop && j == pad && L[j] == 0.0f) tied = true;  // another point in its place
     }
-    // exactly these points are within the K-th distance, no two equal (and
-    // what is missing is not there: points infinitely far would be)
+    // the points within the K-th distance, from the leaves scanned
+    const float tau = mine ? fminf(fminf(L[KCAP - 1], bound), FLT_MAX) : -1.0f;
+    for (int i = 0; i < scanned; ++i) {
+      const u32 l = leaves[i];
+      const float4 mate = mate_of(l);
+      const float at = box_d2(own, t.box[0], t.stride[0], l) <= tau ? tau : -1.0f;
+      if (!stage_leaf(l, at, mate)) continue;
+      test_staged(at, drop && l == packet ? lane : -1, [&](int c, float d) {
+        if (cnt < PCAP) pbuf[cnt][lane] = make_uint2(__float_as_uint(d), l * 32 + c);
+        ++cnt;
+      });
+    }
+    // exactly these are within the K-th distance, no two equal (and what is
+    // missing is not there: points infinitely far would be)
     exact = mine && cnt == have && !tied &&
-            (have == K || bound < INFINITY || (u32)have == t.n);
-    // each to its rank among the sorted distances
+            (have == KL || bound < INFINITY || (u32)(have + (drop ? 1 : 0)) == t.n);
+    // each to its rank among the sorted distances, behind the point itself
+    const int r0 = drop ? 1 : 0;
     if (exact) {
+      if (drop) {
+        if constexpr (MODE == TREE_PAIRS) {
+          if (o.idx) o.idx[(size_t)qidx * K] = (int32_t)qidx;
+          if (o.d2) o.d2[(size_t)qidx * K] = 0.0f;
+        } else {
+          sorted[0][lane] = qi;
+        }
+      }
       for (int i = 0; i < have; ++i) {
         const uint2 b = pbuf[i][lane];
         const float d = __uint_as_float(b.x);
-        int r = -pad;
+        int r = r0 - pad;
 #pragma unroll
         for (int j = 0; j < KCAP; ++j) r += L[j] < d ? 1 : 0;
         if constexpr (MODE == TREE_PAIRS) {
@@ -520,6 +688,7 @@ __global__ __launch_bounds__(32, KCAP > 33 ? 8 : 16) void k_knn_tree(TreeView t,
         }
       }
     }
+    have += r0;
   }
   // the others are listed for the second kernel
   const unsigned again = __ballot_sync(0xffffffffu, active && !exact);
@@ -540,12 +709,13 @@ __global__ __launch_bounds__(32, KCAP > 33 ? 8 : 16) void k_knn_tree(TreeView t,
     tree_normal_out<MODE>([&](int j) { return __ldg(&t.pts[sorted[j][lane]]); }, have, q, qidx, o);
   }
 }
+
 // one warp per listed query, lanes over a leaf's points, a list of packed
 // (distance, index) keys over the lanes
 template <int P, int MODE>
 __global__ __launch_bounds__(128) void k_knn_tree_hard(TreeView t, TreeQueries qs, int K,
                                                        float bound, TreeOut o) {
-  __shared__ u32 sorted[4][32 * P];
+  __shared__ float4 near[4][32 * P];  // the neighbours in order
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const u32 n = *qs.hard_count;
   const bool self = qs.n_sort == nullptr || *qs.n_sort == 0;
@@ -612,7 +782,7 @@ __global__ __launch_bounds__(128) void k_knn_tree_hard(TreeView t, TreeQueries q
             if (o.d2) o.d2[at] = j < have ? nbr_d2(W.e[p]) : INFINITY;
           }
         } else {
-          if (j < have) sorted[wib][j] = t.pos_of[nbr_idx(W.e[p])];
+          if (j < have) near[wib][j] = __ldg(&t.pts[t.pos_of[nbr_idx(W.e[p])]]);
         }
       }
       if constexpr (MODE == TREE_PAIRS) {
@@ -620,8 +790,7 @@ __global__ __launch_bounds__(128) void k_knn_tree_hard(TreeView t, TreeQueries q
       } else {
         __syncwarp();
         if (lane == 0)
-          tree_normal_out<MODE>([&](int j) { return __ldg(&t.pts[sorted[wib][j]]); }, have, q,
-                                qidx, o);
+          tree_normal_out<MODE>([&](int j) { return near[wib][j]; }, have, q, qidx, o);
         __syncwarp();
       }
     }
@@ -635,18 +804,23 @@ void launch_tree(rvp_context *ctx, const TreeView &t, const TreeQueries &q, int 
   static_assert(smem <= 48 * 1024, "no opt-in to larger shared memory here");
   k_knn_tree<KCAP, MODE><<<(q.n + 31) / 32, 32, smem, ctx->stream>>>(t, q, K, bound, o);
   RVP_LAUNCH_CHECK(ctx);
-  k_knn_tree_hard<(KCAP > 32 ? 2 : 1), MODE>
-      <<<grid_for(q.n, 4, ctx->num_sms * 8), 128, 0, ctx->stream>>>(t, q, K, bound, o);
+  const unsigned blocks = grid_for(q.n, 4, ctx->num_sms * 8);
+  if (K <= 32)
+    k_knn_tree_hard<1, MODE><<<blocks, 128, 0, ctx->stream>>>(t, q, K, bound, o);
+  else
+    k_knn_tree_hard<2, MODE><<<blocks, 128, 0, ctx->stream>>>(t, q, K, bound, o);
   RVP_LAUNCH_CHECK(ctx);
 }
 
 template <int MODE>
 void launch_tree_k(rvp_context *ctx, const TreeView &t, const TreeQueries &q, int K, float bound,
                    const TreeOut &o) {
-  if (K <= 9) launch_tree<9, MODE>(ctx, t, q, K, bound, o);
-  else if (K <= 17) launch_tree<17, MODE>(ctx, t, q, K, bound, o);
-  else if (K <= 25) launch_tree<25, MODE>(ctx, t, q, K, bound, o);
-  else if (K <= 33) launch_tree<33, MODE>(ctx, t, q, K, bound, o);
+  // the list leaves the point itself out where the host knows that the
+  // queries are the cloud (n_sort: the device finds out)
+  const int KL = q.n_sort || K == 1 ? K : K - 1;
+  if (KL <= 8) launch_tree<8, MODE>(ctx, t, q, K, bound, o);
+  else if (KL <= 16) launch_tree<16, MODE>(ctx, t, q, K, bound, o);
+  else if (KL <= 32) launch_tree<32, MODE>(ctx, t, q, K, bound, o);
   else launch_tree<64, MODE>(ctx, t, q, K, bound, o);
 }
 }  // namespace
