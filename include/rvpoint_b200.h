@@ -96,6 +96,15 @@ RVP_API rvp_status rvp_hash_radius_search(rvp_hash *h, const float *qx, const fl
                                   int max_nn, int mem, int64_t *offsets,
                                   int32_t *indices, float *dists,
                                   size_t capacity, size_t *total);
+/* The same with the lists' memory asked for once their length is known: alloc
+ * is called once, between the two halves of the search, and returns 0 with
+ * room for `total` indices and distances (host or device as `mem`), or another
+ * value if there is none (RVP_ERR_OOM). */
+typedef int (*rvp_alloc_fn)(void *user, size_t total, int32_t **indices, float **dists);
+RVP_API rvp_status rvp_hash_radius_search_alloc(rvp_hash *h, const float *qx, const float *qy,
+                                                const float *qz, size_t nq, float radius,
+                                                int max_nn, int mem, int64_t *offsets,
+                                                rvp_alloc_fn alloc, void *user, size_t *total);
 /* Exact k nearest neighbours (ties by index) of nq queries, k <= 64.
  * radius > 0 bounds the search (radiusSearch with max_nn = k); radius <= 0
  * searches the whole cloud. indices/dists: nq*k row-major; counts[nq]. */

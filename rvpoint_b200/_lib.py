@@ -54,6 +54,10 @@ SZ = C.c_size_t
 F = C.c_float
 I = C.c_int
 
+# rvp_alloc_fn: (user, total, &indices, &dists) -> 0, or 1 without memory
+AllocFn = C.CFUNCTYPE(C.c_int, C.c_void_p, C.c_size_t, C.POINTER(C.c_void_p),
+                      C.POINTER(C.c_void_p))
+
 # name -> (restype, argtypes)
 SIGNATURES = {
     "rvp_context_create": (I, [I, C.POINTER(P)]),
@@ -73,6 +77,8 @@ SIGNATURES = {
     "rvp_hash_build": (I, [P]),
     "rvp_hash_has_collisions": (I, [P, C.POINTER(I)]),
     "rvp_hash_radius_search": (I, [P, P, P, P, SZ, F, I, I, P, P, P, SZ, C.POINTER(SZ)]),
+    "rvp_hash_radius_search_alloc": (I, [P, P, P, P, SZ, F, I, I, P, AllocFn, P,
+                                         C.POINTER(SZ)]),
     "rvp_hash_knn": (I, [P, P, P, P, SZ, I, F, I, P, P, P]),
     "rvp_voxel_grid": (I, [P, P, P, P, SZ, F, I, P, P, C.POINTER(SZ)]),
     "rvp_sor": (I, [P, P, P, P, SZ, I, F, I, P, C.POINTER(SZ), P, P]),

@@ -194,20 +194,35 @@ class SpatialHash:
         dev = mem == MEM_DEVICE
         device = qx.device if dev else None
         offs = _empty((nq + 1,), np.int64, dev, device)
-        cap = capacity if capacity is not None else (nq * max_nn if max_nn > 0 else 0)
         total = C.c_size_t(0)
-        while True:
-            idx = _empty((max(cap, 1),), np.int32, dev, device)
-            d2 = _empty((max(cap, 1),), np.float32, dev, device)
-            st = self.L.rvp_hash_radius_search(self.h, _ptr(qx), _ptr(qy), _ptr(qz), nq,
-                                               float(radius), int(max_nn), mem, _ptr(offs),
-                                               _ptr(idx), _ptr(d2), cap, C.byref(total))
-            if st == _lib.RVP_ERR_CAPACITY:
-                cap = int(total.value)
-                continue
-            check(st, self.ctx.h)
-            t = int(total.value)
-            return offs, idx[:t], d2[:t]
+        args = (self.h, _ptr(qx), _ptr(qy), _ptr(qz), nq, float(radius), int(max_nn), mem,
+                _ptr(offs))
+        lists = []
+
+        def room(size):
+            lists[:] = [_empty((max(size, 1),), t, dev, device) for t in (np.int32, np.float32)]
+
+        def alloc(_user, size, idx, d2):
+            try:
+                room(size)
+                idx[0], d2[0] = (_ptr(a).value if dev else a.ctypes.data for a in lists)
+                return 0
+            except Exception:
+                return 1
+
+        st = _lib.RVP_ERR_CAPACITY
+        if capacity is not None:  # one call when the lists fit
+            room(capacity)
+            st = self.L.rvp_hash_radius_search(*args, _ptr(lists[0]), _ptr(lists[1]), capacity,
+                                               C.byref(total))
+        if st == _lib.RVP_ERR_CAPACITY:
+            st = self.L.rvp_hash_radius_search_alloc(*args, _lib.AllocFn(alloc), None,
+                                                     C.byref(total))
+        check(st, self.ctx.h)
+        t = int(total.value)
+        if not lists:
+            room(0)
+        return offs, lists[0][:t], lists[1][:t]
 
     def knn(self, qx, qy, qz, k: int, radius: float = 0.0):
         """Exact k nearest (ties by index); radius > 0 bounds the search like
@@ -228,7 +243,8 @@ class SpatialHash:
 
     def close(self):
         if getattr(self, "h", None):
-            self.L.rvp_hash_destroy(self.h)
+            if self.ctx.h:  # (at exit the context may go first, and its memory with it)
+                self.L.rvp_hash_destroy(self.h)
             self.h = None
 
     def __del__(self):  # pragma: no cover
@@ -413,7 +429,8 @@ class Octree:
 
     def close(self):
         if getattr(self, "h", None):
-            self.L.rvp_octree_destroy(self.h)
+            if self.ctx.h:  # (at exit the context may go first, and its memory with it)
+                self.L.rvp_octree_destroy(self.h)
             self.h = None
 
     def __del__(self):  # pragma: no cover
@@ -915,7 +932,8 @@ class Pipeline:
 
     def close(self):
         if getattr(self, "h", None):
-            self.L.rvp_pipeline_destroy(self.h)
+            if self.ctx.h:  # (at exit the context may go first, and its memory with it)
+                self.L.rvp_pipeline_destroy(self.h)
             self.h = None
 
     def __del__(self):  # pragma: no cover

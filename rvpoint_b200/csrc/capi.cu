@@ -90,8 +90,8 @@ struct rvp_hash {
   size_t n = 0;
   float cell = 0.0f;
   long long p1 = 73856093LL, p2 = 19349663LL;
-  rvp::Grid grid;
-  rvp::KnnTree tree;  // k nearest: built by the first search that needs it
+  rvp::Grid grid;     // the reference's buckets, where cells may share a key
+  rvp::KnnTree tree;  // searched unless cells share a key
   rvp::TreeView tree_view{};
   bool has_cloud = false, built = false, tree_built = false;
   int collision = 0;
@@ -166,6 +166,32 @@ int64_t *single_frame_offsets(rvp_context *ctx, int slot, size_t n) {
   return d;
 }
 
+__global__ void k_pack(const int32_t *idx, const float *d2, size_t total, u64 *pairs) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
+       i += (size_t)gridDim.x * blockDim.x)
+    pairs[i] = rvp::pack_nbr(d2[i], idx[i]);
+}
+
+__global__ void k_scatter3(const float *x, const float *y, const float *z, const u32 *to, size_t n,
+                           float *ox, float *oy, float *oz) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x) {
+    ox[to[i]] = x[i];
+    oy[to[i]] = y[i];
+    oz[to[i]] = z[i];
+  }
+}
+
+__global__ void k_copy3(const float *x, const float *y, const float *z, size_t n, float *ox,
+                        float *oy, float *oz) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x) {
+    ox[i] = x[i];
+    oy[i] = y[i];
+    oz[i] = z[i];
+  }
+}
+
 __global__ void k_unpack(const u64 *pairs, size_t total, int32_t *idx, float *d2) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
        i += (size_t)gridDim.x * blockDim.x) {
@@ -230,14 +256,19 @@ void knn_cloud(rvp_context *ctx, const float *x, const float *y, const float *z,
   rvp::tree_knn(ctx, t, rvp::tree_queries(ctx, w, t, x, y, z, x, y, z, n), K, 0.0f, mode, o);
 }
 
-// the same among a hash's points
+// the tree over a hash's points (kept until it takes another cloud)
+void hash_tree(rvp_hash *h) {
+  if (h->tree_built) return;
+  h->tree_view = rvp::tree_build(h->ctx, h->tree, h->x.as<float>(), h->y.as<float>(),
+                                 h->z.as<float>(), h->n);
+  h->tree_built = true;
+}
+
+// the k nearest among a hash's points
 void knn_hash(rvp_hash *h, const float *qx, const float *qy, const float *qz, size_t nq, int K,
               float radius, int mode, const rvp::TreeOut &o) {
   const float *x = h->x.as<float>(), *y = h->y.as<float>(), *z = h->z.as<float>();
-  if (!h->tree_built) {
-    h->tree_view = rvp::tree_build(h->ctx, h->tree, x, y, z, h->n);
-    h->tree_built = true;
-  }
+  hash_tree(h);
   // (32-bit query numbers in the kernels: a billion at a time)
   constexpr size_t kMost = (size_t)1 << 30;
   for (size_t a = 0; a < nq; a += kMost) {
@@ -389,15 +420,15 @@ rvp_status rvp_hash_set_input_cloud(rvp_hash *h, const float *x, const float *y,
     h->tree_built = false;
     h->n = 0;
     h->x.reserve(n * 4 + 16); h->y.reserve(n * 4 + 16); h->z.reserve(n * 4 + 16);
-    h->offs.reserve(16);
-    if (n) {
-      const cudaMemcpyKind k = mem == RVP_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-      RVP_CUDA_TRY(cudaMemcpyAsync(h->x.ptr, x, n * 4, k, ctx->stream));
-      RVP_CUDA_TRY(cudaMemcpyAsync(h->y.ptr, y, n * 4, k, ctx->stream));
-      RVP_CUDA_TRY(cudaMemcpyAsync(h->z.ptr, z, n * 4, k, ctx->stream));
+    if (n && mem == RVP_MEM_DEVICE) {
+      k_copy3<<<rvp::grid_for(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(
+          x, y, z, n, h->x.as<float>(), h->y.as<float>(), h->z.as<float>());
+      RVP_LAUNCH_CHECK(ctx);
+    } else if (n) {
+      RVP_CUDA_TRY(cudaMemcpyAsync(h->x.ptr, x, n * 4, cudaMemcpyHostToDevice, ctx->stream));
+      RVP_CUDA_TRY(cudaMemcpyAsync(h->y.ptr, y, n * 4, cudaMemcpyHostToDevice, ctx->stream));
+      RVP_CUDA_TRY(cudaMemcpyAsync(h->z.ptr, z, n * 4, cudaMemcpyHostToDevice, ctx->stream));
     }
-    int64_t o[2] = {0, (int64_t)n};
-    RVP_CUDA_TRY(cudaMemcpyAsync(h->offs.ptr, o, 16, cudaMemcpyHostToDevice, ctx->stream));
     sync(ctx);
     h->n = n;
     h->cell = cell_size;
@@ -415,10 +446,20 @@ rvp_status rvp_hash_build(rvp_hash *h) {
     h->built = false;  // set again only when this build has completed
     h->collision = 0;
     if (h->n > 0) {
-      rvp::grid_build(ctx, h->grid, h->x.as<float>(), h->y.as<float>(), h->z.as<float>(),
-                      h->offs.as<int64_t>(), 1, h->n, h->cell, rvp::KEY_REF_HASH, h->p1, h->p2,
-                      nullptr);
-      h->collision = read_back(ctx, h->grid.d_collision);
+      hash_tree(h);
+      int *flag = static_cast<int *>(scratch(ctx, 4, 256));
+      rvp::hash_collision_check(ctx, h->tree_view, h->cell, h->p1, h->p2, flag);
+      if (read_back(ctx, flag)) {
+        // cells may share a key: the reference's own buckets tell whether
+        // occupied ones do (and are searched if so)
+        h->offs.reserve(16);
+        const int64_t o[2] = {0, (int64_t)h->n};
+        RVP_CUDA_TRY(cudaMemcpyAsync(h->offs.ptr, o, 16, cudaMemcpyHostToDevice, ctx->stream));
+        rvp::grid_build(ctx, h->grid, h->x.as<float>(), h->y.as<float>(), h->z.as<float>(),
+                        h->offs.as<int64_t>(), 1, h->n, h->cell, rvp::KEY_REF_HASH, h->p1, h->p2,
+                        nullptr);
+        h->collision = read_back(ctx, h->grid.d_collision);
+      }
     }
     h->built = true;
   });
@@ -430,110 +471,163 @@ rvp_status rvp_hash_has_collisions(rvp_hash *h, int *out) {
   return RVP_OK;
 }
 
+}  // extern "C"
+
+// outputs(total, &indices, &dists): where the caller wants them; false: nowhere
+// (the search then ends with the offsets and the total)
+template <class Outputs>
+static void radius_search(rvp_hash *h, const float *qx, const float *qy, const float *qz,
+                          size_t nq, float radius, int max_nn, int mem, int64_t *offsets,
+                          size_t *total, Outputs &&outputs) {
+  rvp_context *ctx = h->ctx;
+  RVP_REQUIRE(h->built, "build before radiusSearch");
+  RVP_REQUIRE(offsets && total, "offsets/total required");
+  RVP_REQUIRE(nq == 0 || (qx && qy && qz), "null query pointer");
+  set_device(ctx);
+  *total = 0;
+  RVP_REQUIRE(radius >= 0.0f, "radius must be >= 0");
+  u64 *offs_d = reinterpret_cast<u64 *>(out_dev(ctx, 0, offsets, nq + 1, mem));
+  int32_t *indices = nullptr;
+  float *dists = nullptr;
+  if (nq == 0 || h->n == 0) {
+    RVP_CUDA_TRY(cudaMemsetAsync(offs_d, 0, (nq + 1) * 8, ctx->stream));
+    out_copy(ctx, offsets, reinterpret_cast<int64_t *>(offs_d), nq + 1, mem);
+    sync(ctx);
+    outputs(0, &indices, &dists);
+    return;
+  }
+  const float *dqx = in_dev(ctx, 1, qx, nq, mem);
+  const float *dqy = in_dev(ctx, 2, qy, nq, mem);
+  const float *dqz = in_dev(ctx, 3, qz, nq, mem);
+  const bool refwin = h->collision != 0;
+  void *scan_tmp = scratch(ctx, 4, rvp::scan_temp_bytes(nq + 1));
+  auto finish = [&](size_t tot) {
+    out_copy(ctx, offsets, reinterpret_cast<int64_t *>(offs_d), nq + 1, mem);
+    out_copy(ctx, indices, static_cast<int32_t *>(ctx->scratch[8].ptr), tot, mem);
+    out_copy(ctx, dists, static_cast<float *>(ctx->scratch[9].ptr), tot, mem);
+    sync(ctx);
+  };
+  if (max_nn > 0 && max_nn <= 64 && !refwin) {
+    const int K = max_nn;
+    rvp::TreeOut o;
+    o.idx = static_cast<int32_t *>(scratch(ctx, 5, nq * (size_t)K * 8));
+    o.d2 = reinterpret_cast<float *>(o.idx + nq * (size_t)K);
+    int32_t *cnt = o.counts = static_cast<int32_t *>(scratch(ctx, 6, nq * 4));
+    knn_hash(h, dqx, dqy, dqz, nq, K, radius, rvp::TREE_PAIRS, o);
+    u32 *ucnt = static_cast<u32 *>(scratch(ctx, 7, nq * 4));
+    k_i32_to_u32<<<rvp::grid_for(nq, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(cnt, nq, ucnt);
+    RVP_LAUNCH_CHECK(ctx);
+    rvp::exclusive_scan_u32_to_u64(ctx, ucnt, offs_d, nq, nullptr, scan_tmp);
+    const u64 tot = read_back(ctx, offs_d + nq);
+    *total = (size_t)tot;
+    if (!outputs((size_t)tot, &indices, &dists)) return finish(0);
+    int32_t *di = out_dev(ctx, 8, indices, tot, mem);
+    float *dd = out_dev(ctx, 9, dists, tot, mem);
+    k_rows_to_csr<<<rvp::grid_for(nq * K, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
+        o.idx, o.d2, K, cnt, offs_d, nq, di, dd);
+    RVP_LAUNCH_CHECK(ctx);
+    return finish(tot);
+  }
+  // the lists' lengths, their offsets, and the lists (cut: the offsets of the
+  // cut ones beside the full ones)
+  const bool tree = !refwin && nq <= ((size_t)1 << 30);
+  rvp::QuerySet qs{dqx, dqy, dqz, nq, nullptr, nullptr, nullptr};
+  const rvp::GridView gv = refwin ? h->grid.view(rvp::KEY_REF_HASH, h->p1, h->p2)
+                                  : rvp::GridView{};
+  rvp::TreeQueries tq{};
+  u32 *cnt = static_cast<u32 *>(scratch(ctx, 6, nq * 4 + 256));
+  u64 *full = max_nn > 0 ? static_cast<u64 *>(scratch(ctx, 10, (nq + 2) * 8)) : offs_d;
+  u32 *most_d = cnt + nq;
+  u32 most = 0;
+  if (tree) {
+    if (rvp::tree_radius_few(nq)) tq.n = (u32)nq;
+    else
+      tq = rvp::tree_queries(ctx, h->tree, h->tree_view, h->x.as<float>(), h->y.as<float>(),
+                             h->z.as<float>(), dqx, dqy, dqz, nq);
+    rvp::tree_radius_count(ctx, h->tree_view, tq, dqx, dqy, dqz, radius, cnt, most_d);
+  } else {
+    RVP_REQUIRE(refwin, "at most 2^30 queries at a time");
+    rvp::grid_radius_count(ctx, gv, qs, radius, refwin, cnt);
+  }
+  rvp::exclusive_scan_u32_to_u64(ctx, cnt, full, nq, nullptr, scan_tmp);
+  u64 tot = 0;
+  if (max_nn > 0) {
+    u32 *ccut = static_cast<u32 *>(scratch(ctx, 7, nq * 4));
+    k_min_counts<<<rvp::grid_for(nq, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(
+        cnt, nq, (u32)max_nn, ccut);
+    RVP_LAUNCH_CHECK(ctx);
+    rvp::exclusive_scan_u32_to_u64(ctx, ccut, offs_d, nq, nullptr, scan_tmp);
+    RVP_CUDA_TRY(cudaMemcpyAsync(&tot, offs_d + nq, 8, cudaMemcpyDeviceToHost, ctx->stream));
+  }
+  u64 tot_full = 0;
+  RVP_CUDA_TRY(cudaMemcpyAsync(&tot_full, full + nq, 8, cudaMemcpyDeviceToHost, ctx->stream));
+  if (tree)
+    RVP_CUDA_TRY(cudaMemcpyAsync(&most, most_d, 4, cudaMemcpyDeviceToHost, ctx->stream));
+  sync(ctx);
+  if (max_nn <= 0) tot = tot_full;
+  *total = (size_t)tot;
+  if (!outputs((size_t)tot, &indices, &dists)) return finish(0);
+  int32_t *di = out_dev(ctx, 8, indices, tot, mem);
+  float *dd = out_dev(ctx, 9, dists, tot, mem);
+  const u32 cut = max_nn > 0 ? (u32)max_nn : 0;
+  if (tree) {
+    const bool big = most > rvp::tree_radius_cap();
+    u64 *pairs = big ? static_cast<u64 *>(scratch(ctx, 5, tot_full * 8)) : nullptr;
+    u32 *list = big ? static_cast<u32 *>(scratch(ctx, 11, nq * 4 + 16)) : nullptr;
+    rvp::tree_radius_fill(ctx, h->tree_view, tq, dqx, dqy, dqz, radius, full, offs_d, cut, di, dd,
+                          pairs, list, big ? list + nq : nullptr);
+    return finish(tot);
+  }
+  u64 *pairs = static_cast<u64 *>(scratch(ctx, 5, (tot_full ? tot_full : 1) * 8));
+  u32 *big = static_cast<u32 *>(scratch(ctx, 11, nq * 4 + 16));
+  u32 *big_count = big + nq;
+  rvp::grid_radius_fill(ctx, gv, qs, radius, refwin, full, 0, pairs, big, big_count);
+  rvp::sort_big_segments(ctx, full, pairs, big, big_count, (u32)std::min<size_t>(nq, 4096));
+  if (max_nn > 0) {
+    k_csr_cut<<<rvp::grid_for(nq, 128, ctx->num_sms * 16), 128, 0, ctx->stream>>>(
+        pairs, full, offs_d, nq, di, dd);
+  } else {
+    k_unpack<<<rvp::grid_for(tot, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(pairs, tot, di, dd);
+  }
+  RVP_LAUNCH_CHECK(ctx);
+  finish(tot);
+}
+
+extern "C" {
 rvp_status rvp_hash_radius_search(rvp_hash *h, const float *qx, const float *qy, const float *qz,
                                   size_t nq, float radius, int max_nn, int mem, int64_t *offsets,
                                   int32_t *indices, float *dists, size_t capacity, size_t *total) {
   if (!h) return RVP_ERR_INVALID_ARG;
-  rvp_context *ctx = h->ctx;
-  bool cap_fail = false;
-  rvp_status s = guard(ctx, [&] {
-    RVP_REQUIRE(h->built, "build before radiusSearch");
-    RVP_REQUIRE(offsets && total, "offsets/total required");
-    RVP_REQUIRE(nq == 0 || (qx && qy && qz), "null query pointer");
-    set_device(ctx);
-    *total = 0;
-    RVP_REQUIRE(radius >= 0.0f, "radius must be >= 0");
-    u64 *offs_d = reinterpret_cast<u64 *>(out_dev(ctx, 0, offsets, nq + 1, mem));
-    if (nq == 0 || h->n == 0) {
-      RVP_CUDA_TRY(cudaMemsetAsync(offs_d, 0, (nq + 1) * 8, ctx->stream));
-      out_copy(ctx, offsets, reinterpret_cast<int64_t *>(offs_d), nq + 1, mem);
-      sync(ctx);
-      return;
-    }
-    const float *dqx = in_dev(ctx, 1, qx, nq, mem);
-    const float *dqy = in_dev(ctx, 2, qy, nq, mem);
-    const float *dqz = in_dev(ctx, 3, qz, nq, mem);
-    rvp::QuerySet qs{dqx, dqy, dqz, nq, nullptr, nullptr, nullptr};
-    const rvp::GridView gv = h->grid.view(rvp::KEY_REF_HASH, h->p1, h->p2);
-    const bool refwin = h->collision != 0;
-    void *scan_tmp = scratch(ctx, 4, rvp::scan_temp_bytes(nq + 1));
-    if (max_nn > 0 && max_nn <= 64 && !refwin) {
-      const int K = max_nn;
-      rvp::TreeOut o;
-      o.idx = static_cast<int32_t *>(scratch(ctx, 5, nq * (size_t)K * 8));
-      o.d2 = reinterpret_cast<float *>(o.idx + nq * (size_t)K);
-      int32_t *cnt = o.counts = static_cast<int32_t *>(scratch(ctx, 6, nq * 4));
-      knn_hash(h, dqx, dqy, dqz, nq, K, radius, rvp::TREE_PAIRS, o);
-      u32 *ucnt = static_cast<u32 *>(scratch(ctx, 7, nq * 4));
-      k_i32_to_u32<<<rvp::grid_for(nq, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(cnt, nq, ucnt);
-      RVP_LAUNCH_CHECK(ctx);
-      rvp::exclusive_scan_u32_to_u64(ctx, ucnt, offs_d, nq, nullptr, scan_tmp);
-      const u64 tot = read_back(ctx, offs_d + nq);
-      *total = (size_t)tot;
-      if (tot > capacity) {
-        out_copy(ctx, offsets, reinterpret_cast<int64_t *>(offs_d), nq + 1, mem);
-        sync(ctx);
-        cap_fail = true;
-        return;
-      }
-      int32_t *di = out_dev(ctx, 8, indices, tot, mem);
-      float *dd = out_dev(ctx, 9, dists, tot, mem);
-      k_rows_to_csr<<<rvp::grid_for(nq * K, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
-          o.idx, o.d2, K, cnt, offs_d, nq, di, dd);
-      RVP_LAUNCH_CHECK(ctx);
-      out_copy(ctx, offsets, reinterpret_cast<int64_t *>(offs_d), nq + 1, mem);
-      out_copy(ctx, indices, di, tot, mem);
-      out_copy(ctx, dists, dd, tot, mem);
-      sync(ctx);
-      return;
-    }
-    u32 *cnt = static_cast<u32 *>(scratch(ctx, 6, nq * 4));
-    rvp::grid_radius_count(ctx, gv, qs, radius, refwin, cnt);
-    u64 *full = static_cast<u64 *>(scratch(ctx, 10, (nq + 1) * 8));
-    rvp::exclusive_scan_u32_to_u64(ctx, cnt, full, nq, nullptr, scan_tmp);
-    const u64 tot_full = read_back(ctx, full + nq);
-    u64 tot = tot_full;
-    if (max_nn > 0) {
-      u32 *ccut = static_cast<u32 *>(scratch(ctx, 7, nq * 4));
-      k_min_counts<<<rvp::grid_for(nq, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(
-          cnt, nq, (u32)max_nn, ccut);
-      RVP_LAUNCH_CHECK(ctx);
-      rvp::exclusive_scan_u32_to_u64(ctx, ccut, offs_d, nq, nullptr, scan_tmp);
-      tot = read_back(ctx, offs_d + nq);
-    } else {
-      RVP_CUDA_TRY(cudaMemcpyAsync(offs_d, full, (nq + 1) * 8, cudaMemcpyDeviceToDevice, ctx->stream));
-    }
-    *total = (size_t)tot;
-    if (tot > capacity) {
-      out_copy(ctx, offsets, reinterpret_cast<int64_t *>(offs_d), nq + 1, mem);
-      sync(ctx);
-      cap_fail = true;
-      return;
-    }
-    u64 *pairs = static_cast<u64 *>(scratch(ctx, 5, (tot_full ? tot_full : 1) * 8));
-    u32 *big = static_cast<u32 *>(scratch(ctx, 11, nq * 4 + 16));
-    u32 *big_count = big + nq;
-    rvp::grid_radius_fill(ctx, gv, qs, radius, refwin, full, 0, pairs, big, big_count);
-    rvp::sort_big_segments(ctx, full, pairs, big, big_count, (u32)std::min<size_t>(nq, 4096));
-    int32_t *di = out_dev(ctx, 8, indices, tot, mem);
-    float *dd = out_dev(ctx, 9, dists, tot, mem);
-    if (max_nn > 0) {
-      k_csr_cut<<<rvp::grid_for(nq, 128, ctx->num_sms * 16), 128, 0, ctx->stream>>>(
-          pairs, full, offs_d, nq, di, dd);
-    } else {
-      k_unpack<<<rvp::grid_for(tot, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(pairs, tot, di, dd);
-    }
-    RVP_LAUNCH_CHECK(ctx);
-    out_copy(ctx, offsets, reinterpret_cast<int64_t *>(offs_d), nq + 1, mem);
-    out_copy(ctx, indices, di, tot, mem);
-    out_copy(ctx, dists, dd, tot, mem);
-    sync(ctx);
+  bool fits = true;
+  rvp_status s = guard(h->ctx, [&] {
+    radius_search(h, qx, qy, qz, nq, radius, max_nn, mem, offsets, total,
+                  [&](size_t tot, int32_t **i, float **d) {
+                    fits = tot <= capacity;
+                    *i = indices;
+                    *d = dists;
+                    return fits;
+                  });
   });
-  if (s == RVP_OK && cap_fail) {
-    ctx->last_error = "radius search: output capacity too small";
+  if (s == RVP_OK && !fits) {
+    h->ctx->last_error = "radius search: output capacity too small";
     return RVP_ERR_CAPACITY;
   }
   return s;
+}
+
+rvp_status rvp_hash_radius_search_alloc(rvp_hash *h, const float *qx, const float *qy,
+                                        const float *qz, size_t nq, float radius, int max_nn,
+                                        int mem, int64_t *offsets, rvp_alloc_fn alloc, void *user,
+                                        size_t *total) {
+  if (!h || !alloc) return RVP_ERR_INVALID_ARG;
+  return guard(h->ctx, [&] {
+    radius_search(h, qx, qy, qz, nq, radius, max_nn, mem, offsets, total,
+                  [&](size_t tot, int32_t **i, float **d) {
+                    if (alloc(user, tot, i, d) != 0 || (tot && (!*i || !*d)))
+                      throw rvp::Error{RVP_ERR_OOM, "radius search: no memory for the lists"};
+                    return true;
+                  });
+  });
 }
 
 rvp_status rvp_hash_knn(rvp_hash *h, const float *qx, const float *qy, const float *qz, size_t nq,
@@ -706,22 +800,69 @@ rvp_status rvp_normals_radius(rvp_hash *h, float radius, float vp_x, float vp_y,
     RVP_REQUIRE(nx && ny && nz, "null output");
     set_device(ctx);
     const float *dx = h->x.as<float>(), *dy = h->y.as<float>(), *dz = h->z.as<float>();
-    rvp::QuerySet qs{dx, dy, dz, n, nullptr, nullptr, nullptr};
-    const rvp::GridView gv = h->grid.view(rvp::KEY_REF_HASH, h->p1, h->p2);
-    const bool refwin = h->collision != 0;
-    u32 *cnt = static_cast<u32 *>(scratch(ctx, 6, n * 4));
-    rvp::grid_radius_count(ctx, gv, qs, radius, refwin, cnt);
-    u64 *offs = static_cast<u64 *>(scratch(ctx, 10, (n + 1) * 8));
-    rvp::exclusive_scan_u32_to_u64(ctx, cnt, offs, n, nullptr, scratch(ctx, 4, rvp::scan_temp_bytes(n + 1)));
-    const u64 tot = read_back(ctx, offs + n);
-    u64 *pairs = static_cast<u64 *>(scratch(ctx, 5, (tot ? tot : 1) * 8));
-    u32 *big = static_cast<u32 *>(scratch(ctx, 11, n * 4 + 16));
-    rvp::grid_radius_fill(ctx, gv, qs, radius, refwin, offs, 0, pairs, big, big + n);
-    rvp::sort_big_segments(ctx, offs, pairs, big, big + n, (u32)std::min<size_t>(n, 4096));
     float *dnx = out_dev(ctx, 12, nx, n, mem), *dny = out_dev(ctx, 13, ny, n, mem),
           *dnz = out_dev(ctx, 14, nz, n, mem);
-    rvp::normals_from_lists(ctx, dx, dy, dz, pairs, offs, nullptr, 0, n, nullptr, false,
-                            eigen_iters, vp_x, vp_y, vp_z, dx, dy, dz, dnx, dny, dnz);
+    // the points of `list` (or all) from their lists in memory
+    auto from_lists = [&](const u32 *list, size_t m) {
+      const float *lx = dx, *ly = dy, *lz = dz;
+      if (list) {
+        float *g = static_cast<float *>(scratch(ctx, 7, m * 12));
+        rvp::gather_queries(ctx, dx, dy, dz, list, m, g, g + m, g + 2 * m);
+        lx = g;
+        ly = g + m;
+        lz = g + 2 * m;
+      }
+      u32 *cnt = static_cast<u32 *>(scratch(ctx, 6, m * 4 + 256));
+      u64 *offs = static_cast<u64 *>(scratch(ctx, 10, (m + 1) * 8));
+      void *scan_tmp = scratch(ctx, 4, rvp::scan_temp_bytes(m + 1));
+      u32 *big = static_cast<u32 *>(scratch(ctx, 11, m * 4 + 16));
+      rvp::QuerySet qs{lx, ly, lz, m, nullptr, nullptr, nullptr};
+      const rvp::GridView gv = h->grid.view(rvp::KEY_REF_HASH, h->p1, h->p2);
+      rvp::TreeQueries tq{};
+      if (h->collision) {
+        rvp::grid_radius_count(ctx, gv, qs, radius, true, cnt);
+      } else {
+        tq = rvp::tree_queries(ctx, h->tree, h->tree_view, dx, dy, dz, lx, ly, lz, m);
+        rvp::tree_radius_count(ctx, h->tree_view, tq, lx, ly, lz, radius, cnt, cnt + m);
+      }
+      rvp::exclusive_scan_u32_to_u64(ctx, cnt, offs, m, nullptr, scan_tmp);
+      const u64 tot = read_back(ctx, offs + m);
+      u64 *pairs = static_cast<u64 *>(scratch(ctx, 5, (tot ? tot : 1) * 8));
+      if (h->collision) {
+        rvp::grid_radius_fill(ctx, gv, qs, radius, true, offs, 0, pairs, big, big + m);
+        rvp::sort_big_segments(ctx, offs, pairs, big, big + m, (u32)std::min<size_t>(m, 4096));
+      } else {
+        u64 *rows = static_cast<u64 *>(scratch(ctx, 8, (tot ? tot : 1) * 8));
+        int32_t *ri = reinterpret_cast<int32_t *>(rows);
+        float *rd = reinterpret_cast<float *>(ri + tot);
+        rvp::tree_radius_fill(ctx, h->tree_view, tq, lx, ly, lz, radius, offs, offs, 0, ri, rd,
+                              pairs, big, big + m);
+        k_pack<<<rvp::grid_for(tot, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(ri, rd, tot,
+                                                                                  pairs);
+        RVP_LAUNCH_CHECK(ctx);
+      }
+      float *o[3] = {dnx, dny, dnz};
+      if (list) {
+        float *g = static_cast<float *>(scratch(ctx, 9, m * 12));
+        for (int a = 0; a < 3; ++a) o[a] = g + a * m;
+      }
+      rvp::normals_from_lists(ctx, dx, dy, dz, pairs, offs, nullptr, 0, m, nullptr, false,
+                              eigen_iters, vp_x, vp_y, vp_z, lx, ly, lz, o[0], o[1], o[2]);
+      if (list) {
+        k_scatter3<<<rvp::grid_for(m, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(
+            o[0], o[1], o[2], list, m, dnx, dny, dnz);
+        RVP_LAUNCH_CHECK(ctx);
+      }
+    };
+    if (h->collision) {
+      from_lists(nullptr, n);
+    } else {
+      u32 *hard = static_cast<u32 *>(scratch(ctx, 15, n * 4 + 16));
+      rvp::tree_radius_normals(ctx, h->tree_view, radius, eigen_iters, vp_x, vp_y, vp_z, dnx, dny,
+                               dnz, hard, hard + n);
+      const u32 m = read_back(ctx, hard + n);
+      if (m) from_lists(hard, m);
+    }
     out_copy(ctx, nx, dnx, n, mem);
     out_copy(ctx, ny, dny, n, mem);
     out_copy(ctx, nz, dnz, n, mem);

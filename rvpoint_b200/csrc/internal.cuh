@@ -417,6 +417,28 @@ TreeQueries tree_queries(rvp_context *ctx, KnnTree &w, const TreeView &t, const 
 // radius > 0: neighbours with d2 <= radius * radius only
 void tree_knn(rvp_context *ctx, const TreeView &t, const TreeQueries &q, int k, float radius,
               int mode, const TreeOut &o);
+// radius searches over the tree (radius_tree.cu). *flag = 1: cells of the hash
+// may share a key (or the check cannot tell)
+void hash_collision_check(rvp_context *ctx, const TreeView &t, float cell, long long p1,
+                          long long p2, int *flag);
+// few queries are taken in their own order (qx, qy, qz); else from q. counts
+// by query index; *most: the longest list, if past tree_radius_cap(); fill
+// then needs big_pairs (one per pair), big (one per query) and big_count
+bool tree_radius_few(size_t nq);
+u32 tree_radius_cap();
+void tree_radius_count(rvp_context *ctx, const TreeView &t, const TreeQueries &q, const float *qx,
+                       const float *qy, const float *qz, float radius, u32 *counts, u32 *most);
+void tree_radius_fill(rvp_context *ctx, const TreeView &t, const TreeQueries &q, const float *qx,
+                      const float *qy, const float *qz, float radius, const u64 *full,
+                      const u64 *offsets, u32 cut, int32_t *idx, float *d2, u64 *big_pairs,
+                      u32 *big, u32 *big_count);
+// normals of the cloud's own points; those with more neighbours than a lane
+// holds are listed in hard
+void tree_radius_normals(rvp_context *ctx, const TreeView &t, float radius, int iters, float vpx,
+                         float vpy, float vpz, float *nx, float *ny, float *nz, u32 *hard,
+                         u32 *hard_count);
+void gather_queries(rvp_context *ctx, const float *x, const float *y, const float *z,
+                    const u32 *list, size_t n, float *qx, float *qy, float *qz);
 // bounds of a cloud, folded into bb (min x, y, z, max x, y, z)
 void cloud_bbox(rvp_context *ctx, const float *x, const float *y, const float *z, size_t n,
                 float *bb);

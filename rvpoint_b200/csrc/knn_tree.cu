@@ -38,9 +38,11 @@
 #include "grid_device.cuh"
 #include "internal.cuh"
 #include "normals_device.cuh"
+#include "tree_device.cuh"
 
 namespace rvp {
 using namespace gd;
+using namespace td;
 
 namespace {
 inline size_t al(size_t b) { return (b + 255) & ~(size_t)255; }
@@ -219,48 +221,6 @@ __global__ void k_tree_queries(const float *__restrict__ x, const float *__restr
 // ---------------------------------------------------------------------------
 // search
 // ---------------------------------------------------------------------------
-// two single-precision operations at once, each rounded by itself
-__device__ __forceinline__ u64 add2(u64 a, u64 b) {
-  u64 d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-// (a product as fma(a, b, -0): mul.rn.f32x2 is contracted with the add that
-// follows, one rounding for both; the zero comes from a kernel argument, so it
-// is no constant to the compiler)
-__device__ __forceinline__ u64 mul2(u64 a, u64 b, u64 minus_zero) {
-  u64 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(minus_zero));
-  return d;
-}
-__device__ __forceinline__ u64 pack2(float a, float b) {
-  return (u64)__float_as_uint(a) | ((u64)__float_as_uint(b) << 32);
-}
-__device__ __forceinline__ float half2f(u64 v, int i) { return __uint_as_float((u32)(v >> (32 * i))); }
-// dist2 of two points: p + (-q) is p - q
-__device__ __forceinline__ u64 dist2x2(u64 px, u64 py, u64 pz, u64 nqx, u64 nqy, u64 nqz,
-                                        u64 mz) {
-  const u64 dx = add2(px, nqx), dy = add2(py, nqy), dz = add2(pz, nqz);
-  return add2(add2(mul2(dx, dx, mz), mul2(dy, dy, mz)), mul2(dz, dz, mz));
-}
-
-// the squared distance between two boxes (a point is a box), with the
-// operations of dist2
-__device__ __forceinline__ float box_gap(float alo, float ahi, float blo, float bhi) {
-  return fmaxf(fmaxf(fsub(blo, ahi), fsub(alo, bhi)), 0.0f);
-}
-struct Box {
-  float lo[3], hi[3];
-};
-__device__ __forceinline__ float box_d2(const Box &q, const float *box, u32 stride, u32 c) {
-  float g[3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-    g[a] = box_gap(q.lo[a], q.hi[a], __ldg(&box[(size_t)a * stride + c]),
-                   __ldg(&box[(size_t)(3 + a) * stride + c]));
-  return fadd(fadd(fmul(g[0], g[0]), fmul(g[1], g[1])), fmul(g[2], g[2]));
-}
-
 // Walks every leaf within limit() of the box q, nearest child first. All
 // lanes take part; limit() is uniform and may shrink on the way.
 template <int LV, class Limit, class Leaf>
@@ -420,16 +380,6 @@ __device__ __forceinline__ void bitonic_sort(float (&v)[N]) {
       }
     }
   }
-}
-
-// the leaf where a query of this key would lie
-__device__ __forceinline__ u32 leaf_of_key(const TreeView &t, u64 key) {
-  u32 lo = 0, hi = t.n - 1;
-  while (lo < hi) {
-    const u32 m = (lo + hi) >> 1;
-    if (t.keys[m] < key) lo = m + 1; else hi = m;
-  }
-  return lo / 32;
 }
 
 // sor_sc's mean (statistical_outlier_removal.cpp:36-40): the ascending sum of
@@ -608,18 +558,7 @@ __global__ __launch_bounds__(32, KCAP > 32 ? 10 : 16) void k_knn_tree(TreeView t
       mine = mine && lim <= kLoner * ref;
       limits();
     }
-    const float v[3] = {q.x, q.y, q.z};
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      float lo = mine ? v[a] : INFINITY, hi = mine ? v[a] : -INFINITY;
-#pragma unroll
-      for (int i = 16; i; i >>= 1) {
-        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, i));
-        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, i));
-      }
-      pk.lo[a] = lo;
-      pk.hi[a] = hi;
-    }
+    pk = warp_box(q, mine);
   }
 
   // ---- results of the packet

@@ -162,7 +162,8 @@ class PlaneScorer:
 
     def close(self):
         if getattr(self, "h", None):
-            self.L.rvp_scorer_destroy(self.h)
+            if self.ctx.h:  # (at exit the context may go first, and its memory with it)
+                self.L.rvp_scorer_destroy(self.h)
             self.h = None
 
     def __del__(self):  # pragma: no cover

@@ -105,3 +105,77 @@ def _means(p, k):
             s = np.float32(s + v)
         out[i] = s / np.float32(k)
     return out
+
+
+def brute_radius(p, q, r):
+    d = [p[None, :, a] - q[:, None, a] for a in range(3)]
+    d2 = (d[0] * d[0] + d[1] * d[1]) + d[2] * d[2]
+    r2 = np.float32(r) * np.float32(r)
+    offs, idx, dist = [0], [], []
+    for row in d2:
+        o = np.argsort(row, kind="stable")
+        o = o[row[o] <= r2]
+        idx.append(o)
+        dist.append(row[o])
+        offs.append(offs[-1] + len(o))
+    return np.asarray(offs), np.concatenate(idx).astype(np.int32), np.concatenate(dist)
+
+
+# radius lists over the tree: lists of up to 32, 64, 512 and 1024 points are
+# ordered in different ways, longer ones apart; up to 2048 queries go one per
+# warp in their own order
+@pytest.mark.parametrize("n,radius", [(1, 1.0), (33, 0.0), (700, 0.4), (2047, 0.8), (2049, 0.8),
+                                      (3000, 1.1), (3000, 20.0)])
+@pytest.mark.parametrize("cloud", ["room", "lattice"])
+def test_tree_radius(gpu_ctx, n, radius, cloud):
+    from rvpoint_b200 import api
+    if cloud == "lattice":
+        i = np.arange(n)
+        c = D.Cloud.from_xyz(np.stack([i % 13, (i // 13) % 11, i // 143], 1) % 9 * 0.25)
+    else:
+        c = D.room_cloud(n=max(n, 50), seed=n).subset(np.arange(n))
+    p = c.aos()
+    h = api.SpatialHash()
+    h.setInputCloud(c, 0.5)
+    h.build()
+    assert not h.hasCollisions()
+    q = np.concatenate([p[: n // 3] + np.float32(0.02), p[::-1]])[: max(1, n - 1)]
+    for q in (p, np.ascontiguousarray(q)):
+        offs, idx, d2 = h.radiusSearchBatch(q[:, 0], q[:, 1], q[:, 2], radius)
+        offs2, idx2, dist2 = brute_radius(p, q, radius)
+        assert np.array_equal(offs, offs2) and np.array_equal(idx, idx2)
+        assert np.array_equal(bits(d2), bits(dist2))
+        cut, idx3, _ = h.radiusSearchBatch(q[:, 0], q[:, 1], q[:, 2], radius, max_nn=70)
+        first = np.concatenate([idx2[a:min(a + 70, b)] for a, b in zip(offs2, offs2[1:])])
+        assert np.array_equal(np.diff(cut), np.minimum(np.diff(offs2), 70))
+        assert np.array_equal(idx3, first)
+
+
+@pytest.mark.parametrize("radius", [0.0, 0.03, 0.3, 2.0])  # 0, tens, hundreds, all as neighbours
+def test_radius_normals_lists(gpu_ctx, restatement, radius):
+    from rvpoint_b200 import api
+    c = D.room_cloud(n=1500, seed=3)
+    h = api.SpatialHash()
+    h.setInputCloud(c, 0.1)
+    h.build()
+    got = np.stack(api.normal_estimation_rvv(c, h, 10, radius), 1)
+    want = np.asarray(restatement.normals_radius(c, 0.1, radius))
+    assert np.array_equal((got != 0).any(1), (want != 0).any(1))
+    # (the rotations branch on the largest entry: a few differ by more)
+    assert (np.abs(got - want).max(1) < 1e-4).mean() > 0.995
+
+
+@pytest.mark.parametrize("primes,collide", [((73856093, 19349663), False), ((1, 1), True),
+                                            ((-73856093, 19349663), False), ((0, 5), True),
+                                            ((1 << 41, 3), True)])  # (3, 0, 0) and (0, 0, 1)
+def test_collisions_found(gpu_ctx, restatement, primes, collide):
+    from rvpoint_b200 import api
+    c = D.room_cloud(n=4000, seed=5)
+    h = api.SpatialHash()
+    h.setHashPrimes(*primes)
+    h.setInputCloud(c, 0.1)
+    h.build()
+    assert h.hasCollisions() == collide
+    offs, idx, _ = h.radiusSearchBatch(c.x, c.y, c.z, 0.1)
+    o2, i2, _ = restatement.radius_search(c, 0.1, 0.1, p1=primes[0], p2=primes[1])
+    assert np.array_equal(offs, o2) and np.array_equal(idx, i2)
