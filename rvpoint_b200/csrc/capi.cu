@@ -538,9 +538,9 @@ static void radius_search(rvp_hash *h, const float *qx, const float *qy, const f
   u32 *cnt = static_cast<u32 *>(scratch(ctx, 6, nq * 4 + 256));
   u64 *full = max_nn > 0 ? static_cast<u64 *>(scratch(ctx, 10, (nq + 2) * 8)) : offs_d;
   u32 *most_d = cnt + nq;
-  u32 most = 0;
+  u32 most[2] = {0, 0};
   if (tree) {
-    if (rvp::tree_radius_few(nq)) tq.n = (u32)nq;
+    if (rvp::tree_radius_few(nq)) tq = rvp::tree_queries_as_given(ctx, h->tree, nq);
     else
       tq = rvp::tree_queries(ctx, h->tree, h->tree_view, h->x.as<float>(), h->y.as<float>(),
                              h->z.as<float>(), dqx, dqy, dqz, nq);
@@ -562,7 +562,7 @@ static void radius_search(rvp_hash *h, const float *qx, const float *qy, const f
   u64 tot_full = 0;
   RVP_CUDA_TRY(cudaMemcpyAsync(&tot_full, full + nq, 8, cudaMemcpyDeviceToHost, ctx->stream));
   if (tree)
-    RVP_CUDA_TRY(cudaMemcpyAsync(&most, most_d, 4, cudaMemcpyDeviceToHost, ctx->stream));
+    RVP_CUDA_TRY(cudaMemcpyAsync(most, most_d, 8, cudaMemcpyDeviceToHost, ctx->stream));
   sync(ctx);
   if (max_nn <= 0) tot = tot_full;
   *total = (size_t)tot;
@@ -571,10 +571,10 @@ static void radius_search(rvp_hash *h, const float *qx, const float *qy, const f
   float *dd = out_dev(ctx, 9, dists, tot, mem);
   const u32 cut = max_nn > 0 ? (u32)max_nn : 0;
   if (tree) {
-    const bool big = most > rvp::tree_radius_cap();
+    const bool big = most[0] > rvp::tree_radius_cap();
     u64 *pairs = big ? static_cast<u64 *>(scratch(ctx, 5, tot_full * 8)) : nullptr;
     u32 *list = big ? static_cast<u32 *>(scratch(ctx, 11, nq * 4 + 16)) : nullptr;
-    rvp::tree_radius_fill(ctx, h->tree_view, tq, dqx, dqy, dqz, radius, full, offs_d, cut, di, dd,
+    rvp::tree_radius_fill(ctx, h->tree_view, tq, dqx, dqy, dqz, radius, full, offs_d, cut, most[1], di, dd,
                           pairs, list, big ? list + nq : nullptr);
     return finish(tot);
   }
@@ -826,7 +826,11 @@ rvp_status rvp_normals_radius(rvp_hash *h, float radius, float vp_x, float vp_y,
         rvp::tree_radius_count(ctx, h->tree_view, tq, lx, ly, lz, radius, cnt, cnt + m);
       }
       rvp::exclusive_scan_u32_to_u64(ctx, cnt, offs, m, nullptr, scan_tmp);
-      const u64 tot = read_back(ctx, offs + m);
+      u64 tot = 0;
+      u32 most[2] = {0, 0};
+      RVP_CUDA_TRY(cudaMemcpyAsync(&tot, offs + m, 8, cudaMemcpyDeviceToHost, ctx->stream));
+      RVP_CUDA_TRY(cudaMemcpyAsync(most, cnt + m, 8, cudaMemcpyDeviceToHost, ctx->stream));
+      sync(ctx);
       u64 *pairs = static_cast<u64 *>(scratch(ctx, 5, (tot ? tot : 1) * 8));
       if (h->collision) {
         rvp::grid_radius_fill(ctx, gv, qs, radius, true, offs, 0, pairs, big, big + m);
@@ -835,7 +839,7 @@ rvp_status rvp_normals_radius(rvp_hash *h, float radius, float vp_x, float vp_y,
         u64 *rows = static_cast<u64 *>(scratch(ctx, 8, (tot ? tot : 1) * 8));
         int32_t *ri = reinterpret_cast<int32_t *>(rows);
         float *rd = reinterpret_cast<float *>(ri + tot);
-        rvp::tree_radius_fill(ctx, h->tree_view, tq, lx, ly, lz, radius, offs, offs, 0, ri, rd,
+        rvp::tree_radius_fill(ctx, h->tree_view, tq, lx, ly, lz, radius, offs, offs, 0, most[1], ri, rd,
                               pairs, big, big + m);
         k_pack<<<rvp::grid_for(tot, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(ri, rd, tot,
                                                                                   pairs);

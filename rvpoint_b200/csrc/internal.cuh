@@ -382,6 +382,7 @@ struct TreeQueries {
   const u64 *n_sort = nullptr;   // null, or 0 there: the queries are the cloud
   u32 *hard_count = nullptr;     // queries left for the warp-per-query kernel
   u32 *hard = nullptr;           // (their places in q, or in the tree)
+  u32 *longer = nullptr;         // queries with long radius lists
   u32 n = 0;
   u64 minus_zero = 0x8000000080000000ull;  // two of them
 };
@@ -414,6 +415,8 @@ TreeView tree_build(rvp_context *ctx, KnnTree &w, const float *x, const float *y
 TreeQueries tree_queries(rvp_context *ctx, KnnTree &w, const TreeView &t, const float *x,
                          const float *y, const float *z, const float *qx, const float *qy,
                          const float *qz, size_t nq);
+// the same for queries in their own order (tree_radius_few)
+TreeQueries tree_queries_as_given(rvp_context *ctx, KnnTree &w, size_t nq);
 // radius > 0: neighbours with d2 <= radius * radius only
 void tree_knn(rvp_context *ctx, const TreeView &t, const TreeQueries &q, int k, float radius,
               int mode, const TreeOut &o);
@@ -422,16 +425,17 @@ void tree_knn(rvp_context *ctx, const TreeView &t, const TreeQueries &q, int k, 
 void hash_collision_check(rvp_context *ctx, const TreeView &t, float cell, long long p1,
                           long long p2, int *flag);
 // few queries are taken in their own order (qx, qy, qz); else from q. counts
-// by query index; *most: the longest list, if past tree_radius_cap(); fill
-// then needs big_pairs (one per pair), big (one per query) and big_count
+// by query index; most[0]: the longest list, or 0 if it is short; most[1]: how
+// many are longer (fill's n_long). Past tree_radius_cap() fill needs big_pairs
+// (one per pair), big (one per query) and big_count
 bool tree_radius_few(size_t nq);
 u32 tree_radius_cap();
 void tree_radius_count(rvp_context *ctx, const TreeView &t, const TreeQueries &q, const float *qx,
                        const float *qy, const float *qz, float radius, u32 *counts, u32 *most);
 void tree_radius_fill(rvp_context *ctx, const TreeView &t, const TreeQueries &q, const float *qx,
                       const float *qy, const float *qz, float radius, const u64 *full,
-                      const u64 *offsets, u32 cut, int32_t *idx, float *d2, u64 *big_pairs,
-                      u32 *big, u32 *big_count);
+                      const u64 *offsets, u32 cut, u32 n_long, int32_t *idx, float *d2,
+                      u64 *big_pairs, u32 *big, u32 *big_count);
 // normals of the cloud's own points; those with more neighbours than a lane
 // holds are listed in hard
 void tree_radius_normals(rvp_context *ctx, const TreeView &t, float radius, int iters, float vpx,

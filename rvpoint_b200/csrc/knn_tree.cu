@@ -1,6 +1,6 @@
 // Exact k nearest neighbours in one cloud (k <= 64) over a 32-wide box tree.
 //
-// Build: the points sorted by the Morton code of their quantised position
+// Build: the points sorted by the Hilbert code of their quantised position
 // (32 bits, one power-of-two cell for all axes), every 32 consecutive points
 // a leaf with its bounding box, every 32 leaves a node, and so on, four levels
 // in all. No cell size is chosen and nothing depends on the
@@ -99,11 +99,28 @@ __device__ __forceinline__ u32 tree_key(const TreeFrame &F, float x, float y, fl
     q[a] = t > 0.0f ? (t < 4.0e9f ? min((u32)t, last) : last) : 0u;
     top = max(top, F.bits[a]);
   }
-  u32 key = 0;
+  // Compact Hilbert index (C. Hamilton, A. Rau-Chaplin, "Compact Hilbert
+  // indices", 2008): per level the Gray code rank of the point's octant in the
+  // frame of the entry e and direction d, over the axes that have this bit.
+  // Consecutive codes are neighbouring cells (but for a few jumps where an
+  // axis has run out of bits), so a leaf's box is small: with Morton codes
+  // packets tested 19 to 41 leaves, one that spans a jump all of a large box.
+  constexpr u32 kGray = 0x54672310u, kEntry = 0x56633000u, kDir = 0x01122110u;
+  auto rotr = [](u32 v, u32 k) { return ((v >> k) | (v << (3 - k))) & 7u; };
+  u32 key = 0, e = 0, d = 0;
   for (int b = top - 1; b >= 0; --b) {
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-      if (b < F.bits[a]) key = (key << 1) | ((q[a] >> b) & 1u);
+    const u32 mask = (b < F.bits[0] ? 1u : 0u) | (b < F.bits[1] ? 2u : 0u) |
+                     (b < F.bits[2] ? 4u : 0u);
+    const u32 l = ((q[0] >> b) & 1u) | (((q[1] >> b) & 1u) << 1) | (((q[2] >> b) & 1u) << 2);
+    const u32 k = d == 2 ? 0 : d + 1;
+    const u32 w = (kGray >> (4 * rotr(l ^ e, k))) & 7u;
+    const u32 mu = rotr(mask, k);
+    if (mu & 4u) key = (key << 1) | (w >> 2);
+    if (mu & 2u) key = (key << 1) | ((w >> 1) & 1u);
+    if (mu & 1u) key = (key << 1) | (w & 1u);
+    e ^= rotr((kEntry >> (4 * w)) & 7u, 3 - k);
+    d += ((kDir >> (4 * w)) & 7u) + 1;
+    d = d >= 3 ? d - 3 : d;
   }
   return key;
 }
@@ -326,9 +343,9 @@ constexpr int kTreeExtra = 3;  // collected points past the list, for equal dist
 // a query joins its packet's walk if its limit (a squared distance) is within
 // this factor of the median one
 constexpr float kLoner = 16.0f;
-// leaves a packet tests before it gives up. Packets test 19 to 41 leaves on
-// average (k 16 to 32); one that spans a jump of the Morton order has every
-// leaf of a large box to test, up to 2 ms, with no other work left to hide it
+// leaves a packet tests before it gives up: one with points far apart has every
+// leaf of a large box to test (milliseconds, with no other work left to hide
+// them), most test 20 to 40
 constexpr int kLeafBudget = 128;
 
 // shared memory of a packet: the staged leaf, the leaves scanned, the buffered
@@ -821,15 +838,21 @@ TreeView tree_build(rvp_context *ctx, KnnTree &w, const float *x, const float *y
   return t;
 }
 
+TreeQueries tree_queries_as_given(rvp_context *ctx, KnnTree &w, size_t nq) {
+  TreeQueries q{};
+  q.n = (u32)nq;
+  w.hard.reserve(nq * 8 + 256);
+  q.hard_count = w.hard.as<u32>();
+  q.hard = q.hard_count + 64;
+  q.longer = q.hard + nq;
+  RVP_CUDA_TRY(cudaMemsetAsync(q.hard_count, 0, 4, ctx->stream));
+  return q;
+}
+
 TreeQueries tree_queries(rvp_context *ctx, KnnTree &w, const TreeView &t, const float *x,
                          const float *y, const float *z, const float *qx, const float *qy,
                          const float *qz, size_t nq) {
-  TreeQueries q{};
-  q.n = (u32)nq;
-  w.hard.reserve(nq * 4 + 256);
-  q.hard_count = w.hard.as<u32>();
-  q.hard = q.hard_count + 64;
-  RVP_CUDA_TRY(cudaMemsetAsync(q.hard_count, 0, 4, ctx->stream));
+  TreeQueries q = tree_queries_as_given(ctx, w, nq);
   if (qx == x && qy == y && qz == z && nq == t.n) return q;
   w.qkeys.reserve(nq * 8);
   w.qvals.reserve(nq * 4);

@@ -26,7 +26,7 @@ using namespace td;
 
 namespace {
 constexpr int FT_WARPS = 4;
-constexpr u32 FT_CAP = 1024;   // pairs a warp orders in shared memory
+constexpr u32 FT_SHORT = 256, FT_CAP = 1024;  // pairs a warp orders in shared memory
 constexpr u32 FT_BINS = 512;
 constexpr size_t kFewQueries = 2048;
 
@@ -66,6 +66,11 @@ __global__ __launch_bounds__(1024) void k_hash_check(const float *bb, float cell
 // ---------------------------------------------------------------------------
 // count
 // ---------------------------------------------------------------------------
+// leaves a packet tests before its queries go one per warp: of 3277 packets of
+// a LiDAR frame a few have every leaf of a wide box to test, and the kernel
+// waited for them (468 us; 256 leaves: 140 us and 8 us for the listed ones)
+constexpr int kLeafBudget = 128;
+
 __global__ __launch_bounds__(32) void k_radius_packets(TreeView t, TreeQueries qs, float r2,
                                                        u32 *counts, u32 *most) {
   __shared__ __align__(16) float stage[3][32];
@@ -80,7 +85,9 @@ __global__ __launch_bounds__(32) void k_radius_packets(TreeView t, TreeQueries q
   const Box pk = warp_box(q, true);
   const u64 nqx = pack2(-q.x, -q.x), nqy = pack2(-q.y, -q.y), nqz = pack2(-q.z, -q.z);
   u32 cnt = 0;
+  int budget = kLeafBudget;
   auto leaf = [&](u32 l) {
+    if (--budget < 0) return;
     const u32 i = l * 32 + lane;
     const float4 mate = i < t.n ? __ldg(&t.pts[i]) : make_float4(NAN, NAN, NAN, 0.0f);
     const float at = box_d2(own, t.box[0], t.stride[0], l) <= r2 ? r2 : -1.0f;
@@ -104,46 +111,107 @@ __global__ __launch_bounds__(32) void k_radius_packets(TreeView t, TreeQueries q
     }
   };
   tree_visit_all(t, pk, r2, leaf);
+  if (budget < 0) {  // points far apart: one warp each (k_radius_listed)
+    u32 at = 0;
+    if (lane == 0) at = atomicAdd(qs.hard_count, min(32u, qs.n - packet * 32));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (active) qs.hard[at + lane] = qi;
+    return;
+  }
   if (active) counts[__float_as_uint(q.w)] = cnt;
-  const u32 m = __reduce_max_sync(0xffffffffu, active ? cnt : 0u);
-  if (lane == 0 && m > FT_CAP) atomicMax(most, m);
+  const unsigned b = __ballot_sync(0xffffffffu, active && cnt > FT_SHORT);
+  if (b) {  // listed for k_radius_fill_long
+    const u32 m = __reduce_max_sync(0xffffffffu, active ? cnt : 0u);
+    u32 at = 0;
+    if (lane == 0) {
+      atomicMax(&most[0], m);
+      at = atomicAdd(&most[1], (u32)__popc(b));
+    }
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if ((b >> lane) & 1u) qs.longer[at + __popc(b & ((1u << lane) - 1))] = qi;
+  }
 }
 
-// hit(d, i, any) for the leaf's point i of every lane, d < 0 past the radius
-template <class Hit>
+// hit(pass, d, index): the lane's point of a leaf. Two leaves' points are
+// loaded at a time. Every SPLIT-th leaf of a node, from `part` on.
+template <int SPLIT, class Hit>
 __device__ __forceinline__ void radius_walk(const TreeView &t, float qx, float qy, float qz,
-                                            float r2, Hit &&hit) {
+                                            float r2, int part, Hit &&hit) {
   const int lane = threadIdx.x & 31;
   const Box own{{qx, qy, qz}, {qx, qy, qz}};
-  auto leaf = [&](u32 l) {
+  auto load = [&](u32 l) {
     const u32 i = l * 32 + lane;
-    bool pass = false;
-    float d = 0.0f;
-    u32 idx = 0;
-    if (i < t.n) {
-      const float4 p = __ldg(&t.pts[i]);
-      d = dist2(p.x, p.y, p.z, qx, qy, qz);
-      idx = __float_as_uint(p.w);
-      pass = d <= r2;
-    }
-    hit(pass, d, idx, i);
+    return i < t.n ? __ldg(&t.pts[i]) : make_float4(NAN, NAN, NAN, 0.0f);
   };
-  tree_visit_all(t, own, r2, leaf);
+  auto take = [&](const float4 &p) {
+    const float d = dist2(p.x, p.y, p.z, qx, qy, qz);
+    hit(d <= r2, d, __float_as_uint(p.w));
+  };
+  auto parent = [&](u32 node) {  // the leaves of a level-1 node
+    const u32 first = node * 32, c = first + lane;
+    unsigned m = __ballot_sync(
+        0xffffffffu, c < t.count[0] && box_d2(own, t.box[0], t.stride[0], c) <= r2);
+    if (SPLIT > 1) {  // this part's leaves: by their rank among those near
+      const unsigned mine = __ballot_sync(
+          0xffffffffu, __popc(m & ((1u << lane) - 1)) % SPLIT == part);
+      m &= mine;
+    }
+    while (m) {
+      const int s = __ffs(m) - 1;
+      m &= m - 1;
+      const float4 p = load(first + s);
+      if (m) {
+        const int s2 = __ffs(m) - 1;
+        m &= m - 1;
+        const float4 p2 = load(first + s2);
+        take(p);
+        take(p2);
+      } else {
+        take(p);
+      }
+    }
+  };
+  tree_visit_all<1>(t, own, r2, parent);
 }
 
 // queries in their own order, one per warp
 __global__ __launch_bounds__(128) void k_radius_each(TreeView t, const float *qx, const float *qy,
                                                      const float *qz, u32 nq, float r2,
-                                                     u32 *counts, u32 *most) {
+                                                     u32 *counts, u32 *most, u32 *longer) {
   const u32 w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (w >= nq) return;
   u32 cnt = 0;
-  radius_walk(t, qx[w], qy[w], qz[w], r2, [&](bool pass, float, u32, u32) {
+  radius_walk<1>(t, qx[w], qy[w], qz[w], r2, 0, [&](bool pass, float, u32) {
     cnt += __popc(__ballot_sync(0xffffffffu, pass));
   });
   if ((threadIdx.x & 31) == 0) {
     counts[w] = cnt;
-    if (cnt > FT_CAP) atomicMax(most, cnt);
+    if (cnt > FT_SHORT) {
+      atomicMax(&most[0], cnt);
+      longer[atomicAdd(&most[1], 1u)] = w;
+    }
+  }
+}
+
+// the queries packets gave up on
+__global__ __launch_bounds__(128) void k_radius_listed(TreeView t, TreeQueries qs, float r2,
+                                                       u32 *counts, u32 *most) {
+  const u32 n = *qs.hard_count;
+  const bool self = qs.n_sort == nullptr || *qs.n_sort == 0;
+  for (u32 w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n;
+       w += (gridDim.x * blockDim.x) >> 5) {
+    const float4 q = self ? t.pts[qs.hard[w]] : qs.q[qs.hard[w]];
+    u32 cnt = 0;
+    radius_walk<1>(t, q.x, q.y, q.z, r2, 0, [&](bool pass, float, u32) {
+      cnt += __popc(__ballot_sync(0xffffffffu, pass));
+    });
+    if ((threadIdx.x & 31) == 0) {
+      counts[__float_as_uint(q.w)] = cnt;
+      if (cnt > FT_SHORT) {
+        atomicMax(&most[0], cnt);
+        qs.longer[atomicAdd(&most[1], 1u)] = qs.hard[w];
+      }
+    }
   }
 }
 
@@ -155,31 +223,41 @@ __device__ __forceinline__ u32 bin_of(u64 key, float scale, u32 bins) {
   return b < (float)(bins - 1) ? (u32)b : bins - 1;
 }
 
-// the cnt keys of `keys` ordered: write(rank, key), by one warp
-template <class Write>
+// The cnt keys of `keys` ordered: write(rank, key), by the TH threads of a warp
+// or a block. Bin b lies at bin_at(b): the run of bins that a thread scans is
+// then free of bank conflicts.
+template <u32 TH, u32 BINS, class Write>
 __device__ __forceinline__ void order_keys(const u64 *keys, u32 cnt, float r2, u32 *bins,
-                                           unsigned short *perm, Write &&write) {
-  const u32 lane = threadIdx.x & 31;
+                                           unsigned short *perm, u32 *warp_sum, Write &&write) {
+  const u32 tid = threadIdx.x & (TH - 1), lane = threadIdx.x & 31;
+  auto sync = [] {
+    if constexpr (TH == 32) __syncwarp();
+    else __syncthreads();
+  };
   if (cnt <= 32) {
-    if (lane < cnt) {
-      const u64 k = keys[lane];
+    if (tid < cnt) {
+      const u64 k = keys[tid];
       u32 rank = 0;
       for (u32 j = 0; j < cnt; ++j) rank += keys[j] < k;
       write(rank, k);
     }
     return;
   }
-  u32 nb = 64;
-  while (nb < cnt && nb < FT_BINS) nb <<= 1;
+  u32 nb = 2 * TH, per_log = 1;  // bins, bins per thread
+  while (nb < cnt && nb < BINS) {
+    nb <<= 1;
+    ++per_log;
+  }
+  const u32 per = 1u << per_log;
+  auto bin_at = [&](u32 b) { return (b & (per - 1)) * TH + (b >> per_log); };
   const float scale = r2 > 0.0f ? fdiv((float)nb, r2) : 0.0f;
-  for (u32 i = lane; i < nb; i += 32) bins[i] = 0;
-  __syncwarp();
-  for (u32 i = lane; i < cnt; i += 32) atomicAdd(&bins[bin_of(keys[i], scale, nb)], 1u);
-  __syncwarp();
-  {  // exclusive scan: nb / 32 bins per lane
-    const u32 per = nb / 32;
+  for (u32 i = tid; i < nb; i += TH) bins[i] = 0;
+  sync();
+  for (u32 i = tid; i < cnt; i += TH) atomicAdd(&bins[bin_at(bin_of(keys[i], scale, nb))], 1u);
+  sync();
+  {  // exclusive scan of the bins
     u32 sum = 0;
-    for (u32 j = 0; j < per; ++j) sum += bins[lane * per + j];
+    for (u32 j = 0; j < per; ++j) sum += bins[j * TH + tid];
     u32 incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -187,22 +265,27 @@ __device__ __forceinline__ void order_keys(const u64 *keys, u32 cnt, float r2, u
       if (lane >= (u32)o) incl += v;
     }
     u32 run = incl - sum;
+    if constexpr (TH > 32) {
+      if (lane == 31) warp_sum[tid >> 5] = incl;
+      sync();
+      for (u32 w = 0; w < tid >> 5; ++w) run += warp_sum[w];
+    }
     for (u32 j = 0; j < per; ++j) {
-      const u32 c = bins[lane * per + j];
-      bins[lane * per + j] = run;
+      const u32 c = bins[j * TH + tid];
+      bins[j * TH + tid] = run;
       run += c;
     }
   }
-  __syncwarp();
-  for (u32 i = lane; i < cnt; i += 32) {
-    const u32 at = atomicAdd(&bins[bin_of(keys[i], scale, nb)], 1u);
+  sync();
+  for (u32 i = tid; i < cnt; i += TH) {
+    const u32 at = atomicAdd(&bins[bin_at(bin_of(keys[i], scale, nb))], 1u);
     perm[at] = (unsigned short)i;
   }
-  __syncwarp();  // bins[b] is now the end of bin b
-  for (u32 p = lane; p < cnt; p += 32) {
+  sync();  // a bin now holds its end
+  for (u32 p = tid; p < cnt; p += TH) {
     const u64 k = keys[perm[p]];
     const u32 b = bin_of(k, scale, nb);
-    const u32 s = b ? bins[b - 1] : 0, e = bins[b];
+    const u32 s = b ? bins[bin_at(b - 1)] : 0, e = bins[bin_at(b)];
     u32 rank = s;
     if (e - s > 1)
       for (u32 j = s; j < e; ++j) rank += keys[perm[j]] < k;
@@ -211,46 +294,89 @@ __device__ __forceinline__ void order_keys(const u64 *keys, u32 cnt, float r2, u
 }
 
 // Query w: the w-th in tree order (or of the sorted queries), or with qx the
-// w-th in its own order. Lists over FT_CAP go unordered to big_pairs and are
-// listed. cut > 0: only the first cut of a list are written.
+// w-th in its own order. cut > 0: only the first cut of a list are written.
+__device__ __forceinline__ float4 fill_query(const TreeView &t, const TreeQueries &qs,
+                                             const float *qx, const float *qy, const float *qz,
+                                             u32 w) {
+  if (qx) return make_float4(qx[w], qy[w], qz[w], __uint_as_float(w));
+  const bool self = qs.n_sort == nullptr || *qs.n_sort == 0;
+  return self ? t.pts[w] : qs.q[w];
+}
+
+// lists of up to FT_SHORT points, one warp each
 __global__ __launch_bounds__(FT_WARPS * 32) void k_radius_fill(
     TreeView t, TreeQueries qs, const float *qx, const float *qy, const float *qz, float r2,
-    const u64 *full, const u64 *offsets, u32 cut, int32_t *out_idx, float *out_d2, u64 *big_pairs,
-    u32 *big, u32 *big_count) {
-  __shared__ u64 s_keys[FT_WARPS][FT_CAP];
-  __shared__ u32 s_bins[FT_WARPS][FT_BINS];
-  __shared__ unsigned short s_perm[FT_WARPS][FT_CAP];
+    const u64 *full, const u64 *offsets, u32 cut, int32_t *out_idx, float *out_d2) {
+  __shared__ u64 s_keys[FT_WARPS][FT_SHORT];
+  __shared__ u32 s_bins[FT_WARPS][FT_SHORT];
+  __shared__ unsigned short s_perm[FT_WARPS][FT_SHORT];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const u32 w = blockIdx.x * FT_WARPS + wib;
   if (w >= qs.n) return;
-  const bool self = qs.n_sort == nullptr || *qs.n_sort == 0;
-  float4 q;
-  if (qx) q = make_float4(qx[w], qy[w], qz[w], __uint_as_float(w));
-  else q = self ? t.pts[w] : qs.q[w];
+  const float4 q = fill_query(t, qs, qx, qy, qz, w);
   const u32 qi = __float_as_uint(q.w);
   const u64 from = full[qi];
   const u32 cnt = (u32)(full[qi + 1] - from);
-  if (cnt == 0) return;
-  const bool small = cnt <= FT_CAP;
-  u64 *to = small ? s_keys[wib] : big_pairs + from;
+  if (cnt == 0 || cnt > FT_SHORT) return;
   u32 pos = 0;
-  radius_walk(t, q.x, q.y, q.z, r2, [&](bool pass, float d, u32 idx, u32) {
+  radius_walk<1>(t, q.x, q.y, q.z, r2, 0, [&](bool pass, float d, u32 idx) {
     const unsigned b = __ballot_sync(0xffffffffu, pass);
     const u32 at = pos + __popc(b & ((1u << lane) - 1));
-    if (pass && at < cnt) to[at] = pack_nbr(d, (int)idx);
+    if (pass && at < cnt) s_keys[wib][at] = pack_nbr(d, (int)idx);
     pos += __popc(b);
   });
   __syncwarp();
+  const u64 off = offsets[qi];
+  order_keys<32, FT_SHORT>(s_keys[wib], cnt, r2, s_bins[wib], s_perm[wib], nullptr,
+                           [&](u32 rank, u64 k) {
+                             if (cut && rank >= cut) return;
+                             out_idx[off + rank] = nbr_idx(k);
+                             out_d2[off + rank] = nbr_d2(k);
+                           });
+}
+
+// The queries with longer lists, one block each: its warps take turns at the
+// leaves and order the list together. (One warp per list, with shared memory
+// for 1024 pairs each, left 16 warps to an SM: 394 us for the 15M pairs of a
+// LiDAR frame's lists over 256 points.) Lists over FT_CAP go unordered to
+// big_pairs and are listed in big.
+__global__ __launch_bounds__(FT_WARPS * 32) void k_radius_fill_long(
+    TreeView t, TreeQueries qs, const float *qx, const float *qy, const float *qz, float r2,
+    const u64 *full, const u64 *offsets, u32 cut, int32_t *out_idx, float *out_d2, u64 *big_pairs,
+    u32 *big, u32 *big_count) {
+  __shared__ u64 s_keys[FT_CAP];
+  __shared__ u32 s_bins[FT_BINS];
+  __shared__ unsigned short s_perm[FT_CAP];
+  __shared__ u32 s_pos, s_warp[FT_WARPS];
+  const int lane = threadIdx.x & 31;
+  const float4 q = fill_query(t, qs, qx, qy, qz, qs.longer[blockIdx.x]);
+  const u32 qi = __float_as_uint(q.w);
+  const u64 from = full[qi];
+  const u32 cnt = (u32)(full[qi + 1] - from);
+  const bool small = cnt <= FT_CAP;
+  u64 *to = small ? s_keys : big_pairs + from;
+  if (threadIdx.x == 0) s_pos = 0;
+  __syncthreads();
+  radius_walk<FT_WARPS>(t, q.x, q.y, q.z, r2, threadIdx.x >> 5, [&](bool pass, float d, u32 idx) {
+    const unsigned b = __ballot_sync(0xffffffffu, pass);
+    if (!b) return;
+    u32 at = 0;
+    if (lane == 0) at = atomicAdd(&s_pos, (u32)__popc(b));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(b & ((1u << lane) - 1));
+    if (pass && at < cnt) to[at] = pack_nbr(d, (int)idx);
+  });
+  __syncthreads();
   if (!small) {
-    if (lane == 0) big[atomicAdd(big_count, 1u)] = qi;
+    if (threadIdx.x == 0) big[atomicAdd(big_count, 1u)] = qi;
     return;
   }
   const u64 off = offsets[qi];
-  order_keys(s_keys[wib], cnt, r2, s_bins[wib], s_perm[wib], [&](u32 rank, u64 k) {
-    if (cut && rank >= cut) return;
-    out_idx[off + rank] = nbr_idx(k);
-    out_d2[off + rank] = nbr_d2(k);
-  });
+  order_keys<FT_WARPS * 32, FT_BINS>(s_keys, cnt, r2, s_bins, s_perm, s_warp,
+                                     [&](u32 rank, u64 k) {
+                                       if (cut && rank >= cut) return;
+                                       out_idx[off + rank] = nbr_idx(k);
+                                       out_d2[off + rank] = nbr_d2(k);
+                                     });
 }
 
 // the listed long lists, ordered in place in `pairs`
@@ -376,25 +502,36 @@ u32 tree_radius_cap() { return FT_CAP; }
 void tree_radius_count(rvp_context *ctx, const TreeView &t, const TreeQueries &q, const float *qx,
                        const float *qy, const float *qz, float radius, u32 *counts, u32 *most) {
   const float r2 = square_of(radius);
-  RVP_CUDA_TRY(cudaMemsetAsync(most, 0, 4, ctx->stream));
+  RVP_CUDA_TRY(cudaMemsetAsync(most, 0, 8, ctx->stream));
   if (tree_radius_few(q.n))
-    k_radius_each<<<(q.n + 3) / 4, 128, 0, ctx->stream>>>(t, qx, qy, qz, q.n, r2, counts, most);
+    k_radius_each<<<(q.n + 3) / 4, 128, 0, ctx->stream>>>(t, qx, qy, qz, q.n, r2, counts, most,
+                                                             q.longer);
   else
     k_radius_packets<<<(q.n + 31) / 32, 32, 0, ctx->stream>>>(t, q, r2, counts, most);
   RVP_LAUNCH_CHECK(ctx);
+  if (!tree_radius_few(q.n)) {
+    k_radius_listed<<<ctx->num_sms * 4, 128, 0, ctx->stream>>>(t, q, r2, counts, most);
+    RVP_LAUNCH_CHECK(ctx);
+  }
 }
 
 void tree_radius_fill(rvp_context *ctx, const TreeView &t, const TreeQueries &q, const float *qx,
                       const float *qy, const float *qz, float radius, const u64 *full,
-                      const u64 *offsets, u32 cut, int32_t *idx, float *d2, u64 *big_pairs,
-                      u32 *big, u32 *big_count) {
+                      const u64 *offsets, u32 cut, u32 n_long, int32_t *idx, float *d2,
+                      u64 *big_pairs, u32 *big, u32 *big_count) {
   const float r2 = square_of(radius);
   if (big_count) RVP_CUDA_TRY(cudaMemsetAsync(big_count, 0, 4, ctx->stream));
   const bool few = tree_radius_few(q.n);
-  k_radius_fill<<<(q.n + FT_WARPS - 1) / FT_WARPS, FT_WARPS * 32, 0, ctx->stream>>>(
-      t, q, few ? qx : nullptr, qy, qz, r2, full, offsets, cut, idx, d2, big_pairs, big,
-      big_count);
+  const unsigned blocks = (q.n + FT_WARPS - 1) / FT_WARPS;
+  k_radius_fill<<<blocks, FT_WARPS * 32, 0, ctx->stream>>>(t, q, few ? qx : nullptr, qy, qz, r2,
+                                                          full, offsets, cut, idx, d2);
   RVP_LAUNCH_CHECK(ctx);
+  if (n_long) {
+    k_radius_fill_long<<<n_long, FT_WARPS * 32, 0, ctx->stream>>>(
+        t, q, few ? qx : nullptr, qy, qz, r2, full, offsets, cut, idx, d2, big_pairs, big,
+        big_count);
+    RVP_LAUNCH_CHECK(ctx);
+  }
   if (big_count) {  // lists past a warp's reach
     sort_big_segments(ctx, full, big_pairs, big, big_count, std::min(q.n, 4096u));
     k_radius_big_out<<<std::min(q.n, 4096u), 256, 0, ctx->stream>>>(big_pairs, big, big_count, full,

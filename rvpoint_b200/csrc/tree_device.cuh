@@ -77,9 +77,9 @@ __device__ __forceinline__ Box warp_box(const float4 &q, bool in) {
   return b;
 }
 
-// Visits every leaf within sqrt(lim) of the box q, in tree order. All lanes
-// take part.
-template <int LV, class Leaf>
+// Visits every node of level END within sqrt(lim) of the box q, in tree order
+// (END 0: leaves). All lanes take part.
+template <int LV, int END, class Leaf>
 __device__ __forceinline__ void tree_visit(const TreeView &t, const Box &q, u32 first, float lim,
                                            Leaf &leaf) {
   const u32 c = first + (threadIdx.x & 31);
@@ -88,15 +88,15 @@ __device__ __forceinline__ void tree_visit(const TreeView &t, const Box &q, u32 
   while (m) {
     const int s = __ffs(m) - 1;
     m &= m - 1;
-    if constexpr (LV == 0) leaf(first + s);
-    else tree_visit<LV - 1>(t, q, (first + s) * 32, lim, leaf);
+    if constexpr (LV == END) leaf(first + s);
+    else tree_visit<LV - 1, END>(t, q, (first + s) * 32, lim, leaf);
   }
 }
-template <class Leaf>
+template <int END = 0, class Leaf>
 __device__ __forceinline__ void tree_visit_all(const TreeView &t, const Box &q, float lim,
                                                Leaf &leaf) {
   for (u32 f = 0; f < t.count[kTreeLevels - 1]; f += 32)
-    tree_visit<kTreeLevels - 1>(t, q, f, lim, leaf);
+    tree_visit<kTreeLevels - 1, END>(t, q, f, lim, leaf);
 }
 
 }  // namespace td
