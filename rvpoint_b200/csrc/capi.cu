@@ -342,6 +342,7 @@ rvp_status rvp_context_destroy(rvp_context *ctx) {
   cudaStreamSynchronize(ctx->stream);
   for (auto &b : ctx->scratch) b.release();
   for (auto &b : ctx->pinned) b.release();
+  ctx->rand_table.release();
   if (ctx->grid) {
     ctx->grid->release();
     delete ctx->grid;
@@ -967,57 +968,66 @@ rvp_status rvp_ransac_plane(rvp_context *ctx, const float *x, const float *y, co
     const float *dz = in_dev(ctx, 3, z, n, mem);
     const size_t R = 3 * (size_t)max_iters;
     const bool own_stream = rand_stream == nullptr;
-    std::vector<int32_t> rs;
+    int *drand = nullptr;
     if (own_stream) {
       // the reference's srand(0) + rand() sequence, drawn from libc itself
-      srand(0);
-      rs.resize(R);
-      for (size_t i = 0; i < R; ++i) rs[i] = rand();
-    }
-    int *drand = static_cast<int *>(scratch(ctx, 4, R * 4 + 16));
-    if (R) {
-      if (own_stream)
-        RVP_CUDA_TRY(cudaMemcpyAsync(drand, rs.data(), R * 4, cudaMemcpyHostToDevice, ctx->stream));
-      else
+      // once per context: it is the same for every call
+      if (ctx->rand_count < R) {
+        ctx->rand_count = 0;
+        ctx->rand_table.reserve(R * 4 + 16);
+        std::vector<int32_t> rs(R);
+        srand(0);
+        for (size_t i = 0; i < R; ++i) rs[i] = rand();
+        RVP_CUDA_TRY(cudaMemcpyAsync(ctx->rand_table.ptr, rs.data(), R * 4,
+                                     cudaMemcpyHostToDevice, ctx->stream));
+        sync(ctx);
+        ctx->rand_count = R;
+      }
+      drand = ctx->rand_table.as<int>();
+    } else {
+      drand = static_cast<int *>(scratch(ctx, 4, R * 4 + 16));
+      if (R)
         RVP_CUDA_TRY(cudaMemcpyAsync(drand, rand_stream, R * 4,
                                      mem == RVP_MEM_DEVICE ? cudaMemcpyDeviceToDevice
                                                            : cudaMemcpyHostToDevice,
                                      ctx->stream));
     }
-    int64_t *offs = single_frame_offsets(ctx, 5, n);
-    float *dm = static_cast<float *>(scratch(ctx, 6, 64));
-    int32_t *db = reinterpret_cast<int32_t *>(dm + 8);
-    int32_t *di = db + 2;
-    int32_t *dcounts = counts ? static_cast<int32_t *>(scratch(ctx, 7, (size_t)max_iters * 4 + 4))
-                              : nullptr;
     double pc = (double)probability;
     pc = pc < 0.5 ? 0.5 : (pc > 0.9999 ? 0.9999 : pc);
     rvp::RansacParams prm{dist_thresh, max_iters, collinear_thresh, log(1.0 - pc)};
-    if (max_iters > 0)
-      rvp::ransac_frames(ctx, dx, dy, dz, offs, 1, drand, prm, dm, db, di, dcounts,
-                         counts != nullptr, rvp::RansacSampler{}, 8);
-    float hm[4] = {0, 0, 0, 0};
-    int32_t hb = 0, hi = 0;
-    if (max_iters > 0) {
-      RVP_CUDA_TRY(cudaMemcpyAsync(hm, dm, 16, cudaMemcpyDeviceToHost, ctx->stream));
-      RVP_CUDA_TRY(cudaMemcpyAsync(&hb, db, 4, cudaMemcpyDeviceToHost, ctx->stream));
-      RVP_CUDA_TRY(cudaMemcpyAsync(&hi, di, 4, cudaMemcpyDeviceToHost, ctx->stream));
-      if (counts)
-        RVP_CUDA_TRY(cudaMemcpyAsync(counts, dcounts, (size_t)max_iters * 4,
-                                     mem == RVP_MEM_DEVICE ? cudaMemcpyDeviceToDevice
-                                                           : cudaMemcpyDeviceToHost,
-                                     ctx->stream));
+    rvp::RansacState r{};
+    if (max_iters > 0 && !counts) {
+      rvp::RansacState *dstate = static_cast<rvp::RansacState *>(scratch(ctx, 6, 64));
+      rvp::ransac_one(ctx, dx, dy, dz, n, drand, prm, dstate,
+                      scratch(ctx, 7, rvp::ransac_one_bytes()));
+      RVP_CUDA_TRY(cudaMemcpyAsync(&r, dstate, sizeof(r), cudaMemcpyDeviceToHost, ctx->stream));
+    } else if (max_iters > 0) {
+      // every hypothesis's count is wanted: none is left out
+      int64_t *offs = single_frame_offsets(ctx, 5, n);
+      float *dm = static_cast<float *>(scratch(ctx, 6, 64));
+      int32_t *db = reinterpret_cast<int32_t *>(dm + 8);
+      int32_t *di = db + 2;
+      int32_t *dcounts = static_cast<int32_t *>(scratch(ctx, 7, (size_t)max_iters * 4 + 4));
+      rvp::ransac_frames(ctx, dx, dy, dz, offs, 1, drand, prm, dm, db, di, dcounts, true,
+                         rvp::RansacSampler{}, 8);
+      RVP_CUDA_TRY(cudaMemcpyAsync(&r.model, dm, 16, cudaMemcpyDeviceToHost, ctx->stream));
+      RVP_CUDA_TRY(cudaMemcpyAsync(&r.best, db, 4, cudaMemcpyDeviceToHost, ctx->stream));
+      RVP_CUDA_TRY(cudaMemcpyAsync(&r.iters, di, 4, cudaMemcpyDeviceToHost, ctx->stream));
+      RVP_CUDA_TRY(cudaMemcpyAsync(counts, dcounts, (size_t)max_iters * 4,
+                                   mem == RVP_MEM_DEVICE ? cudaMemcpyDeviceToDevice
+                                                         : cudaMemcpyDeviceToHost,
+                                   ctx->stream));
     }
     sync(ctx);
     if (own_stream) {
       // leave libc's generator where the reference leaves it: srand(0) and
       // three rand() calls per executed iteration
       srand(0);
-      for (long i = 0; i < 3L * hi; ++i) (void)rand();
+      for (long i = 0; i < 3L * r.iters; ++i) (void)rand();
     }
-    memcpy(model, hm, 16);
-    *best_count = hb;
-    if (iters_run) *iters_run = hi;
+    memcpy(model, &r.model, 16);
+    *best_count = r.best;
+    if (iters_run) *iters_run = r.iters;
   });
 }
 

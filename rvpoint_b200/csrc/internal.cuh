@@ -84,6 +84,8 @@ struct rvp_context {
   rvp::Grid *grid = nullptr;        // grid of the clustering entry point
   rvp::KnnTree *tree = nullptr;     // tree reused by one-shot kNN entry points
   rvp::VoxelWork *vwork = nullptr;  // voxel scratch of rvp_voxel_grid
+  rvp::DevBuf rand_table;           // the first rand_count values after srand(0)
+  size_t rand_count = 0;
 };
 
 namespace rvp {
@@ -123,6 +125,29 @@ __device__ __forceinline__ float dist2(float px, float py, float pz, float qx,
   const float dx = fsub(px, qx), dy = fsub(py, qy), dz = fsub(pz, qz);
   return fadd(fadd(fmul(dx, dx), fmul(dy, dy)), fmul(dz, dz));
 }
+
+// two single-precision operations at once, each rounded by itself
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+  u64 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+  u64 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+// (a product as fma(a, b, -0): mul.rn.f32x2 is contracted with the add that
+// follows, one rounding for both; the zero comes from a kernel argument
+// (kMinusZero2), so it is no constant to the compiler)
+__device__ __forceinline__ u64 mul2(u64 a, u64 b, u64 minus_zero) {
+  return fma2(a, b, minus_zero);
+}
+__device__ __forceinline__ u64 pack2(float a, float b) {
+  return (u64)__float_as_uint(a) | ((u64)__float_as_uint(b) << 32);
+}
+__device__ __forceinline__ float half2f(u64 v, int i) { return __uint_as_float((u32)(v >> (32 * i))); }
+constexpr u64 kMinusZero2 = 0x8000000080000000ull;
 
 // (d2, idx) packed so that unsigned order == std::pair<float,int> order for
 // d2 >= 0 and idx >= 0 (spatial_hashing.cpp:149-154).
@@ -384,7 +409,7 @@ struct TreeQueries {
   u32 *hard = nullptr;           // (their places in q, or in the tree)
   u32 *longer = nullptr;         // queries with long radius lists
   u32 n = 0;
-  u64 minus_zero = 0x8000000080000000ull;  // two of them
+  u64 minus_zero = kMinusZero2;
 };
 // TREE_MEAN: SOR's mean distance; TREE_PAIRS: rows of k indices and squared
 // distances (-1 and infinity past the found) and counts; TREE_NORMALS /
@@ -517,13 +542,6 @@ struct RansacSampler {
   const double *cdf = nullptr;
   u64 seed = 0;
   const int32_t *targets = nullptr;
-  // given hypotheses instead of drawn ones: n_models planes per frame (a NaN
-  // first coefficient marks an empty slot)
-  const float4 *models = nullptr;
-  int n_models = 0;
-  // start each frame from an earlier best (count and model), not from zero
-  const int32_t *best_in = nullptr;
-  const float *model_in = nullptr;
 };
 // One cluster of `cluster` blocks (1-8, fewer if the device cannot hold them)
 // per frame over SoA clouds; frame f = [off[f], off[f+1]).
@@ -533,6 +551,16 @@ void ransac_frames(rvp_context *ctx, const float *x, const float *y,
                    float *model, int32_t *best, int32_t *iters_run,
                    int32_t *counts_all, bool eval_all,
                    const RansacSampler &smp = RansacSampler{}, int cluster = 1);
+// RANSAC on one cloud over the whole device (the rand() stream; hypotheses
+// past the early stop are counted in part, in rounds): *state afterwards holds
+// the result. scratch: ransac_one_bytes().
+struct RansacState {
+  float4 model;
+  int best, k_iters, stop, iters;
+};
+size_t ransac_one_bytes();
+void ransac_one(rvp_context *ctx, const float *x, const float *y, const float *z, size_t n,
+                const int *rand_dev, const RansacParams &p, RansacState *state, void *scratch);
 // Euclidean clusters of one cloud (cluster.cu): CSR offsets (capacity
 // n + 1) and indices (capacity n) on the device, count in n_clusters_dev.
 // temp: euclidean_temp_bytes(n). Synchronizes.

@@ -544,7 +544,7 @@ void tree_radius_normals(rvp_context *ctx, const TreeView &t, float radius, int 
                          float vpy, float vpz, float *nx, float *ny, float *nz, u32 *hard,
                          u32 *hard_count) {
   RVP_CUDA_TRY(cudaMemsetAsync(hard_count, 0, 4, ctx->stream));
-  k_radius_normals<<<(t.n + 31) / 32, 32, 0, ctx->stream>>>(t, TreeQueries{}.minus_zero, square_of(radius), iters,
+  k_radius_normals<<<(t.n + 31) / 32, 32, 0, ctx->stream>>>(t, kMinusZero2, square_of(radius), iters,
                                                            vpx, vpy, vpz, nx, ny, nz, hard,
                                                            hard_count);
   RVP_LAUNCH_CHECK(ctx);

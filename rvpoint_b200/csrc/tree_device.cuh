@@ -7,24 +7,6 @@
 namespace rvp {
 namespace td {
 
-// two single-precision operations at once, each rounded by itself
-__device__ __forceinline__ u64 add2(u64 a, u64 b) {
-  u64 d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-// (a product as fma(a, b, -0): mul.rn.f32x2 is contracted with the add that
-// follows, one rounding for both; the zero comes from a kernel argument, so it
-// is no constant to the compiler)
-__device__ __forceinline__ u64 mul2(u64 a, u64 b, u64 minus_zero) {
-  u64 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(minus_zero));
-  return d;
-}
-__device__ __forceinline__ u64 pack2(float a, float b) {
-  return (u64)__float_as_uint(a) | ((u64)__float_as_uint(b) << 32);
-}
-__device__ __forceinline__ float half2f(u64 v, int i) { return __uint_as_float((u32)(v >> (32 * i))); }
 // dist2 of two points: p + (-q) is p - q
 __device__ __forceinline__ u64 dist2x2(u64 px, u64 py, u64 pz, u64 nqx, u64 nqy, u64 nqz,
                                         u64 mz) {

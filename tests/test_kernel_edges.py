@@ -179,3 +179,21 @@ def test_collisions_found(gpu_ctx, restatement, primes, collide):
     offs, idx, _ = h.radiusSearchBatch(c.x, c.y, c.z, 0.1)
     o2, i2, _ = restatement.radius_search(c, 0.1, 0.1, p1=primes[0], p2=primes[1])
     assert np.array_equal(offs, o2) and np.array_equal(idx, i2)
+
+
+# RANSAC on one cloud: hypotheses are counted in rounds of 64 to 1024, over
+# chunks of 2048 points, 64 hypotheses at a time; the stop and the libc state
+# are the sequential loop's
+@pytest.mark.parametrize("n,iters", [(3, 5), (50, 1), (2047, 63), (2049, 65), (20_000, 2500),
+                                     (1_700_000, 300)])
+def test_ransac_rounds(gpu_ctx, restatement, n, iters):
+    from oracle import oracle as O
+    from rvpoint_b200 import api
+    c = D.room_cloud(n=max(n, 50), seed=n).subset(np.arange(n))
+    stream = O.libc_rand_stream(3 * iters)
+    best, model, _, _, ran = restatement.ransac_plane(c, 0.01, iters, stream)
+    for kw in ({}, {"rand_stream": stream}):
+        got, m = api.ransac_plane_rvv(c, 0.01, iters, **kw)
+        assert got == best and np.array_equal(bits(m), bits(np.asarray(model, np.float32)))
+    best2, _, _, ran2 = api.ransac_plane_rvv(c, 0.01, iters, return_counts=True)
+    assert best2 == best and ran2 == ran
