@@ -11,8 +11,9 @@
 //           and a rank among the few of the same bin. (A bitonic sort of the
 //           same lists in shared memory took 1855 us of the 2650 us that all
 //           neighbours within 0.5 m of 105k LiDAR points, 20M pairs, cost.)
-//   normals one warp per packet, the lists (radius_normals: 10 to 30 points)
-//           in a column of shared memory per lane, ordered there by rank
+//   normals one warp per packet, the lists (10 to 30 points usually) in a
+//           column of shared memory per lane, ordered there by rank; points
+//           with longer ones go one per warp
 #include <math.h>
 
 #include <algorithm>
@@ -447,7 +448,7 @@ __global__ __launch_bounds__(32) void k_radius_normals(TreeView t, u64 minus_zer
   if (!active) return;
   const u32 qidx = __float_as_uint(q.w);
   if (cnt > RN_CAP) {
-    hard[atomicAdd(hard_count, 1u)] = qidx;
+    hard[atomicAdd(hard_count, 1u)] = qi;
     return;
   }
   float ax = 0.0f, ay = 0.0f, az = 0.0f;
@@ -470,6 +471,45 @@ __global__ __launch_bounds__(32) void k_radius_normals(TreeView t, u64 minus_zer
   nx[qidx] = ax;
   ny[qidx] = ay;
   nz[qidx] = az;
+}
+
+// The points with more neighbours than a lane holds (hard: places in the tree),
+// one warp each; those past FT_CAP neighbours go on to `huge` (indices).
+__global__ __launch_bounds__(32) void k_radius_normals_listed(
+    TreeView t, float r2, int iters, float vpx, float vpy, float vpz, float *nx, float *ny,
+    float *nz, const u32 *hard, const u32 *hard_count, u32 *huge, u32 *huge_count) {
+  __shared__ u64 s_keys[FT_CAP];
+  __shared__ u32 s_bins[FT_BINS], s_near[FT_CAP];
+  __shared__ unsigned short s_perm[FT_CAP];
+  const int lane = threadIdx.x;
+  for (u32 w = blockIdx.x; w < *hard_count; w += gridDim.x) {
+    const float4 q = t.pts[hard[w]];
+    const u32 qidx = __float_as_uint(q.w);
+    u32 cnt = 0;
+    radius_walk<1>(t, q.x, q.y, q.z, r2, 0, [&](bool pass, float d, u32 idx) {
+      const unsigned b = __ballot_sync(0xffffffffu, pass);
+      const u32 at = cnt + __popc(b & ((1u << lane) - 1));
+      if (pass && at < FT_CAP) s_keys[at] = pack_nbr(d, (int)idx);
+      cnt += __popc(b);
+    });
+    __syncwarp();
+    if (cnt > FT_CAP) {
+      if (lane == 0) huge[atomicAdd(huge_count, 1u)] = qidx;
+      continue;
+    }
+    order_keys<32, FT_BINS>(s_keys, cnt, r2, s_bins, s_perm, nullptr,
+                            [&](u32 rank, u64 k) { s_near[rank] = t.pos_of[nbr_idx(k)]; });
+    __syncwarp();
+    if (lane == 0) {
+      float ax, ay, az;
+      nd::normal_from_points([&](int j) { return __ldg(&t.pts[s_near[j]]); }, (int)cnt, false,
+                             iters, q.x, q.y, q.z, vpx, vpy, vpz, ax, ay, az);
+      nx[qidx] = ax;
+      ny[qidx] = ay;
+      nz[qidx] = az;
+    }
+    __syncwarp();
+  }
 }
 
 // listed queries: their coordinates
@@ -542,11 +582,14 @@ void tree_radius_fill(rvp_context *ctx, const TreeView &t, const TreeQueries &q,
 
 void tree_radius_normals(rvp_context *ctx, const TreeView &t, float radius, int iters, float vpx,
                          float vpy, float vpz, float *nx, float *ny, float *nz, u32 *hard,
-                         u32 *hard_count) {
-  RVP_CUDA_TRY(cudaMemsetAsync(hard_count, 0, 4, ctx->stream));
-  k_radius_normals<<<(t.n + 31) / 32, 32, 0, ctx->stream>>>(t, kMinusZero2, square_of(radius), iters,
-                                                           vpx, vpy, vpz, nx, ny, nz, hard,
-                                                           hard_count);
+                         u32 *huge, u32 *counts) {
+  const float r2 = square_of(radius);
+  RVP_CUDA_TRY(cudaMemsetAsync(counts, 0, 8, ctx->stream));
+  k_radius_normals<<<(t.n + 31) / 32, 32, 0, ctx->stream>>>(t, kMinusZero2, r2, iters, vpx, vpy,
+                                                           vpz, nx, ny, nz, hard, counts);
+  RVP_LAUNCH_CHECK(ctx);
+  k_radius_normals_listed<<<grid_for(t.n, 1, ctx->num_sms * 14), 32, 0, ctx->stream>>>(
+      t, r2, iters, vpx, vpy, vpz, nx, ny, nz, hard, counts, huge, counts + 1);
   RVP_LAUNCH_CHECK(ctx);
 }
 
