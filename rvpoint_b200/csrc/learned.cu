@@ -600,8 +600,9 @@ __global__ __launch_bounds__(FWD_THREADS) void k_mlp_forward(const float *__rest
 // and dW1 = delta1^T X as MMAs over the iteration's 64 points, accumulated in
 // registers across iterations; the vector entries are added in warp order.
 // Every gradient entry of a block is written by one thread, and the blocks'
-// shares are added in block order afterwards (k_grad_reduce): the same batch
-// always gives the same gradient.
+// shares are added in a fixed order afterwards (k_grad_reduce): the same batch
+// always gives the same gradient. Two blocks per SM: an iteration is a chain
+// of small steps, bound by their latency.
 // ---------------------------------------------------------------------------
 constexpr int TB = 128;                 // threads per training block
 constexpr int TP = 64;                  // points per block iteration
@@ -872,18 +873,34 @@ __global__ __launch_bounds__(TB) void k_mlp_train(const float *__restrict__ feat
   }
 }
 
-// the blocks' gradient shares and losses, added in block order
-__global__ void k_grad_reduce(const float *part, const double *part_loss, int blocks, float *grad,
-                              double *loss_sum) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < NP; p += gridDim.x * blockDim.x) {
-    float t = 0.0f;
-    for (int b = 0; b < blocks; ++b) t += part[(size_t)b * NP + p];
+// The blocks' gradient shares and losses, added up: 32 entries per block of
+// threads, eight runs of consecutive shares each, the runs in order. (A thread
+// per entry over all 148 shares took 17 us, one load after the other.)
+constexpr int GR_RUNS = 8;
+__global__ __launch_bounds__(32 * GR_RUNS) void k_grad_reduce(const float *part,
+                                                              const double *part_loss, int blocks,
+                                                              float *grad, double *loss_sum) {
+  __shared__ float run[GR_RUNS][32];
+  const int lane = threadIdx.x & 31, r = threadIdx.x >> 5, p = blockIdx.x * 32 + lane;
+  const int per = (blocks + GR_RUNS - 1) / GR_RUNS, b1 = min(blocks, (r + 1) * per);
+  float t = 0.0f;
+  if (p < NP) {
+#pragma unroll 8
+    for (int b = r * per; b < b1; ++b) t += part[(size_t)b * NP + p];
+  }
+  run[r][lane] = t;
+  __syncthreads();
+  if (r == 0 && p < NP) {
+#pragma unroll
+    for (int q = 1; q < GR_RUNS; ++q) t += run[q][lane];
     grad[p] = t;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    double t = 0.0;
-    for (int b = 0; b < blocks; ++b) t += part_loss[b];
-    *loss_sum = t;
+  if (blockIdx.x == 0 && r == 1) {
+    double l = 0.0;
+    for (int b = lane; b < blocks; b += 32) l += part_loss[b];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    if (lane == 0) *loss_sum = l;
   }
 }
 
@@ -1282,7 +1299,7 @@ void mlp_grad(rvp_scorer *s, const float *features, const float *labels, size_t 
               size_t n_src = 0, u64 sample_seed = 0) {
   rvp_context *ctx = s->ctx;
   const unsigned blocks =
-      (unsigned)std::min<size_t>((n + rvp::TP - 1) / rvp::TP, (size_t)ctx->num_sms);
+      (unsigned)std::min<size_t>((n + rvp::TP - 1) / rvp::TP, 2 * (size_t)ctx->num_sms);
   s->gpart.reserve((size_t)blocks * rvp::NP * 4 + (size_t)blocks * 8 + 256);
   float *part = s->gpart.as<float>();
   double *part_loss = reinterpret_cast<double *>(
@@ -1291,7 +1308,7 @@ void mlp_grad(rvp_scorer *s, const float *features, const float *labels, size_t 
       features, labels, n, n_src ? n_src : n, sample_seed, s->wq.as<__nv_bfloat16>(),
       s->norm.as<float>(), part, part_loss);
   RVP_LAUNCH_CHECK(ctx);
-  rvp::k_grad_reduce<<<(rvp::NP + 255) / 256, 256, 0, ctx->stream>>>(
+  rvp::k_grad_reduce<<<(rvp::NP + 31) / 32, 32 * rvp::GR_RUNS, 0, ctx->stream>>>(
       part, part_loss, (int)blocks, s->grad.as<float>(), s->loss.as<double>());
   RVP_LAUNCH_CHECK(ctx);
 }
