@@ -407,6 +407,15 @@ void cloud_bbox(rvp_context *ctx, const float *x, const float *y, const float *z
   RVP_LAUNCH_CHECK(ctx);
 }
 
+void frames_bbox(rvp_context *ctx, const float *x, const float *y, const float *z,
+                 const int64_t *offs, int n_frames, size_t n_max, float *bb) {
+  k_bbox_init<<<grid_for(n_frames, 256, 64), 256, 0, ctx->stream>>>(bb, n_frames);
+  RVP_LAUNCH_CHECK(ctx);
+  k_bbox<<<grid_for(n_max, 256, ctx->num_sms * kBoxBlocks), 256, 0, ctx->stream>>>(
+      x, y, z, offs, n_frames, n_max, reinterpret_cast<const u64 *>(offs + n_frames), bb);
+  RVP_LAUNCH_CHECK(ctx);
+}
+
 void grid_build(rvp_context *ctx, Grid &g, const float *x, const float *y, const float *z,
                 const int64_t *offs, int n_frames, size_t n_points, float cell, int mode,
                 long long p1, long long p2, const u64 *n_dev_opt, int base_level,

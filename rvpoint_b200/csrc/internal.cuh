@@ -369,6 +369,8 @@ bool normals_from_sor_lists(rvp_context *ctx, const GridView &g, const TileArgs 
                             int kn);
 bool grid_knn_tile(rvp_context *ctx, const GridView &g, int k, int mode, const TileArgs &a,
                    int blocks, u32 *stats = nullptr);
+// the positions whose qlevel is `level`, in order: a.open_list, a.open_n
+void list_open(rvp_context *ctx, const u64 *n_points, int level, const TileArgs &a);
 // The hard slots that carry a bound tau (TileArgs::hard, hard_tau; n_hard on
 // the device): one thread per slot scans the tight window of sqrt(tau) at the
 // finest level where it spans at most 27 cells -- exact, since at least K
@@ -399,7 +401,12 @@ struct TreeView {  // what the search reads
   float *box[kTreeLevels];    // per level: lo x, y, z, hi x, y, z (stride each)
   u32 stride[kTreeLevels];
   u32 count[kTreeLevels];     // nodes per level (level 0: leaves of 32 points)
-  u32 n;
+  u32 n;                      // points (positions, with frames)
+  // many frames (knn_tree_frames.cu): the frame of each level-1 node (or
+  // 0xFFFFFFFF), each frame's nodes (first, end), the positions in use
+  const u32 *node_frame;
+  const uint2 *frame_nodes;
+  const u64 *n_positions;
 };
 struct TreeQueries {
   const float4 *q = nullptr;     // {x, y, z, index} in key order
@@ -408,13 +415,16 @@ struct TreeQueries {
   u32 *hard_count = nullptr;     // queries left for the warp-per-query kernel
   u32 *hard = nullptr;           // (their places in q, or in the tree)
   u32 *longer = nullptr;         // queries with long radius lists
+  const u32 *list = nullptr;     // with frames: these positions only
+  const u64 *n_list = nullptr;
   u32 n = 0;
   u64 minus_zero = kMinusZero2;
 };
 // TREE_MEAN: SOR's mean distance; TREE_PAIRS: rows of k indices and squared
 // distances (-1 and infinity past the found) and counts; TREE_NORMALS /
 // TREE_PRECISE: normals of the k nearest (k <= n)
-enum TreeMode { TREE_MEAN = 0, TREE_PAIRS = 1, TREE_NORMALS = 2, TREE_PRECISE = 3 };
+// TREE_LIST (frames): the mean and rows of k tree positions, by position
+enum TreeMode { TREE_MEAN = 0, TREE_PAIRS = 1, TREE_NORMALS = 2, TREE_PRECISE = 3, TREE_LIST = 4 };
 struct TreeOut {  // by query index; null pointers are skipped
   float *mean = nullptr;
   bool radius_mode = false;
@@ -428,9 +438,12 @@ struct TreeOut {  // by query index; null pointers are skipped
   double cond_fp64 = 0.0;
   float *cond = nullptr;
   uint8_t *used64 = nullptr;
+  u32 *rows = nullptr;
+  const u64 *out_pos = nullptr;  // where a point's normal goes (null: its index)
 };
 struct KnnTree {
   DevBuf keys, vals, sort, pts, pos, boxes, misc, qkeys, qvals, qpts, hard;
+  void reserve_frames(size_t n_max, int n_frames);
   void release();
 };
 TreeView tree_build(rvp_context *ctx, KnnTree &w, const float *x, const float *y, const float *z,
@@ -445,6 +458,19 @@ TreeQueries tree_queries_as_given(rvp_context *ctx, KnnTree &w, size_t nq);
 // radius > 0: neighbours with d2 <= radius * radius only
 void tree_knn(rvp_context *ctx, const TreeView &t, const TreeQueries &q, int k, float radius,
               int mode, const TreeOut &o);
+// The tree of a batch's frames (points by x, y, z and interleaved; offsets and
+// counts on the device), its positions for n_max points, the marking of
+// removed points (keep by index), and the search for every point (list null)
+// or the listed positions. keys, vals, sort_temp: room for n_max (sort_temp_bytes).
+size_t tree_frames_positions(size_t n_max, int n_frames);
+TreeView tree_build_frames(rvp_context *ctx, KnnTree &w, const float *x, const float *y,
+                           const float *z, const float *aos, const int64_t *offs, int n_frames,
+                           size_t n_max, u64 *keys, u32 *vals, void *sort_temp);
+void tree_frames_mark_removed(rvp_context *ctx, const TreeView &t, const uint8_t *keep);
+void tree_knn_frames(rvp_context *ctx, KnnTree &w, const TreeView &t, const u32 *list,
+                     const u64 *n_list, int k, int mode, const TreeOut &o);
+void frames_bbox(rvp_context *ctx, const float *x, const float *y, const float *z,
+                 const int64_t *offs, int n_frames, size_t n_max, float *bb);
 // radius searches over the tree (radius_tree.cu). *flag = 1: cells of the hash
 // may share a key (or the check cannot tell)
 void hash_collision_check(rvp_context *ctx, const TreeView &t, float cell, long long p1,

@@ -1589,6 +1589,16 @@ bool normals_from_sor_lists(rvp_context *ctx, const GridView &g, const TileArgs 
   return true;
 }
 
+void list_open(rvp_context *ctx, const u64 *n_points, int level, const TileArgs &a) {
+  const unsigned gb = grid_for(a.n_max, 256, ctx->num_sms * 16);
+  k_open_flags<<<gb, 256, 0, ctx->stream>>>(a.qlevel, n_points, level, a.open_flags);
+  RVP_LAUNCH_CHECK(ctx);
+  exclusive_scan_u32_to_u64(ctx, a.open_flags, a.open_pos, a.n_max, n_points, a.scan_tmp);
+  k_open_scatter<<<gb, 256, 0, ctx->stream>>>(a.open_flags, a.open_pos, n_points, a.open_list,
+                                              a.open_n);
+  RVP_LAUNCH_CHECK(ctx);
+}
+
 bool grid_knn_tau(rvp_context *ctx, const GridView &g, int k, int mode, const TileArgs &a,
                   const u64 *n_hard, u64 *slot_pairs, int32_t *slot_counts, u32 *stats) {
   if (g.mode != KEY_DENSE || !a.hard || !a.hard_tau) return false;

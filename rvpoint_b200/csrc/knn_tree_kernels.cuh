@@ -1,0 +1,716 @@
+// Kernels of the box tree (knn_tree.cu, knn_tree_frames.cu): keys, boxes and
+// the search for the k nearest.
+#pragma once
+
+#include <float.h>
+#include <math.h>
+
+#include "grid_device.cuh"
+#include "internal.cuh"
+#include "normals_device.cuh"
+#include "tree_device.cuh"
+
+namespace rvp {
+using namespace gd;
+using namespace td;
+
+namespace {
+constexpr int kTreeKeyBits = 32;
+
+struct TreeFrame {  // the quantisation of the cloud's box
+  float lo[3];
+  float inv;    // cells per unit (a power of two)
+  int bits[3];  // of each axis
+};
+
+// the finest power-of-two cell whose codes fit `key_bits`
+__device__ __forceinline__ void tree_frame(const float *bb, int key_bits, TreeFrame &F) {
+  float ext[3], emax = 0.0f;
+  for (int a = 0; a < 3; ++a) {
+    const float lo = bb[a], hi = bb[3 + a];
+    F.lo[a] = lo < INFINITY && lo > -INFINITY ? lo : 0.0f;
+    float e = fsub(hi, lo);
+    e = e > 0.0f ? fminf(e, 1e30f) : 0.0f;  // (NaN and empty axes: one cell)
+    ext[a] = e;
+    emax = fmaxf(emax, e);
+  }
+  int k = emax > 0.0f ? ilogbf(emax) - key_bits : -60;
+  k = max(k, -100);
+  for (;; ++k) {
+    int sum = 0;
+    for (int a = 0; a < 3; ++a) {
+      const float q = ldexpf(ext[a], -k);  // cells along the axis
+      F.bits[a] = q < 1.0f ? 0 : ilogbf(q) + 1;
+      sum += F.bits[a];
+    }
+    if (sum <= key_bits) break;
+  }
+  F.inv = ldexpf(1.0f, -k);
+}
+
+__device__ __forceinline__ u32 tree_key(const TreeFrame &F, float x, float y, float z) {
+  const float v[3] = {x, y, z};
+  u32 q[3];
+  int top = 0;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const float t = fmul(fsub(v[a], F.lo[a]), F.inv);
+    const u32 last = F.bits[a] >= 32 ? 0xFFFFFFFFu : (1u << F.bits[a]) - 1u;
+    q[a] = t > 0.0f ? (t < 4.0e9f ? min((u32)t, last) : last) : 0u;
+    top = max(top, F.bits[a]);
+  }
+  // Compact Hilbert index (C. Hamilton, A. Rau-Chaplin, "Compact Hilbert
+  // indices", 2008): per level the Gray code rank of the point's octant in the
+  // frame of the entry e and direction d, over the axes that have this bit.
+  // Consecutive codes are neighbouring cells (but for a few jumps where an
+  // axis has run out of bits), so a leaf's box is small: with Morton codes
+  // packets tested 19 to 41 leaves, one that spans a jump all of a large box.
+  constexpr u32 kGray = 0x54672310u, kEntry = 0x56633000u, kDir = 0x01122110u;
+  auto rotr = [](u32 v, u32 k) { return ((v >> k) | (v << (3 - k))) & 7u; };
+  u32 key = 0, e = 0, d = 0;
+  for (int b = top - 1; b >= 0; --b) {
+    const u32 mask = (b < F.bits[0] ? 1u : 0u) | (b < F.bits[1] ? 2u : 0u) |
+                     (b < F.bits[2] ? 4u : 0u);
+    const u32 l = ((q[0] >> b) & 1u) | (((q[1] >> b) & 1u) << 1) | (((q[2] >> b) & 1u) << 2);
+    const u32 k = d == 2 ? 0 : d + 1;
+    const u32 w = (kGray >> (4 * rotr(l ^ e, k))) & 7u;
+    const u32 mu = rotr(mask, k);
+    if (mu & 4u) key = (key << 1) | (w >> 2);
+    if (mu & 2u) key = (key << 1) | ((w >> 1) & 1u);
+    if (mu & 1u) key = (key << 1) | (w & 1u);
+    e ^= rotr((kEntry >> (4 * w)) & 7u, 3 - k);
+    d += ((kDir >> (4 * w)) & 7u) + 1;
+    d = d >= 3 ? d - 3 : d;
+  }
+  return key;
+}
+
+// box reduction over a warp; lane 0 writes node `c` of a level
+__device__ __forceinline__ void box_out(float (&m)[6], float *box, u32 stride, u32 c) {
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      const float t = __shfl_xor_sync(0xffffffffu, m[k], o);
+      m[k] = k < 3 ? fminf(m[k], t) : fmaxf(m[k], t);
+    }
+  }
+  if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) box[(size_t)k * stride + c] = m[k];
+  }
+}
+
+// one warp per node of the next level: the box of up to 32 children
+__device__ __forceinline__ void parent_box(const float *kid, u32 kid_stride, u32 kids, float *box,
+                                           u32 stride, u32 c) {
+  const u32 i = c * 32 + (threadIdx.x & 31);
+  float m[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  if (i < kids) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) m[k] = kid[(size_t)k * kid_stride + i];
+  }
+  box_out(m, box, stride, c);
+}
+
+// ---------------------------------------------------------------------------
+// search
+// ---------------------------------------------------------------------------
+// Walks every leaf within limit() of the box q, nearest child first. All
+// lanes take part; limit() is uniform and may shrink on the way.
+template <int LV, class Limit, class Leaf>
+__device__ __forceinline__ void tree_walk(const TreeView &t, const Box &q, u32 first, u32 end,
+                                          Limit &limit, Leaf &leaf) {
+  const int lane = threadIdx.x & 31;
+  const u32 c = first + lane;
+  const float lb = c < end ? box_d2(q, t.box[LV], t.stride[LV], c) : 0.0f;
+  bool open = c < end && lb <= limit();
+  while (true) {
+    // (the low bits of the distance give way to the lane)
+    const u32 key = open ? (__float_as_uint(lb) & ~31u) | lane : 0xFFFFFFFFu;
+    const u32 best = __reduce_min_sync(0xffffffffu, key);
+    if (best == 0xFFFFFFFFu) break;
+    const int s = best & 31;
+    if (lane == s) open = false;
+    if (__uint_as_float(best & ~31u) > limit()) break;  // and so are all that are left
+    if (__shfl_sync(0xffffffffu, lb, s) > limit()) continue;
+    if constexpr (LV == 0) leaf(first + s);
+    else tree_walk<LV - 1>(t, q, (first + s) * 32, t.count[LV - 1], limit, leaf);
+  }
+}
+// The nodes a search starts from: one cloud's top level (at most 32 nodes up to
+// 33.5M points), or a frame's level-1 nodes; 32 at a time.
+struct Roots {
+  u32 first, end;
+};
+template <bool FRAMES>
+constexpr int tree_top() { return FRAMES ? 1 : kTreeLevels - 1; }
+template <bool FRAMES, class Limit, class Leaf>
+__device__ __forceinline__ void tree_walk_all(const TreeView &t, const Roots &r, const Box &q,
+                                              Limit &limit, Leaf &leaf) {
+  for (u32 f = r.first; f < r.end; f += 32)
+    tree_walk<tree_top<FRAMES>()>(t, q, f, r.end, limit, leaf);
+}
+
+// The same walk leaf by leaf, for a caller whose leaf code is too long to be
+// inlined more than once (it would not fit the instruction cache).
+// element l of v without an index (v stays in registers)
+template <int N, class A>
+__device__ __forceinline__ auto by_level(const A &v, int l) {
+  auto r = v[0];
+#pragma unroll
+  for (int i = 1; i < N; ++i) r = i == l ? v[i] : r;
+  return r;
+}
+template <int N, class T>
+__device__ __forceinline__ void set_level(T (&v)[N], int l, T x) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = i == l ? x : v[i];
+}
+
+template <int TOP>
+struct TreeWalk {
+  static constexpr int N = TOP + 1;
+  float lb[N];   // per level: the lane's child's distance
+  u32 open[N];   // children left (a mask, uniform)
+  u32 first[N];  // their numbers start here
+  int level;     // where the walk stands
+  u32 top, end;  // the next group of top nodes, and their end
+  __device__ __forceinline__ void begin(const Roots &r) {
+    level = N;
+    top = r.first;
+    end = r.end;
+#pragma unroll
+    for (int l = 0; l < N; ++l) {
+      lb[l] = 0.0f;
+      open[l] = first[l] = 0;
+    }
+  }
+  // the next leaf within `limit` of q; false at the end
+  __device__ __forceinline__ bool next(const TreeView &t, const Box &q, float limit, u32 &leaf) {
+    const int lane = threadIdx.x & 31;
+    while (true) {
+      u32 f = top;
+      int to = TOP;
+      if (level == N) {
+        if (top >= end) return false;
+        top += 32;
+      } else {
+        const u32 mask = by_level<N>(open, level);
+        const float v = by_level<N>(lb, level);
+        // (the low bits of the distance give way to the lane)
+        const u32 best = __reduce_min_sync(
+            0xffffffffu,
+            (mask >> lane) & 1u ? (__float_as_uint(v) & ~31u) | lane : 0xFFFFFFFFu);
+        if (best == 0xFFFFFFFFu || __uint_as_float(best & ~31u) > limit) {  // none near enough
+          ++level;
+          continue;
+        }
+        const int s = best & 31;
+        set_level<N>(open, level, mask & ~(1u << s));
+        if (__shfl_sync(0xffffffffu, v, s) > limit) continue;
+        f = by_level<N>(first, level) + s;
+        if (level == 0) {
+          leaf = f;
+          return true;
+        }
+        f *= 32;
+        to = level - 1;
+      }
+      const u32 c = f + lane, n = to == TOP ? end : by_level<N>(t.count, to);
+      const float d =
+          c < n ? box_d2(q, by_level<N>(t.box, to), by_level<N>(t.stride, to), c) : 0.0f;
+      set_level<N>(lb, to, d);
+      set_level<N>(open, to, __ballot_sync(0xffffffffu, c < n && d <= limit));
+      set_level<N>(first, to, f);
+      level = to;
+    }
+  }
+};
+
+constexpr int kTreeBuf = 64;   // buffered distances per lane, flushed above 32
+constexpr int kTreeExtra = 3;  // collected points past the list, for equal distances
+// a query joins its packet's walk if its limit (a squared distance) is within
+// this factor of the median one
+constexpr float kLoner = 16.0f;
+// leaves a packet tests before it gives up: one with points far apart has every
+// leaf of a large box to test (milliseconds, with no other work left to hide
+// them), most test 20 to 40
+constexpr int kLeafBudget = 128;
+
+// shared memory of a packet: the staged leaf, the leaves scanned, the buffered
+// distances and later (in the same place) the collected points, and the
+// positions in order where a normal follows
+constexpr int kTreeLeaves = (kLeafBudget + 3 + 3) & ~3;
+template <int KCAP, int MODE>
+constexpr size_t tree_buffer() {
+  constexpr size_t dist = (size_t)kTreeBuf * 32 * 4;
+  constexpr size_t near = (size_t)(KCAP + kTreeExtra) * 32 * 8;
+  return MODE != TREE_MEAN && near > dist ? near : dist;
+}
+template <int KCAP, int MODE>
+constexpr size_t tree_smem() {
+  return 3 * 32 * 4 + kTreeLeaves * 4 + tree_buffer<KCAP, MODE>() +
+         (MODE == TREE_NORMALS || MODE == TREE_PRECISE ? (size_t)(KCAP + 1) * 32 * 4 : 0);
+}
+
+// Compare-exchange networks over registers. They are straight code: batches of
+// 32 took fewer steps than 16, but the kernel then waited for instructions
+// (4.7 of 9 cycles per issue).
+__device__ __forceinline__ void order2(float &a, float &b) {
+  const float l = fminf(a, b), h = fmaxf(a, b);
+  a = l;
+  b = h;
+}
+template <int N>
+__device__ __forceinline__ void bitonic_merge(float (&v)[N]) {
+#pragma unroll
+  for (int j = N / 2; j > 0; j >>= 1) {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if ((i ^ j) > i) order2(v[i], v[i ^ j]);
+  }
+}
+template <int N>
+__device__ __forceinline__ void bitonic_sort(float (&v)[N]) {
+#pragma unroll
+  for (int k = 2; k <= N; k <<= 1) {
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) {
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        const int l = i ^ j;
+        if (l > i) {
+          if ((i & k) == 0) order2(v[i], v[l]);
+          else order2(v[l], v[i]);
+        }
+      }
+    }
+  }
+}
+
+// sor_sc's mean (statistical_outlier_removal.cpp:36-40): the ascending sum of
+// sqrtf(d2_j), j = 1 .. k, over k; within a radius over those found, and the
+// radius itself for a point without neighbours (:246-270)
+__device__ __forceinline__ void tree_mean_out(float sum, int have, const float4 &q, u32 qidx,
+                                              const TreeOut &o) {
+  float m = have > 1 ? fdiv(sum, (float)(have - 1)) : 0.0f;
+  if (o.radius_mode && have <= 1) m = o.fallback;
+  const float none = dist2(q.x, q.y, q.z, q.x, q.y, q.z);  // NaN without a position
+  o.mean[qidx] = none == 0.0f ? m : none;
+}
+
+// the normal of a query from its sorted neighbours nbr(0 .. have - 1)
+template <int MODE, class Nbr>
+__device__ __forceinline__ void tree_normal_out(Nbr nbr, int have, const float4 &q, u32 qidx,
+                                                const TreeOut &o) {
+  float nx = 0.0f, ny = 0.0f, nz = 0.0f;
+  if constexpr (MODE == TREE_NORMALS) {
+    if (have >= 3)
+      nd::normal_from_points(nbr, have, true, o.iters, q.x, q.y, q.z, o.vpx, o.vpy, o.vpz, nx, ny,
+                             nz);
+  } else {
+    float cond;
+    bool wide;
+    nd::precise_normal(nbr, have, q.x, q.y, q.z, o.vpx, o.vpy, o.vpz, o.cond_fp64, nx, ny, nz,
+                       cond, wide);
+    if (o.cond) o.cond[qidx] = cond;
+    if (o.used64) o.used64[qidx] = wide ? 1 : 0;
+  }
+  const size_t at = o.out_pos ? (size_t)o.out_pos[qidx] : (size_t)qidx;
+  o.nx[at] = nx;
+  o.ny[at] = ny;
+  o.nz[at] = nz;
+}
+
+// One warp (block) per packet of 32 queries. The list holds the K nearest, or
+// for the cloud's own points the K - 1 nearest others (the point itself, at
+// distance 0, is the first of its row); KCAP is at least that, a power of two.
+// FRAMES: a tree of many frames (tree_build_frames), whose own points, all or
+// those listed, are the queries.
+template <int KCAP, int MODE, bool FRAMES>
+__global__ __launch_bounds__(32, KCAP > 32 ? 10 : 16) void k_knn_tree(TreeView t, TreeQueries qs,
+                                                                      int K, float bound,
+                                                                      TreeOut o) {
+  extern __shared__ __align__(16) unsigned char tree_sm[];
+  constexpr bool MEAN = MODE == TREE_MEAN;  // distances only
+  constexpr int PCAP = KCAP + kTreeExtra;
+  constexpr int SORTED = KCAP < 16 ? KCAP : 16;  // distances sorted at once
+  float(*stage)[32] = reinterpret_cast<float(*)[32]>(tree_sm);  // x, y, z
+  u32 *leaves = reinterpret_cast<u32 *>(tree_sm + 384);
+  unsigned char *buf = tree_sm + 384 + kTreeLeaves * 4;
+  float(*fbuf)[32] = reinterpret_cast<float(*)[32]>(buf);
+  uint2(*pbuf)[32] = reinterpret_cast<uint2(*)[32]>(buf);
+  u32(*sorted)[32] = reinterpret_cast<u32(*)[32]>(buf + tree_buffer<KCAP, MODE>());
+  const int lane = threadIdx.x;
+  const u32 packet = blockIdx.x;
+  // the cloud's own points (leaf `packet`), or 32 of the sorted queries
+  const bool self = FRAMES || qs.n_sort == nullptr || *qs.n_sort == 0;
+  const float4 *src = self ? t.pts : qs.q;
+  u32 qi = packet * 32 + lane, start = packet;
+  bool active = qi < qs.n, mine = active;  // (mine: answered with the packet)
+  Roots roots{0, t.count[kTreeLevels - 1]};
+  u32 leaf0 = 0, leaf1 = t.count[0] - 1;  // the leaves there are
+  if constexpr (FRAMES) {
+    if (qs.list) {
+      const u64 n = *qs.n_list;
+      if (packet * 32 >= n) return;
+      active = qi < n;
+      qi = qs.list[active ? qi : packet * 32];
+      start = __shfl_sync(0xffffffffu, qi, 0) / 32;
+    }
+    const u32 frame = t.node_frame[start / 32];
+    if (frame == 0xFFFFFFFFu) return;
+    active = active && !(__float_as_uint(src[qi].w) & kRemovedBit);  // (or no point at all)
+    if (!__any_sync(0xffffffffu, active)) return;
+    mine = active && t.node_frame[qi / 1024] == frame;
+    const uint2 nodes = t.frame_nodes[frame];
+    roots = Roots{nodes.x, nodes.y};
+    leaf0 = nodes.x * 32;
+    leaf1 = nodes.y * 32 - 1;
+  } else if (!self) {
+    start = leaf_of_key(t, qs.keys[min(packet * 32 + 16, qs.n - 1)]);
+  }
+  const float4 q = src[FRAMES || active ? qi : packet * 32];
+  const u32 qidx = __float_as_uint(q.w) & (FRAMES ? 0x7FFFFFFFu : 0xFFFFFFFFu);
+  const Box own{{q.x, q.y, q.z}, {q.x, q.y, q.z}};
+
+  // ---- the sorted distances: slots 0 .. pad - 1 hold -1 and never move
+  const bool drop = self && K > 1;  // the point itself is not in the list
+  const int KL = drop ? K - 1 : K, pad = KCAP - KL;
+  float L[KCAP];
+#pragma unroll
+  for (int j = 0; j < KCAP; ++j) L[j] = j < pad ? -1.0f : INFINITY;
+  int cnt = 0;  // buffered distances
+  float lim = -1.0f, pmax = -1.0f;  // what the buffer takes: d2 <= lim; its largest
+  auto limits = [&]() {
+    lim = mine ? fminf(fminf(L[KCAP - 1], bound), FLT_MAX) : -1.0f;
+    pmax = __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(lim)));
+  };
+  limits();
+  auto flush = [&]() {
+    const int most = __reduce_max_sync(0xffffffffu, cnt);
+    int i = 0;
+    // a sorted batch merged at once; the last few one by one
+    for (; i + SORTED / 4 < most; i += SORTED) {
+      float S[SORTED];
+#pragma unroll
+      for (int j = 0; j < SORTED; ++j) S[j] = i + j < cnt ? fbuf[i + j][lane] : INFINITY;
+      bitonic_sort<SORTED>(S);
+#pragma unroll
+      for (int j = 0; j < SORTED; ++j)
+        L[KCAP - SORTED + j] = fminf(L[KCAP - SORTED + j], S[SORTED - 1 - j]);
+      bitonic_merge<KCAP>(L);
+    }
+    for (; i < most; ++i) {
+      const float key = i < cnt ? fbuf[i][lane] : INFINITY;
+#pragma unroll
+      for (int j = KCAP - 1; j > 0; --j) L[j] = fmaxf(L[j - 1], fminf(L[j], key));
+      L[0] = fminf(L[0], key);
+    }
+    cnt = 0;
+    limits();
+  };
+  int scanned = 0, budget = kLeafBudget;
+  auto stage_leaf = [&](u32 l, float at, const float4 &mate) {
+    if (!__any_sync(0xffffffffu, at >= 0.0f)) return false;
+    __syncwarp();
+    stage[0][lane] = mate.x;
+    stage[1][lane] = mate.y;
+    stage[2][lane] = mate.z;
+    __syncwarp();
+    return true;
+  };
+  const u64 nqx = pack2(-q.x, -q.x), nqy = pack2(-q.y, -q.y), nqz = pack2(-q.z, -q.z);
+  // hit(c, d2) for the staged points c within `at`, except `skip`
+  auto test_staged = [&](float at, int skip, auto &&hit) {
+#pragma unroll 2
+    for (int c = 0; c < 32; c += 4) {
+      const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(&stage[0][c]);
+      const ulonglong2 y = *reinterpret_cast<const ulonglong2 *>(&stage[1][c]);
+      const ulonglong2 z = *reinterpret_cast<const ulonglong2 *>(&stage[2][c]);
+      const u64 a = dist2x2(x.x, y.x, z.x, nqx, nqy, nqz, qs.minus_zero);
+      const u64 b = dist2x2(x.y, y.y, z.y, nqx, nqy, nqz, qs.minus_zero);
+      const float d[4] = {half2f(a, 0), half2f(a, 1), half2f(b, 0), half2f(b, 1)};
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (d[u] <= at && c + u != skip) hit(c + u, d[u]);
+    }
+  };
+  auto mate_of = [&](u32 l) {  // the lane's point of leaf l
+    const u32 i = l * 32 + lane;
+    return i < t.n ? __ldg(&t.pts[i]) : make_float4(INFINITY, INFINITY, INFINITY, 0.0f);
+  };
+  auto scan_leaf = [&](u32 l) {
+    if (--budget < 0) {  // (uniform) nothing is left open: the walk ends
+      mine = false;
+      pmax = -1.0f;
+      return;
+    }
+    const float4 mate = mate_of(l);
+    const float at = box_d2(own, t.box[0], t.stride[0], l) <= lim ? lim : -1.0f;
+    if (!stage_leaf(l, at, mate)) return;
+    leaves[scanned++] = l;
+    const int skip = drop && l == qi / 32 ? (int)(qi & 31) : -1;  // the point itself
+    float *to = &fbuf[cnt][lane];
+    test_staged(at, skip, [&](int, float d) {
+      *to = d;
+      to += 32;
+    });
+    cnt = (int)(to - &fbuf[0][lane]) >> 5;
+  };
+  // the leaves around the packet's place first (they set the limits), then
+  // the walk
+  const u32 s0 = start > leaf0 ? start - 1 : leaf0, s1 = min(start + 1, leaf1);
+  const int near = (int)(s1 - s0) + 1;
+  Box pk{};  // the box of the packet
+  TreeWalk<tree_top<FRAMES>()> walk;
+  walk.begin(roots);
+  for (int step = 0;; ++step) {
+    bool more = true;
+    u32 l = step == 0 ? start : (step == 1 && s0 < start ? s0 : s1);
+    if (step >= near) more = walk.next(t, pk, pmax, l);
+    if (more && (step < near || l < s0 || l > s1)) scan_leaf(l);
+    if (!more || step == 0 || step == near - 1 || __any_sync(0xffffffffu, cnt > kTreeBuf - 32))
+      flush();
+    if (!more) break;
+    if (step != near - 1) continue;
+    // A query whose limit is far above the others' (four times the median
+    // radius) would take the packet through all the leaves around it
+    int rank = 0;
+    for (int i = 0; i < 32; ++i) {
+      const float other = __shfl_sync(0xffffffffu, mine ? lim : INFINITY, i);
+      rank += other < lim || (other == lim && i < lane) ? 1 : 0;
+    }
+    const unsigned mid = __ballot_sync(0xffffffffu, mine && rank == 16);
+    if (mid) {
+      const float ref = __shfl_sync(0xffffffffu, lim, __ffs(mid) - 1);
+      mine = mine && lim <= kLoner * ref;
+      limits();
+    }
+    pk = warp_box(q, mine);
+  }
+
+  // ---- results of the packet
+  bool exact = mine;
+  int have = 0;  // distances in the list
+  float sum = 0.0f;
+  if constexpr (MEAN || MODE == TREE_LIST) {
+    // (without a radius they are all there, some infinitely far perhaps)
+    bool first = !drop;  // the nearest of all does not count
+#pragma unroll
+    for (int j = 0; j < KCAP; ++j) {
+      if (j >= pad && (!o.radius_mode || L[j] < INFINITY)) {
+        if (!first) sum = fadd(sum, __fsqrt_rn(L[j]));
+        first = false;
+        ++have;
+      }
+    }
+    if (MEAN && exact) tree_mean_out(sum, have + (drop ? 1 : 0), q, qidx, o);
+  }
+  if constexpr (!MEAN) {
+    have = 0;
+    bool tied = false;
+#pragma unroll
+    for (int j = 0; j < KCAP; ++j) {
+      if (j >= pad && L[j] < INFINITY) ++have;
+      if (j > pad && L[j] < INFINITY && L[j] == L[j - (j > 0)]) tied = true;
+      if (drop && j == pad && L[j] == 0.0f) tied = true;  // another point in its place
+    }
+    // the points within the K-th distance, from the leaves scanned
+    const float tau = mine ? fminf(fminf(L[KCAP - 1], bound), FLT_MAX) : -1.0f;
+    for (int i = 0; i < scanned; ++i) {
+      const u32 l = leaves[i];
+      const float4 mate = mate_of(l);
+      const float at = box_d2(own, t.box[0], t.stride[0], l) <= tau ? tau : -1.0f;
+      if (!stage_leaf(l, at, mate)) continue;
+      test_staged(at, drop && l == qi / 32 ? (int)(qi & 31) : -1, [&](int c, float d) {
+        if (cnt < PCAP) pbuf[cnt][lane] = make_uint2(__float_as_uint(d), l * 32 + c);
+        ++cnt;
+      });
+    }
+    // exactly these are within the K-th distance, no two equal (and what is
+    // missing is not there: points infinitely far would be)
+    exact = mine && cnt == have && !tied &&
+            (have == KL || bound < INFINITY || (!FRAMES && (u32)(have + (drop ? 1 : 0)) == t.n));
+    // each to its rank among the sorted distances, behind the point itself
+    const int r0 = drop ? 1 : 0;
+    if (exact) {
+      if (drop) {
+        if constexpr (MODE == TREE_PAIRS) {
+          if (o.idx) o.idx[(size_t)qidx * K] = (int32_t)qidx;
+          if (o.d2) o.d2[(size_t)qidx * K] = 0.0f;
+        } else if constexpr (MODE == TREE_LIST) {
+          o.rows[(size_t)qi * K] = qi;
+        } else {
+          sorted[0][lane] = qi;
+        }
+      }
+      for (int i = 0; i < have; ++i) {
+        const uint2 b = pbuf[i][lane];
+        const float d = __uint_as_float(b.x);
+        int r = r0 - pad;
+#pragma unroll
+        for (int j = 0; j < KCAP; ++j) r += L[j] < d ? 1 : 0;
+        if constexpr (MODE == TREE_PAIRS) {
+          const size_t at = (size_t)qidx * K + r;
+          if (o.idx) o.idx[at] = (int32_t)__float_as_uint(__ldg(&t.pts[b.y]).w);
+          if (o.d2) o.d2[at] = d;
+        } else if constexpr (MODE == TREE_LIST) {
+          o.rows[(size_t)qi * K + r] = b.y;
+        } else {
+          sorted[r][lane] = b.y;
+        }
+      }
+    }
+    have += r0;
+    if (MODE == TREE_LIST && exact) tree_mean_out(sum, have, q, qidx, o);
+  }
+  // the others are listed for the second kernel
+  const unsigned again = __ballot_sync(0xffffffffu, active && !exact);
+  if (again) {
+    u32 at = 0;
+    if (lane == 0) at = atomicAdd(qs.hard_count, (u32)__popc(again));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (active && !exact) qs.hard[at + __popc(again & ((1u << lane) - 1))] = qi;
+  }
+  if (!exact) return;
+  if constexpr (MODE == TREE_PAIRS) {
+    for (int j = have; j < K; ++j) {
+      if (o.idx) o.idx[(size_t)qidx * K + j] = -1;
+      if (o.d2) o.d2[(size_t)qidx * K + j] = INFINITY;
+    }
+    if (o.counts) o.counts[qidx] = have;
+  } else if constexpr (MODE == TREE_NORMALS || MODE == TREE_PRECISE) {
+    tree_normal_out<MODE>([&](int j) { return __ldg(&t.pts[sorted[j][lane]]); }, have, q, qidx, o);
+  }
+}
+
+// one warp per listed query, lanes over a leaf's points, a list of packed
+// (distance, index) keys over the lanes
+template <int P, int MODE, bool FRAMES>
+__global__ __launch_bounds__(128) void k_knn_tree_hard(TreeView t, TreeQueries qs, int K,
+                                                       float bound, TreeOut o) {
+  __shared__ float4 near[4][32 * P];  // the neighbours in order
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const u32 n = *qs.hard_count;
+  const bool self = FRAMES || qs.n_sort == nullptr || *qs.n_sort == 0;
+  for (u32 w = blockIdx.x * 4 + wib; w < n; w += gridDim.x * 4) {
+    const u32 qi = qs.hard[w];
+    const float4 q = self ? t.pts[qi] : qs.q[qi];
+    const u32 qidx = __float_as_uint(q.w) & (FRAMES ? 0x7FFFFFFFu : 0xFFFFFFFFu);
+    u32 start = qi / 32;
+    Roots roots{0, t.count[kTreeLevels - 1]};
+    u32 leaf0 = 0, leaf1 = t.count[0] - 1;
+    if constexpr (FRAMES) {
+      const uint2 nodes = t.frame_nodes[t.node_frame[qi / 1024]];
+      roots = Roots{nodes.x, nodes.y};
+      leaf0 = nodes.x * 32;
+      leaf1 = nodes.y * 32 - 1;
+    } else if (!self) {
+      start = leaf_of_key(t, qs.keys[qi]);
+    }
+    WarpList<P> W;
+    W.init();
+    u64 key_thr = ~0ull;
+    u32 found = 0;
+    const Box own{{q.x, q.y, q.z}, {q.x, q.y, q.z}};
+    auto limit = [&]() {
+      return key_thr == ~0ull ? bound : fminf(nbr_d2(key_thr), bound);
+    };
+    auto scan = [&](u32 l) {
+      const u32 i = l * 32 + lane;
+      u64 key = ~0ull;
+      if (i < t.n) {
+        const float4 p = __ldg(&t.pts[i]);
+        const float d = dist2(p.x, p.y, p.z, q.x, q.y, q.z);
+        if (d <= bound) key = pack_nbr(d, (int)__float_as_uint(p.w));
+      }
+      found += __popc(__ballot_sync(0xffffffffu, key != ~0ull));
+      unsigned m = __ballot_sync(0xffffffffu, key < key_thr);
+      if constexpr (P == 1) {
+        if (__popc(m) > 4) {  // many at once: one merge instead of serial inserts
+          W.merge_lanes((m >> lane) & 1u ? key : ~0ull);
+          key_thr = W.get(K - 1);
+          m = 0;
+        }
+      }
+      while (m) {
+        const int b = __ffs(m) - 1;
+        m &= m - 1;
+        const u64 k = __shfl_sync(0xffffffffu, key, b);
+        if (k < key_thr) {
+          W.insert(k);
+          key_thr = W.get(K - 1);
+        }
+      }
+    };
+    const u32 s0 = start > leaf0 ? start - 1 : leaf0, s1 = min(start + 1, leaf1);
+    for (u32 l = s0; l <= s1; ++l) scan(l);
+    auto leaf = [&](u32 l) {
+      if (l < s0 || l > s1) scan(l);
+    };
+    tree_walk_all<FRAMES>(t, roots, own, limit, leaf);
+    const int have = min((int)found, K);
+    if constexpr (MODE == TREE_MEAN || MODE == TREE_LIST) {
+      float sum = 0.0f;
+      for (int j = 1; j < have; ++j) sum = fadd(sum, __fsqrt_rn(nbr_d2(W.get(j))));
+      if (lane == 0) tree_mean_out(sum, have, q, qidx, o);
+    }
+    if constexpr (MODE != TREE_MEAN) {
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        const int j = p * 32 + lane;
+        if constexpr (MODE == TREE_PAIRS) {
+          if (j < K) {
+            const size_t at = (size_t)qidx * K + j;
+            if (o.idx) o.idx[at] = j < have ? nbr_idx(W.e[p]) : -1;
+            if (o.d2) o.d2[at] = j < have ? nbr_d2(W.e[p]) : INFINITY;
+          }
+        } else if constexpr (MODE == TREE_LIST) {
+          if (j < K)
+            o.rows[(size_t)qi * K + j] =
+                j < have ? t.pos_of[(u32)nbr_idx(W.e[p]) & 0x7FFFFFFFu] : 0xFFFFFFFFu;
+        } else {
+          if (j < have) near[wib][j] = __ldg(&t.pts[t.pos_of[(u32)nbr_idx(W.e[p]) & 0x7FFFFFFFu]]);
+        }
+      }
+      if constexpr (MODE == TREE_PAIRS) {
+        if (lane == 0 && o.counts) o.counts[qidx] = have;
+      } else if constexpr (MODE != TREE_LIST) {
+        __syncwarp();
+        if (lane == 0)
+          tree_normal_out<MODE>([&](int j) { return near[wib][j]; }, have, q, qidx, o);
+        __syncwarp();
+      }
+    }
+  }
+}
+
+// packets: how many there can be
+template <int KCAP, int MODE, bool FRAMES>
+void launch_tree(rvp_context *ctx, const TreeView &t, const TreeQueries &q, u32 packets, int K,
+                 float bound, const TreeOut &o) {
+  constexpr size_t smem = tree_smem<KCAP, MODE>();
+  static_assert(smem <= 48 * 1024, "no opt-in to larger shared memory here");
+  k_knn_tree<KCAP, MODE, FRAMES><<<packets, 32, smem, ctx->stream>>>(t, q, K, bound, o);
+  RVP_LAUNCH_CHECK(ctx);
+  const unsigned blocks = grid_for(packets * 32, 4, ctx->num_sms * 8);
+  if (K <= 32)
+    k_knn_tree_hard<1, MODE, FRAMES><<<blocks, 128, 0, ctx->stream>>>(t, q, K, bound, o);
+  else
+    k_knn_tree_hard<2, MODE, FRAMES><<<blocks, 128, 0, ctx->stream>>>(t, q, K, bound, o);
+  RVP_LAUNCH_CHECK(ctx);
+}
+
+// listed: distances a list needs room for
+template <int MODE, bool FRAMES>
+void launch_tree_k(rvp_context *ctx, const TreeView &t, const TreeQueries &q, u32 packets, int K,
+                   int listed, float bound, const TreeOut &o) {
+  if (listed <= 8) launch_tree<8, MODE, FRAMES>(ctx, t, q, packets, K, bound, o);
+  else if (listed <= 16) launch_tree<16, MODE, FRAMES>(ctx, t, q, packets, K, bound, o);
+  else if (listed <= 32) launch_tree<32, MODE, FRAMES>(ctx, t, q, packets, K, bound, o);
+  else launch_tree<64, MODE, FRAMES>(ctx, t, q, packets, K, bound, o);
+}
+}  // namespace
+}  // namespace rvp

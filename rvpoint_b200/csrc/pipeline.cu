@@ -35,6 +35,13 @@ struct rvp_pipeline {
   int grid_base = 2;    // the grid is sorted by cells of cell / 2^grid_base
   rvp::VoxelWork vw;
   rvp::Grid grid;
+  // kernel mode 0 searches a box tree of the frames instead of the grid.
+  // tree_fits: its frames, padded to 1024 positions each, stay within twice
+  // the points (a batch of many tiny frames keeps the grid)
+  rvp::KnnTree tree;
+  bool tree_fits = false;
+  bool grid_built = false;  // by the last run
+  size_t points_last = 0;
   rvp::DevBuf in_x, in_y, in_z, in_offs;
   rvp::DevBuf vox_aos, vox_x, vox_y, vox_z, vox_offs, vox_frame;
   rvp::DevBuf sor_list, knn_counts, mean, keep, sor_tmp;
@@ -160,6 +167,7 @@ void release_pipeline(rvp_pipeline *p) {
   for (auto *b : bufs) b->release();
   p->vw.release();
   p->grid.release();
+  p->tree.release();
   for (auto e : p->events) cudaEventDestroy(e);
   if (p->graph) cudaGraphExecDestroy(p->graph);
   for (auto e : p->ev_stage)
@@ -171,6 +179,108 @@ void release_pipeline(rvp_pipeline *p) {
     if (e) cudaEventDestroy(e);
   for (auto *b : {&p->in2_x, &p->in2_y, &p->in2_z, &p->in2_offs}) b->release();
   delete p;
+}
+
+// stages 2 to 4 over the box tree of the batch: SOR means with the k+1 nearest
+// of every voxel point as rows of tree positions, the statistics and the copy,
+// then the normals, from the rows whose points all survived, else searched
+// again among the kept points
+void run_tree(rvp_pipeline *p, int n_frames, size_t N) {
+  rvp_context *ctx = p->ctx;
+  const rvp_pipeline_config &c = p->cfg;
+  cudaStream_t st = ctx->stream;
+  int64_t *vox_offs = p->vox_offs.as<int64_t>(), *sor_offs = p->sor_offs.as<int64_t>();
+  const u64 *n_vox = reinterpret_cast<const u64 *>(vox_offs + n_frames);
+  const float *x = p->vox_x.as<float>(), *y = p->vox_y.as<float>(), *z = p->vox_z.as<float>();
+  RVP_CUDA_TRY(cudaMemsetAsync(p->grid.d_collision, 0, 8, st));  // nothing to overflow
+  const rvp::TreeView t = rvp::tree_build_frames(
+      ctx, p->tree, x, y, z, p->vox_aos.as<float>(), vox_offs, n_frames, N, p->vw.keys.as<u64>(),
+      p->vw.vals.as<u32>(), p->vw.sort.ptr);
+  p->mark(2);
+  // the search kernels' time goes to the first of the timed kernels
+  auto timed = [&](int stage, auto &&search) {
+    cudaEvent_t *ev = p->level_events(stage);
+    p->empty_level_events(ev);
+    if (ev) cudaEventRecord(ev[0], st);
+    search();
+    if (ev) cudaEventRecord(ev[1], st);
+  };
+  const int ks = c.sor_k + 1, kn = c.normal_k + 1;
+  const bool lists = kn <= ks;
+  rvp::TreeOut o;
+  o.mean = p->mean.as<float>();
+  o.rows = p->sor_list.as<u32>();
+  timed(0, [&] {
+    rvp::tree_knn_frames(ctx, p->tree, t, nullptr, nullptr, ks,
+                         lists ? rvp::TREE_LIST : rvp::TREE_MEAN, o);
+  });
+  p->mark(3);
+  if (p->wait_before[1]) RVP_CUDA_TRY(cudaStreamWaitEvent(st, p->wait_before[1], 0));
+  rvp::sor_filter_frames(ctx, x, y, z, p->mean.as<float>(), vox_offs, n_frames, N, n_vox,
+                         c.sor_alpha, p->keep.as<uint8_t>(), p->sor_aos.as<float>(), sor_offs,
+                         nullptr, p->sor_tmp.ptr, p->sor_x.as<float>(), p->sor_y.as<float>(),
+                         p->sor_z.as<float>(), p->sor_src.as<u32>());
+  p->mark(4);
+  if (p->record_stages) RVP_CUDA_TRY(cudaEventRecord(p->ev_stage[1], st));
+  if (p->wait_before[2]) RVP_CUDA_TRY(cudaStreamWaitEvent(st, p->wait_before[2], 0));
+  rvp::tree_frames_mark_removed(ctx, t, p->keep.as<uint8_t>());
+  o.nx = p->nx.as<float>();
+  o.ny = p->ny.as<float>();
+  o.nz = p->nz.as<float>();
+  o.iters = c.eigen_iters;
+  o.vpx = c.vp_x;
+  o.vpy = c.vp_y;
+  o.vpz = c.vp_z;
+  o.out_pos = rvp::sor_positions(p->sor_tmp.ptr, N);
+  rvp::TileArgs a{};
+  a.sor_list = o.rows;
+  a.qlevel = p->qlevel.as<uint8_t>();
+  a.out_pos = o.out_pos;
+  a.nx = o.nx;
+  a.ny = o.ny;
+  a.nz = o.nz;
+  a.iters = o.iters;
+  a.vpx = o.vpx;
+  a.vpy = o.vpy;
+  a.vpz = o.vpz;
+  a.n_max = t.n;
+  {
+    auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    char *op = p->open.as<char>();
+    a.open_flags = reinterpret_cast<u32 *>(op); op += al(a.n_max * 4);
+    a.open_pos = reinterpret_cast<u64 *>(op); op += al(a.n_max * 8 + 8);
+    a.open_list = reinterpret_cast<u32 *>(op); op += al(a.n_max * 4);
+    a.open_n = reinterpret_cast<u64 *>(op); op += 256;
+    a.scan_tmp = op;
+  }
+  rvp::GridView gv{};  // the tree's records by position
+  gv.mode = rvp::KEY_DENSE;
+  gv.pts = t.pts;
+  gv.n_points = t.n_positions;
+  const bool from_rows = lists && rvp::normals_from_sor_lists(ctx, gv, a, ks, kn);
+  if (from_rows) rvp::list_open(ctx, t.n_positions, 0, a);
+  timed(1, [&] {
+    rvp::tree_knn_frames(ctx, p->tree, t, from_rows ? a.open_list : nullptr, a.open_n, kn,
+                         rvp::TREE_NORMALS, o);
+  });
+  p->mark(5);
+}
+
+// stage 5: RANSAC per frame on the kept points
+void run_ransac(rvp_pipeline *p, int n_frames) {
+  rvp_context *ctx = p->ctx;
+  const rvp_pipeline_config &c = p->cfg;
+  p->mark(6);
+  if (p->wait_before[3]) RVP_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, p->wait_before[3], 0));
+  double pc = (double)c.ransac_prob;
+  pc = pc < 0.5 ? 0.5 : (pc > 0.9999 ? 0.9999 : pc);
+  rvp::RansacParams prm{c.ransac_thresh, c.ransac_iters, c.ransac_collinear, log(1.0 - pc)};
+  rvp::ransac_frames(ctx, p->sor_x.as<float>(), p->sor_y.as<float>(), p->sor_z.as<float>(),
+                     p->sor_offs.as<int64_t>(), n_frames, p->r_rand.as<int>(), prm,
+                     p->r_model.as<float>(), p->r_best.as<int32_t>(), p->r_iters.as<int32_t>(),
+                     nullptr, false, rvp::RansacSampler{}, 4);
+  p->mark(7);
+  if (!p->capturing && p->runs_cap > 0 && p->runs_recorded < p->runs_cap) p->runs_recorded++;
 }
 }  // namespace
 
@@ -209,7 +319,11 @@ rvp_status rvp_pipeline_create(rvp_context *ctx, const rvp_pipeline_config *cfg,
     p->vox_offs.reserve(F1 * 8);
     p->vox_frame.reserve(N * 4);
     const int ks = cfg->sor_k + 1, kn = cfg->normal_k + 1;
-    p->sor_list.reserve(N * (size_t)ks * 4);
+    p->tree_fits = (size_t)max_frames * 1024 <= N + 65536;
+    // (tree positions, or grid positions)
+    const size_t P = p->tree_fits ? rvp::tree_frames_positions(N, max_frames) : N;
+    if (p->tree_fits) p->tree.reserve_frames(N, max_frames);
+    p->sor_list.reserve(P * (size_t)ks * 4);
     p->knn_counts.reserve(N * 4);
     p->mean.reserve(N * 4);
     p->keep.reserve(N);
@@ -221,11 +335,12 @@ rvp_status rvp_pipeline_create(rvp_context *ctx, const rvp_pipeline_config *cfg,
     p->sor_src.reserve(N * 4);
     p->nrm_pairs.reserve(N * (size_t)kn * 8);
     p->hard.reserve(N * 8 + 256);
-    p->qlevel.reserve(N);
+    p->qlevel.reserve(P);
     p->qtau.reserve(N * 4);
     p->routed.reserve(256);
-    p->open.reserve(((N * 4 + 255) & ~(size_t)255) + ((N * 8 + 8 + 255) & ~(size_t)255) +
-                    ((N * 4 + 255) & ~(size_t)255) + 256 + rvp::scan_temp_bytes(N));
+    p->open.reserve(((P * 4 + 255) & ~(size_t)255) + ((P * 8 + 8 + 255) & ~(size_t)255) +
+                    ((P * 4 + 255) & ~(size_t)255) + 256 + rvp::scan_temp_bytes(P));
+    RVP_CUDA_TRY(cudaMemset(p->grid.d_collision, 0, 8));
     p->nrm_counts.reserve(N * 4);
     p->nx.reserve(N * 4); p->ny.reserve(N * 4); p->nz.reserve(N * 4);
     p->r_model.reserve((size_t)max_frames * 16);
@@ -285,6 +400,13 @@ rvp_status rvp_pipeline_run_device(rvp_pipeline *p, const float *x, const float 
                         p->vox_y.as<float>(), p->vox_z.as<float>());
     p->mark(1);
     if (p->record_stages) RVP_CUDA_TRY(cudaEventRecord(p->ev_stage[0], st));
+    p->points_last = N;
+    p->grid_built = !(p->tree_fits && c.queries_per_warp == 0);
+    if (!p->grid_built) {
+      run_tree(p, n_frames, N);
+      run_ransac(p, n_frames);
+      return;
+    }
     // 2) grid over the voxel points of every frame: cells of `cell` for the
     //    searches, the points sorted by cells of cell / 4 inside them (so
     //    that consecutive points, a warp's queries, lie close together)
@@ -425,18 +547,7 @@ rvp_status rvp_pipeline_run_device(rvp_pipeline *p, const float *x, const float 
                             p->vox_x.as<float>(), p->vox_y.as<float>(), p->vox_z.as<float>(),
                             p->nx.as<float>(), p->ny.as<float>(), p->nz.as<float>(), hard,
                             sor_pos);
-    p->mark(6);
-    if (p->wait_before[3]) RVP_CUDA_TRY(cudaStreamWaitEvent(st, p->wait_before[3], 0));
-    // 5) RANSAC per frame on the kept points
-    double pc = (double)c.ransac_prob;
-    pc = pc < 0.5 ? 0.5 : (pc > 0.9999 ? 0.9999 : pc);
-    rvp::RansacParams prm{c.ransac_thresh, c.ransac_iters, c.ransac_collinear, log(1.0 - pc)};
-    rvp::ransac_frames(ctx, p->sor_x.as<float>(), p->sor_y.as<float>(), p->sor_z.as<float>(),
-                       sor_offs, n_frames, p->r_rand.as<int>(), prm, p->r_model.as<float>(),
-                       p->r_best.as<int32_t>(), p->r_iters.as<int32_t>(), nullptr, false,
-                       rvp::RansacSampler{}, 4);
-    p->mark(7);
-    if (!p->capturing && p->runs_cap > 0 && p->runs_recorded < p->runs_cap) p->runs_recorded++;
+    run_ransac(p, n_frames);
   });
 }
 
@@ -497,6 +608,14 @@ rvp_status rvp_pipeline_fit_tables(rvp_pipeline *p) {
   if (!p) return RVP_ERR_INVALID_ARG;
   return guard(p->ctx, [&] {
     RVP_CUDA_TRY(cudaSetDevice(p->ctx->device));
+    if (p->n_frames_last < 1) return;  // no run to measure
+    if (!p->grid_built) {  // it used the tree: the buckets its grid would have
+      const int64_t *offs = p->vox_offs.as<int64_t>();
+      rvp::grid_build(p->ctx, p->grid, p->vox_x.as<float>(), p->vox_y.as<float>(),
+                      p->vox_z.as<float>(), offs, p->n_frames_last, p->points_last, p->cell,
+                      rvp::KEY_DENSE, 0, 0, reinterpret_cast<const u64 *>(offs + p->n_frames_last),
+                      p->grid_base, p->vox_aos.as<float>());
+    }
     u64 nb[rvp::kHeadLevels] = {};
     RVP_CUDA_TRY(cudaMemcpyAsync(nb, p->grid.d_nbuckets, 8 * rvp::kHeadLevels, cudaMemcpyDeviceToHost,
                                  p->ctx->stream));
