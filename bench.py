@@ -438,15 +438,13 @@ def kernel_name(stage: str, coop: bool) -> str:
         return "k_knn_coop<17,SOR_LIST> (cells of c)"
     if coop and stage == "sor_knn_l0":
         return "k_knn_adapt<17,SOR_LIST> (per-thread windows)"
-    cells = {"sor_knn_l0": "c", "sor_knn_l1": "4c", "sor_knn_l2": "16c"}[stage]
-    return f"k_knn_wt<17,SOR_LIST> (cells of {cells})"
+    return f"k_knn_tree<16,TREE_LIST> (box tree of all frames, {stage})"
 
 
 def kernel_units(stage: str, coop: bool, counts, n_vox: int):
     """Queries one launch of a SOR kNN kernel processes: in cooperative mode
     the cooperative pass's and the adaptive kernel's (counts); without it
-    the per-lane kernel on cells of c takes every query (on the coarser
-    cells only the ones left open, a count the line does not carry)."""
+    the box tree's packets take every query."""
     if coop:
         return {"sor_knn_coop": counts[0], "sor_knn_l0": counts[1]}.get(stage)
     if stage == "sor_knn_l0":
@@ -836,8 +834,8 @@ def main():
 
     # ---- roofline of the longest kernel timed live (per-level SOR kNN
     # kernels and RANSAC)
-    coop = int(pipe.cfg.queries_per_warp) == 3
-    counts = pipe.knn_counts() if coop else None
+    counts = pipe.knn_counts()
+    coop = sum(counts) > 0  # (zeros: the box tree, or one query per lane)
     routed = counts[0] if coop else None
     cand = {}
     for k in LEVEL_STAGES + ("ransac",):

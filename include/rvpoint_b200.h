@@ -282,10 +282,11 @@ typedef struct {
   float cell_size;       /* grid cell for the neighbour searches (0 = auto) */
   int block_threads;     /* warp-per-query kNN kernel block size: 32..256, a multiple
                             of 32 (0 = 256) */
-  int queries_per_warp;  /* kNN kernel mode: 0 one query per lane at every grid level
-                            (default), 1 one warp per query, 2 shared-memory tiles,
-                            3 a cooperative level-0 pass (all lanes test the same
-                            candidate) before the per-lane kernels */
+  int queries_per_warp;  /* kNN kernel mode: 0 (default) and 3 a box tree of all frames;
+                            on the neighbour grid: 1 one warp per query, 2 shared-memory
+                            tiles, and, for batches of many tiny frames, which keep the
+                            grid, 0 one query per lane at every level, 3 a cooperative
+                            level-0 pass before per-thread windows */
 } rvp_pipeline_config;
 
 RVP_API rvp_status rvp_pipeline_create(rvp_context *ctx, const rvp_pipeline_config *cfg,
@@ -341,7 +342,7 @@ RVP_API rvp_status rvp_pipeline_check(rvp_pipeline *p);
  * 16c (c = the pipeline's cell size). */
 #define RVP_GRID_LEVELS 5
 /* Queries of the last run's SOR kNN kernels in cooperative mode
- * (queries_per_warp 3; zeros otherwise): out[0] the cooperative pass took
+ * (queries_per_warp 3 on the grid; zeros otherwise): out[0] the cooperative pass took
  * (points whose own cell holds at least ceil(rfac^2 k) points), out[1] the
  * adaptive per-thread kernel took (what the cooperative pass left open).
  * out[2]. */
@@ -349,7 +350,8 @@ RVP_API rvp_status rvp_pipeline_knn_routed(rvp_pipeline *p, uint64_t *out);
 /* Diagnostics: enable != 0 makes the kNN kernels count which search path
  * settled each query: out20[0..7] SOR, [8..15] normals (warp-per-query
  * kernel: first-level ring, tight window of a bound, second-level ring,
- * coarser ring, whole frame; per-lane chain levels 1, 2, 3), [16] SOR and
+ * coarser ring, whole frame; per-lane chain levels 1, 2, 3; on the box tree
+ * the first of each: the warp-per-query kernel, the packets), [16] SOR and
  * [17] normals settled by the per-thread tight window of a handed-on bound,
  * [18..19] reserved. Reads (if out20) and clears the counters. */
 RVP_API rvp_status rvp_pipeline_knn_stats(rvp_pipeline *p, int enable, uint32_t *out20);

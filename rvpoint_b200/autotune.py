@@ -46,8 +46,9 @@ def tune(pipe, x, y, z, offsets, n_frames: int, n_points: int,
     """Returns (best setting, all trials) and applies the best to `pipe`.
 
     Two stages: every combination of cell size, kNN kernel mode
-    (queries_per_warp: 0 one query per lane at every grid level, 3 a
-    cooperative pass over dense cells, then one query per thread with its
+    (queries_per_warp: 0 and 3 the box tree, which no other setting changes;
+    for batches of many tiny frames 0 one query per lane at every grid level,
+    3 a cooperative pass over dense cells, then one query per thread with its
     own adaptive window), first-pass radius factor and per-lane grid levels
     (mode 0 only) at the default block shape; then the block shape of the
     warp-per-query kernel at the best of those."""

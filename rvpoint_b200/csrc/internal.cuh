@@ -440,6 +440,7 @@ struct TreeOut {  // by query index; null pointers are skipped
   uint8_t *used64 = nullptr;
   u32 *rows = nullptr;
   const u64 *out_pos = nullptr;  // where a point's normal goes (null: its index)
+  u32 *n_packets = nullptr, *n_hard = nullptr;  // counters: queries of each kernel
 };
 struct KnnTree {
   DevBuf keys, vals, sort, pts, pos, boxes, misc, qkeys, qvals, qpts, hard;

@@ -574,6 +574,10 @@ __global__ __launch_bounds__(32, KCAP > 32 ? 10 : 16) void k_knn_tree(TreeView t
     at = __shfl_sync(0xffffffffu, at, 0);
     if (active && !exact) qs.hard[at + __popc(again & ((1u << lane) - 1))] = qi;
   }
+  if (o.n_packets) {
+    const unsigned b = __ballot_sync(0xffffffffu, exact);
+    if (lane == 0) atomicAdd(o.n_packets, (u32)__popc(b));
+  }
   if (!exact) return;
   if constexpr (MODE == TREE_PAIRS) {
     for (int j = have; j < K; ++j) {
@@ -652,6 +656,7 @@ __global__ __launch_bounds__(128) void k_knn_tree_hard(TreeView t, TreeQueries q
     };
     tree_walk_all<FRAMES>(t, roots, own, limit, leaf);
     const int have = min((int)found, K);
+    if (o.n_hard && lane == 0) atomicAdd(o.n_hard, 1u);
     if constexpr (MODE == TREE_MEAN || MODE == TREE_LIST) {
       float sum = 0.0f;
       for (int j = 1; j < have; ++j) sum = fadd(sum, __fsqrt_rn(nbr_d2(W.get(j))));
