@@ -187,12 +187,27 @@ struct SortTemp {
   u32 *vals_alt = nullptr;
   u32 *tile_hist = nullptr;    // 256 x tiles(n_max)
   u32 *global_hist = nullptr;  // 256 digit totals of the current pass
-  int *pass_info = nullptr;    // OR and AND of all keys (2 x u64)
+  int *pass_info = nullptr;    // bits that some key has set, that some has clear (2 x u64)
 };
 size_t sort_temp_bytes(size_t n_max);
 void sort_temp_carve(SortTemp &t, void *base, size_t n_max);
+// bits: sort_key_bits, filled by the kernel that wrote the keys
+// (note_key_bits); null: the sort reads the keys for them
 void radix_sort_pairs(rvp_context *ctx, u64 *keys, u32 *vals, size_t n_max,
-                      const u64 *n_dev, const SortTemp &t);
+                      const u64 *n_dev, const SortTemp &t, u64 *bits = nullptr);
+// cleared words for the keys' bits; null where the sort needs none
+u64 *sort_key_bits(rvp_context *ctx, const SortTemp &t, size_t n_max);
+// by whole warps: the bits set (clear) in some of the warp's keys
+__device__ __forceinline__ void note_key_bits(u64 ones, u64 zeros, u64 *bits) {
+  const unsigned ol = __reduce_or_sync(0xffffffffu, (unsigned)ones);
+  const unsigned oh = __reduce_or_sync(0xffffffffu, (unsigned)(ones >> 32));
+  const unsigned zl = __reduce_or_sync(0xffffffffu, (unsigned)zeros);
+  const unsigned zh = __reduce_or_sync(0xffffffffu, (unsigned)(zeros >> 32));
+  if ((threadIdx.x & 31) == 0) {
+    atomicOr(&bits[0], ((u64)oh << 32) | ol);
+    atomicOr(&bits[1], ((u64)zh << 32) | zl);
+  }
+}
 
 // exclusive scan of u32/u64 flags -> u64 offsets (scan.cu). n may be on the
 // device. out[n] receives the total. temp: scan_temp_bytes(n_max).

@@ -51,16 +51,24 @@ __global__ __launch_bounds__(256) void k_tree_keys(const float *__restrict__ x,
                                                    const float *__restrict__ y,
                                                    const float *__restrict__ z, size_t n_max,
                                                    const u64 *n_dev, const float *bb, u64 *keys,
-                                                   u32 *vals) {
+                                                   u32 *vals, u64 *bits) {
   __shared__ TreeFrame F;
+  __shared__ unsigned short table[192];
   const size_t n = n_dev ? *n_dev : n_max;
-  if (threadIdx.x == 0) tree_frame(bb, kTreeKeyBits, F);
+  if (n == 0) return;
+  if (threadIdx.x == 255) tree_frame(bb, tree_key_bits(n_max), F);
+  tree_key_table(table);
   __syncthreads();
+  u64 ones = 0, zeros = 0;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
-    keys[i] = tree_key(F, x[i], y[i], z[i]);
+    const u64 k = tree_key(F, table, x[i], y[i], z[i]);
+    keys[i] = k;
     vals[i] = (u32)i;
+    ones |= k;
+    zeros |= ~k;
   }
+  if (bits) note_key_bits(ones, zeros, bits);
 }
 
 // one warp per leaf: its records in tree order and its box
@@ -168,12 +176,13 @@ TreeView tree_build(rvp_context *ctx, KnnTree &w, const float *x, const float *y
   k_tree_init<<<1, 32, 0, st>>>(w.misc.as<float>());
   RVP_LAUNCH_CHECK(ctx);
   cloud_bbox(ctx, x, y, z, n, w.misc.as<float>());
-  k_tree_keys<<<grid_for(n, 256, sms * 8), 256, 0, st>>>(x, y, z, n, nullptr, t.bb,
-                                                         w.keys.as<u64>(), w.vals.as<u32>());
-  RVP_LAUNCH_CHECK(ctx);
   SortTemp tmp;
   sort_temp_carve(tmp, w.sort.ptr, n);
-  radix_sort_pairs(ctx, w.keys.as<u64>(), w.vals.as<u32>(), n, nullptr, tmp);
+  u64 *bits = sort_key_bits(ctx, tmp, n);
+  k_tree_keys<<<grid_for(n, 256, sms * 8), 256, 0, st>>>(x, y, z, n, nullptr, t.bb,
+                                                         w.keys.as<u64>(), w.vals.as<u32>(), bits);
+  RVP_LAUNCH_CHECK(ctx);
+  radix_sort_pairs(ctx, w.keys.as<u64>(), w.vals.as<u32>(), n, nullptr, tmp, bits);
   k_tree_leaves<<<(unsigned)((t.count[0] + 7) / 8), 256, 0, st>>>(
       x, y, z, w.vals.as<u32>(), t.n, w.pts.as<float4>(), w.pos.as<u32>(), t.box[0], t.stride[0]);
   RVP_LAUNCH_CHECK(ctx);
@@ -217,12 +226,13 @@ TreeQueries tree_queries(rvp_context *ctx, KnnTree &w, const TreeView &t, const 
     k_tree_same<<<gb, 256, 0, st>>>(qx, qy, qz, x, y, z, nq, n_sort);
     RVP_LAUNCH_CHECK(ctx);
   }
-  k_tree_keys<<<gb, 256, 0, st>>>(qx, qy, qz, nq, n_sort, t.bb, w.qkeys.as<u64>(),
-                                  w.qvals.as<u32>());
-  RVP_LAUNCH_CHECK(ctx);
   SortTemp tmp;
   sort_temp_carve(tmp, w.sort.ptr, nq);
-  radix_sort_pairs(ctx, w.qkeys.as<u64>(), w.qvals.as<u32>(), nq, n_sort, tmp);
+  u64 *bits = sort_key_bits(ctx, tmp, nq);
+  k_tree_keys<<<gb, 256, 0, st>>>(qx, qy, qz, nq, n_sort, t.bb, w.qkeys.as<u64>(),
+                                  w.qvals.as<u32>(), bits);
+  RVP_LAUNCH_CHECK(ctx);
+  radix_sort_pairs(ctx, w.qkeys.as<u64>(), w.qvals.as<u32>(), nq, n_sort, tmp, bits);
   k_tree_queries<<<gb, 256, 0, st>>>(qx, qy, qz, w.qvals.as<u32>(), n_sort, w.qpts.as<float4>());
   RVP_LAUNCH_CHECK(ctx);
   q.q = w.qpts.as<float4>();

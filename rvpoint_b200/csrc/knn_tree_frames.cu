@@ -63,9 +63,12 @@ __global__ __launch_bounds__(256) void k_frames_keys(const float *__restrict__ x
                                                      const float *__restrict__ z,
                                                      const int64_t *offs, int n_frames,
                                                      const TreeFrame *F, int key_bits, u64 *keys,
-                                                     u32 *vals) {
+                                                     u32 *vals, u64 *bits) {
   const int64_t n = offs[n_frames];
   __shared__ int s_lo, s_hi;
+  __shared__ unsigned short table[192];
+  tree_key_table(table);
+  u64 ones = 0, zeros = 0;
   for (int64_t base = (int64_t)blockIdx.x * FK_CHUNK; base < n;
        base += (int64_t)gridDim.x * FK_CHUNK) {
     const int64_t end = base + FK_CHUNK < n ? base + FK_CHUNK : n;
@@ -75,11 +78,15 @@ __global__ __launch_bounds__(256) void k_frames_keys(const float *__restrict__ x
     const int lo = s_lo, hi = s_hi;
     for (int64_t i = base + threadIdx.x; i < end; i += 256) {
       const int f = frame_of(offs, lo, hi, i);
-      keys[i] = ((u64)f << key_bits) | tree_key(F[f], x[i], y[i], z[i]);
+      const u64 k = ((u64)f << key_bits) | tree_key(F[f], table, x[i], y[i], z[i]);
+      keys[i] = k;
       vals[i] = (u32)i;
+      ones |= k;
+      zeros |= ~k;
     }
     __syncthreads();
   }
+  if (bits) note_key_bits(ones, zeros, bits);
 }
 
 // one block per level-1 node: its 1024 records, 32 leaf boxes and own box
@@ -193,12 +200,14 @@ TreeView tree_build_frames(rvp_context *ctx, KnnTree &w, const float *x, const f
   frames_bbox(ctx, x, y, z, offs, n_frames, n_max, bb);
   k_frames_setup<<<1, 1024, 0, st>>>(bb, offs, n_frames, key_bits, F, nodes, n_positions);
   RVP_LAUNCH_CHECK(ctx);
-  k_frames_keys<<<grid_for(n_max, FK_CHUNK, ctx->num_sms * 8), 256, 0, st>>>(
-      x, y, z, offs, n_frames, F, key_bits, keys, vals);
-  RVP_LAUNCH_CHECK(ctx);
   SortTemp tmp;
   sort_temp_carve(tmp, sort_temp, n_max);
-  radix_sort_pairs(ctx, keys, vals, n_max, reinterpret_cast<const u64 *>(offs + n_frames), tmp);
+  u64 *bits = sort_key_bits(ctx, tmp, n_max);
+  k_frames_keys<<<grid_for(n_max, FK_CHUNK, ctx->num_sms * 8), 256, 0, st>>>(
+      x, y, z, offs, n_frames, F, key_bits, keys, vals, bits);
+  RVP_LAUNCH_CHECK(ctx);
+  radix_sort_pairs(ctx, keys, vals, n_max, reinterpret_cast<const u64 *>(offs + n_frames), tmp,
+                   bits);
   k_frames_nodes<<<t.count[1], 1024, 0, st>>>(x, y, z, aos, vals, offs, n_frames,
                                               nodes, t, node_frame);
   RVP_LAUNCH_CHECK(ctx);

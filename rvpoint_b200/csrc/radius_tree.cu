@@ -35,7 +35,7 @@ constexpr size_t kFewQueries = 2048;
 // Can two cells of the grid have one key ix + iy * p1 + iz * p2
 // (spatial_hashing.h:43-45)? Only if dx + dy * p1 + dz * p2 = 0 for some
 // difference of cells, and with |p1| at least the cells along x each dz leaves
-// two candidates for dy. *flag = 1 when there is one, or when this does not
+// two candidates for dy. *flag is 1 when there is one, else 0, or when this does not
 // settle it (tiny or huge primes, huge grids): the caller then builds the
 // reference's grid and looks at the cells that are occupied.
 // ---------------------------------------------------------------------------
@@ -61,7 +61,8 @@ __global__ __launch_bounds__(1024) void k_hash_check(const float *bb, float cell
       if (y < g[1] && -y < g[1] && s < g[0] && -s < g[0]) hit = true;
     }
   }
-  if (__syncthreads_or(hit) && threadIdx.x == 0) *flag = 1;
+  const int any = __syncthreads_or(hit);
+  if (threadIdx.x == 0) *flag = any ? 1 : 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -525,7 +526,6 @@ __global__ void k_gather_queries(const float *x, const float *y, const float *z,
 
 void hash_collision_check(rvp_context *ctx, const TreeView &t, float cell, long long p1,
                           long long p2, int *flag) {
-  RVP_CUDA_TRY(cudaMemsetAsync(flag, 0, 4, ctx->stream));
   k_hash_check<<<1, 1024, 0, ctx->stream>>>(t.bb, cell, p1, p2, flag);
   RVP_LAUNCH_CHECK(ctx);
 }

@@ -3,7 +3,7 @@
 // Per live 8-bit digit: (1) tile histogram, (2) per-digit scan over tiles,
 // (3) tile-local stable ranking with ballots, reorder in shared
 // memory, coalesced scatter of each digit run. A digit is live when the keys
-// differ in it (global OR ^ AND of all keys), so a 64-bit key with 30 live
+// differ in it (some have a one, some a zero there), so a 64-bit key with 30 live
 // bits costs 4 passes. The key count and the live mask are read from device
 // memory; nothing returns to the host, so a sort can sit in a graph.
 //
@@ -31,8 +31,9 @@ __host__ __device__ inline size_t tiles_for(size_t n) { return (n + TILE - 1) / 
 
 inline size_t al(size_t b) { return (b + 255) & ~(size_t)255; }
 
-__device__ __forceinline__ u64 live_mask(const u64 *orand) {
-  return orand[0] ^ orand[1];
+// the bits in which keys differ: some key has a one there, some a zero
+__device__ __forceinline__ u64 live_mask(const u64 *bits) {
+  return bits[0] & bits[1];
 }
 __device__ __forceinline__ bool pass_live(u64 live, int pass) {
   return ((live >> (8 * pass)) & 0xFFull) != 0;
@@ -58,24 +59,17 @@ __device__ __forceinline__ int pass_src(u64 live, int pass) {
   return c & 1;
 }
 
-__global__ void k_orand(const u64 *__restrict__ keys, size_t n_max,
-                        const u64 *__restrict__ n_dev, u64 *orand) {
+__global__ void k_key_bits(const u64 *__restrict__ keys, size_t n_max,
+                           const u64 *__restrict__ n_dev, u64 *bits) {
   const size_t n = n_dev ? *n_dev : n_max;
-  u64 o = 0, a = ~0ull;
+  u64 ones = 0, zeros = 0;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
     const u64 k = keys[i];
-    o |= k;
-    a &= k;
+    ones |= k;
+    zeros |= ~k;
   }
-  unsigned olo = __reduce_or_sync(0xffffffffu, (unsigned)o);
-  unsigned ohi = __reduce_or_sync(0xffffffffu, (unsigned)(o >> 32));
-  unsigned alo = __reduce_and_sync(0xffffffffu, (unsigned)a);
-  unsigned ahi = __reduce_and_sync(0xffffffffu, (unsigned)(a >> 32));
-  if ((threadIdx.x & 31) == 0) {
-    atomicOr(&orand[0], ((u64)ohi << 32) | olo);
-    atomicAnd(&orand[1], ((u64)ahi << 32) | alo);
-  }
+  note_key_bits(ones, zeros, bits);
 }
 
 // ---------------------------------------------------------------------------
@@ -246,14 +240,14 @@ __device__ __forceinline__ void scatter_tile(const u64 *kin, const u32 *vin, u64
 
 __global__ __launch_bounds__(TH, 4) void k_sort_tiles(u64 *k0, u32 *v0, u64 *k1, u32 *v1,
                                                       size_t n_max, const u64 *n_dev,
-                                                      const u64 *orand, u32 *tile_hist,
+                                                      const u64 *bits, u32 *tile_hist,
                                                       size_t t_max, u32 *totals) {
   namespace cg = cooperative_groups;
   cg::grid_group grid = cg::this_grid();
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ u32 wsum[WARPS];
   const size_t n = n_dev ? *n_dev : n_max;
-  const u64 live = n ? live_mask(orand) : 0;
+  const u64 live = n ? live_mask(bits) : 0;
   const size_t T = tiles_for(n);
   int src = 0;
   for (int pass = 0; pass < 8; ++pass) {
@@ -284,10 +278,10 @@ __global__ __launch_bounds__(TH, 4) void k_sort_tiles(u64 *k0, u32 *v0, u64 *k1,
 
 // the same steps as kernels of their own, a block per tile (or digit)
 __global__ __launch_bounds__(TH) void k_hist(const u64 *k0, const u64 *k1, size_t n_max,
-                                             const u64 *n_dev, const u64 *orand, int pass,
+                                             const u64 *n_dev, const u64 *bits, int pass,
                                              u32 *tile_hist, size_t t_max) {
   __shared__ u32 h[WARPS][256];
-  const u64 live = live_mask(orand);
+  const u64 live = live_mask(bits);
   if (!pass_live(live, pass)) return;
   const size_t n = n_dev ? *n_dev : n_max;
   if ((size_t)blockIdx.x * TILE >= n) return;
@@ -295,22 +289,22 @@ __global__ __launch_bounds__(TH) void k_hist(const u64 *k0, const u64 *k1, size_
 }
 
 __global__ __launch_bounds__(TH) void k_scan_digit(u32 *tile_hist, size_t t_max, size_t n_max,
-                                                   const u64 *n_dev, const u64 *orand, int pass,
+                                                   const u64 *n_dev, const u64 *bits, int pass,
                                                    u32 *totals) {
   __shared__ u32 wsum[WARPS];
-  if (!pass_live(live_mask(orand), pass)) return;
+  if (!pass_live(live_mask(bits), pass)) return;
   const size_t n = n_dev ? *n_dev : n_max;
   scan_digit(tile_hist + (size_t)blockIdx.x * t_max, tiles_for(n), &totals[blockIdx.x], wsum);
 }
 
 __global__ __launch_bounds__(TH, 3) void k_scatter(u64 *k0, u32 *v0, u64 *k1, u32 *v1,
                                                    size_t n_max, const u64 *n_dev,
-                                                   const u64 *orand, int pass,
+                                                   const u64 *bits, int pass,
                                                    const u32 *tile_scan, size_t t_max,
                                                    const u32 *totals) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ u32 wsum[WARPS];
-  const u64 live = live_mask(orand);
+  const u64 live = live_mask(bits);
   if (!pass_live(live, pass)) return;
   const int src = pass_src(live, pass);
   const size_t n = n_dev ? *n_dev : n_max;
@@ -322,8 +316,8 @@ __global__ __launch_bounds__(TH, 3) void k_scatter(u64 *k0, u32 *v0, u64 *k1, u3
 }
 
 __global__ void k_copy_back(u64 *k0, u32 *v0, const u64 *k1, const u32 *v1, size_t n_max,
-                            const u64 *n_dev, const u64 *orand) {
-  if (!pass_src(live_mask(orand), 8)) return;
+                            const u64 *n_dev, const u64 *bits) {
+  if (!pass_src(live_mask(bits), 8)) return;
   const size_t n = n_dev ? *n_dev : n_max;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
@@ -339,13 +333,13 @@ __global__ void k_copy_back(u64 *k0, u32 *v0, const u64 *k1, const u32 *v1, size
 // them in shared memory (stable, as k_scatter), writes its digit counts, and
 // after a grid barrier adds up the other blocks' counts for its offsets and
 // scatters; a second barrier ends the pass. Bound by the barriers and the
-// latency of the steps (about 6 us per live digit at 100k keys); the launches
-// it replaces took 27 us per live digit and 8 us per dead one.
+// latency of the steps (about 12 us per live digit at 105k keys, 4 us at
+// 2,500); the launches it replaces took 27 us per live digit and 8 us per dead one.
 constexpr int CO_TH = 512, CO_WARPS = CO_TH / 32, CO_ITEMS = 8;
 constexpr int kCoopItems = CO_TH * CO_ITEMS;  // keys per block
 
 __global__ __launch_bounds__(CO_TH) void k_sort_coop(u64 *k0, u32 *v0, u64 *k1, u32 *v1,
-                                                     size_t n_max, const u64 *n_dev, u64 *orand,
+                                                     size_t n_max, const u64 *n_dev,
                                                      u32 *counts) {
   namespace cg = cooperative_groups;
   cg::grid_group grid = cg::this_grid();
@@ -353,6 +347,7 @@ __global__ __launch_bounds__(CO_TH) void k_sort_coop(u64 *k0, u32 *v0, u64 *k1, 
   __shared__ u32 part[2][256], part_all[2][256];
   __shared__ u32 dbase[256];
   __shared__ u32 wsum[8];
+  __shared__ u64 s_bits[2];
   const u32 n = (u32)(n_dev ? *n_dev : n_max);
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
   const u32 G = gridDim.x, b = blockIdx.x;
@@ -362,29 +357,33 @@ __global__ __launch_bounds__(CO_TH) void k_sort_coop(u64 *k0, u32 *v0, u64 *k1, 
   const unsigned lt = (1u << lane) - 1;
   u64 key[CO_ITEMS];
   u32 val[CO_ITEMS];
-  u64 o = 0, a = ~0ull;
+  u64 ones = 0, zeros = 0;
 #pragma unroll
   for (int r = 0; r < CO_ITEMS; ++r) {
     const u32 i = base + r * 32;
     if (r < rows && i < n) {
       key[r] = k0[i];
       val[r] = v0[i];
-      o |= key[r];
-      a &= key[r];
+      ones |= key[r];
+      zeros |= ~key[r];
     }
   }
-  {
-    const unsigned olo = __reduce_or_sync(0xffffffffu, (unsigned)o);
-    const unsigned ohi = __reduce_or_sync(0xffffffffu, (unsigned)(o >> 32));
-    const unsigned alo = __reduce_and_sync(0xffffffffu, (unsigned)a);
-    const unsigned ahi = __reduce_and_sync(0xffffffffu, (unsigned)(a >> 32));
-    if (lane == 0) {
-      atomicOr(&orand[0], ((u64)ohi << 32) | olo);
-      atomicAnd(&orand[1], ((u64)ahi << 32) | alo);
-    }
-  }
+  // the bits that differ: the block's to memory, then everybody's
+  u64 *bits = reinterpret_cast<u64 *>(counts + (size_t)G * 256);
+  if (tid < 2) s_bits[tid] = 0;
+  __syncthreads();
+  note_key_bits(ones, zeros, s_bits);
+  __syncthreads();
+  if (tid < 2) __stcg(&bits[2 * b + tid], s_bits[tid]);
   grid.sync();
-  const u64 live = n ? __ldcg(&orand[0]) ^ __ldcg(&orand[1]) : 0;
+  ones = zeros = 0;
+  for (u32 t = tid; t < G; t += CO_TH) {
+    ones |= __ldcg(&bits[2 * t]);
+    zeros |= __ldcg(&bits[2 * t + 1]);
+  }
+  if ((tid & ~31) < G) note_key_bits(ones, zeros, s_bits);
+  __syncthreads();
+  const u64 live = n ? live_mask(s_bits) : 0;
   int src = 0;
   bool loaded = true;  // the first live pass has its keys already
   for (int pass = 0; pass < 8; ++pass) {
@@ -439,7 +438,7 @@ __global__ __launch_bounds__(CO_TH) void k_sort_coop(u64 *k0, u32 *v0, u64 *k1, 
     {  // the digit's count in the blocks before this one, and in all
       const int d = tid & 255, half = tid >> 8;
       u32 before = 0, all = 0;
-#pragma unroll 8
+#pragma unroll 16
       for (u32 t = half; t < G; t += 2) {
         const u32 c = __ldcg(&counts[t * 256 + d]);
         all += c;
@@ -508,19 +507,29 @@ void sort_temp_carve(SortTemp &t, void *base, size_t n_max) {
   t.pass_info = reinterpret_cast<int *>(p);                      // or/and words
 }
 
+// A block's warps take a row of 32 keys each, up to 32 blocks; then four rows:
+// at 105k keys of 24 live bits 52 blocks take 38 us, 103 (two rows) 41, 148
+// 51 and 26 44, the barriers and counts against the rows. Beyond that all SMs.
+static size_t coop_blocks(const rvp_context *ctx, size_t n_max) {
+  const size_t most = std::min(ctx->num_sms, 1024), rows4 = (n_max + 4 * CO_TH - 1) / (4 * CO_TH);
+  return std::min({(n_max + CO_TH - 1) / CO_TH, std::max<size_t>(rows4, 32), most});
+}
+
+u64 *sort_key_bits(rvp_context *ctx, const SortTemp &t, size_t n_max) {
+  if (n_max <= coop_blocks(ctx, n_max) * kCoopItems) return nullptr;  // finds them itself
+  u64 *bits = reinterpret_cast<u64 *>(t.pass_info);
+  RVP_CUDA_TRY(cudaMemsetAsync(bits, 0, 16, ctx->stream));
+  return bits;
+}
+
 void radix_sort_pairs(rvp_context *ctx, u64 *keys, u32 *vals, size_t n_max,
-                      const u64 *n_dev, const SortTemp &t) {
+                      const u64 *n_dev, const SortTemp &t, u64 *bits) {
   if (n_max == 0) return;
-  u64 *orand = reinterpret_cast<u64 *>(t.pass_info);
-  RVP_CUDA_TRY(cudaMemsetAsync(orand, 0x00, 8, ctx->stream));
-  RVP_CUDA_TRY(cudaMemsetAsync(orand + 1, 0xFF, 8, ctx->stream));
   u64 *k0 = keys, *k1 = t.keys_alt;
   u32 *v0 = vals, *v1 = t.vals_alt, *counts = t.tile_hist, *totals = t.global_hist;
-  // one block per SM, each with at least one row of keys per warp
-  const size_t G = std::min<size_t>((n_max + CO_TH - 1) / CO_TH,
-                                    (size_t)std::min(ctx->num_sms, 1024));
+  const size_t G = coop_blocks(ctx, n_max);
   if (n_max <= G * kCoopItems) {
-    void *args[] = {&k0, &v0, &k1, &v1, &n_max, &n_dev, &orand, &counts};
+    void *args[] = {&k0, &v0, &k1, &v1, &n_max, &n_dev, &counts};
     RVP_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(k_sort_coop),
                                              dim3((unsigned)G), dim3(CO_TH), args, 0,
                                              ctx->stream));
@@ -539,12 +548,15 @@ void radix_sort_pairs(rvp_context *ctx, u64 *keys, u32 *vals, size_t n_max,
     RVP_REQUIRE(b > 0, "the sort kernel does not fit on the device");
     per_sm[dev] = b;
   }
-  k_orand<<<grid_for(n_max, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(keys, n_max, n_dev,
-                                                                           orand);
-  RVP_LAUNCH_CHECK(ctx);
+  if (!bits) {
+    bits = sort_key_bits(ctx, t, n_max);
+    k_key_bits<<<grid_for(n_max, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(keys, n_max, n_dev,
+                                                                                bits);
+    RVP_LAUNCH_CHECK(ctx);
+  }
   size_t T = tiles_for(n_max);
   if (T <= (size_t)ctx->num_sms * per_sm[dev]) {
-    void *args[] = {&k0, &v0, &k1, &v1, &n_max, &n_dev, &orand, &counts, &T, &totals};
+    void *args[] = {&k0, &v0, &k1, &v1, &n_max, &n_dev, &bits, &counts, &T, &totals};
     RVP_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(k_sort_tiles),
                                              dim3((unsigned)T), dim3(TH), args, kTilesSmem,
                                              ctx->stream));
@@ -552,16 +564,16 @@ void radix_sort_pairs(rvp_context *ctx, u64 *keys, u32 *vals, size_t n_max,
     return;
   }
   for (int pass = 0; pass < 8; ++pass) {
-    k_hist<<<(unsigned)T, TH, 0, ctx->stream>>>(k0, k1, n_max, n_dev, orand, pass, counts, T);
+    k_hist<<<(unsigned)T, TH, 0, ctx->stream>>>(k0, k1, n_max, n_dev, bits, pass, counts, T);
     RVP_LAUNCH_CHECK(ctx);
-    k_scan_digit<<<256, TH, 0, ctx->stream>>>(counts, T, n_max, n_dev, orand, pass, totals);
+    k_scan_digit<<<256, TH, 0, ctx->stream>>>(counts, T, n_max, n_dev, bits, pass, totals);
     RVP_LAUNCH_CHECK(ctx);
-    k_scatter<<<(unsigned)T, TH, kTilesSmem, ctx->stream>>>(k0, v0, k1, v1, n_max, n_dev, orand,
+    k_scatter<<<(unsigned)T, TH, kTilesSmem, ctx->stream>>>(k0, v0, k1, v1, n_max, n_dev, bits,
                                                            pass, counts, T, totals);
     RVP_LAUNCH_CHECK(ctx);
   }
   k_copy_back<<<grid_for(n_max, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(
-      k0, v0, k1, v1, n_max, n_dev, orand);
+      k0, v0, k1, v1, n_max, n_dev, bits);
   RVP_LAUNCH_CHECK(ctx);
 }
 
@@ -708,6 +720,52 @@ __global__ __launch_bounds__(SC_TH) void k_scan_apply(const u32 *in, size_t n_ma
 }
 }  // namespace
 
+// Up to kScanOne items: one block, 16384 at a time with a carry. The three
+// kernels of the general case take 12 us and two more launches however few
+// items there are; this 5.4 us for 2,500 and 7.7 us for 7,106.
+namespace {
+constexpr size_t kScanOne = 49152;
+constexpr int S1_TH = 1024;
+__global__ __launch_bounds__(S1_TH) void k_scan_one(const u32 *in, size_t n_max, const u64 *n_dev,
+                                                    u64 *out) {
+  __shared__ u64 warp_tot[S1_TH / 32];
+  const size_t n = n_dev ? *n_dev : n_max;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  u64 carry = 0;
+  for (size_t base = 0; base < n; base += S1_TH * SC_IT) {
+    const size_t i0 = base + (size_t)threadIdx.x * SC_IT;
+    u32 v[SC_IT];
+    scan_load(in, i0, n, v);
+    u64 s = 0;
+#pragma unroll
+    for (int j = 0; j < SC_IT; ++j) s += v[j];
+    u64 incl = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const u64 t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    if (lane == 31) warp_tot[w] = incl;
+    __syncthreads();
+    u64 t = warp_tot[lane], ti = t;  // every warp scans the warps' totals
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const u64 p = __shfl_up_sync(0xffffffffu, ti, o);
+      if (lane >= o) ti += p;
+    }
+    u64 run = carry + incl - s + __shfl_sync(0xffffffffu, ti - t, w);
+    carry += __shfl_sync(0xffffffffu, ti, 31);
+#pragma unroll
+    for (int j = 0; j < SC_IT; ++j) {
+      if (i0 + j < n) out[i0 + j] = run;
+      run += v[j];
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) out[n] = carry;
+}
+}  // namespace
+
 size_t scan_temp_bytes(size_t n_max) {
   return al(((n_max + SC_TILE - 1) / SC_TILE + 1) * 8);
 }
@@ -720,6 +778,11 @@ void exclusive_scan_u32_to_u64(rvp_context *ctx, const u32 *in, u64 *out, size_t
 void exclusive_scan_u32_to_u64_batch(rvp_context *ctx, const u32 *in, size_t in_stride, u64 *out,
                                      size_t out_stride, int batch, size_t n_max,
                                      const u64 *n_dev, void *temp) {
+  if (batch == 1 && n_max <= kScanOne) {
+    k_scan_one<<<1, S1_TH, 0, ctx->stream>>>(in, n_max, n_dev, out);
+    RVP_LAUNCH_CHECK(ctx);
+    return;
+  }
   const size_t nt = (n_max + SC_TILE - 1) / SC_TILE;
   const size_t ts_stride = scan_temp_bytes(n_max) / 8;
   u64 *tsum = static_cast<u64 *>(temp);

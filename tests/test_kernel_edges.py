@@ -151,6 +151,22 @@ def test_tree_radius(gpu_ctx, n, radius, cloud):
         assert np.array_equal(idx3, first)
 
 
+# list offsets: one block scans up to 49152 counts, 16384 at a time
+@pytest.mark.parametrize("n", [16_383, 16_385, 49_152, 49_153])
+def test_radius_offsets(gpu_ctx, n):
+    from rvpoint_b200 import api
+    i = np.arange(n)
+    c = D.Cloud.from_xyz(np.stack([i % 37, (i // 37) % 41, i // 1517], 1) * 0.25)
+    h = api.SpatialHash()
+    h.setInputCloud(c, 0.5)
+    h.build()
+    q = c.aos()
+    q[::3, 2] = 1e3  # nothing near these
+    offs, idx, d2 = h.radiusSearchBatch(q[:, 0], q[:, 1], q[:, 2], 0.1)
+    assert np.array_equal(np.diff(offs), (i % 3 != 0).astype(np.int64))
+    assert np.array_equal(idx, i[i % 3 != 0]) and not d2.any()
+
+
 @pytest.mark.parametrize("radius", [0.0, 0.03, 0.3, 2.0])  # 0, tens, hundreds, all as neighbours
 def test_radius_normals_lists(gpu_ctx, restatement, radius):
     from rvpoint_b200 import api
