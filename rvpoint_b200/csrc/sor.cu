@@ -5,6 +5,8 @@
 //    threshold; k_sor_stats reproduces those roundings in parallel;
 //  * keep mean <= mu + alpha * sigma and copy kept points out in input order
 //    (flag scan + scatter).
+#include <cooperative_groups.h>
+
 #include "internal.cuh"
 
 namespace rvp {
@@ -26,17 +28,25 @@ __device__ __forceinline__ int frame_of_index(const int64_t *offs, int n_frames,
 // u = 2^(e-23), and adding v >= 0, v = (q + r) u, moves S by an integer: q
 // (r < 1/2), q + 1 (r > 1/2), or, on a tie, to the even neighbour. Without
 // ties the moves do not depend on S: they are summed (exactly, as floats
-// below 2^24 u) by a block scan. With a tie among them every value becomes a
-// pair of increments (S even, S odd), which compose associatively, and the
-// scan runs over the pairs. Either way S after every value has exactly the
-// roundings of the loop. The thread in whose run S first reaches 2^24 (the
-// next binade) adds its own values one by one in float, and the rest of the
-// chunk is scanned again from there: about log2(n) times over the whole sum,
-// so the chunks start at 512 values and double up to 8192.
-//   Bound by one SM's issue and the scans' latency (a block per frame): 89,343
-// values 544 us with one lane adding in order (a dependent add per value),
-// 123 us here; 256 frames of 11 M values 379 and 182 us.
-constexpr int ST_TH = 512, ST_IT = 16, ST_CHUNK = ST_TH * ST_IT;
+// below 2^24 u). With a tie among them every value becomes a pair of
+// increments (S even, S odd), which compose associatively. Either way S after
+// every value has exactly the roundings of the loop.
+//   Three steps, twice (the mean, then the squares about it): the blocks of a
+// cluster add up their shares in double; knowing about where the sum stands,
+// each warp makes the pair of each of its segments of 256 values for that
+// binade; and the first block composes the pairs from the true sum, 512
+// segments at a time. Where a segment's binade was not foreseen, or the sum
+// leaves it within the segment (about log2(n / 256) times), one lane adds the
+// segment's values in order; after a run of such segments (sums that rounding
+// has taken far from their true values) the block takes 4096 values at a time
+// in the binade that it is in.
+//   Bound by the first block's steps at each binade: 89,343 values 544 us with
+// one lane adding in order (a dependent add per value), 123 us with one block
+// making the pairs as it went, 52 us here; 256 frames of 11 M values 379, 182
+// and 95 us.
+constexpr int ST_TH = 512, ST_IT = 8, ST_CHUNK = ST_TH * ST_IT;
+constexpr int ST_SEG = 256;         // values of a segment
+constexpr int ST_FEW = 4 * ST_SEG;  // up to these one lane adds all
 constexpr u32 ST_TOP = 1u << 24, ST_CAP = 1u << 30;
 
 struct Incr {  // increments of S when it is even / odd, capped at ST_CAP
@@ -71,187 +81,300 @@ __device__ __forceinline__ Incr incr_of(float v, int ex) {
   return Incr{q + (q & 1), q + ((q & 1) ^ 1)};
 }
 
-__global__ __launch_bounds__(ST_TH) void k_sor_stats(const float *__restrict__ mean,
+// S as the sum again: below 2^24 in the binade of exponent ex, else past it
+__device__ __forceinline__ float st_float(u32 t, int ex) {
+  return t >= ST_TOP ? __uint_as_float((u32)(ex + 1) << 23)
+                     : __uint_as_float(t >= 0x800000u ? ((u32)ex << 23) | (t & 0x7FFFFFu) : t);
+}
+// what pass 1 adds for a value
+__device__ __forceinline__ float st_value(float v, int pass, float mu) {
+  if (pass == 0) return v;
+  v = fsub(v, mu);
+  return fmul(v, v);
+}
+// the moves of S without ties: rounded to units by adding and taking away
+// 1.5 * 2^23 u, which needs v < 2^22 u
+struct StMoves {
+  float magic, half, most;
+  __device__ __forceinline__ explicit StMoves(int ex) {
+    magic = __uint_as_float(((u32)ex << 23) | 0x400000u);
+    half = ex > 30 ? __uint_as_float((u32)(ex - 24) << 23) : 0.0f;  // u / 2
+    most = __uint_as_float((u32)(ex - 1) << 23);                    // 2^22 u
+  }
+  __device__ __forceinline__ float of(float v, bool &hard) const {
+    const float q = fsub(fadd(v, magic), magic);
+    hard = hard || fabsf(fsub(v, q)) == half || !(v < most);
+    return q;
+  }
+};
+// inclusive scan of a block's pairs (warp_tot: one per warp)
+__device__ __forceinline__ Incr incr_scan(Incr v, Incr *warp_tot, Incr &before) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  auto up = [&](Incr x, int o) {
+    return Incr{__shfl_up_sync(0xffffffffu, x.a, o), __shfl_up_sync(0xffffffffu, x.b, o)};
+  };
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const Incr p = up(v, o);
+    if (lane >= o) v = incr_then(p, v);
+  }
+  if (lane == 31) warp_tot[warp] = v;
+  __syncthreads();
+  Incr t = lane < ST_TH / 32 ? warp_tot[lane] : Incr{0, 0};  // every warp scans the totals
+#pragma unroll
+  for (int o = 1; o < ST_TH / 32; o <<= 1) {
+    const Incr p = up(t, o);
+    if (lane >= o) t = incr_then(p, t);
+  }
+  const int w = warp > 0 ? warp - 1 : 0;
+  Incr pre{__shfl_sync(0xffffffffu, t.a, w), __shfl_sync(0xffffffffu, t.b, w)};
+  if (warp == 0) pre = Incr{0, 0};
+  before = up(v, 1);
+  before = incr_then(pre, lane == 0 ? Incr{0, 0} : before);
+  return incr_then(pre, v);
+}
+
+// a segment's pair for the binade ex (0: none), as 16 bytes
+struct StSeg {
+  u64 pair, ex;
+};
+
+// by a whole block: acc after m <= ST_CHUNK values, whatever they are
+__device__ float st_chunk(const float *mean, int m, int pass, float mu, float acc, float *buf,
+                          Incr *warp_tot, float *s_acc, int *s_next) {
+  const int tid = threadIdx.x;
+  bool odd = false;  // a value the increments cannot express
+  for (int i = tid; i < m; i += ST_TH) {
+    const float v = st_value(__ldg(&mean[i]), pass, mu);
+    odd = odd || !(v >= 0.0f && v < INFINITY);
+    buf[i + i / ST_IT] = v;  // (a gap per run: no bank conflicts)
+  }
+  odd = __syncthreads_or(odd) || !(acc < INFINITY);
+  if (odd) {  // (infinities, NaN, negative values): one lane, in order
+    if (tid == 0) {
+      float s = acc;
+      for (int i = 0; i < m; ++i) s = fadd(s, buf[i + i / ST_IT]);
+      *s_acc = s;
+    }
+    __syncthreads();
+    return *s_acc;
+  }
+  const int runs = (m + ST_IT - 1) / ST_IT;  // threads with values
+  float v[ST_IT];
+#pragma unroll
+  for (int j = 0; j < ST_IT; ++j)
+    v[j] = tid * ST_IT + j < m ? buf[tid * (ST_IT + 1) + j] : 0.0f;
+  int from = 0;  // threads before it are added already
+  while (from < runs) {
+    const int ex = st_exp(acc);
+    const float top = __uint_as_float((u32)(ex + 1) << 23);  // 2^24 u (inf past the last)
+    const bool mine = tid >= from && tid < runs;
+    Incr run{0, 0};
+    if (mine) {
+      Incr t[ST_IT];
+#pragma unroll
+      for (int j = 0; j < ST_IT; ++j) t[j] = incr_of(v[j], ex);
+#pragma unroll
+      for (int w = 1; w < ST_IT; w <<= 1)  // pairwise, in order: a short chain
+#pragma unroll
+        for (int j = 0; j < ST_IT; j += 2 * w) t[j] = incr_then(t[j], t[j + w]);
+      run = t[0];
+    }
+    const u32 s0 = st_sig(acc);
+    Incr pre;
+    const Incr end = incr_scan(run, warp_tot, pre);
+    const float pre_acc = st_float(s0 + (s0 & 1 ? pre.b : pre.a), ex);
+    const float end_acc = st_float(s0 + (s0 & 1 ? end.b : end.a), ex);
+    if (tid == ST_TH - 1 && end_acc < top) *s_acc = end_acc, *s_next = runs;
+    if (mine && pre_acc < top && !(end_acc < top)) {  // one thread leaves the binade
+      float s = pre_acc;
+#pragma unroll
+      for (int j = 0; j < ST_IT; ++j) s = fadd(s, v[j]);
+      *s_acc = s;
+      *s_next = tid + 1;
+    }
+    __syncthreads();
+    acc = *s_acc;
+    from = *s_next;
+    if (!(acc < INFINITY)) break;  // overflow: every later sum is infinite too
+    __syncthreads();
+  }
+  __syncthreads();
+  return acc;
+}
+
+__global__ __launch_bounds__(ST_TH, 2) void k_sor_stats(const float *__restrict__ mean_all,
                                                      const int64_t *offs, int n_frames,
-                                                     float alpha, float *thresh) {
-  __shared__ float buf[ST_CHUNK + ST_CHUNK / ST_IT];  // a gap per run: no bank conflicts
+                                                     float alpha, float *thresh, u64 *temp) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  __shared__ float buf[ST_CHUNK + ST_CHUNK / ST_IT];
   __shared__ Incr warp_tot[ST_TH / 32];
-  __shared__ float warp_sum[ST_TH / 32];
-  __shared__ float s_acc;
+  __shared__ double share[ST_TH / 32];  // sums of the warps' shares
+  __shared__ float s_acc, s_mu;
   __shared__ int s_next;
-  const int f = blockIdx.x;
-  if (f >= n_frames) return;
+  const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int f = blockIdx.x / C;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int64_t a = offs[f], n = offs[f + 1] - a;
-  if (n <= 0) {
-    if (tid == 0) thresh[f] = 0.0f;
+  if (n <= 0) {  // (the whole cluster)
+    if (rank == 0 && tid == 0) thresh[f] = 0.0f;
     return;
   }
-  mean += a;
+  const float *mean = mean_all + a;
+  StSeg *segs = reinterpret_cast<StSeg *>(temp + 2 * ((a + 1) / 2));
+  const int64_t n_seg = (n + ST_SEG - 1) / ST_SEG;
+  const bool ahead = n > ST_FEW;  // (few enough: nothing is foreseen)
+  // each warp's share of the segments
+  const int W = C * (ST_TH / 32), me = rank * (ST_TH / 32) + warp;
+  const int64_t lo = ahead ? n_seg * me / W : 0, hi = ahead ? n_seg * (me + 1) / W : 0;
+  constexpr int IT = ST_SEG / 32;
   float mu = 0.0f;
   for (int pass = 0; pass < 2; ++pass) {
-    float acc = 0.0f;
-    float nxt[ST_IT];
-    auto chunk_at = [&](int64_t base) {
-      const int64_t len = base < 512 ? 512 : (base < ST_CHUNK ? base : ST_CHUNK);
-      return (int)(n - base < len ? n - base : len);
-    };
-    auto fetch = [&](int64_t base) {
-      const int m = base < n ? chunk_at(base) : 0;
+    if (ahead) {
+      double sum = 0.0;
+      for (int64_t i = lo * ST_SEG + lane, e = min(hi * ST_SEG, n); i < e; i += 32)
+        sum += st_value(__ldg(&mean[i]), pass, mu);
 #pragma unroll
-      for (int j = 0; j < ST_IT; ++j) {
-        const int i = j * ST_TH + tid;
-        nxt[j] = i < m ? __ldg(&mean[base + i]) : mu;
-      }
-    };
-    fetch(0);
-    for (int64_t base = 0; base < n;) {
-      const int m = chunk_at(base);
-      bool odd = false;  // a value the increments cannot express
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (lane == 0) share[warp] = sum;
+      cluster.sync();
+      double at = 0.0;  // about the sum before the warp's share
+      for (int w = lane; w < me; w += 32)
+        at += *cluster.map_shared_rank(&share[w % (ST_TH / 32)], w / (ST_TH / 32));
 #pragma unroll
-      for (int j = 0; j < ST_IT; ++j) {
-        const int i = j * ST_TH + tid;
-        if (j * ST_TH >= m) break;  // (uniform) rows past the chunk's end
-        float v = nxt[j];
-        if (pass == 1) {
-          v = fsub(v, mu);
-          v = fmul(v, v);
+      for (int o = 16; o > 0; o >>= 1) at += __shfl_xor_sync(0xffffffffu, at, o);
+      for (int64_t g = lo; g < hi; ++g) {
+        const int m = (int)min((int64_t)ST_SEG, n - g * ST_SEG);
+        float v[IT];
+        bool odd = false;
+        float part = 0.0f;
+#pragma unroll
+        for (int j = 0; j < IT; ++j) {  // (lane's run is IT consecutive values)
+          const int i = lane * IT + j;
+          v[j] = i < m ? st_value(__ldg(&mean[g * ST_SEG + i]), pass, mu) : 0.0f;
+          odd = odd || !(v[j] >= 0.0f && v[j] < INFINITY);
+          part += v[j];
         }
-        odd = odd || !(v >= 0.0f && v < INFINITY);
-        buf[i + i / ST_IT] = v;
-      }
-      odd = __syncthreads_or(odd) || !(acc < INFINITY);
-      base += m;
-      if (odd) {  // (infinities, NaN, negative values): one lane, in order
-        if (tid == 0) {
-          float s = acc;
-          for (int i = 0; i < m; ++i) s = fadd(s, buf[i + i / ST_IT]);
-          s_acc = s;
-        }
-        fetch(base);
-        __syncthreads();
-        acc = s_acc;
-        continue;
-      }
-      const int runs = (m + ST_IT - 1) / ST_IT;  // threads with values
-      float v[ST_IT];
+        double total = part;
 #pragma unroll
-      for (int j = 0; j < ST_IT; ++j) v[j] = tid < runs ? buf[tid * (ST_IT + 1) + j] : 0.0f;
-      fetch(base);
-      int from = 0;  // threads before it are added already
-      while (from < runs) {
-        const int ex = st_exp(acc);
-        const bool mine = tid >= from && tid < runs;
-        // moves without ties: rounded to units by adding and taking away
-        // 1.5 * 2^23 u, which needs v < 2^22 u
-        const float magic = __uint_as_float(((u32)ex << 23) | 0x400000u);
-        const float top = __uint_as_float((u32)(ex + 1) << 23);  // 2^24 u (inf past the last)
-        const float half = ex > 30 ? __uint_as_float((u32)(ex - 24) << 23) : 0.0f;  // u / 2
-        const float most = __uint_as_float((u32)(ex - 1) << 23);  // 2^22 u
-        float sum = 0.0f;
-        bool hard = ex <= 30;
-        if (mine) {
+        for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+        const int ex = st_exp((float)at);
+        at += total;
+        StSeg r{0, 0};
+        if (!__any_sync(0xffffffffu, odd) && at < 3.0e38 && ex == st_exp((float)at)) {
+          const StMoves mv(ex);
+          bool hard = ex <= 30;
+          float q = 0.0f;
 #pragma unroll
-          for (int j = 0; j < ST_IT; ++j) {
-            const float q = fsub(fadd(v[j], magic), magic);
-            hard = hard || fabsf(fsub(v[j], q)) == half || !(v[j] < most);
-            sum = fadd(sum, q);
+          for (int j = 0; j < IT; ++j) q = fadd(q, mv.of(v[j], hard));
+          if (!__any_sync(0xffffffffu, hard)) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) q = fadd(q, __shfl_xor_sync(0xffffffffu, q, o));
+            // (2^(150 - ex): units per one; capped as the pairs are)
+            const float units = fmul(q, __uint_as_float((u32)(277 - ex) << 23));
+            const u32 k = units < 1073741824.0f ? (u32)units : ST_CAP;
+            r.pair = ((u64)k << 32) | k;
+          } else {
+            Incr t{0, 0};
+#pragma unroll
+            for (int j = 0; j < IT; ++j) t = incr_then(t, incr_of(v[j], ex));
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+              const Incr p{__shfl_up_sync(0xffffffffu, t.a, o),
+                           __shfl_up_sync(0xffffffffu, t.b, o)};
+              if (lane >= o) t = incr_then(p, t);
+            }
+            r.pair = ((u64)__shfl_sync(0xffffffffu, t.b, 31) << 32) |
+                     __shfl_sync(0xffffffffu, t.a, 31);
           }
+          r.ex = (u64)ex;
         }
-        float incl = sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const float p = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl = fadd(p, incl);
+        if (lane == 0) {
+          __stcg(&segs[g].pair, r.pair);
+          __stcg(&segs[g].ex, r.ex);
         }
-        if (lane == 31) warp_sum[warp] = incl;
-        hard = __syncthreads_or(hard);
-        float pre_acc, end_acc, all_acc;  // the sum before and after this run, and at the end
-        if (!hard) {
-          float before = 0.0f, total = 0.0f;
-#pragma unroll
-          for (int w = 0; w < ST_TH / 32; ++w) {
-            if (w == warp) before = total;
-            total = fadd(total, warp_sum[w]);
-          }
-          float pre = __shfl_up_sync(0xffffffffu, incl, 1);
-          pre = fadd(before, lane == 0 ? 0.0f : pre);
-          pre_acc = fadd(acc, pre);
-          end_acc = fadd(acc, fadd(before, incl));
-          all_acc = fadd(acc, total);
-        } else {
+      }
+      cluster.sync();
+    }
+    if (rank == 0) {
+      float acc = 0.0f;
+      int alone = 0;  // segments in a row that were not foreseen
+      for (int64_t w0 = 0; w0 < n_seg;) {
+        const int count = (int)min((int64_t)ST_TH, n_seg - w0);
+        StSeg r{0, 0};
+        if (ahead && tid < count) {
+          r.pair = __ldcg(&segs[w0 + tid].pair);
+          r.ex = __ldcg(&segs[w0 + tid].ex);
+        }
+        int from = 0;
+        while (from < count) {
+          const int ex = st_exp(acc);
           const u32 s0 = st_sig(acc);
-          auto to_float = [&](u32 t) {  // below 2^24: in acc's binade; else past it
-            return t >= ST_TOP ? top
-                               : __uint_as_float(t >= 0x800000u ? ((u32)ex << 23) | (t & 0x7FFFFFu)
-                                                                : t);
-          };
-          Incr run{0, 0};
-          if (mine) {
-            Incr t[ST_IT];
-#pragma unroll
-            for (int j = 0; j < ST_IT; ++j) t[j] = incr_of(v[j], ex);
-#pragma unroll
-            for (int w = 1; w < ST_IT; w <<= 1)  // pairwise, in order: a short chain
-#pragma unroll
-              for (int j = 0; j < ST_IT; j += 2 * w) t[j] = incr_then(t[j], t[j + w]);
-            run = t[0];
-          }
-          Incr upto = run;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            Incr p;
-            p.a = __shfl_up_sync(0xffffffffu, upto.a, o);
-            p.b = __shfl_up_sync(0xffffffffu, upto.b, o);
-            if (lane >= o) upto = incr_then(p, upto);
-          }
-          if (lane == 31) warp_tot[warp] = upto;
+          const bool fits = tid >= from && tid < count && (int)r.ex == ex;
+          // (uniform: the next segment was not foreseen)
+          if (tid == from) s_next = fits ? ST_TH : from;
           __syncthreads();
-          Incr before{0, 0}, total{0, 0};
-#pragma unroll
-          for (int w = 0; w < ST_TH / 32; ++w) {
-            if (w == warp) before = total;
-            total = incr_then(total, warp_tot[w]);
+          if (s_next > from) {
+            Incr pre;
+            const Incr run = fits ? Incr{(u32)r.pair, (u32)(r.pair >> 32)} : Incr{0, 0};
+            const Incr end = incr_scan(run, warp_tot, pre);
+            const u32 s1 = s0 + (s0 & 1 ? end.b : end.a), s = s0 + (s0 & 1 ? pre.b : pre.a);
+            const bool stop = tid >= from && (!fits || s1 >= ST_TOP);
+            if (stop) atomicMin(&s_next, tid);
+            if (tid == ST_TH - 1) s_acc = st_float(s1, ex);
+            __syncthreads();
+            if (tid == s_next) s_acc = st_float(s, ex);  // the sum before it
+            __syncthreads();
+            acc = s_acc;
+            if (s_next > from) alone = 0;
+            from = s_next;
           }
-          Incr pre;  // everything before this thread's run
-          pre.a = __shfl_up_sync(0xffffffffu, upto.a, 1);
-          pre.b = __shfl_up_sync(0xffffffffu, upto.b, 1);
-          if (lane == 0) pre = Incr{0, 0};
-          pre = incr_then(before, pre);
-          const Incr end = incr_then(pre, run);
-          const bool p0 = s0 & 1;
-          pre_acc = to_float(s0 + (p0 ? pre.b : pre.a));
-          end_acc = to_float(s0 + (p0 ? end.b : end.a));
-          all_acc = to_float(s0 + (p0 ? total.b : total.a));
-        }
-        if (all_acc < top) {
-          acc = all_acc;
-          break;
-        }
-        if (mine && pre_acc < top && !(end_acc < top)) {  // one thread
-          float s = pre_acc;
-#pragma unroll
-          for (int j = 0; j < ST_IT; ++j) s = fadd(s, v[j]);
-          s_acc = s;
-          s_next = tid + 1;
+          if (from >= count) break;
+          const int64_t i0 = (w0 + from) * ST_SEG;
+          if (alone < 8) {
+            const int m = (int)min((int64_t)ST_SEG, n - i0);
+            __syncthreads();
+            if (tid < ST_SEG) buf[tid] = tid < m ? st_value(__ldg(&mean[i0 + tid]), pass, mu) : 0.0f;
+            __syncthreads();
+            if (tid == 0) {
+              float s = acc;
+              if (m == ST_SEG) {
+#pragma unroll 32
+                for (int i = 0; i < ST_SEG; ++i) s = fadd(s, buf[i]);
+              } else {
+                for (int i = 0; i < m; ++i) s = fadd(s, buf[i]);
+              }
+              s_acc = s;
+            }
+            __syncthreads();
+            acc = s_acc;
+            ++alone;
+            ++from;
+          } else {
+            const int m = (int)min((int64_t)ST_CHUNK, n - i0);
+            __syncthreads();
+            acc = st_chunk(mean + i0, m, pass, mu, acc, buf, warp_tot, &s_acc, &s_next);
+            alone = 8 - 1;  // the next one may be foreseen again
+            from += (m + ST_SEG - 1) / ST_SEG;
+          }
         }
         __syncthreads();
-        acc = s_acc;
-        from = s_next;
-        if (!(acc < INFINITY)) {  // overflow: every later sum is infinite too
-          acc = INFINITY;
-          break;
-        }
+        w0 += from;
       }
-      __syncthreads();  // buf and the warps' totals are refilled
+      if (pass == 0) {
+        if (tid == 0) s_mu = fdiv(acc, (float)n);
+      } else if (tid == 0) {
+        const float sd = __fsqrt_rn(fdiv(acc, (float)n));
+        thresh[f] = fadd(mu, fmul(alpha, sd));
+      }
     }
     if (pass == 0) {
-      mu = fdiv(acc, (float)n);
-    } else if (tid == 0) {
-      const float sd = __fsqrt_rn(fdiv(acc, (float)n));
-      thresh[f] = fadd(mu, fmul(alpha, sd));
+      cluster.sync();
+      mu = *cluster.map_shared_rank(&s_mu, 0);
     }
   }
+  cluster.sync();  // (its shared memory is read until here)
 }
 
 __global__ void k_sor_keep(const float *mean, const int64_t *offs, int n_frames, size_t n_max,
@@ -317,8 +440,23 @@ void sor_filter_frames(rvp_context *ctx, const float *x, const float *y, const f
   p += al((size_t)(n_frames + 1) * 4);
   void *scan_tmp = p;
   cudaStream_t st = ctx->stream;
-  k_sor_stats<<<(unsigned)(n_frames > 0 ? n_frames : 1), ST_TH, 0, st>>>(mean, offs, n_frames,
-                                                                       alpha, thresh);
+  // 8 blocks per frame while the device holds them all at once (2 per SM: one
+  // frame of 89,343 values 52 us); a block each for more frames, whose first
+  // blocks would wait their turn with seven idle ones beside them
+  const int frames = n_frames > 0 ? n_frames : 1;
+  const unsigned C = frames * 8 <= ctx->num_sms * 2 ? 8 : 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)frames * C);
+  cfg.blockDim = dim3(ST_TH);
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = C;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  // (pos is free until the scan: 8 bytes per value, a segment needs 16)
+  RVP_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_sor_stats, mean, offs, n_frames, alpha, thresh, pos));
   RVP_LAUNCH_CHECK(ctx);
   k_sor_keep<<<grid_for(n_max, 256, ctx->num_sms * 16), 256, 0, st>>>(mean, offs, n_frames, n_max,
                                                                      n_dev, thresh, keep, flags);

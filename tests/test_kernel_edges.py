@@ -29,6 +29,36 @@ def test_sor_statistics_sum_in_order(gpu_ctx, restatement, n, cloud):
     assert np.array_equal(keep, keep2) and np.array_equal(bits(out), bits(out2))
 
 
+# SOR statistics from 1025 values on: pairs of segments of 256, 512 at a time;
+# one value near 2^20 first takes the float sum away from the true one (0.1 is
+# rounded to 0.125), so the binades foreseen for whole runs are not the sum's
+@pytest.mark.parametrize("n,far", [(1024, 0), (1025, 0), (30_000, 0), (30_000, 2**20 - 2000),
+                                   (131_330, 0)])
+def test_sor_statistics_segments(gpu_ctx, n, far):
+    from rvpoint_b200.api import sor_rvv
+    i = np.arange(n)
+    p = np.stack([i % 31, (i // 31) % 37, i // 1147], 1).astype(np.float32) * np.float32(0.1)
+    if far:
+        p[0] = [-far, 0, 0]
+    else:
+        p += np.random.default_rng(n).uniform(0, 0.05, p.shape).astype(np.float32)
+    c = D.Cloud.from_xyz(p)
+    _, mean, _ = sor_rvv(c, 3, 0.5, return_stats=True)
+    f = np.float32
+    mu = np.add.accumulate(mean)[-1] / f(n)  # in order, in float
+    sd = np.sqrt(np.add.accumulate((mean - mu) * (mean - mu))[-1] / f(n))
+    # a threshold on a value: one unit less would drop its point
+    target = np.sort(mean)[int(0.7 * n)] if not far else np.sort(mean)[-2]
+    alpha = f((target - mu) / sd)
+    for _ in range(64):
+        t = mu + alpha * sd
+        if t == target:
+            break
+        alpha = np.nextafter(alpha, f(np.inf) if t < target else f(-np.inf))
+    _, _, keep = sor_rvv(c, 3, float(alpha), return_stats=True)
+    assert np.array_equal(keep.astype(bool), mean <= mu + alpha * sd)
+
+
 # the voxel grid sorts its keys: up to 148 x 4096 of them in one cooperative
 # kernel (512 threads, up to eight keys each), more in tiles of 4096
 @pytest.mark.parametrize("n", [1, 31, 513, 4097, 75_777, 606_208, 606_209, 2_424_833])
