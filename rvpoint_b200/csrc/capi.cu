@@ -253,7 +253,13 @@ void knn_cloud(rvp_context *ctx, const float *x, const float *y, const float *z,
                int mode, const rvp::TreeOut &o) {
   rvp::KnnTree &w = ctx_tree(ctx);
   const rvp::TreeView t = rvp::tree_build(ctx, w, x, y, z, n);
-  rvp::tree_knn(ctx, t, rvp::tree_queries(ctx, w, t, x, y, z, x, y, z, n), K, 0.0f, mode, o);
+  rvp::TreeOut out = o;
+  if (mode == rvp::TREE_PRECISE) {
+    const u32 packets = (u32)((n + 31) / 32);
+    w.rows.reserve((size_t)rvp::tree_precise_packets(packets, K) * K * 128);
+    out.rows = w.rows.as<u32>();
+  }
+  rvp::tree_knn(ctx, t, rvp::tree_queries(ctx, w, t, x, y, z, x, y, z, n), K, 0.0f, mode, out);
 }
 
 // the tree over a hash's points (kept until it takes another cloud)

@@ -453,12 +453,18 @@ struct TreeOut {  // by query index; null pointers are skipped
   double cond_fp64 = 0.0;
   float *cond = nullptr;
   uint8_t *used64 = nullptr;
-  u32 *rows = nullptr;
+  u32 *rows = nullptr;   // (TREE_PRECISE: room for tree_precise_packets packets of k * 32)
+  u32 packet0 = 0;       // TREE_PRECISE: the first packet of a part
   const u64 *out_pos = nullptr;  // where a point's normal goes (null: its index)
   u32 *n_packets = nullptr, *n_hard = nullptr;  // counters: queries of each kernel
 };
+// TREE_PRECISE keeps rows for this many packets at once (at most 512 MB)
+inline u32 tree_precise_packets(u32 packets, int k) {
+  const u32 most = (u32)((512u << 20) / ((size_t)k * 128));
+  return packets < most ? packets : most;
+}
 struct KnnTree {
-  DevBuf keys, vals, sort, pts, pos, boxes, misc, qkeys, qvals, qpts, hard;
+  DevBuf keys, vals, sort, pts, pos, boxes, misc, qkeys, qvals, qpts, hard, rows;
   void reserve_frames(size_t n_max, int n_frames);
   void release();
 };
@@ -482,6 +488,12 @@ size_t tree_frames_positions(size_t n_max, int n_frames);
 TreeView tree_build_frames(rvp_context *ctx, KnnTree &w, const float *x, const float *y,
                            const float *z, const float *aos, const int64_t *offs, int n_frames,
                            size_t n_max, u64 *keys, u32 *vals, void *sort_temp);
+// the same for many small frames of up to kSmallFrame points (x, y, z finite
+// and below 1e18); other frames get no tree and skipped[f] = 1
+constexpr int kSmallFrame = 2048;
+TreeView tree_build_small_frames(rvp_context *ctx, KnnTree &w, const float *x, const float *y,
+                                 const float *z, const int64_t *offs, int n_frames, size_t n_max,
+                                 int32_t *skipped);
 void tree_frames_mark_removed(rvp_context *ctx, const TreeView &t, const uint8_t *keep);
 void tree_knn_frames(rvp_context *ctx, KnnTree &w, const TreeView &t, const u32 *list,
                      const u64 *n_list, int k, int mode, const TreeOut &o);

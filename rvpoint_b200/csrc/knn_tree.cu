@@ -142,6 +142,7 @@ __global__ void k_tree_queries(const float *__restrict__ x, const float *__restr
 void KnnTree::release() {
   keys.release(); vals.release(); sort.release(); pts.release(); pos.release(); boxes.release();
   misc.release(); qkeys.release(); qvals.release(); qpts.release(); hard.release();
+  rows.release();
 }
 
 TreeView tree_build(rvp_context *ctx, KnnTree &w, const float *x, const float *y, const float *z,

@@ -273,16 +273,20 @@ constexpr int kLeafBudget = 128;
 // distances and later (in the same place) the collected points, and the
 // positions in order where a normal follows
 constexpr int kTreeLeaves = (kLeafBudget + 3 + 3) & ~3;
-template <int KCAP, int MODE>
-constexpr size_t tree_buffer() {
-  constexpr size_t dist = (size_t)kTreeBuf * 32 * 4;
-  constexpr size_t near = (size_t)(KCAP + kTreeExtra) * 32 * 8;
-  return MODE != TREE_MEAN && near > dist ? near : dist;
-}
+// leaves whose hits are noted before they are collected (with lists of up to
+// 16 the notes fit behind them in the buffer)
+constexpr int kTreeNotes = 24;
+// the buffer: distances; then the collected points and, behind them, the notes
+// and after these the sorted positions (each lane in its own column)
+template <int KCAP>
+constexpr size_t tree_near() { return (size_t)(KCAP + kTreeExtra) * 32 * 8; }
 template <int KCAP, int MODE>
 constexpr size_t tree_smem() {
-  return 3 * 32 * 4 + kTreeLeaves * 4 + tree_buffer<KCAP, MODE>() +
-         (MODE == TREE_NORMALS || MODE == TREE_PRECISE ? (size_t)(KCAP + 1) * 32 * 4 : 0);
+  constexpr size_t dist = (size_t)kTreeBuf * 32 * 4;
+  constexpr bool normals = MODE == TREE_NORMALS || MODE == TREE_PRECISE;
+  constexpr size_t behind = (normals && KCAP + 1 > kTreeNotes ? KCAP + 1 : kTreeNotes) * 32 * 4;
+  constexpr size_t list = tree_near<KCAP>() + behind;
+  return 3 * 32 * 4 + kTreeLeaves * 4 + (MODE != TREE_MEAN && list > dist ? list : dist);
 }
 
 // Compare-exchange networks over registers. They are straight code: batches of
@@ -372,9 +376,10 @@ __global__ __launch_bounds__(32, KCAP > 32 ? 10 : 16) void k_knn_tree(TreeView t
   unsigned char *buf = tree_sm + 384 + kTreeLeaves * 4;
   float(*fbuf)[32] = reinterpret_cast<float(*)[32]>(buf);
   uint2(*pbuf)[32] = reinterpret_cast<uint2(*)[32]>(buf);
-  u32(*sorted)[32] = reinterpret_cast<u32(*)[32]>(buf + tree_buffer<KCAP, MODE>());
+  u32(*notes)[32] = reinterpret_cast<u32(*)[32]>(buf + tree_near<KCAP>());
+  u32(*sorted)[32] = notes;
   const int lane = threadIdx.x;
-  const u32 packet = blockIdx.x;
+  const u32 packet = blockIdx.x + (MODE == TREE_PRECISE ? o.packet0 : 0u);
   // the cloud's own points (leaf `packet`), or 32 of the sorted queries
   const bool self = FRAMES || qs.n_sort == nullptr || *qs.n_sort == 0;
   const float4 *src = self ? t.pts : qs.q;
@@ -453,8 +458,8 @@ __global__ __launch_bounds__(32, KCAP > 32 ? 10 : 16) void k_knn_tree(TreeView t
     return true;
   };
   const u64 nqx = pack2(-q.x, -q.x), nqy = pack2(-q.y, -q.y), nqz = pack2(-q.z, -q.z);
-  // hit(c, d2) for the staged points c within `at`, except `skip`
-  auto test_staged = [&](float at, int skip, auto &&hit) {
+  // hit(c, d2) for the staged points c within `at`
+  auto test_staged = [&](float at, auto &&hit) {
 #pragma unroll 2
     for (int c = 0; c < 32; c += 4) {
       const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(&stage[0][c]);
@@ -465,7 +470,7 @@ __global__ __launch_bounds__(32, KCAP > 32 ? 10 : 16) void k_knn_tree(TreeView t
       const float d[4] = {half2f(a, 0), half2f(a, 1), half2f(b, 0), half2f(b, 1)};
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (d[u] <= at && c + u != skip) hit(c + u, d[u]);
+        if (d[u] <= at) hit(c + u, d[u]);
     }
   };
   auto mate_of = [&](u32 l) {  // the lane's point of leaf l
@@ -481,14 +486,27 @@ __global__ __launch_bounds__(32, KCAP > 32 ? 10 : 16) void k_knn_tree(TreeView t
     const float4 mate = mate_of(l);
     const float at = box_d2(own, t.box[0], t.stride[0], l) <= lim ? lim : -1.0f;
     if (!stage_leaf(l, at, mate)) return;
-    leaves[scanned++] = l;
     const int skip = drop && l == qi / 32 ? (int)(qi & 31) : -1;  // the point itself
     float *to = &fbuf[cnt][lane];
-    test_staged(at, skip, [&](int, float d) {
-      *to = d;
-      to += 32;
-    });
-    cnt = (int)(to - &fbuf[0][lane]) >> 5;
+    // (mostly the first leaf only; larger kernels wait for instructions: 2.88 ms
+    // with and 2.72 without the second loop for 2 M lists of 30; 5.68 and 5.76 ms
+    // for 14.5 M lists of 16)
+    if (KCAP > 16 || __any_sync(0xffffffffu, skip >= 0)) {
+      test_staged(at, [&](int c, float d) {
+        if (c == skip) return;
+        *to = d;
+        to += 32;
+      });
+    } else {
+      test_staged(at, [&](int, float d) {
+        *to = d;
+        to += 32;
+      });
+    }
+    const int now = (int)(to - &fbuf[0][lane]) >> 5;
+    // (without hits now it has none later)
+    if (MEAN || __any_sync(0xffffffffu, now != cnt)) leaves[scanned++] = l;
+    cnt = now;
   };
   // the leaves around the packet's place first (they set the limits), then
   // the walk
@@ -550,15 +568,37 @@ __global__ __launch_bounds__(32, KCAP > 32 ? 10 : 16) void k_knn_tree(TreeView t
     }
     // the points within the K-th distance, from the leaves scanned
     const float tau = mine ? fminf(fminf(L[KCAP - 1], bound), FLT_MAX) : -1.0f;
-    for (int i = 0; i < scanned; ++i) {
-      const u32 l = leaves[i];
-      const float4 mate = mate_of(l);
-      const float at = box_d2(own, t.box[0], t.stride[0], l) <= tau ? tau : -1.0f;
-      if (!stage_leaf(l, at, mate)) continue;
-      test_staged(at, drop && l == qi / 32 ? (int)(qi & 31) : -1, [&](int c, float d) {
-        if (cnt < PCAP) pbuf[cnt][lane] = make_uint2(__float_as_uint(d), l * 32 + c);
+    // (a leaf's hits are few and uneven over the lanes: they are noted for some
+    // leaves, then each lane collects its own, about as many as any other; leaf
+    // by leaf this was 36% of the kernel, 14.5 M lists of 16 in 5.94 ms, now 5.68)
+    for (int i0 = 0; i0 < scanned; i0 += kTreeNotes) {
+      u32 some = 0;  // leaves with hits of this lane
+      for (int i = 0; i < min(kTreeNotes, scanned - i0); ++i) {
+        const u32 l = leaves[i0 + i];
+        const float4 mate = mate_of(l);
+        const float at = box_d2(own, t.box[0], t.stride[0], l) <= tau ? tau : -1.0f;
+        if (!stage_leaf(l, at, mate)) continue;
+        u32 m = 0;
+        test_staged(at, [&](int c, float) { m |= 1u << c; });
+        if (drop && l == qi / 32) m &= ~(1u << (qi & 31));
+        notes[i][lane] = m;
+        some |= m ? 1u << i : 0u;
+      }
+      u32 m = 0, p0 = 0;
+      while (some | m) {
+        if (m == 0) {
+          const int i = __ffs(some) - 1;
+          some &= some - 1;
+          m = notes[i][lane];
+          p0 = leaves[i0 + i] * 32;
+        }
+        const u32 p = p0 + __ffs(m) - 1;
+        m &= m - 1;
+        const float4 v = __ldg(&t.pts[p]);
+        const float d = dist2(v.x, v.y, v.z, q.x, q.y, q.z);
+        if (cnt < PCAP) pbuf[cnt][lane] = make_uint2(__float_as_uint(d), p);
         ++cnt;
-      });
+      }
     }
     // exactly these are within the K-th distance, no two equal (and what is
     // missing is not there: points infinitely far would be)
@@ -596,6 +636,11 @@ __global__ __launch_bounds__(32, KCAP > 32 ? 10 : 16) void k_knn_tree(TreeView t
     }
     have += r0;
     if (MODE == TREE_LIST && exact) tree_mean_out(sum, have, q, qidx, o);
+    if constexpr (MODE == TREE_PRECISE) {  // for k_tree_precise
+      u32 *row = o.rows + (size_t)blockIdx.x * K * 32 + lane;
+      for (int j = 0; j < K; ++j, row += 32)
+        *row = exact && j < have ? sorted[j][lane] : 0xFFFFFFFFu;
+    }
   }
   // the others are listed for the second kernel
   const unsigned again = __ballot_sync(0xffffffffu, active && !exact);
@@ -616,7 +661,7 @@ __global__ __launch_bounds__(32, KCAP > 32 ? 10 : 16) void k_knn_tree(TreeView t
       if (o.d2) o.d2[(size_t)qidx * K + j] = INFINITY;
     }
     if (o.counts) o.counts[qidx] = have;
-  } else if constexpr (MODE == TREE_NORMALS || MODE == TREE_PRECISE) {
+  } else if constexpr (MODE == TREE_NORMALS) {
     tree_normal_out<MODE>([&](int j) { return __ldg(&t.pts[sorted[j][lane]]); }, have, q, qidx, o);
   }
 }
@@ -723,14 +768,48 @@ __global__ __launch_bounds__(128) void k_knn_tree_hard(TreeView t, TreeQueries q
   }
 }
 
+// Normals in high precision from the rows of positions that a search left, a
+// thread per query. Bound by the latency of the gather (rows, then points) and
+// of the sums. Inside the search, at 14 warps per SM and among code that the
+// instruction cache does not hold, this took 650 us for 2 M points of 30
+// neighbours; here, with the rows (248 MB), 326.
+constexpr int TP_TH = 128;
+__global__ __launch_bounds__(TP_TH, 6) void k_tree_precise(TreeView t, int K, u32 packets,
+                                                           TreeOut o) {
+  const u32 g = blockIdx.x * TP_TH + threadIdx.x, packet = g / 32, lane = g & 31;
+  const u32 qi = o.packet0 * 32 + g;
+  if (packet >= packets || qi >= t.n) return;
+  const u32 *row = o.rows + (size_t)packet * K * 32 + lane;
+  int have = 0;
+#pragma unroll 8
+  for (int j = 0; j < K; ++j) have += row[(size_t)j * 32] != 0xFFFFFFFFu;
+  if (have == 0) return;  // left for the second search
+  const float4 q = __ldg(&t.pts[qi]);
+  tree_normal_out<TREE_PRECISE>(
+      [&](int j) { return __ldg(&t.pts[row[(size_t)j * 32]]); }, have, q, __float_as_uint(q.w), o);
+}
+
 // packets: how many there can be
 template <int KCAP, int MODE, bool FRAMES>
 void launch_tree(rvp_context *ctx, const TreeView &t, const TreeQueries &q, u32 packets, int K,
                  float bound, const TreeOut &o) {
   constexpr size_t smem = tree_smem<KCAP, MODE>();
   static_assert(smem <= 48 * 1024, "no opt-in to larger shared memory here");
-  k_knn_tree<KCAP, MODE, FRAMES><<<packets, 32, smem, ctx->stream>>>(t, q, K, bound, o);
-  RVP_LAUNCH_CHECK(ctx);
+  if constexpr (MODE == TREE_PRECISE) {
+    const u32 most = tree_precise_packets(packets, K);  // as many as have rows
+    TreeOut part = o;
+    for (u32 p0 = 0; p0 < packets; p0 += most) {
+      const u32 n = std::min(most, packets - p0);
+      part.packet0 = p0;
+      k_knn_tree<KCAP, MODE, FRAMES><<<n, 32, smem, ctx->stream>>>(t, q, K, bound, part);
+      RVP_LAUNCH_CHECK(ctx);
+      k_tree_precise<<<(n + 3) / 4, TP_TH, 0, ctx->stream>>>(t, K, n, part);
+      RVP_LAUNCH_CHECK(ctx);
+    }
+  } else {
+    k_knn_tree<KCAP, MODE, FRAMES><<<packets, 32, smem, ctx->stream>>>(t, q, K, bound, o);
+    RVP_LAUNCH_CHECK(ctx);
+  }
   const unsigned blocks = grid_for(packets * 32, 4, ctx->num_sms * 8);
   if (K <= 32)
     k_knn_tree_hard<1, MODE, FRAMES><<<blocks, 128, 0, ctx->stream>>>(t, q, K, bound, o);

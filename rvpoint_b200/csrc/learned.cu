@@ -1,7 +1,8 @@
 // Learned hypothesis proposal for batched RANSAC plane fitting.
 //
 // Per-point features come from the k = 16 nearest neighbours (17 with the
-// point itself) found by the batched grid kNN: the shifted covariance of
+// point itself), found by the batched grid kNN or, among drawn candidates, by
+// a box tree of each scene's: the shifted covariance of
 // the neighbourhood, its eigen-decomposition (cyclic Jacobi, FP32), the
 // K-th neighbour distance and the point's offset from the neighbourhood
 // centroid. A per-point MLP 8 -> 64 -> 64 -> 1 (ReLU) scores how likely
@@ -118,10 +119,15 @@ __device__ __forceinline__ void plane_features(const float (&dx)[KF], const floa
   f[7] = sqrtf(cx * cx + cy * cy + cz * cz) / r;
 }
 
+// rows of neighbours as packed (d2, index) keys, or as indices
+__device__ __forceinline__ u32 row_index(u64 e) { return (u32)(nbr_idx(e) & 0x7FFFFFFF); }
+__device__ __forceinline__ u32 row_index(int32_t e) { return (u32)(e & 0x7FFFFFFF); }
+
+template <class Row>
 __global__ __launch_bounds__(256) void k_features(const float *__restrict__ x,
                                                   const float *__restrict__ y,
                                                   const float *__restrict__ z,
-                                                  const u64 *__restrict__ pairs,
+                                                  const Row *__restrict__ rows,
                                                   const int32_t *__restrict__ counts,
                                                   const u32 *__restrict__ cand, size_t n_cand,
                                                   size_t n, float *__restrict__ feat) {
@@ -133,16 +139,15 @@ __global__ __launch_bounds__(256) void k_features(const float *__restrict__ x,
     if (m >= 3) {
       const float px = x[i], py = y[i], pz = z[i];
       float dx[KF], dy[KF], dz[KF];
-      float r2 = 0.0f;
+      const u32 far = min(row_index(rows[(size_t)i * KF + m - 1]), (u32)(n - 1));
+      const float r2 = dist2(x[far], y[far], z[far], px, py, pz);
 #pragma unroll
       for (int j = 0; j < KF; ++j) {
         if (j < m) {
-          const u64 key = pairs[(size_t)i * KF + j];
-          const u32 q = min((u32)(nbr_idx(key) & 0x7FFFFFFF), (u32)(n - 1));
+          const u32 q = min(row_index(rows[(size_t)i * KF + j]), (u32)(n - 1));
           dx[j] = x[q] - px;
           dy[j] = y[q] - py;
           dz[j] = z[q] - pz;
-          r2 = nbr_d2(key);
         } else {
           dx[j] = dy[j] = dz[j] = 0.0f;
         }
@@ -166,33 +171,6 @@ __global__ void k_frame_of(const int64_t *offs, int n_frames, size_t n, int32_t 
   }
 }
 
-// Feature neighbourhoods among one scene's candidates (a few thousand
-// points at most): each of CK_SLICES blocks per scene keeps the scene's
-// candidates in shared memory, sorted into a small grid of its own
-// (counting sort over at most CK_CELLS cells of at least the given cell
-// size), and answers the queries of a run of whole cells (about one
-// CK_SLICES-th of them, in cell order); every query, one per
-// thread, takes the exact KF nearest by rings of cells around its own cell
-// (the own cell, then shells at Chebyshev distance 1, 2, ...) until the KF-th
-// distance lies inside the covered box (its distance to every face that has
-// cells beyond it, less a rounding slack) or the box covers the grid,
-// skipping cells whose box lies beyond the KF-th distance so far; the
-// queries go in cell order, so a warp's lanes walk the same cells. Keys
-// are packed (d2, index), so the list is the exact (d2, index) order the
-// grid kNN gives; d2 is computed as there. A scene of more than CK_MAX
-// candidates is searched by brute force over global memory (exact, slow;
-// not reached with the proposal's candidate counts).
-constexpr int CK_MAX = 2048, CK_CELLS = 2048, CK_TH = 256;
-constexpr int CK_SLICES = 2;  // blocks per scene (each builds the scene's grid)
-// the 26 cells around a cell, nearest first: 6 faces, 12 edges, 8 corners
-__constant__ signed char kNbr26[26][3] = {
-    {-1, 0, 0},  {1, 0, 0},   {0, -1, 0},  {0, 1, 0},   {0, 0, -1},  {0, 0, 1},
-    {-1, -1, 0}, {1, -1, 0},  {-1, 1, 0},  {1, 1, 0},   {-1, 0, -1}, {1, 0, -1},
-    {-1, 0, 1},  {1, 0, 1},   {0, -1, -1}, {0, 1, -1},  {0, -1, 1},  {0, 1, 1},
-    {-1, -1, -1}, {1, -1, -1}, {-1, 1, -1}, {1, 1, -1}, {-1, -1, 1}, {1, -1, 1},
-    {-1, 1, 1},  {1, 1, 1}};
-constexpr size_t CK_SMEM = (size_t)CK_MAX * 16 + (size_t)(2 * CK_CELLS + 1) * 4 + CK_MAX * 2;
-
 __device__ __forceinline__ void insert_u64(u64 (&L)[KF], u64 key) {
 #pragma unroll
   for (int j = KF - 1; j > 0; --j) {
@@ -202,216 +180,36 @@ __device__ __forceinline__ void insert_u64(u64 (&L)[KF], u64 key) {
   L[0] = key < L[0] ? key : L[0];
 }
 
-__global__ __launch_bounds__(CK_TH) void k_cand_knn(const float *__restrict__ x,
-                                                    const float *__restrict__ y,
-                                                    const float *__restrict__ z,
-                                                    const int64_t *offs, int n_frames,
-                                                    float cell, u64 *pairs, int32_t *counts) {
-  extern __shared__ __align__(16) unsigned char ck_smem[];
-  float4 *sp = reinterpret_cast<float4 *>(ck_smem);                // sorted points
-  u32 *cstart = reinterpret_cast<u32 *>(sp + CK_MAX);             // CK_CELLS + 1
-  u32 *cursor = cstart + CK_CELLS + 1;                            // CK_CELLS
-  uint16_t *cellof = reinterpret_cast<uint16_t *>(cursor + CK_CELLS);  // CK_MAX
-  __shared__ float s_bb[3];
-  __shared__ float s_wmn[CK_TH / 32][3], s_wmx[CK_TH / 32][3];
-  __shared__ int s_dim[3];
-  __shared__ float s_cell;
-  const int tid = threadIdx.x;
-  // work items: (scene, slice); each of a scene's CK_SLICES blocks builds
-  // the scene's grid and answers its slice's run of cells
-  for (int item = blockIdx.x; item < n_frames * CK_SLICES; item += gridDim.x) {
-    const int f = item / CK_SLICES, slice = item % CK_SLICES;
-    const int64_t a = offs[f], b = offs[f + 1];
-    const int m = (int)(b - a);
-    if (m <= 0) continue;
-    if (m > CK_MAX) {  // brute force over global memory
-      for (int i = tid + slice * CK_TH; i < m; i += CK_SLICES * CK_TH) {
-        const float qx = x[a + i], qy = y[a + i], qz = z[a + i];
-        u64 L[KF];
-#pragma unroll
-        for (int j = 0; j < KF; ++j) L[j] = ~0ull;
-        for (int t = 0; t < m; ++t) {
-          const u64 key = pack_nbr(dist2(x[a + t], y[a + t], z[a + t], qx, qy, qz), (int)(a + t));
-          if (key < L[KF - 1]) insert_u64(L, key);
-        }
-#pragma unroll
-        for (int j = 0; j < KF; ++j) pairs[(size_t)(a + i) * KF + j] = L[j];
-        counts[a + i] = min(m, KF);
-      }
-      continue;
-    }
-    // bounding box
-    float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (int i = tid; i < m; i += CK_TH) {
-      const float v[3] = {x[a + i], y[a + i], z[a + i]};
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        mn[k] = fminf(mn[k], v[k]);
-        mx[k] = fmaxf(mx[k], v[k]);
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-      for (int o = 16; o; o >>= 1) {
-        mn[k] = fminf(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
-        mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
-      }
-    // the block's min / max through a per-warp table
-    if ((tid & 31) == 0)
-      for (int k = 0; k < 3; ++k) {
-        s_wmn[tid >> 5][k] = mn[k];
-        s_wmx[tid >> 5][k] = mx[k];
-      }
-    __syncthreads();
-    if (tid == 0) {
-      float bmn[3] = {INFINITY, INFINITY, INFINITY}, bmx[3] = {-INFINITY, -INFINITY, -INFINITY};
-      for (int w = 0; w < CK_TH / 32; ++w)
-        for (int k = 0; k < 3; ++k) {
-          bmn[k] = fminf(bmn[k], s_wmn[w][k]);
-          bmx[k] = fmaxf(bmx[k], s_wmx[w][k]);
-        }
-      // the grid: cells of at least `cell`, at most CK_CELLS of them
-      float c = cell;
-      int d[3];
-      for (int it = 0; it < 64; ++it) {
-        long long tot = 1;
-        for (int k = 0; k < 3; ++k) {
-          d[k] = (int)floorf((bmx[k] - bmn[k]) / c) + 1;
-          d[k] = max(d[k], 1);
-          tot *= d[k];
-        }
-        if (tot <= CK_CELLS) break;
-        c *= 1.26f;
-      }
-      for (int k = 0; k < 3; ++k) {
-        s_bb[k] = bmn[k];
-        s_dim[k] = d[k];
-      }
-      s_cell = c;
-    }
-    __syncthreads();
-    const float c = s_cell, ic = 1.0f / c;
-    const int GX = s_dim[0], GY = s_dim[1], GZ = s_dim[2];
-    const float mnx = s_bb[0], mny = s_bb[1], mnz = s_bb[2];
-    auto cax = [&](float v, float m0, int G) { return min(max((int)((v - m0) * ic), 0), G - 1); };
-    // counting sort into the cells
-    for (int j = tid; j < CK_CELLS; j += CK_TH) cursor[j] = 0;
-    __syncthreads();
-    for (int i = tid; i < m; i += CK_TH) {
-      const int cid = (cax(z[a + i], mnz, GZ) * GY + cax(y[a + i], mny, GY)) * GX +
-                      cax(x[a + i], mnx, GX);
-      cellof[i] = (uint16_t)cid;
-      atomicAdd(&cursor[cid], 1u);
-    }
-    __syncthreads();
-    if (tid < 32) {  // exclusive scan of the cell counts (one warp)
-      u32 run = 0;
-      for (int base = 0; base < CK_CELLS; base += 32) {
-        const u32 v = cursor[base + tid];
-        u32 incl = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const u32 t = __shfl_up_sync(0xffffffffu, incl, o);
-          if (tid >= o) incl += t;
-        }
-        cstart[base + tid] = run + incl - v;
-        run += __shfl_sync(0xffffffffu, incl, 31);
-      }
-      if (tid == 0) cstart[CK_CELLS] = run;
-    }
-    __syncthreads();
-    for (int j = tid; j < CK_CELLS; j += CK_TH) cursor[j] = cstart[j];
-    __syncthreads();
-    for (int i = tid; i < m; i += CK_TH) {
-      const u32 p = atomicAdd(&cursor[cellof[i]], 1u);
-      sp[p] = make_float4(x[a + i], y[a + i], z[a + i], __int_as_float((int)(a + i)));
-    }
-    __syncthreads();
-    // this block's queries: a run of whole cells in cell order, from the
-    // start of the cell holding sorted position slice * m / CK_SLICES to
-    // that of the next slice (the cell starts are the same in every block
-    // of the scene, while the order inside a cell is not: whole cells keep
-    // the split exact); a warp's lanes work on neighbouring points, the same
-    // cells, the same ring counts
-    auto slice_start = [&](int k) -> int {
-      if (k <= 0) return 0;
-      if (k >= CK_SLICES) return m;
-      const u32 pos = (u32)((long long)k * m / CK_SLICES);
-      int lo = 0, hi = CK_CELLS - 1;  // the last cell starting at or before pos
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (cstart[mid] <= pos) lo = mid; else hi = mid - 1;
-      }
-      return (int)cstart[lo];
-    };
-    const int q0 = slice_start(slice), q1 = slice_start(slice + 1);
-    for (int j = q0 + tid; j < q1; j += CK_TH) {
-      const float4 qp = sp[j];
-      const float qx = qp.x, qy = qp.y, qz = qp.z;
-      const int64_t qo = __float_as_int(qp.w);  // its index in the candidate cloud
-      const int cx = cax(qx, mnx, GX), cy = cax(qy, mny, GY), cz = cax(qz, mnz, GZ);
+// Feature neighbourhoods among one scene's candidates: a box tree of all
+// scenes answers them; the scenes it leaves out (more than kSmallFrame
+// candidates, or coordinates that are not finite) are searched here by brute
+// force, exactly and slowly (the proposal draws far fewer). 512 scenes of 1024
+// candidates: a grid in shared memory per scene 762 us, the tree 41 to build and
+// 460 to search.
+constexpr int CB_TH = 256;
+__global__ __launch_bounds__(CB_TH) void k_cand_brute(const float *__restrict__ x,
+                                                      const float *__restrict__ y,
+                                                      const float *__restrict__ z,
+                                                      const int64_t *offs, int n_frames,
+                                                      const int32_t *skipped, int32_t *idx,
+                                                      int32_t *counts) {
+  for (int f = blockIdx.x; f < n_frames; f += gridDim.x) {
+    if (!skipped[f]) continue;
+    const int64_t a = offs[f];
+    const int m = (int)(offs[f + 1] - a);
+    for (int i = threadIdx.x; i < m; i += CB_TH) {
+      const float qx = x[a + i], qy = y[a + i], qz = z[a + i];
       u64 L[KF];
 #pragma unroll
       for (int j = 0; j < KF; ++j) L[j] = ~0ull;
-      int found = 0;
-      // rounding slack of the cell function and the face positions
-      const float sl = 4e-6f * (fabsf(mnx) + fabsf(mny) + fabsf(mnz) + fabsf(qx) + fabsf(qy) +
-                                fabsf(qz) + (float)(GX + GY + GZ + 3) * c) + 1e-6f;
-      // one cell: skipped when its box lies beyond the current KF-th
-      // distance (once the list is full), else its points tested
-      auto visit = [&](int ux, int uy, int uz, bool test_box) {
-        if (ux < 0 || ux >= GX || uy < 0 || uy >= GY || uz < 0 || uz >= GZ) return;
-        if (test_box) {
-          const float lx = mnx + (float)ux * c, ly = mny + (float)uy * c,
-                      lz = mnz + (float)uz * c;
-          const float gx = fmaxf(fmaxf(lx - sl - qx, qx - (lx + c + sl)), 0.0f);
-          const float gy = fmaxf(fmaxf(ly - sl - qy, qy - (ly + c + sl)), 0.0f);
-          const float gz = fmaxf(fmaxf(lz - sl - qz, qz - (lz + c + sl)), 0.0f);
-          if ((gx * gx + gy * gy + gz * gz) * (1.0f - 1e-5f) > nbr_d2(L[KF - 1])) return;
-        }
-        const int cid = (uz * GY + uy) * GX + ux;
-        for (u32 t = cstart[cid]; t < cstart[cid + 1]; ++t) {
-          const float4 p = sp[t];
-          const u64 key = pack_nbr(dist2(p.x, p.y, p.z, qx, qy, qz), __float_as_int(p.w));
-          ++found;
-          if (key < L[KF - 1]) insert_u64(L, key);
-        }
-      };
-      for (int r = 0;; ++r) {
-        if (r == 0) {
-          visit(cx, cy, cz, false);
-        } else if (r == 1) {  // nearest first: faces, edges, corners
-          for (int t = 0; t < 26; ++t)
-            visit(cx + kNbr26[t][0], cy + kNbr26[t][1], cz + kNbr26[t][2], true);
-        } else {
-          for (int dz = -r; dz <= r; ++dz)
-            for (int dy = -r; dy <= r; ++dy) {
-              const bool edge = dz == -r || dz == r || dy == -r || dy == r;
-              for (int dx = -r; dx <= r; dx += (edge ? 1 : 2 * r))
-                visit(cx + dx, cy + dy, cz + dz, true);
-            }
-        }
-        // the box of rings 0..r: all points found, or the KF-th inside it
-        const bool all = cx - r <= 0 && cy - r <= 0 && cz - r <= 0 && cx + r >= GX - 1 &&
-                         cy + r >= GY - 1 && cz + r >= GZ - 1;
-        if (all) break;
-        if (found >= KF) {
-          float cov = INFINITY;
-          if (cx - r > 0) cov = fminf(cov, qx - (mnx + (float)(cx - r) * c));
-          if (cx + r < GX - 1) cov = fminf(cov, (mnx + (float)(cx + r + 1) * c) - qx);
-          if (cy - r > 0) cov = fminf(cov, qy - (mny + (float)(cy - r) * c));
-          if (cy + r < GY - 1) cov = fminf(cov, (mny + (float)(cy + r + 1) * c) - qy);
-          if (cz - r > 0) cov = fminf(cov, qz - (mnz + (float)(cz - r) * c));
-          if (cz + r < GZ - 1) cov = fminf(cov, (mnz + (float)(cz + r + 1) * c) - qz);
-          cov -= sl;
-          if (cov > 0.0f && nbr_d2(L[KF - 1]) < cov * cov * (1.0f - 1e-5f)) break;
-        }
+      for (int t = 0; t < m; ++t) {
+        const u64 key = pack_nbr(dist2(x[a + t], y[a + t], z[a + t], qx, qy, qz), (int)(a + t));
+        if (key < L[KF - 1]) insert_u64(L, key);
       }
 #pragma unroll
-      for (int j = 0; j < KF; ++j) pairs[(size_t)qo * KF + j] = L[j];
-      counts[qo] = min(m, KF);
+      for (int j = 0; j < KF; ++j) idx[(size_t)(a + i) * KF + j] = nbr_idx(L[j]);
+      counts[a + i] = min(m, KF);
     }
-    __syncthreads();  // the shared arrays are reused by the next scene
   }
 }
 
@@ -975,6 +773,8 @@ struct rvp_scorer {
   rvp::DevBuf frame_of, is_cand, pairs, counts, hard, qlevel, qtau, open;
   rvp::DevBuf w, wq, m, v, grad, norm, loss;
   rvp::DevBuf cand_xyz;  // candidates' own coordinates (neighbours among candidates)
+  rvp::KnnTree tree;     // of the candidates, scene by scene
+  rvp::DevBuf skipped;   // scenes without a tree
   rvp::DevBuf gpart;     // per-block gradient shares of a training step
   int adam_step = 0;
   size_t fitted_points = 0;  // batch size and cell the bucket table was fitted to
@@ -1075,9 +875,10 @@ rvp_status rvp_scorer_destroy(rvp_scorer *s) {
   cudaStreamSynchronize(s->ctx->stream);
   rvp::DevBuf *bufs[] = {&s->frame_of, &s->is_cand, &s->pairs, &s->counts, &s->hard, &s->qlevel,
                          &s->qtau, &s->open, &s->w, &s->wq, &s->m, &s->v, &s->grad, &s->norm,
-                         &s->loss, &s->cand_xyz, &s->gpart};
+                         &s->loss, &s->cand_xyz, &s->gpart, &s->skipped};
   for (auto *b : bufs) b->release();
   s->grid.release();
+  s->tree.release();
   delete s;
   return RVP_OK;
 }
@@ -1204,27 +1005,27 @@ rvp_status rvp_scorer_features(rvp_scorer *s, const float *x, const float *y, co
     RVP_LAUNCH_CHECK(ctx);
   });
   if (st != RVP_OK) return st;
-  // CK_SLICES blocks per scene, each with the scene's candidates in shared
-  // memory (no global grid, sort or table)
   return sguard(ctx, [&] {
     RVP_REQUIRE(cell_size > 0.0f, "cell_size must be > 0");
     RVP_REQUIRE(n_frames >= 1 && n_frames <= s->max_frames, "n_frames out of range");
-    const float *gx = s->cand_xyz.as<float>();
-    static bool attr[64] = {false};
-    if (ctx->device < 64 && !attr[ctx->device]) {
-      RVP_CUDA_TRY(cudaFuncSetAttribute(rvp::k_cand_knn,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)rvp::CK_SMEM));
-      attr[ctx->device] = true;
-    }
-    const unsigned blocks = (unsigned)std::min(n_frames * rvp::CK_SLICES, ctx->num_sms * 8);
-    rvp::k_cand_knn<<<blocks, rvp::CK_TH, rvp::CK_SMEM, ctx->stream>>>(
-        gx, gx + n_cand, gx + 2 * n_cand, cand_offsets_dev, n_frames, cell_size,
-        s->pairs.as<u64>(), s->counts.as<int32_t>());
+    cudaStream_t st = ctx->stream;
+    const float *gx = s->cand_xyz.as<float>(), *gy = gx + n_cand, *gz = gy + n_cand;
+    int32_t *idx = s->pairs.as<int32_t>();
+    int32_t *counts = s->counts.as<int32_t>();
+    s->skipped.reserve((size_t)n_frames * 4);
+    int32_t *skipped = s->skipped.as<int32_t>();
+    const rvp::TreeView t = rvp::tree_build_small_frames(ctx, s->tree, gx, gy, gz,
+                                                         cand_offsets_dev, n_frames, n_cand,
+                                                         skipped);
+    rvp::TreeOut o;
+    o.idx = idx;
+    o.counts = counts;
+    rvp::tree_knn_frames(ctx, s->tree, t, nullptr, nullptr, rvp::KF, rvp::TREE_PAIRS, o);
+    rvp::k_cand_brute<<<(unsigned)std::min(n_frames, ctx->num_sms * 8), rvp::CB_TH, 0, st>>>(
+        gx, gy, gz, cand_offsets_dev, n_frames, skipped, idx, counts);
     RVP_LAUNCH_CHECK(ctx);
-    rvp::k_features<<<rvp::grid_for(n_cand, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
-        gx, gx + n_cand, gx + 2 * n_cand, s->pairs.as<u64>(), s->counts.as<int32_t>(), nullptr,
-        n_cand, n_cand, features);
+    rvp::k_features<<<rvp::grid_for(n_cand, 256, ctx->num_sms * 16), 256, 0, st>>>(
+        gx, gy, gz, idx, counts, nullptr, n_cand, n_cand, features);
     RVP_LAUNCH_CHECK(ctx);
   });
 }

@@ -307,6 +307,7 @@ __device__ __forceinline__ void precise_normal(Nbr nbr, int kk, float qx, float 
                                                bool &wide) {
   // shifted, compensated centroid of (p - q)
   float sx = 0, sy = 0, sz = 0, ex = 0, ey = 0, ez = 0;
+#pragma unroll 4
   for (int t = 0; t < kk; ++t) {
     const float4 p = nbr(t);
     kahan_add(sx, ex, fsub(p.x, qx));
@@ -316,6 +317,7 @@ __device__ __forceinline__ void precise_normal(Nbr nbr, int kk, float qx, float 
   const float inv = fdiv(1.0f, (float)kk);
   const float cx = fmul(sx, inv), cy = fmul(sy, inv), cz = fmul(sz, inv);
   float s[6] = {0, 0, 0, 0, 0, 0}, e[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll 4
   for (int t = 0; t < kk; ++t) {
     const float4 p = nbr(t);
     const float dx = fsub(fsub(p.x, qx), cx);

@@ -59,6 +59,49 @@ def test_sor_statistics_segments(gpu_ctx, n, far):
     assert np.array_equal(keep.astype(bool), mean <= mu + alpha * sd)
 
 
+# neighbourhoods among the candidates: scenes of up to 1024 and up to 2048
+# candidates have a tree each, larger ones are searched by brute force; a point
+# that is not finite takes its scene there as well
+@pytest.mark.parametrize("sizes", [(3, 17, 33, 1), (1023, 1024, 1025), (2047, 2048, 2049, 40)])
+@pytest.mark.parametrize("lattice", [False, True])
+def test_candidate_neighbourhoods(gpu_ctx, sizes, lattice):
+    import torch
+    from rvpoint_b200.learned import DeviceBatch, PlaneScorer
+    n = sum(sizes)
+    rng = np.random.default_rng(n)
+    i = np.arange(n)
+    p = (np.stack([i % 13, (i // 13) % 11, i // 143], 1) % 9 * 0.25 if lattice
+         else rng.uniform(-5, 5, (n, 3)) * [1, 1, 0.1]).astype(np.float32)
+    offs = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    b = DeviceBatch.from_host(D.Batch(p[:, 0].copy(), p[:, 1].copy(), p[:, 2].copy(), offs))
+    s = PlaneScorer(n, len(sizes), ctx=gpu_ctx)
+    cand = torch.arange(n, dtype=torch.int32, device="cuda")
+    coffs = torch.from_numpy(offs).cuda()
+    ref = s.features(b, 1.0).cpu().numpy()  # among all points, by the grid
+    got = s.features(b, 1.0, cand, coffs, among_candidates=True).cpu().numpy()
+    assert np.array_equal(bits(got), bits(ref))
+    b.x[0] = float("inf")  # (the other scenes are as before)
+    got = s.features(b, 1.0, cand, coffs, among_candidates=True).cpu().numpy()
+    assert np.array_equal(bits(got[sizes[0]:]), bits(ref[sizes[0]:]))
+    s.close()
+
+
+# rows of neighbours for the normals in high precision: K = 4, 17, 33 and 64
+@pytest.mark.parametrize("n,k", [(5, 3), (33, 16), (64, 32), (1025, 63), (4097, 16)])
+def test_precise_rows(gpu_ctx, n, k):
+    from rvpoint_b200.api import normal_estimation_precise
+    c = D.room_cloud(n=max(n, 50), seed=n).subset(np.arange(n))
+    k = min(k, n - 1)
+    normals, _, _ = normal_estimation_precise(c, k)
+    p = c.aos().astype(np.float64)
+    idx, _ = brute_knn(c.aos(), c.aos(), k + 1)
+    q = p[idx] - p[idx].mean(1, keepdims=True)
+    w, v = np.linalg.eigh(np.einsum("nki,nkj->nij", q, q))
+    a = np.abs((normals * v[:, :, 0]).sum(1))
+    clear = w[:, 0] < 0.5 * w[:, 1]  # a normal that is well defined
+    assert clear.any() and (1 - a[clear] < 1e-5).all()
+
+
 # the voxel grid sorts its keys: up to 148 x 4096 of them in one cooperative
 # kernel (512 threads, up to eight keys each), more in tiles of 4096
 @pytest.mark.parametrize("n", [1, 31, 513, 4097, 75_777, 606_208, 606_209, 2_424_833])
