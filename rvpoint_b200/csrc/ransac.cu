@@ -54,6 +54,14 @@ __device__ __forceinline__ bool is_inlier(const float4 &m, float x, float y, flo
   return fabsf(fadd(fadd(fadd(fmul(m.x, x), fmul(m.y, y)), fmul(m.z, z)), m.w)) <= t;
 }
 
+// ++c if v <= t: a compare and a predicated add (with c += v <= t the compiler
+// made a select and an addition of it, on the pipes that the products need)
+__device__ __forceinline__ void count_le(u32 &c, float v, float t) {
+  asm("{\n\t.reg .pred p;\n\tsetp.le.f32 p, %1, %2;\n\t@p add.u32 %0, %0, 1;\n\t}"
+      : "+r"(c)
+      : "f"(v), "f"(t));
+}
+
 // One weighted draw: the candidate whose prefix-sum interval holds u * total,
 // returned relative to the frame's first point (a0).
 __device__ __forceinline__ u32 weighted_draw(const RansacSampler &smp, int f, int it, int k,
@@ -327,7 +335,7 @@ __global__ __launch_bounds__(PE_THREADS) void k_preempt_count(
     if (isnan(mdl.x)) continue;
     const u64 ma = pack2(mdl.x, mdl.x), mb = pack2(mdl.y, mdl.y), mc = pack2(mdl.z, mdl.z),
               md = pack2(mdl.w, mdl.w);
-    int c = 0;
+    u32 c = 0;
 #pragma unroll 4
     for (int j = 4 * cs; j < mp; j += 4 * S) {
       const ulonglong2 px = *reinterpret_cast<const ulonglong2 *>(&P[0][j]);
@@ -335,12 +343,12 @@ __global__ __launch_bounds__(PE_THREADS) void k_preempt_count(
       const ulonglong2 pz = *reinterpret_cast<const ulonglong2 *>(&P[2][j]);
       const u64 v = fma2(ma, px.x, fma2(mb, py.x, fma2(mc, pz.x, md)));
       const u64 w = fma2(ma, px.y, fma2(mb, py.y, fma2(mc, pz.y, md)));
-      c += fabsf(half2f(v, 0)) <= prm.thresh;
-      c += fabsf(half2f(v, 1)) <= prm.thresh;
-      c += fabsf(half2f(w, 0)) <= prm.thresh;
-      c += fabsf(half2f(w, 1)) <= prm.thresh;
+      count_le(c, fabsf(half2f(v, 0)), prm.thresh);
+      count_le(c, fabsf(half2f(v, 1)), prm.thresh);
+      count_le(c, fabsf(half2f(w, 0)), prm.thresh);
+      count_le(c, fabsf(half2f(w, 1)), prm.thresh);
     }
-    if (c) atomicAdd(&hcnt[h], c);
+    if (c) atomicAdd(&hcnt[h], (int)c);
   }
   __syncthreads();
   for (int h = threadIdx.x; h < nh; h += blockDim.x) {
@@ -430,15 +438,18 @@ __global__ void k_fill_i32(int32_t *p, int n, int v) {
 // counting many hypotheses over many points
 // ---------------------------------------------------------------------------
 // Block b of a frame's `blocks` takes every blocks-th chunk of CM_CHUNK points
-// (and, of gridDim.y, its share of the tiles of hypotheses): a thread keeps CM_PTS of them in registers, two to a
-// 64-bit pair, and goes over the hypotheses, a tile of which sits in shared
-// memory with every coefficient doubled. Per hypothesis and pair: three
-// products and three sums as f32x2 instructions (each rounded by itself, as
-// is_inlier), two compares and two adds; the warp's counts meet once per
-// hypothesis and eight points per lane. Bound by issue, about 5.5 instructions
-// per test. The one-ballot-per-test loop of k_ransac ran 819M tests (512
-// frames of 50k points, 32 hypotheses) in 505 us, this in 190 us.
-constexpr int CM_THREADS = 256, CM_PTS = 8, CM_CHUNK = CM_THREADS * CM_PTS, CM_TILE = 64;
+// (and, of gridDim.y, its share of the tiles of hypotheses): a thread keeps
+// CM_PTS of them in registers, two to a 64-bit pair, and goes over the
+// hypotheses, a tile of which sits in shared memory. Per hypothesis and pair:
+// six products, three sums as f32x2 instructions (each rounded by itself, as
+// is_inlier; products as f32x2 take a third operand, a zero, to stay apart from
+// the sums, and were slower), two compares and two predicated adds; the warp's
+// counts meet once per hypothesis and sixteen points per lane. Bound by the
+// FP32 pipes and issue, about 7.5 instructions per test. 512 frames of 50k
+// points: 64 hypotheses 510 us with packed products, selects for the counts and
+// eight points per lane, 449 here; 32 hypotheses in the one-ballot-per-test
+// loop of k_ransac 505 us, here 236.
+constexpr int CM_THREADS = 128, CM_PTS = 16, CM_CHUNK = CM_THREADS * CM_PTS, CM_TILE = 64;
 
 // frames: offs, or one frame of n_one points. models: `stride` per frame, the
 // first n_models of them counted into counts (same stride), which start at 0;
@@ -446,9 +457,9 @@ constexpr int CM_THREADS = 256, CM_PTS = 8, CM_CHUNK = CM_THREADS * CM_PTS, CM_T
 __global__ __launch_bounds__(CM_THREADS) void k_count_models(
     const float *__restrict__ X, const float *__restrict__ Y, const float *__restrict__ Z,
     const int64_t *offs, u32 n_one, int blocks, const float4 *__restrict__ models, int stride,
-    int n_models, u32 *counts, float thresh, u64 minus_zero, const RansacState *state,
+    int n_models, u32 *counts, float thresh, const RansacState *state,
     const int32_t *best_now, const int32_t *targets) {
-  __shared__ __align__(16) ulonglong2 hyp[CM_TILE][2];  // (a a, b b), (c c, d d)
+  __shared__ float4 hyp[CM_TILE];
   __shared__ u32 cnt[CM_TILE];
   const int f = blockIdx.x / blocks, part = blockIdx.x % blocks;
   if (state && state->stop) return;
@@ -462,9 +473,7 @@ __global__ __launch_bounds__(CM_THREADS) void k_count_models(
   for (int h0 = blockIdx.y * CM_TILE; h0 < n_models; h0 += gridDim.y * CM_TILE) {
     const int nh = min(CM_TILE, n_models - h0);
     if (tid < nh) {
-      const float4 m = models[h0 + tid];
-      hyp[tid][0] = make_ulonglong2(pack2(m.x, m.x), pack2(m.y, m.y));
-      hyp[tid][1] = make_ulonglong2(pack2(m.z, m.z), pack2(m.w, m.w));
+      hyp[tid] = models[h0 + tid];
       cnt[tid] = 0;
     }
     __syncthreads();
@@ -484,16 +493,17 @@ __global__ __launch_bounds__(CM_THREADS) void k_count_models(
         const int last = min(32, nh - 32 * t);
 #pragma unroll 2
         for (int h = 0; h < last; ++h) {
-          const ulonglong2 ab = hyp[32 * t + h][0], cd = hyp[32 * t + h][1];
+          const float4 m = hyp[32 * t + h];
+          const u64 dd = pack2(m.w, m.w);
           u32 c = 0;
 #pragma unroll
           for (int r = 0; r < CM_PTS / 2; ++r) {
-            const u64 v = add2(add2(add2(mul2(ab.x, px[r], minus_zero),
-                                         mul2(ab.y, py[r], minus_zero)),
-                                    mul2(cd.x, pz[r], minus_zero)),
-                               cd.y);
-            c += fabsf(half2f(v, 0)) <= thresh;
-            c += fabsf(half2f(v, 1)) <= thresh;
+            const u64 u = pack2(fmul(m.x, half2f(px[r], 0)), fmul(m.x, half2f(px[r], 1)));
+            const u64 v = pack2(fmul(m.y, half2f(py[r], 0)), fmul(m.y, half2f(py[r], 1)));
+            const u64 w = pack2(fmul(m.z, half2f(pz[r], 0)), fmul(m.z, half2f(pz[r], 1)));
+            const u64 d = add2(add2(add2(u, v), w), dd);
+            count_le(c, fabsf(half2f(d, 0)), thresh);
+            count_le(c, fabsf(half2f(d, 1)), thresh);
           }
           c = __reduce_add_sync(0xffffffffu, c);
           if (lane == h) acc[t] += c;
@@ -758,7 +768,7 @@ void ransac_preemptive(rvp_context *ctx, const float *x, const float *y, const f
       // (blocks per frame: some 2000 in all keep every SM busy to the end)
       const int blocks = std::min(64, std::max(4, 2048 / n_frames));
       k_count_models<<<(unsigned)n_frames * blocks, CM_THREADS, 0, st>>>(
-          x, y, z, offs, 0, blocks, models + h0, PE_KALL, nh, counts, p.thresh, kMinusZero2,
+          x, y, z, offs, 0, blocks, models + h0, PE_KALL, nh, counts, p.thresh,
           nullptr, from_best ? best : nullptr, smp0.targets);
       RVP_LAUNCH_CHECK(ctx);
       k_decide_models<<<n_frames, 32, 0, st>>>(offs, models + h0, PE_KALL, nh, counts, p,
@@ -812,7 +822,7 @@ void ransac_one(rvp_context *ctx, const float *x, const float *y, const float *z
     const dim3 grid((unsigned)blocks,
                     (unsigned)std::min(tiles, std::max(1, ctx->num_sms * 8 / blocks)));
     k_count_models<<<grid, CM_THREADS, 0, st>>>(x, y, z, nullptr, (u32)n, blocks, models,
-                                                kRoundMost, round, counts, p.thresh, kMinusZero2,
+                                                kRoundMost, round, counts, p.thresh,
                                                 state, nullptr, nullptr);
     RVP_LAUNCH_CHECK(ctx);
     k_decide_one<<<1, 32, 0, st>>>(models, counts, it0, round, p, (u32)n, state);
