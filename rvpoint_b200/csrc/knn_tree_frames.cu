@@ -354,7 +354,6 @@ TreeView tree_build_small_frames(rvp_context *ctx, KnnTree &w, const float *x, c
                                  const float *z, const int64_t *offs, int n_frames, size_t n_max,
                                  int32_t *skipped) {
   const size_t nf = (size_t)n_frames, P = nf * kSmallFrame;
-  RVP_REQUIRE(P <= 0x7FFFFFFFu, "too many frames");
   w.pts.reserve(P * 16);
   w.pos.reserve(n_max * 4);
   w.hard.reserve(P * 4 + 256);

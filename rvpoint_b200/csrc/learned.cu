@@ -1014,13 +1014,16 @@ rvp_status rvp_scorer_features(rvp_scorer *s, const float *x, const float *y, co
     int32_t *counts = s->counts.as<int32_t>();
     s->skipped.reserve((size_t)n_frames * 4);
     int32_t *skipped = s->skipped.as<int32_t>();
-    const rvp::TreeView t = rvp::tree_build_small_frames(ctx, s->tree, gx, gy, gz,
-                                                         cand_offsets_dev, n_frames, n_cand,
-                                                         skipped);
     rvp::TreeOut o;
     o.idx = idx;
     o.counts = counts;
-    rvp::tree_knn_frames(ctx, s->tree, t, nullptr, nullptr, rvp::KF, rvp::TREE_PAIRS, o);
+    // (positions for 2048 points per scene: 8192 scenes at a time)
+    for (int f0 = 0; f0 < n_frames; f0 += 8192) {
+      const rvp::TreeView t = rvp::tree_build_small_frames(
+          ctx, s->tree, gx, gy, gz, cand_offsets_dev + f0, std::min(n_frames - f0, 8192), n_cand,
+          skipped + f0);
+      rvp::tree_knn_frames(ctx, s->tree, t, nullptr, nullptr, rvp::KF, rvp::TREE_PAIRS, o);
+    }
     rvp::k_cand_brute<<<(unsigned)std::min(n_frames, ctx->num_sms * 8), rvp::CB_TH, 0, st>>>(
         gx, gy, gz, cand_offsets_dev, n_frames, skipped, idx, counts);
     RVP_LAUNCH_CHECK(ctx);

@@ -102,6 +102,37 @@ def test_precise_rows(gpu_ctx, n, k):
     assert clear.any() and (1 - a[clear] < 1e-5).all()
 
 
+# the batched pipeline: its trees, with frames that end at a leaf, a node or
+# after one point, empty ones among them, and the grid where many tiny frames
+# would leave the trees mostly empty (130 frames in a batch of 4000 points)
+@pytest.mark.parametrize("sizes,points", [((1023, 0, 1024, 1025, 33, 2049, 1, 0), 8192),
+                                          ((40, 31, 1, 0, 65) * 26, 4000)])
+def test_pipeline_frames(gpu_ctx, sizes, points):
+    import torch
+    from rvpoint_b200.api import Pipeline
+    rng = np.random.default_rng(len(sizes))
+    n = sum(sizes)
+    assert (1024 * len(sizes) <= points + 65_536) == (len(sizes) == 8)
+    # one point per voxel of 0.1: a frame's voxels are its points
+    p = []
+    for m in sizes:
+        i = rng.choice(64 * 64 * 4, m, replace=False)
+        p.append(np.stack([i % 64, i // 64 % 64, i // 4096], 1) * 0.1 + rng.uniform(0.02, 0.08, (m, 3)))
+    p = np.concatenate(p).astype(np.float32)
+    offs = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    batch = D.Batch(p[:, 0].copy(), p[:, 1].copy(), p[:, 2].copy(), offs)
+    got = []
+    for mode in (0, 3, 1):  # trees (or the grid), and a warp per query on the grid
+        pipe = Pipeline(points, len(sizes), leaf_size=0.1, sor_k=16, normal_k=16,
+                        ransac_iters=20, queries_per_warp=mode, ctx=gpu_ctx)
+        got.append(pipe.run_host(batch))
+        pipe.close()
+    for g in got[:2]:
+        assert g.keys() == got[2].keys()
+        for k in g:
+            assert np.array_equal(np.asarray(g[k]), np.asarray(got[2][k]), equal_nan=True), k
+
+
 # the voxel grid sorts its keys: up to 148 x 4096 of them in one cooperative
 # kernel (512 threads, up to eight keys each), more in tiles of 4096
 @pytest.mark.parametrize("n", [1, 31, 513, 4097, 75_777, 606_208, 606_209, 2_424_833])
