@@ -400,6 +400,13 @@ __global__ void k_radius_big_out(const u64 *pairs, const u32 *big, const u32 *bi
 // ---------------------------------------------------------------------------
 // normals
 // ---------------------------------------------------------------------------
+// A packet of 32 queries per warp, each lane with its own neighbours; points
+// with more than a lane holds, and packets of points far apart (past
+// kLeafBudget leaves; one such packet kept the kernel busy for 421 us where the
+// others take 119), go one per warp. Bound by issue and, with many long lists,
+// by the listed points. 87,477 points of a room, radius 0.03 (10 neighbours
+// each): 119 us and 18 for the listed ones; 100,000 and 0.05 (28 each) 165 and
+// 356 (64 neighbours a lane: 258 and 281).
 constexpr int RN_CAP = 48;  // neighbours a lane holds
 
 __global__ __launch_bounds__(32) void k_radius_normals(TreeView t, u64 minus_zero, float r2,
@@ -416,8 +423,9 @@ __global__ __launch_bounds__(32) void k_radius_normals(TreeView t, u64 minus_zer
   const Box own{{q.x, q.y, q.z}, {q.x, q.y, q.z}};
   const Box pk = warp_box(q, true);
   const u64 nqx = pack2(-q.x, -q.x), nqy = pack2(-q.y, -q.y), nqz = pack2(-q.z, -q.z);
-  int cnt = 0;
+  int cnt = 0, budget = kLeafBudget;
   auto leaf = [&](u32 l) {
+    if (--budget < 0) return;
     const u32 i = l * 32 + lane;
     const float4 mate = i < t.n ? __ldg(&t.pts[i]) : make_float4(NAN, NAN, NAN, 0.0f);
     const float at = active && box_d2(own, t.box[0], t.stride[0], l) <= r2 ? r2 : -1.0f;
@@ -448,7 +456,7 @@ __global__ __launch_bounds__(32) void k_radius_normals(TreeView t, u64 minus_zer
   __syncwarp();
   if (!active) return;
   const u32 qidx = __float_as_uint(q.w);
-  if (cnt > RN_CAP) {
+  if (cnt > RN_CAP || budget < 0) {  // (or a packet of points far apart)
     hard[atomicAdd(hard_count, 1u)] = qi;
     return;
   }
@@ -474,13 +482,14 @@ __global__ __launch_bounds__(32) void k_radius_normals(TreeView t, u64 minus_zer
   nz[qidx] = az;
 }
 
-// The points with more neighbours than a lane holds (hard: places in the tree),
-// one warp each; those past FT_CAP neighbours go on to `huge` (indices).
+// The points with more neighbours than a lane holds, and those of wide packets
+// (hard: places in the tree), one warp each; those past FT_CAP neighbours go on to `huge` (indices).
 __global__ __launch_bounds__(32) void k_radius_normals_listed(
     TreeView t, float r2, int iters, float vpx, float vpy, float vpz, float *nx, float *ny,
     float *nz, const u32 *hard, const u32 *hard_count, u32 *huge, u32 *huge_count) {
   __shared__ u64 s_keys[FT_CAP];
-  __shared__ u32 s_bins[FT_BINS], s_near[FT_CAP];
+  __shared__ u32 s_bins[FT_BINS];
+  __shared__ float s_near[3][FT_CAP];  // in order: gathered by all lanes, summed by one
   __shared__ unsigned short s_perm[FT_CAP];
   const int lane = threadIdx.x;
   for (u32 w = blockIdx.x; w < *hard_count; w += gridDim.x) {
@@ -499,12 +508,19 @@ __global__ __launch_bounds__(32) void k_radius_normals_listed(
       continue;
     }
     order_keys<32, FT_BINS>(s_keys, cnt, r2, s_bins, s_perm, nullptr,
-                            [&](u32 rank, u64 k) { s_near[rank] = t.pos_of[nbr_idx(k)]; });
+                            [&](u32 rank, u64 k) {
+                              const float4 p = __ldg(&t.pts[t.pos_of[nbr_idx(k)]]);
+                              s_near[0][rank] = p.x;
+                              s_near[1][rank] = p.y;
+                              s_near[2][rank] = p.z;
+                            });
     __syncwarp();
     if (lane == 0) {
-      float ax, ay, az;
-      nd::normal_from_points([&](int j) { return __ldg(&t.pts[s_near[j]]); }, (int)cnt, false,
-                             iters, q.x, q.y, q.z, vpx, vpy, vpz, ax, ay, az);
+      float ax = 0.0f, ay = 0.0f, az = 0.0f;
+      if (cnt >= 3)  // normal_estimation.cpp:203
+        nd::normal_from_points(
+            [&](int j) { return make_float4(s_near[0][j], s_near[1][j], s_near[2][j], 0.0f); },
+            (int)cnt, false, iters, q.x, q.y, q.z, vpx, vpy, vpz, ax, ay, az);
       nx[qidx] = ax;
       ny[qidx] = ay;
       nz[qidx] = az;

@@ -285,6 +285,21 @@ def test_radius_normals_lists(gpu_ctx, restatement, radius):
     assert (np.abs(got - want).max(1) < 1e-4).mean() > 0.995
 
 
+# a leaf of points around a dense cloud: its packet would test all the leaves
+def test_radius_normals_of_scattered_points(gpu_ctx, restatement):
+    from rvpoint_b200 import api
+    rng = np.random.default_rng(7)
+    near = rng.uniform(-1, 1, (12_000, 3)) * [1, 1, 0.01]
+    c = D.Cloud.from_xyz(np.concatenate([near, rng.uniform(-6, 6, (60, 3))])[rng.permutation(12_060)])
+    h = api.SpatialHash()
+    h.setInputCloud(c, 0.1)
+    h.build()
+    got = np.stack(api.normal_estimation_rvv(c, h, 10, 0.06), 1)
+    want = np.asarray(restatement.normals_radius(c, 0.1, 0.06))
+    assert np.array_equal((got != 0).any(1), (want != 0).any(1))
+    assert (np.abs(got - want).max(1) < 1e-4).mean() > 0.995
+
+
 @pytest.mark.parametrize("primes,collide", [((73856093, 19349663), False), ((1, 1), True),
                                             ((-73856093, 19349663), False), ((0, 5), True),
                                             ((1 << 41, 3), True)])  # (3, 0, 0) and (0, 0, 1)
