@@ -99,8 +99,6 @@ struct rvp_hash {
 
 namespace {
 
-inline size_t al(size_t b) { return (b + 255) & ~(size_t)255; }
-
 template <class F>
 rvp_status guard(rvp_context *ctx, F &&f) {
   try {

@@ -37,8 +37,6 @@
 namespace rvp {
 
 namespace {
-inline size_t al(size_t b) { return (b + 255) & ~(size_t)255; }
-
 // ---------------------------------------------------------------------------
 // build
 // ---------------------------------------------------------------------------

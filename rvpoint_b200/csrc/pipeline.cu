@@ -401,7 +401,6 @@ rvp_status rvp_pipeline_run_device(rvp_pipeline *p, const float *x, const float 
     int64_t *vox_offs = p->vox_offs.as<int64_t>();
     const u64 *n_vox = reinterpret_cast<const u64 *>(vox_offs + n_frames);
     int64_t *sor_offs = p->sor_offs.as<int64_t>();
-    const u64 *n_sor = reinterpret_cast<const u64 *>(sor_offs + n_frames);
 
     p->mark(0);
     if (p->wait_before[0]) RVP_CUDA_TRY(cudaStreamWaitEvent(st, p->wait_before[0], 0));
