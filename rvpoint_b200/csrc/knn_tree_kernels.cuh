@@ -325,14 +325,16 @@ __device__ __forceinline__ void bitonic_sort(float (&v)[N]) {
 }
 
 // sor_sc's mean (statistical_outlier_removal.cpp:36-40): the ascending sum of
-// sqrtf(d2_j), j = 1 .. k, over k; within a radius over those found, and the
-// radius itself for a point without neighbours (:246-270)
+// sqrtf(d2_j), j = 1 .. k, over k, NaN for a point without a position (its
+// distances are); within a radius over those found, and the radius itself for a
+// point without neighbours (:246-270), one without a position among them
 __device__ __forceinline__ void tree_mean_out(float sum, int have, const float4 &q, u32 qidx,
                                               const TreeOut &o) {
+  const float self = dist2(q.x, q.y, q.z, q.x, q.y, q.z);
   float m = have > 1 ? fdiv(sum, (float)(have - 1)) : 0.0f;
-  if (o.radius_mode && have <= 1) m = o.fallback;
-  const float none = dist2(q.x, q.y, q.z, q.x, q.y, q.z);  // NaN without a position
-  o.mean[qidx] = none == 0.0f ? m : none;
+  if (o.radius_mode) m = have > 1 ? m : o.fallback;
+  else if (!(self == 0.0f)) m = self;
+  o.mean[qidx] = m;
 }
 
 // the normal of a query from its sorted neighbours nbr(0 .. have - 1)
