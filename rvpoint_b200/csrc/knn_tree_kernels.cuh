@@ -412,6 +412,9 @@ __global__ __launch_bounds__(32, KCAP > 32 ? 10 : 16) void k_knn_tree(TreeView t
   const float4 q = src[FRAMES || active ? qi : packet * 32];
   const u32 qidx = __float_as_uint(q.w) & (FRAMES ? 0x7FFFFFFFu : 0xFFFFFFFFu);
   const Box own{{q.x, q.y, q.z}, {q.x, q.y, q.z}};
+  // (a point without a position, NaN or infinite, is not at distance 0 from
+  // itself, as the packet takes for granted: the second kernel answers it)
+  mine = mine && dist2(q.x, q.y, q.z, q.x, q.y, q.z) == 0.0f;
 
   // ---- the sorted distances: slots 0 .. pad - 1 hold -1 and never move
   const bool drop = self && K > 1;  // the point itself is not in the list
@@ -728,11 +731,14 @@ __global__ __launch_bounds__(128) void k_knn_tree_hard(TreeView t, TreeQueries q
       }
     };
     const u32 s0 = start > leaf0 ? start - 1 : leaf0, s1 = min(start + 1, leaf1);
-    for (u32 l = s0; l <= s1; ++l) scan(l);
     auto leaf = [&](u32 l) {
       if (l < s0 || l > s1) scan(l);
     };
-    tree_walk_all<FRAMES>(t, roots, own, limit, leaf);
+    const bool unplaced = isnan(q.x) || isnan(q.y) || isnan(q.z);  // near nothing
+    if (!unplaced) {
+      for (u32 l = s0; l <= s1; ++l) scan(l);
+      tree_walk_all<FRAMES>(t, roots, own, limit, leaf);
+    }
     const int have = min((int)found, K);
     if (o.n_hard && lane == 0) atomicAdd(o.n_hard, 1u);
     if constexpr (MODE == TREE_MEAN || MODE == TREE_LIST) {

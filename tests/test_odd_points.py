@@ -34,3 +34,32 @@ def test_sor_within_a_radius_of_odd_points(gpu_ctx, restatement, odd, k):
     out2, mean2, keep2 = restatement.sor_radius(c, 0.2, k, 1.0, 0.2)
     assert np.array_equal(bits(mean), bits(mean2)) and np.array_equal(keep, keep2)
     assert keep.any() and np.array_equal(bits(out), bits(out2))
+
+
+# and it is not its own neighbour either, whichever kernel takes the query
+@pytest.mark.parametrize("odd", ["nan", "nan z", "inf", "-inf"])
+@pytest.mark.parametrize("k", [1, 16, 40])
+@pytest.mark.parametrize("run", [False, True])  # spread over the cloud, or one after the other
+def test_bounded_neighbours_of_odd_points(gpu_ctx, odd, k, run):
+    from rvpoint_b200 import api
+    c = odd_cloud(odd, at=np.arange(70) if run else None)
+    q = c.aos()
+    h = api.SpatialHash()
+    h.setInputCloud(c, 0.2)
+    h.build()
+    for radius in (0.05, 0.5):
+        offs, idx, d2 = h.radiusSearchBatch(c.x, c.y, c.z, radius)
+        n = np.minimum(np.diff(offs), k)
+        cut = np.concatenate([np.arange(a, a + m) for a, m in zip(offs, n)])
+        assert (n[~np.isfinite(q).all(1)] == 0).all()
+        o3, i3, e3 = h.radiusSearchBatch(c.x, c.y, c.z, radius, max_nn=k)
+        assert np.array_equal(np.diff(o3), n)
+        assert np.array_equal(i3, idx[cut]) and np.array_equal(bits(e3), bits(d2[cut]))
+        i4, e4, n4 = h.knn(c.x, c.y, c.z, k, radius=radius)
+        row = np.arange(k)[None] < n[:, None]
+        assert np.array_equal(n4, n) and np.array_equal(i4[row], idx[cut])
+        assert (i4[~row] == -1).all() and np.isinf(e4[~row]).all()
+    i5, _, n5 = h.knn(c.x, c.y, c.z, k)  # without a bound
+    if "nan" in odd:
+        assert (n5[~np.isfinite(q).all(1)] == 0).all()
+    assert (n5[np.isfinite(q).all(1)] == k).all()
