@@ -89,8 +89,9 @@ RVP_API rvp_status rvp_hash_has_collisions(rvp_hash *h, int *out);
 /* radiusSearch, spatial_hashing.cpp:110-168, for nq queries at once.
  * CSR result: offsets[nq+1] (int64), indices/dists hold offsets[nq] entries,
  * each query's list sorted by (d2, index) and cut at max_nn when max_nn > 0.
- * dists are squared distances, as in the reference. If the total exceeds
- * capacity, returns RVP_ERR_CAPACITY with *total and offsets filled. */
+ * dists are squared distances, as in the reference; either may be null (not
+ * wanted). If the total exceeds capacity, returns RVP_ERR_CAPACITY with *total
+ * and offsets filled. */
 RVP_API rvp_status rvp_hash_radius_search(rvp_hash *h, const float *qx, const float *qy,
                                   const float *qz, size_t nq, float radius,
                                   int max_nn, int mem, int64_t *offsets,

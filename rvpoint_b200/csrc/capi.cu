@@ -209,8 +209,8 @@ __global__ void k_rows_to_csr(const int32_t *row_idx, const float *row_d2, int K
     const int j = (int)(t % K);
     if (j >= counts[q]) continue;
     const u64 o = offs[q] + j;
-    idx[o] = row_idx[t];
-    d2[o] = row_d2[t];
+    if (idx) idx[o] = row_idx[t];
+    if (d2) d2[o] = row_d2[t];
   }
 }
 
@@ -222,8 +222,8 @@ __global__ void k_csr_cut(const u64 *pairs, const u64 *offs_in, const u64 *offs_
     const u64 a = offs_in[q], o = offs_out[q], c = offs_out[q + 1] - o;
     for (u64 j = 0; j < c; ++j) {
       const u64 k = pairs[a + j];
-      idx[o + j] = (int32_t)(u32)(k & 0x7FFFFFFFull);
-      d2[o + j] = __uint_as_float((u32)(k >> 32));
+      if (idx) idx[o + j] = (int32_t)(u32)(k & 0x7FFFFFFFull);
+      if (d2) d2[o + j] = __uint_as_float((u32)(k >> 32));
     }
   }
 }

@@ -305,6 +305,12 @@ __device__ __forceinline__ float4 fill_query(const TreeView &t, const TreeQuerie
   return self ? t.pts[w] : qs.q[w];
 }
 
+// one pair of a list; an output that is not wanted is null
+__device__ __forceinline__ void pair_out(u64 key, u64 at, int32_t *idx, float *d2) {
+  if (idx) idx[at] = nbr_idx(key);
+  if (d2) d2[at] = nbr_d2(key);
+}
+
 // lists of up to FT_SHORT points, one warp each
 __global__ __launch_bounds__(FT_WARPS * 32) void k_radius_fill(
     TreeView t, TreeQueries qs, const float *qx, const float *qy, const float *qz, float r2,
@@ -332,8 +338,7 @@ __global__ __launch_bounds__(FT_WARPS * 32) void k_radius_fill(
   order_keys<32, FT_SHORT>(s_keys[wib], cnt, r2, s_bins[wib], s_perm[wib], nullptr,
                            [&](u32 rank, u64 k) {
                              if (cut && rank >= cut) return;
-                             out_idx[off + rank] = nbr_idx(k);
-                             out_d2[off + rank] = nbr_d2(k);
+                             pair_out(k, off + rank, out_idx, out_d2);
                            });
 }
 
@@ -376,8 +381,7 @@ __global__ __launch_bounds__(FT_WARPS * 32) void k_radius_fill_long(
   order_keys<FT_WARPS * 32, FT_BINS>(s_keys, cnt, r2, s_bins, s_perm, s_warp,
                                      [&](u32 rank, u64 k) {
                                        if (cut && rank >= cut) return;
-                                       out_idx[off + rank] = nbr_idx(k);
-                                       out_d2[off + rank] = nbr_d2(k);
+                                       pair_out(k, off + rank, out_idx, out_d2);
                                      });
 }
 
@@ -390,10 +394,8 @@ __global__ void k_radius_big_out(const u64 *pairs, const u32 *big, const u32 *bi
     const u64 from = full[qi], off = offsets[qi];
     u64 cnt = full[qi + 1] - from;
     if (cut && cnt > cut) cnt = cut;
-    for (u64 i = threadIdx.x; i < cnt; i += blockDim.x) {
-      out_idx[off + i] = nbr_idx(pairs[from + i]);
-      out_d2[off + i] = nbr_d2(pairs[from + i]);
-    }
+    for (u64 i = threadIdx.x; i < cnt; i += blockDim.x)
+      pair_out(pairs[from + i], off + i, out_idx, out_d2);
   }
 }
 

@@ -63,3 +63,42 @@ def test_bounded_neighbours_of_odd_points(gpu_ctx, odd, k, run):
     if "nan" in odd:
         assert (n5[~np.isfinite(q).all(1)] == 0).all()
     assert (n5[np.isfinite(q).all(1)] == k).all()
+
+
+# a list that is not wanted has no memory: short lists, longer ones (256 points)
+# and those past shared memory (1024), for few queries and for packets of them
+# (colliding cells repeat a point once per cell of the window: short radius only)
+@pytest.mark.parametrize("radius,primes", [(0.3, None), (2.0, None), (30.0, None), (0.3, (1, 1))])
+@pytest.mark.parametrize("nq", [300, 2100])
+@pytest.mark.parametrize("mem", [0, 1])
+def test_radius_search_without_a_list(gpu_ctx, radius, nq, mem, primes):
+    import ctypes as C
+    import torch
+    from rvpoint_b200 import api
+    c = D.room_cloud(n=2100, seed=4)
+    h = api.SpatialHash()
+    if primes:
+        h.setHashPrimes(*primes)
+    h.setInputCloud(c, 0.5)
+    h.build()
+    assert h.hasCollisions() == bool(primes)
+    q = [torch.from_numpy(np.array(v[:nq])) for v in (c.x, c.y, c.z)]
+    if mem == 1:
+        q = [v.cuda() for v in q]
+    api._prep(gpu_ctx, mem)
+    ptr = lambda t: C.c_void_p(t.data_ptr()) if t is not None else None  # noqa: E731
+    for max_nn in (0, 16, 100):
+        offs, idx, d2 = h.radiusSearchBatch(*[v if mem else v.numpy() for v in q], radius,
+                                            max_nn=max_nn)
+        want = [torch.as_tensor(v) for v in (idx, d2)]
+        for keep in ((0,), (1,), ()):
+            lists = [torch.zeros_like(w) if i in keep else None for i, w in enumerate(want)]
+            o = torch.zeros(nq + 1, dtype=torch.int64, device=q[0].device)
+            total = C.c_size_t(0)
+            st = gpu_ctx.L.rvp_hash_radius_search(
+                h.h, *[ptr(v) for v in q], nq, radius, max_nn, mem, ptr(o), ptr(lists[0]),
+                ptr(lists[1]), len(want[0]), C.byref(total))
+            assert st == 0 and total.value == len(want[0])
+            assert torch.equal(o, torch.as_tensor(offs))
+            for i in keep:
+                assert torch.equal(lists[i].view(torch.int32), want[i].view(torch.int32))
