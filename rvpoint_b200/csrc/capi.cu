@@ -268,15 +268,16 @@ void hash_tree(rvp_hash *h) {
   h->tree_built = true;
 }
 
+// (32-bit query numbers in the tree's kernels: a billion queries at a time)
+constexpr size_t kMostQueries = (size_t)1 << 30;
+
 // the k nearest among a hash's points
 void knn_hash(rvp_hash *h, const float *qx, const float *qy, const float *qz, size_t nq, int K,
               float radius, int mode, const rvp::TreeOut &o) {
   const float *x = h->x.as<float>(), *y = h->y.as<float>(), *z = h->z.as<float>();
   hash_tree(h);
-  // (32-bit query numbers in the kernels: a billion at a time)
-  constexpr size_t kMost = (size_t)1 << 30;
-  for (size_t a = 0; a < nq; a += kMost) {
-    const size_t m = std::min(kMost, nq - a);
+  for (size_t a = 0; a < nq; a += kMostQueries) {
+    const size_t m = std::min(kMostQueries, nq - a);
     rvp::TreeOut p = o;
     if (p.mean) p.mean += a;
     if (p.idx) p.idx += a * K;
@@ -535,25 +536,30 @@ static void radius_search(rvp_hash *h, const float *qx, const float *qy, const f
   }
   // the lists' lengths, their offsets, and the lists (cut: the offsets of the
   // cut ones beside the full ones)
-  const bool tree = !refwin && nq <= ((size_t)1 << 30);
   rvp::QuerySet qs{dqx, dqy, dqz, nq, nullptr, nullptr, nullptr};
   const rvp::GridView gv = refwin ? h->grid.view(rvp::KEY_REF_HASH, h->p1, h->p2)
                                   : rvp::GridView{};
-  rvp::TreeQueries tq{};
   u32 *cnt = static_cast<u32 *>(scratch(ctx, 6, nq * 4 + 256));
   u64 *full = max_nn > 0 ? static_cast<u64 *>(scratch(ctx, 10, (nq + 2) * 8)) : offs_d;
   u32 *most_d = cnt + nq;
   u32 most[2] = {0, 0};
-  if (tree) {
-    if (rvp::tree_radius_few(nq)) tq = rvp::tree_queries_as_given(ctx, h->tree, nq);
+  // counts of the m queries from a on
+  auto count = [&](size_t a, size_t m) {
+    rvp::TreeQueries tq{};
+    if (rvp::tree_radius_few(m)) tq = rvp::tree_queries_as_given(ctx, h->tree, m);
     else
       tq = rvp::tree_queries(ctx, h->tree, h->tree_view, h->x.as<float>(), h->y.as<float>(),
-                             h->z.as<float>(), dqx, dqy, dqz, nq);
-    rvp::tree_radius_count(ctx, h->tree_view, tq, dqx, dqy, dqz, radius, cnt, most_d);
-  } else {
-    RVP_REQUIRE(refwin, "at most 2^30 queries at a time");
+                             h->z.as<float>(), dqx + a, dqy + a, dqz + a, m);
+    rvp::tree_radius_count(ctx, h->tree_view, tq, dqx + a, dqy + a, dqz + a, radius, cnt + a,
+                           most_d);
+    return tq;
+  };
+  rvp::TreeQueries tq{};
+  if (!refwin)
+    for (size_t a = 0; a < nq; a += kMostQueries)
+      tq = count(a, std::min(kMostQueries, nq - a));
+  else
     rvp::grid_radius_count(ctx, gv, qs, radius, refwin, cnt);
-  }
   rvp::exclusive_scan_u32_to_u64(ctx, cnt, full, nq, nullptr, scan_tmp);
   u64 tot = 0;
   if (max_nn > 0) {
@@ -566,7 +572,7 @@ static void radius_search(rvp_hash *h, const float *qx, const float *qy, const f
   }
   u64 tot_full = 0;
   RVP_CUDA_TRY(cudaMemcpyAsync(&tot_full, full + nq, 8, cudaMemcpyDeviceToHost, ctx->stream));
-  if (tree)
+  if (!refwin)
     RVP_CUDA_TRY(cudaMemcpyAsync(most, most_d, 8, cudaMemcpyDeviceToHost, ctx->stream));
   sync(ctx);
   if (max_nn <= 0) tot = tot_full;
@@ -575,12 +581,21 @@ static void radius_search(rvp_hash *h, const float *qx, const float *qy, const f
   int32_t *di = out_dev(ctx, 8, indices, tot, mem);
   float *dd = out_dev(ctx, 9, dists, tot, mem);
   const u32 cut = max_nn > 0 ? (u32)max_nn : 0;
-  if (tree) {
-    const bool big = most[0] > rvp::tree_radius_cap();
-    u64 *pairs = big ? static_cast<u64 *>(scratch(ctx, 5, tot_full * 8)) : nullptr;
-    u32 *list = big ? static_cast<u32 *>(scratch(ctx, 11, nq * 4 + 16)) : nullptr;
-    rvp::tree_radius_fill(ctx, h->tree_view, tq, dqx, dqy, dqz, radius, full, offs_d, cut, most[1], di, dd,
-                          pairs, list, big ? list + nq : nullptr);
+  if (!refwin) {
+    for (size_t a = 0; a < nq; a += kMostQueries) {
+      const size_t m = std::min(kMostQueries, nq - a);
+      if (nq > kMostQueries) {  // (the part's queries and long lists once more)
+        tq = count(a, m);
+        RVP_CUDA_TRY(cudaMemcpyAsync(most, most_d, 8, cudaMemcpyDeviceToHost, ctx->stream));
+        sync(ctx);
+      }
+      const bool big = most[0] > rvp::tree_radius_cap();
+      u64 *pairs = big ? static_cast<u64 *>(scratch(ctx, 5, tot_full * 8)) : nullptr;
+      u32 *list = big ? static_cast<u32 *>(scratch(ctx, 11, m * 4 + 16)) : nullptr;
+      rvp::tree_radius_fill(ctx, h->tree_view, tq, dqx + a, dqy + a, dqz + a, radius, full + a,
+                            offs_d + a, cut, most[1], di, dd, pairs, list,
+                            big ? list + m : nullptr);
+    }
     return finish(tot);
   }
   u64 *pairs = static_cast<u64 *>(scratch(ctx, 5, (tot_full ? tot_full : 1) * 8));

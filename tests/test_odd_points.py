@@ -102,3 +102,31 @@ def test_radius_search_without_a_list(gpu_ctx, radius, nq, mem, primes):
             assert torch.equal(o, torch.as_tensor(offs))
             for i in keep:
                 assert torch.equal(lists[i].view(torch.int32), want[i].view(torch.int32))
+
+
+# more queries than one launch numbers (2^30): taken in parts, short and long
+# lists (this takes some 75 GB)
+@pytest.mark.parametrize("max_nn", [0, 70])
+def test_radius_search_of_a_billion_queries(gpu_ctx, max_nn):
+    import torch
+    from rvpoint_b200 import api
+    if torch.cuda.mem_get_info()[0] < 110 << 30:
+        pytest.skip("needs 110 GB free")
+    most = 1 << 30
+    t = np.linspace(0, 1, 2000, dtype=np.float32)
+    ctx = api.Context(0)
+    h = api.SpatialHash(ctx)
+    h.setInputCloud((t, t, t), 0.1)
+    h.build()
+    near = [0, most - 1, most, most + 4]
+    v = torch.tensor([0.1, 0.5, 0.2, 0.45], device="cuda")
+    q = torch.full((most + 5,), 1e3, device="cuda")
+    q[near] = v
+    offs, idx, d2 = h.radiusSearchBatch(q, q, q, 0.5, max_nn=max_nn)
+    o2, i2, e2 = h.radiusSearchBatch(v, v, v, 0.5, max_nn=max_nn)
+    assert int(o2.diff().max()) > (1024 if max_nn == 0 else 69)
+    assert torch.equal(offs[near], o2[:-1]) and int(offs[-1]) == int(o2[-1])
+    assert int((offs.diff() != 0).sum()) == len(near)
+    assert torch.equal(idx, i2) and torch.equal(d2, e2)
+    h.close()
+    ctx.close()
