@@ -19,6 +19,7 @@ path.
 from __future__ import annotations
 
 import ctypes as C
+import weakref
 from typing import Optional, Sequence
 
 import numpy as np
@@ -74,7 +75,8 @@ def _empty(shape, dtype, like_dev: bool, device=None):
 
 
 class Context:
-    """One CUDA device + stream + scratch arena (rvp_context)."""
+    """One CUDA device + stream + scratch arena (rvp_context). Closing it
+    closes the objects made in it."""
 
     def __init__(self, device: int = 0):
         self.L = _lib.load()
@@ -82,6 +84,17 @@ class Context:
         check(self.L.rvp_context_create(device, C.byref(h)))
         self.h = h
         self.device = device
+        self._objects = {}  # handle -> (its destroy function, weak reference to its owner)
+
+    def _own(self, owner, destroy) -> None:
+        self._objects[owner.h.value] = (destroy, weakref.ref(owner))
+
+    def _give_back(self, owner) -> None:
+        """Destroys an object's handle, unless the context has done so."""
+        h, owner.h = owner.h, None
+        known = self._objects.pop(h.value, None) if self.h else None
+        if known:
+            known[0](h)
 
     def set_stream(self, stream_handle: int) -> None:
         check(self.L.rvp_context_set_stream(self.h, C.c_void_p(stream_handle)), self.h)
@@ -99,6 +112,12 @@ class Context:
 
     def close(self) -> None:
         if getattr(self, "h", None):
+            # (an object's memory is its own, and it needs the context to go)
+            while self._objects:
+                h, (destroy, owner) = self._objects.popitem()
+                if owner() is not None:
+                    owner().h = None
+                destroy(C.c_void_p(h))
             self.L.rvp_context_destroy(self.h)
             self.h = None
 
@@ -147,6 +166,7 @@ class SpatialHash:
         h = C.c_void_p()
         check(self.L.rvp_hash_create(self.ctx.h, C.byref(h)), self.ctx.h)
         self.h = h
+        self.ctx._own(self, self.L.rvp_hash_destroy)
         self.n = 0
 
     def setHashPrimes(self, p1: int, p2: int) -> None:
@@ -243,9 +263,7 @@ class SpatialHash:
 
     def close(self):
         if getattr(self, "h", None):
-            if self.ctx.h:  # (at exit the context may go first, and its memory with it)
-                self.L.rvp_hash_destroy(self.h)
-            self.h = None
+            self.ctx._give_back(self)
 
     def __del__(self):  # pragma: no cover
         try:
@@ -352,6 +370,7 @@ class Octree:
         h = C.c_void_p()
         check(self.L.rvp_octree_create(self.ctx.h, self.KIND, C.byref(h)), self.ctx.h)
         self.h = h
+        self.ctx._own(self, self.L.rvp_octree_destroy)
         self.n = 0
         self._params = [64, 8, 1e-4]
 
@@ -429,9 +448,7 @@ class Octree:
 
     def close(self):
         if getattr(self, "h", None):
-            if self.ctx.h:  # (at exit the context may go first, and its memory with it)
-                self.L.rvp_octree_destroy(self.h)
-            self.h = None
+            self.ctx._give_back(self)
 
     def __del__(self):  # pragma: no cover
         try:
@@ -735,6 +752,7 @@ class Pipeline:
         check(self.L.rvp_pipeline_create(self.ctx.h, C.byref(cfg), int(max_points),
                                          int(max_frames), C.byref(h)), self.ctx.h)
         self.h = h
+        self.ctx._own(self, self.L.rvp_pipeline_destroy)
         self.max_points = max_points
         self.max_frames = max_frames
         self.last_frames = 0
@@ -932,9 +950,7 @@ class Pipeline:
 
     def close(self):
         if getattr(self, "h", None):
-            if self.ctx.h:  # (at exit the context may go first, and its memory with it)
-                self.L.rvp_pipeline_destroy(self.h)
-            self.h = None
+            self.ctx._give_back(self)
 
     def __del__(self):  # pragma: no cover
         try:

@@ -100,6 +100,7 @@ class PlaneScorer:
         check(self.L.rvp_scorer_create(self.ctx.h, int(max_points), int(max_frames),
                                        C.byref(h)), self.ctx.h)
         self.h = h
+        self.ctx._own(self, self.L.rvp_scorer_destroy)
         self.mean = np.zeros(8, np.float32)
         self.std = np.ones(8, np.float32)
 
@@ -162,9 +163,7 @@ class PlaneScorer:
 
     def close(self):
         if getattr(self, "h", None):
-            if self.ctx.h:  # (at exit the context may go first, and its memory with it)
-                self.L.rvp_scorer_destroy(self.h)
-            self.h = None
+            self.ctx._give_back(self)
 
     def __del__(self):  # pragma: no cover
         try:
