@@ -334,7 +334,8 @@ RVP_API rvp_status rvp_pipeline_outputs_get(rvp_pipeline *p, rvp_pipeline_output
  * run (with 25% headroom, 2.5 slots per bucket rounded up to a power of two)
  * so it stays resident in L2. Call after a first run, before capturing a
  * graph; a later batch with more buckets than that makes rvp_pipeline_check
- * report RVP_ERR_CAPACITY (refit then). */
+ * report RVP_ERR_CAPACITY (refit then). After a run on the box tree, which has
+ * no table, the fit is made when rvp_pipeline_set_tuning chooses a grid mode. */
 RVP_API rvp_status rvp_pipeline_fit_tables(rvp_pipeline *p);
 /* RVP_ERR_CAPACITY if the last run's bucket table overflowed (results of
  * that run are then incomplete); synchronizes the stream. */

@@ -349,11 +349,7 @@ void Grid::reserve(size_t n, int nf) {
   b_lstart.reserve(al(kHeadLevels * n_max * 4));
   b_pos.reserve(n_max * 4);
   b_sub.reserve(al(n_max * 2));
-  b_misc.reserve(256);
-  d_n = b_misc.as<u64>();
-  d_nbuckets = d_n + 1;
-  d_collision = reinterpret_cast<int *>(d_n + 1 + kHeadLevels);
-  d_overflow = d_collision + 1;
+  reserve_flags();
   // the buckets of the table levels never exceed kGridLevels n (each holds a
   // point; in practice ~1.4 n): without a measured count the table holds
   // that many, so no insert can fail; rvp_pipeline_fit_tables and the
@@ -367,6 +363,14 @@ void Grid::reserve(size_t n, int nf) {
     b_table.reserve(want * 16);
     table_cap = want;
   }
+}
+
+void Grid::reserve_flags() {
+  b_misc.reserve(256);
+  d_n = b_misc.as<u64>();
+  d_nbuckets = d_n + 1;
+  d_collision = reinterpret_cast<int *>(d_n + 1 + kHeadLevels);
+  d_overflow = d_collision + 1;
 }
 
 void Grid::fit_table(size_t buckets) {

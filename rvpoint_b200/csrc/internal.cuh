@@ -281,6 +281,7 @@ struct Grid {
   int *d_overflow = nullptr;   // a bucket found no free table slot
   GridView view(int mode, long long p1, long long p2) const;
   void reserve(size_t n_max, int n_frames_max);
+  void reserve_flags();  // the counts and flags below only
   // shrink/grow the bucket table to hold `buckets` entries at load <= 1/2.5
   void fit_table(size_t buckets);
   void release();

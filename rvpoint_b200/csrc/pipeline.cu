@@ -39,15 +39,20 @@ struct rvp_pipeline {
   // 256 LiDAR frames (14.6M points) 10.6 ms a run, on the grid 16.7 ms with the
   // cooperative kernels and more with one query per lane.
   // tree_fits: its frames, padded to 1024 positions each, stay within twice
-  // the points (a batch of many tiny frames keeps the grid)
+  // the points (a batch of many tiny frames keeps the grid). The grid and the
+  // buffers of its kernels are reserved once a mode uses them.
   rvp::KnnTree tree;
   bool tree_fits = false;
   bool grid_built = false;  // by the last run
+  bool fit_wanted = false;  // fit_tables after a run on the tree: the next grid
   size_t points_last = 0;
+  bool on_tree() const {
+    return tree_fits && (cfg.queries_per_warp == 0 || cfg.queries_per_warp == 3);
+  }
   rvp::DevBuf in_x, in_y, in_z, in_offs;
   rvp::DevBuf vox_aos, vox_x, vox_y, vox_z, vox_offs, vox_frame;
-  rvp::DevBuf sor_list, knn_counts, mean, keep, sor_tmp;
-  rvp::DevBuf sor_aos, sor_x, sor_y, sor_z, sor_offs, sor_frame, sor_src;
+  rvp::DevBuf sor_list, mean, keep, sor_tmp;
+  rvp::DevBuf sor_aos, sor_x, sor_y, sor_z, sor_offs, sor_src;
   rvp::DevBuf nrm_pairs, nrm_counts, nx, ny, nz;
   rvp::DevBuf r_model, r_best, r_iters, r_rand;
   rvp::DevBuf stats;  // 20 kNN path counters (diagnostics)
@@ -161,8 +166,8 @@ namespace {
 void release_pipeline(rvp_pipeline *p) {
   rvp::DevBuf *bufs[] = {&p->in_x, &p->in_y, &p->in_z, &p->in_offs, &p->vox_aos, &p->vox_x,
                          &p->vox_y, &p->vox_z, &p->vox_offs, &p->vox_frame, &p->sor_list,
-                         &p->knn_counts, &p->mean, &p->keep, &p->sor_tmp, &p->sor_aos, &p->sor_x,
-                         &p->sor_y, &p->sor_z, &p->sor_offs, &p->sor_frame, &p->sor_src,
+                         &p->mean, &p->keep, &p->sor_tmp, &p->sor_aos, &p->sor_x,
+                         &p->sor_y, &p->sor_z, &p->sor_offs, &p->sor_src,
                          &p->nrm_pairs, &p->nrm_counts, &p->nx, &p->ny, &p->nz, &p->r_model,
                          &p->r_best, &p->r_iters, &p->r_rand, &p->stats, &p->hard, &p->qlevel,
                          &p->qtau, &p->open, &p->routed};
@@ -181,6 +186,47 @@ void release_pipeline(rvp_pipeline *p) {
     if (e) cudaEventDestroy(e);
   for (auto *b : {&p->in2_x, &p->in2_y, &p->in2_z, &p->in2_offs}) b->release();
   delete p;
+}
+
+// room for the kernel modes that search the grid
+void reserve_grid(rvp_pipeline *p) {
+  const size_t N = p->max_points;
+  p->grid.reserve(N, p->max_frames);
+  p->vox_frame.reserve(N * 4);
+  p->nrm_pairs.reserve(N * (size_t)(p->cfg.normal_k + 1) * 8);
+  p->nrm_counts.reserve(N * 4);
+  p->hard.reserve(N * 8 + 256);
+  p->qtau.reserve(N * 4);
+}
+
+// the bucket table sized to the buckets of the last grid
+void fit_grid(rvp_pipeline *p) {
+  u64 nb[rvp::kHeadLevels] = {};
+  RVP_CUDA_TRY(cudaMemcpyAsync(nb, p->grid.d_nbuckets, 8 * rvp::kHeadLevels, cudaMemcpyDeviceToHost,
+                               p->ctx->stream));
+  RVP_CUDA_TRY(cudaStreamSynchronize(p->ctx->stream));
+  // a quarter of headroom for batches whose scenes occupy more cells than
+  // this one; the table (2.5 slots per bucket, rounded up to a power of
+  // two) then stays inside L2, where every probe of the kNN kernels lands
+  size_t tot = 0;
+  for (int l = 0; l < rvp::kGridLevels; ++l) tot += (size_t)nb[l];
+  p->grid.fit_table(tot + tot / 4);
+}
+
+// The mode now searches the grid: its memory, and the fit asked for after a
+// run on the tree, from the buckets that run's points would have.
+void enter_grid(rvp_pipeline *p) {
+  reserve_grid(p);
+  if (!p->fit_wanted) return;
+  const int64_t *offs = p->vox_offs.as<int64_t>();
+  rvp::grid_build(p->ctx, p->grid, p->vox_x.as<float>(), p->vox_y.as<float>(),
+                  p->vox_z.as<float>(), offs, p->n_frames_last, p->points_last, p->cell,
+                  rvp::KEY_DENSE, 0, 0, reinterpret_cast<const u64 *>(offs + p->n_frames_last),
+                  p->grid_base, p->vox_aos.as<float>());
+  fit_grid(p);
+  // (no run's overflow)
+  RVP_CUDA_TRY(cudaMemsetAsync(p->grid.d_collision, 0, 8, p->ctx->stream));
+  p->fit_wanted = false;
 }
 
 // stages 2 to 4 over the box tree of the batch: SOR means with the k+1 nearest
@@ -325,35 +371,29 @@ rvp_status rvp_pipeline_create(rvp_context *ctx, const rvp_pipeline_config *cfg,
     p->in_x.reserve(N * 4); p->in_y.reserve(N * 4); p->in_z.reserve(N * 4);
     p->in_offs.reserve(F1 * 8);
     p->vw.reserve(N, max_frames);
-    p->grid.reserve(N, max_frames);
+    p->grid.reserve_flags();
     p->vox_aos.reserve(N * 12);
     p->vox_x.reserve(N * 4); p->vox_y.reserve(N * 4); p->vox_z.reserve(N * 4);
     p->vox_offs.reserve(F1 * 8);
-    p->vox_frame.reserve(N * 4);
-    const int ks = cfg->sor_k + 1, kn = cfg->normal_k + 1;
+    const int ks = cfg->sor_k + 1;
     p->tree_fits = (size_t)max_frames * 1024 <= N + 65536;
     // (tree positions, or grid positions)
     const size_t P = p->tree_fits ? rvp::tree_frames_positions(N, max_frames) : N;
     if (p->tree_fits) p->tree.reserve_frames(N, max_frames);
     p->sor_list.reserve(P * (size_t)ks * 4);
-    p->knn_counts.reserve(N * 4);
     p->mean.reserve(N * 4);
     p->keep.reserve(N);
     p->sor_tmp.reserve(rvp::sor_filter_temp_bytes(N, max_frames));
     p->sor_aos.reserve(N * 12);
     p->sor_x.reserve(N * 4); p->sor_y.reserve(N * 4); p->sor_z.reserve(N * 4);
     p->sor_offs.reserve(F1 * 8);
-    p->sor_frame.reserve(N * 4);
     p->sor_src.reserve(N * 4);
-    p->nrm_pairs.reserve(N * (size_t)kn * 8);
-    p->hard.reserve(N * 8 + 256);
     p->qlevel.reserve(P);
-    p->qtau.reserve(N * 4);
     p->routed.reserve(256);
     p->open.reserve(((P * 4 + 255) & ~(size_t)255) + ((P * 8 + 8 + 255) & ~(size_t)255) +
                     ((P * 4 + 255) & ~(size_t)255) + 256 + rvp::scan_temp_bytes(P));
     RVP_CUDA_TRY(cudaMemset(p->grid.d_collision, 0, 8));
-    p->nrm_counts.reserve(N * 4);
+    if (!p->on_tree()) reserve_grid(p);
     p->nx.reserve(N * 4); p->ny.reserve(N * 4); p->nz.reserve(N * 4);
     p->r_model.reserve((size_t)max_frames * 16);
     p->r_best.reserve((size_t)max_frames * 4);
@@ -412,8 +452,7 @@ rvp_status rvp_pipeline_run_device(rvp_pipeline *p, const float *x, const float 
     p->mark(1);
     if (p->record_stages) RVP_CUDA_TRY(cudaEventRecord(p->ev_stage[0], st));
     p->points_last = N;
-    p->grid_built =
-        !(p->tree_fits && (c.queries_per_warp == 0 || c.queries_per_warp == 3));
+    p->grid_built = !p->on_tree();
     if (!p->grid_built) {
       run_tree(p, n_frames, N);
       run_ransac(p, n_frames);
@@ -621,23 +660,9 @@ rvp_status rvp_pipeline_fit_tables(rvp_pipeline *p) {
   return guard(p->ctx, [&] {
     RVP_CUDA_TRY(cudaSetDevice(p->ctx->device));
     if (p->n_frames_last < 1) return;  // no run to measure
-    if (!p->grid_built) {  // it used the tree: the buckets its grid would have
-      const int64_t *offs = p->vox_offs.as<int64_t>();
-      rvp::grid_build(p->ctx, p->grid, p->vox_x.as<float>(), p->vox_y.as<float>(),
-                      p->vox_z.as<float>(), offs, p->n_frames_last, p->points_last, p->cell,
-                      rvp::KEY_DENSE, 0, 0, reinterpret_cast<const u64 *>(offs + p->n_frames_last),
-                      p->grid_base, p->vox_aos.as<float>());
-    }
-    u64 nb[rvp::kHeadLevels] = {};
-    RVP_CUDA_TRY(cudaMemcpyAsync(nb, p->grid.d_nbuckets, 8 * rvp::kHeadLevels, cudaMemcpyDeviceToHost,
-                                 p->ctx->stream));
-    RVP_CUDA_TRY(cudaStreamSynchronize(p->ctx->stream));
-    // a quarter of headroom for batches whose scenes occupy more cells than
-    // this one; the table (2.5 slots per bucket, rounded up to a power of
-    // two) then stays inside L2, where every probe of the kNN kernels lands
-    size_t tot = 0;
-    for (int l = 0; l < rvp::kGridLevels; ++l) tot += (size_t)nb[l];
-    p->grid.fit_table(tot + tot / 4);
+    // (the tree has no table: the fit waits for a mode that searches the grid)
+    p->fit_wanted = !p->grid_built;
+    if (p->grid_built) fit_grid(p);
   });
 }
 
@@ -709,11 +734,23 @@ rvp_status rvp_pipeline_set_tuning(rvp_pipeline *p, float cell_size, int block_t
   // the warp-per-query kernel is compiled for blocks of at most 256 threads
   if (block_threads < 0 || block_threads > 256 || (block_threads % 32) != 0)
     return RVP_ERR_INVALID_ARG;
-  p->cell = cell_size;
-  p->cfg.cell_size = cell_size;
-  p->cfg.block_threads = block_threads;
-  p->cfg.queries_per_warp = queries_per_warp;
-  return RVP_OK;
+  return guard(p->ctx, [&] {
+    const rvp_pipeline_config before = p->cfg;
+    const float cell = p->cell;
+    p->cell = cell_size;
+    p->cfg.cell_size = cell_size;
+    p->cfg.block_threads = block_threads;
+    p->cfg.queries_per_warp = queries_per_warp;
+    if (p->on_tree()) return;
+    RVP_CUDA_TRY(cudaSetDevice(p->ctx->device));
+    try {
+      enter_grid(p);
+    } catch (...) {  // the former setting stays
+      p->cfg = before;
+      p->cell = cell;
+      throw;
+    }
+  });
 }
 
 rvp_status rvp_pipeline_set_search_radius_factor(rvp_pipeline *p, float rfac) {
