@@ -283,8 +283,15 @@ void knn_hash(rvp_hash *h, const float *qx, const float *qy, const float *qz, si
     if (p.idx) p.idx += a * K;
     if (p.d2) p.d2 += a * K;
     if (p.counts) p.counts += a;
-    const rvp::TreeQueries q = rvp::tree_queries(h->ctx, h->tree, h->tree_view, x, y, z, qx + a,
-                                                 qy + a, qz + a, m);
+    rvp::TreeQueries q{};
+    if (rvp::tree_knn_few(m, radius)) {
+      q.n = (u32)m;
+      q.each[0] = qx + a;
+      q.each[1] = qy + a;
+      q.each[2] = qz + a;
+    } else {
+      q = rvp::tree_queries(h->ctx, h->tree, h->tree_view, x, y, z, qx + a, qy + a, qz + a, m);
+    }
     rvp::tree_knn(h->ctx, h->tree_view, q, K, radius, mode, p);
   }
 }

@@ -431,6 +431,7 @@ struct TreeQueries {
   u32 *hard_count = nullptr;     // queries left for the warp-per-query kernel
   u32 *hard = nullptr;           // (their places in q, or in the tree)
   u32 *longer = nullptr;         // queries with long radius lists
+  const float *each[3] = {};     // or: few queries in their own order, one per warp
   const u32 *list = nullptr;     // with frames: these positions only
   const u64 *n_list = nullptr;
   u32 n = 0;
@@ -478,6 +479,9 @@ TreeQueries tree_queries(rvp_context *ctx, KnnTree &w, const TreeView &t, const 
                          const float *qz, size_t nq);
 // the same for queries in their own order (tree_radius_few)
 TreeQueries tree_queries_as_given(rvp_context *ctx, KnnTree &w, size_t nq);
+// queries that go one per warp, in their own order (TreeQueries::each; TREE_MEAN
+// and TREE_PAIRS)
+bool tree_knn_few(size_t nq, float radius);
 // radius > 0: neighbours with d2 <= radius * radius only
 void tree_knn(rvp_context *ctx, const TreeView &t, const TreeQueries &q, int k, float radius,
               int mode, const TreeOut &o);

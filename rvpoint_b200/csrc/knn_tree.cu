@@ -16,7 +16,8 @@
 // its sorted list, all lanes in step. With the K-th distance known, the leaves
 // scanned are gone over again, the points within it collected and each put at
 // its rank. Queries that do not fit this (far from their packet, equal
-// distances) are listed and answered one per warp by a second kernel.
+// distances) are listed and answered one per warp by a second kernel, as are
+// few queries of their own (tree_knn_few).
 //
 // Pruning needs no slack: every operation of the distance (subtract, square,
 // add) is monotone under rounding, so the distance to a box computed with the
@@ -240,11 +241,24 @@ TreeQueries tree_queries(rvp_context *ctx, KnnTree &w, const TreeView &t, const 
   return q;
 }
 
+// A packet of 32 queries takes some 200 us from end to end (with the sort that
+// makes packets of queries), however few there are; one query per warp takes
+// none of this, but five times the work. Queries among 400,000 LiDAR points, k 16, packets
+// and warps: 1000 queries 309 and 90 us, 16,000 360 and 200, 32,000 338 and 313,
+// 64,000 334 and 590; within 0.3 m 187 and 50, 257 and 74, 243 and 106, 243 and
+// 178, 128,000 292 and 311; within 3 m 32,000 305 and 221, 64,000 305 and 403.
+bool tree_knn_few(size_t nq, float radius) { return nq <= (radius > 0.0f ? 49152u : 24576u); }
+
 void tree_knn(rvp_context *ctx, const TreeView &t, const TreeQueries &q, int k, float radius,
               int mode, const TreeOut &o) {
   // the radius search's bound: d2 <= radius * radius in float
   volatile float r = radius;
   const float bound = radius > 0.0f ? r * r : INFINITY;
+  if (q.each[0]) {
+    if (mode == TREE_MEAN) launch_tree_each<TREE_MEAN, false>(ctx, t, q, q.n, k, bound, o);
+    else launch_tree_each<TREE_PAIRS, false>(ctx, t, q, q.n, k, bound, o);
+    return;
+  }
   const u32 packets = (q.n + 31) / 32;
   // the list leaves the point itself out where the host knows that the
   // queries are the cloud (n_sort: the device finds out)

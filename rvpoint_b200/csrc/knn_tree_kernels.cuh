@@ -147,28 +147,6 @@ __device__ __forceinline__ void parent_box(const float *kid, u32 kid_stride, u32
 // ---------------------------------------------------------------------------
 // search
 // ---------------------------------------------------------------------------
-// Walks every leaf within limit() of the box q, nearest child first. All
-// lanes take part; limit() is uniform and may shrink on the way.
-template <int LV, class Limit, class Leaf>
-__device__ __forceinline__ void tree_walk(const TreeView &t, const Box &q, u32 first, u32 end,
-                                          Limit &limit, Leaf &leaf) {
-  const int lane = threadIdx.x & 31;
-  const u32 c = first + lane;
-  const float lb = c < end ? box_d2(q, t.box[LV], t.stride[LV], c) : 0.0f;
-  bool open = c < end && lb <= limit();
-  while (true) {
-    // (the low bits of the distance give way to the lane)
-    const u32 key = open ? (__float_as_uint(lb) & ~31u) | lane : 0xFFFFFFFFu;
-    const u32 best = __reduce_min_sync(0xffffffffu, key);
-    if (best == 0xFFFFFFFFu) break;
-    const int s = best & 31;
-    if (lane == s) open = false;
-    if (__uint_as_float(best & ~31u) > limit()) break;  // and so are all that are left
-    if (__shfl_sync(0xffffffffu, lb, s) > limit()) continue;
-    if constexpr (LV == 0) leaf(first + s);
-    else tree_walk<LV - 1>(t, q, (first + s) * 32, t.count[LV - 1], limit, leaf);
-  }
-}
 // The nodes a search starts from: one cloud's top level (at most 32 nodes up to
 // 33.5M points), or a frame's level-1 nodes; 32 at a time.
 struct Roots {
@@ -176,15 +154,9 @@ struct Roots {
 };
 template <bool FRAMES>
 constexpr int tree_top() { return FRAMES ? 1 : kTreeLevels - 1; }
-template <bool FRAMES, class Limit, class Leaf>
-__device__ __forceinline__ void tree_walk_all(const TreeView &t, const Roots &r, const Box &q,
-                                              Limit &limit, Leaf &leaf) {
-  for (u32 f = r.first; f < r.end; f += 32)
-    tree_walk<tree_top<FRAMES>()>(t, q, f, r.end, limit, leaf);
-}
 
-// The same walk leaf by leaf, for a caller whose leaf code is too long to be
-// inlined more than once (it would not fit the instruction cache).
+// The leaves nearest first, one by one, for a caller whose leaf code is too long
+// to be inlined more than once (it would not fit the instruction cache).
 // element l of v without an index (v stays in registers)
 template <int N, class A>
 __device__ __forceinline__ auto by_level(const A &v, int l) {
@@ -671,107 +643,189 @@ __global__ __launch_bounds__(32, KCAP > 32 ? 10 : 16) void k_knn_tree(TreeView t
   }
 }
 
-// one warp per listed query, lanes over a leaf's points, a list of packed
-// (distance, index) keys over the lanes
+// ---------------------------------------------------------------------------
+// one query per warp: those the packets leave (qs.hard), or few of their own
+// (qs.each), in any order
+// ---------------------------------------------------------------------------
+// The leaves nearest first, two loaded at a time, a lane per point, a sorted
+// list of packed (distance, index) keys over the lanes: equal distances need no
+// care. Normals are left for the end: a warp takes up to 32 queries, keeps their
+// neighbours in columns of shared memory, and then every lane has one.
+// Bound by issue where there are many (about 1100 instructions per query of 16
+// within a few leaves, 65% of the issue slots), by the chain of one query, four
+// levels of boxes and then leaves, where there are few: 700 queries among
+// 150,000 LiDAR points, k 16, 45 us of a call, as packets 203. Keys collected in
+// shared memory and ranked all at once, or merged 16 at a time, took up to twice
+// the time of this (normals of a 700,000-point lattice 5.4 and 3.8 ms, 3.1 here;
+// 4.0 with a lane of the warp making each normal).
+constexpr int EK_WARPS = 4;
+constexpr int EK_MERGE = 8;  // keys of a leaf that are merged at once
+template <int MODE>
+constexpr size_t each_smem(int K) {
+  constexpr bool normals = MODE == TREE_NORMALS || MODE == TREE_PRECISE;
+  return normals ? (size_t)EK_WARPS * K * 128 : 0;
+}
+
+// Visits the leaves within limit() of the box q, nearest child first: leaf(l, p)
+// with the lane's point of a leaf, from load(l).
+template <int LV, class Limit, class Load, class Leaf>
+__device__ __forceinline__ void each_walk(const TreeView &t, const Box &q, u32 first, u32 end,
+                                          Limit &limit, Load &load, Leaf &leaf) {
+  const int lane = threadIdx.x & 31;
+  const u32 c = first + lane;
+  const float lb = c < end ? box_d2(q, t.box[LV], t.stride[LV], c) : 0.0f;
+  bool open = c < end && lb <= limit();
+  // the nearest open child, no longer open; -1: none (near enough)
+  auto nearest = [&]() {
+    // (the low bits of the distance give way to the lane)
+    const u32 best = __reduce_min_sync(
+        0xffffffffu, open ? (__float_as_uint(lb) & ~31u) | lane : 0xFFFFFFFFu);
+    if (best == 0xFFFFFFFFu || __uint_as_float(best & ~31u) > limit()) return -1;
+    if (lane == (int)(best & 31)) open = false;
+    return (int)(best & 31);
+  };
+  auto near = [&](int s) { return __shfl_sync(0xffffffffu, lb, s) <= limit(); };
+  while (true) {
+    const int s = nearest();
+    if (s < 0) break;
+    if constexpr (LV > 0) {
+      if (near(s))
+        each_walk<LV - 1>(t, q, (first + s) * 32, t.count[LV - 1], limit, load, leaf);
+    } else {
+      const int s2 = nearest();
+      const float4 p = load(first + s);
+      const float4 p2 = s2 >= 0 ? load(first + s2) : p;
+      if (near(s)) leaf(first + s, p);
+      if (s2 < 0) break;
+      if (near(s2)) leaf(first + s2, p2);
+    }
+  }
+}
+
 template <int P, int MODE, bool FRAMES>
-__global__ __launch_bounds__(128) void k_knn_tree_hard(TreeView t, TreeQueries qs, int K,
-                                                       float bound, TreeOut o) {
-  __shared__ float4 near[4][32 * P];  // the neighbours in order
+__global__ __launch_bounds__(EK_WARPS * 32, 6) void k_knn_tree_each(TreeView t, TreeQueries qs,
+                                                                    int K, float bound,
+                                                                    TreeOut o) {
+  extern __shared__ __align__(16) unsigned char tree_sm[];
+  constexpr bool NORMALS = MODE == TREE_NORMALS || MODE == TREE_PRECISE;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const u32 n = *qs.hard_count;
+  u32(*columns)[32] = reinterpret_cast<u32(*)[32]>(tree_sm) + wib * K;
+  const bool each = qs.each[0] != nullptr;
+  const u32 n = each ? qs.n : *qs.hard_count, warps = gridDim.x * EK_WARPS;
   const bool self = FRAMES || qs.n_sort == nullptr || *qs.n_sort == 0;
-  for (u32 w = blockIdx.x * 4 + wib; w < n; w += gridDim.x * 4) {
-    const u32 qi = qs.hard[w];
-    const float4 q = self ? t.pts[qi] : qs.q[qi];
-    const u32 qidx = __float_as_uint(q.w) & (FRAMES ? 0x7FFFFFFFu : 0xFFFFFFFFu);
-    u32 start = qi / 32;
-    Roots roots{0, t.count[kTreeLevels - 1]};
-    u32 leaf0 = 0, leaf1 = t.count[0] - 1;
-    if constexpr (FRAMES) {
-      const uint2 nodes = t.frame_nodes[t.node_frame[qi / 1024]];
-      roots = Roots{nodes.x, nodes.y};
-      leaf0 = nodes.x * 32;
-      leaf1 = nodes.y * 32 - 1;
-    } else if (!self) {
-      start = leaf_of_key(t, qs.keys[qi]);
-    }
-    WarpList<P> W;
-    W.init();
-    u64 key_thr = ~0ull;
-    u32 found = 0;
-    const Box own{{q.x, q.y, q.z}, {q.x, q.y, q.z}};
-    auto limit = [&]() {
-      return key_thr == ~0ull ? bound : fminf(nbr_d2(key_thr), bound);
-    };
-    auto scan = [&](u32 l) {
-      const u32 i = l * 32 + lane;
-      u64 key = ~0ull;
-      if (i < t.n) {
-        const float4 p = __ldg(&t.pts[i]);
+  auto query = [&](u32 w) {
+    if (each) return make_float4(qs.each[0][w], qs.each[1][w], qs.each[2][w], __uint_as_float(w));
+    return self ? t.pts[qs.hard[w]] : qs.q[qs.hard[w]];
+  };
+  auto index_of = [](const float4 &q) {
+    return __float_as_uint(q.w) & (FRAMES ? 0x7FFFFFFFu : 0xFFFFFFFFu);
+  };
+  const u32 chunk = NORMALS ? min(32u, (n + warps - 1) / warps) : 1u;  // queries per turn
+  for (u32 w0 = (blockIdx.x * EK_WARPS + wib) * chunk; w0 < n; w0 += warps * chunk) {
+    const u32 m = min(chunk, n - w0);
+    int mine = 0;  // the lane's query's neighbours
+    for (u32 c = 0; c < m; ++c) {
+      const float4 q = query(w0 + c);
+      const u32 qidx = index_of(q);
+      Roots roots{0, t.count[kTreeLevels - 1]};
+      u32 s0 = 1, s1 = 0;  // leaves tested before the walk: around the cloud's own point
+      if constexpr (FRAMES) {
+        const u32 qi = qs.hard[w0 + c];
+        const uint2 nodes = t.frame_nodes[t.node_frame[qi / 1024]];
+        roots = Roots{nodes.x, nodes.y};
+        s0 = max(qi / 32, nodes.x * 32 + 1) - 1;
+        s1 = min(qi / 32 + 1, nodes.y * 32 - 1);
+      } else if (!each && self) {
+        const u32 leaf = qs.hard[w0 + c] / 32;
+        s0 = max(leaf, 1u) - 1;
+        s1 = min(leaf + 1, t.count[0] - 1);
+      }
+      WarpList<P> W;
+      W.init();
+      u32 found = 0;
+      u64 thr = ~0ull;  // the K-th key, once there are K
+      auto limit = [&]() { return thr == ~0ull ? bound : fminf(nbr_d2(thr), bound); };
+      auto load = [&](u32 l) {
+        const u32 i = l * 32 + lane;
+        return i < t.n ? __ldg(&t.pts[i]) : make_float4(NAN, NAN, NAN, 0.0f);
+      };
+      auto take = [&](const float4 &p) {
         const float d = dist2(p.x, p.y, p.z, q.x, q.y, q.z);
-        if (d <= bound) key = pack_nbr(d, (int)__float_as_uint(p.w));
-      }
-      found += __popc(__ballot_sync(0xffffffffu, key != ~0ull));
-      unsigned m = __ballot_sync(0xffffffffu, key < key_thr);
-      if constexpr (P == 1) {
-        if (__popc(m) > 4) {  // many at once: one merge instead of serial inserts
-          W.merge_lanes((m >> lane) & 1u ? key : ~0ull);
-          key_thr = W.get(K - 1);
-          m = 0;
+        const u64 key = d <= bound ? pack_nbr(d, (int)__float_as_uint(p.w)) : ~0ull;
+        unsigned m = __ballot_sync(0xffffffffu, key < thr);
+        found += __popc(m);  // (more than there are, past the K-th)
+        if constexpr (P == 1) {
+          if (__popc(m) > EK_MERGE) {  // many at once: one merge instead of serial inserts
+            W.merge_lanes((m >> lane) & 1u ? key : ~0ull);
+            thr = W.get(K - 1);
+            m = 0;
+          }
         }
-      }
-      while (m) {
-        const int b = __ffs(m) - 1;
-        m &= m - 1;
-        const u64 k = __shfl_sync(0xffffffffu, key, b);
-        if (k < key_thr) {
-          W.insert(k);
-          key_thr = W.get(K - 1);
+        while (m) {
+          const int b = __ffs(m) - 1;
+          m &= m - 1;
+          const u64 k = __shfl_sync(0xffffffffu, key, b);
+          if (k < thr) {
+            W.insert(k);
+            thr = W.get(K - 1);
+          }
         }
+      };
+      // (a query with a NaN is near nothing)
+      if (!(isnan(q.x) || isnan(q.y) || isnan(q.z))) {
+        const Box own{{q.x, q.y, q.z}, {q.x, q.y, q.z}};
+        if (s0 <= s1) {
+          const float4 a = load(s0), b = load(min(s0 + 1, s1)), e = load(s1);
+          take(a);
+          if (s0 + 1 <= s1) take(b);
+          if (s0 + 2 <= s1) take(e);
+        }
+        auto leaf = [&](u32 l, const float4 &p) {
+          if (l < s0 || l > s1) take(p);
+        };
+        for (u32 f = roots.first; f < roots.end; f += 32)
+          each_walk<tree_top<FRAMES>()>(t, own, f, roots.end, limit, load, leaf);
       }
-    };
-    const u32 s0 = start > leaf0 ? start - 1 : leaf0, s1 = min(start + 1, leaf1);
-    auto leaf = [&](u32 l) {
-      if (l < s0 || l > s1) scan(l);
-    };
-    const bool unplaced = isnan(q.x) || isnan(q.y) || isnan(q.z);  // near nothing
-    if (!unplaced) {
-      for (u32 l = s0; l <= s1; ++l) scan(l);
-      tree_walk_all<FRAMES>(t, roots, own, limit, leaf);
-    }
-    const int have = min((int)found, K);
-    if (o.n_hard && lane == 0) atomicAdd(o.n_hard, 1u);
-    if constexpr (MODE == TREE_MEAN || MODE == TREE_LIST) {
-      float sum = 0.0f;
-      for (int j = 1; j < have; ++j) sum = fadd(sum, __fsqrt_rn(nbr_d2(W.get(j))));
-      if (lane == 0) tree_mean_out(sum, have, q, qidx, o);
-    }
-    if constexpr (MODE != TREE_MEAN) {
+      const int have = min((int)found, K);
+      if (o.n_hard && lane == 0) atomicAdd(o.n_hard, 1u);
+      if constexpr (MODE == TREE_MEAN || MODE == TREE_LIST) {
+        float sum = 0.0f;
 #pragma unroll
-      for (int p = 0; p < P; ++p) {
-        const int j = p * 32 + lane;
-        if constexpr (MODE == TREE_PAIRS) {
-          if (j < K) {
+        for (int p = 0; p < P; ++p) {
+          const float r = __fsqrt_rn(nbr_d2(W.e[p]));
+          for (int j = p == 0 ? 1 : 0; j < min(32, have - p * 32); ++j)
+            sum = fadd(sum, __shfl_sync(0xffffffffu, r, j));
+        }
+        if (lane == 0) tree_mean_out(sum, have, q, qidx, o);
+      }
+      if constexpr (MODE != TREE_MEAN) {
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+          const int j = p * 32 + lane;
+          if (j >= K) continue;
+          if constexpr (MODE == TREE_PAIRS) {
             const size_t at = (size_t)qidx * K + j;
             if (o.idx) o.idx[at] = j < have ? nbr_idx(W.e[p]) : -1;
             if (o.d2) o.d2[at] = j < have ? nbr_d2(W.e[p]) : INFINITY;
-          }
-        } else if constexpr (MODE == TREE_LIST) {
-          if (j < K)
-            o.rows[(size_t)qi * K + j] =
+          } else {
+            const u32 at =
                 j < have ? t.pos_of[(u32)nbr_idx(W.e[p]) & 0x7FFFFFFFu] : 0xFFFFFFFFu;
-        } else {
-          if (j < have) near[wib][j] = __ldg(&t.pts[t.pos_of[(u32)nbr_idx(W.e[p]) & 0x7FFFFFFFu]]);
+            if constexpr (NORMALS) columns[j][c] = at;
+            else o.rows[(size_t)qs.hard[w0 + c] * K + j] = at;
+          }
         }
+        if (MODE == TREE_PAIRS && lane == 0 && o.counts) o.counts[qidx] = have;
+        if (lane == (int)c) mine = have;
       }
-      if constexpr (MODE == TREE_PAIRS) {
-        if (lane == 0 && o.counts) o.counts[qidx] = have;
-      } else if constexpr (MODE != TREE_LIST) {
-        __syncwarp();
-        if (lane == 0)
-          tree_normal_out<MODE>([&](int j) { return near[wib][j]; }, have, q, qidx, o);
-        __syncwarp();
+    }
+    if constexpr (NORMALS) {
+      __syncwarp();
+      if (lane < (int)m) {
+        const float4 q = query(w0 + lane);
+        tree_normal_out<MODE>([&](int j) { return __ldg(&t.pts[columns[j][lane]]); }, mine, q,
+                              index_of(q), o);
       }
+      __syncwarp();
     }
   }
 }
@@ -797,6 +851,22 @@ __global__ __launch_bounds__(TP_TH, 6) void k_tree_precise(TreeView t, int K, u3
       [&](int j) { return __ldg(&t.pts[row[(size_t)j * 32]]); }, have, q, __float_as_uint(q.w), o);
 }
 
+// queries: how many there can be
+template <int MODE, bool FRAMES>
+void launch_tree_each(rvp_context *ctx, const TreeView &t, const TreeQueries &q, size_t queries,
+                      int K, float bound, const TreeOut &o) {
+  static_assert(each_smem<MODE>(64) <= 48 * 1024, "no opt-in to larger shared memory here");
+  const unsigned blocks = grid_for(queries, EK_WARPS, ctx->num_sms * 8);
+  const size_t smem = each_smem<MODE>(K);
+  if (K <= 32)
+    k_knn_tree_each<1, MODE, FRAMES><<<blocks, EK_WARPS * 32, smem, ctx->stream>>>(t, q, K, bound,
+                                                                                  o);
+  else
+    k_knn_tree_each<2, MODE, FRAMES><<<blocks, EK_WARPS * 32, smem, ctx->stream>>>(t, q, K, bound,
+                                                                                  o);
+  RVP_LAUNCH_CHECK(ctx);
+}
+
 // packets: how many there can be
 template <int KCAP, int MODE, bool FRAMES>
 void launch_tree(rvp_context *ctx, const TreeView &t, const TreeQueries &q, u32 packets, int K,
@@ -818,12 +888,7 @@ void launch_tree(rvp_context *ctx, const TreeView &t, const TreeQueries &q, u32 
     k_knn_tree<KCAP, MODE, FRAMES><<<packets, 32, smem, ctx->stream>>>(t, q, K, bound, o);
     RVP_LAUNCH_CHECK(ctx);
   }
-  const unsigned blocks = grid_for(packets * 32, 4, ctx->num_sms * 8);
-  if (K <= 32)
-    k_knn_tree_hard<1, MODE, FRAMES><<<blocks, 128, 0, ctx->stream>>>(t, q, K, bound, o);
-  else
-    k_knn_tree_hard<2, MODE, FRAMES><<<blocks, 128, 0, ctx->stream>>>(t, q, K, bound, o);
-  RVP_LAUNCH_CHECK(ctx);
+  launch_tree_each<MODE, FRAMES>(ctx, t, q, packets * 32, K, bound, o);
 }
 
 // listed: distances a list needs room for

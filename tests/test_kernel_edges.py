@@ -332,3 +332,48 @@ def test_ransac_rounds(gpu_ctx, restatement, n, iters):
         assert got == best and np.array_equal(bits(m), bits(np.asarray(model, np.float32)))
     best2, _, _, ran2 = api.ransac_plane_rvv(c, 0.01, iters, return_counts=True)
     assert best2 == best and ran2 == ran
+
+
+# up to 24576 queries (49152 within a radius) go one per warp, more in packets
+@pytest.mark.parametrize("nq,radius", [(24_576, 0.0), (49_152, 0.3)])
+@pytest.mark.parametrize("k", [1, 9, 17, 40])
+@pytest.mark.parametrize("cloud", ["room", "lattice"])
+def test_few_and_many_queries(gpu_ctx, nq, radius, k, cloud):
+    from rvpoint_b200.api import SpatialHash
+    n = 50_000
+    if cloud == "lattice":
+        i = np.arange(n)
+        c = D.Cloud.from_xyz(np.stack([i % 41, (i // 41) % 43, i // 1763], 1) % 38 * 0.25)
+    else:
+        c = D.room_cloud(n=n, seed=k)
+    p = c.aos()
+    h = SpatialHash()
+    h.setInputCloud(c, 0.5)
+    h.build()
+    rng = np.random.default_rng(nq)
+    q = np.concatenate([p[rng.permutation(n)[:nq - 500]],
+                        rng.uniform(-9, 9, (501, 3)).astype(np.float32)])
+    few = h.knn(*q[:nq].T, k, radius)
+    many = h.knn(*q.T, k, radius)
+    for a, b in zip(few, many):
+        assert np.array_equal(a.view(np.int32), b[:nq].view(np.int32))
+    at = np.concatenate([rng.choice(nq, 100, replace=False), [nq]])
+    idx, d2 = brute_knn(p, q[at], k, np.float32(radius) * np.float32(radius) if radius else np.inf)
+    assert np.array_equal(many[0][at], idx) and np.array_equal(bits(many[1][at]), bits(d2))
+    assert np.array_equal(many[2][at], (idx >= 0).sum(1))
+
+
+# a call for few queries is one kernel (the queries are neither sorted nor
+# compared with the cloud)
+def test_few_queries_are_one_launch(gpu_ctx):
+    import torch
+    from rvpoint_b200.api import SpatialHash
+    c = D.room_cloud(n=60_000, seed=1)
+    v = [torch.from_numpy(np.array(a)).cuda() for a in (c.x, c.y, c.z)]
+    h = SpatialHash()
+    h.setInputCloud(v, 0.5)
+    h.build()
+    for nq, radius in ((1, 0.0), (700, 0.0), (24_576, 0.0), (40_000, 0.3)):
+        before = gpu_ctx.launches
+        h.knn(*[a[:nq] for a in v], 16, radius)
+        assert gpu_ctx.launches - before == 1
