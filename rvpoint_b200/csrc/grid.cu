@@ -404,13 +404,6 @@ GridView Grid::view(int mode, long long p1, long long p2) const {
   return v;
 }
 
-void cloud_bbox(rvp_context *ctx, const float *x, const float *y, const float *z, size_t n,
-                float *bb) {
-  k_bbox<<<grid_for(n, 256, ctx->num_sms * kBoxBlocks), 256, 0, ctx->stream>>>(
-      x, y, z, nullptr, 1, n, nullptr, bb);
-  RVP_LAUNCH_CHECK(ctx);
-}
-
 void frames_bbox(rvp_context *ctx, const float *x, const float *y, const float *z,
                  const int64_t *offs, int n_frames, size_t n_max, float *bb) {
   k_bbox_init<<<grid_for(n_frames, 256, 64), 256, 0, ctx->stream>>>(bb, n_frames);

@@ -527,9 +527,6 @@ void tree_radius_normals(rvp_context *ctx, const TreeView &t, float radius, int 
                          u32 *huge, u32 *counts);
 void gather_queries(rvp_context *ctx, const float *x, const float *y, const float *z,
                     const u32 *list, size_t n, float *qx, float *qy, float *qz);
-// bounds of a cloud, folded into bb (min x, y, z, max x, y, z)
-void cloud_bbox(rvp_context *ctx, const float *x, const float *y, const float *z, size_t n,
-                float *bb);
 
 // ---------------------------------------------------------------------------
 // voxel grid (voxel.cu)

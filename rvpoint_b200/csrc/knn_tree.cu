@@ -1,7 +1,7 @@
 // Exact k nearest neighbours in one cloud (k <= 64) over a 32-wide box tree.
 //
 // Build: the points sorted by the Hilbert code of their quantised position
-// (32 bits, one power-of-two cell for all axes), every 32 consecutive points
+// (32 bits or more, one power-of-two cell for all axes), every 32 consecutive points
 // a leaf with its bounding box, every 32 leaves a node, and so on, four levels
 // in all. No cell size is chosen and nothing depends on the
 // density: a leaf is small where the points are dense.
@@ -41,27 +41,86 @@ namespace {
 // ---------------------------------------------------------------------------
 // build
 // ---------------------------------------------------------------------------
-__global__ void k_tree_init(float *bb) {
-  if (threadIdx.x < 3) bb[threadIdx.x] = INFINITY;
-  else if (threadIdx.x < 6) bb[threadIdx.x] = -INFINITY;
+// KnnTree::misc
+struct TreeMisc {
+  float bb[8];                    // the box
+  alignas(16) TreeSample sample;  // and a sample
+  u64 n_sort;                     // queries to sort
+};
+__global__ void k_tree_init(TreeMisc *m) {
+  if (threadIdx.x < 3) m->bb[threadIdx.x] = INFINITY;
+  else if (threadIdx.x < 6) m->bb[threadIdx.x] = -INFINITY;
+}
+
+// The cloud's box, six atomics per block (at most kBoxBlocks blocks per SM: the
+// atomics meet on the same words), and beside them a block for the sample.
+constexpr int kBoxBlocks = 4;
+__global__ __launch_bounds__(256) void k_tree_box(const float *__restrict__ x,
+                                                  const float *__restrict__ y,
+                                                  const float *__restrict__ z, size_t n,
+                                                  TreeMisc *misc) {
+  __shared__ float part[6][8];
+  __shared__ TreeSample S;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const u32 blocks = gridDim.x - 1;
+  if (blockIdx.x == blocks) {
+    tree_sample(x, y, z, n, &S);
+    __syncthreads();
+    if (tid == 0) misc->sample = S;
+    return;
+  }
+  const size_t per = ((n + blocks - 1) / blocks + 255) & ~(size_t)255;
+  const size_t from = blockIdx.x * per, to = from + per < n ? from + per : n;
+  float m[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll 4
+  for (size_t i = from + tid; i < to; i += 256) {
+    const float v[3] = {x[i], y[i], z[i]};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      m[a] = fminf(m[a], v[a]);
+      m[3 + a] = fmaxf(m[3 + a], v[a]);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      const float t = __shfl_xor_sync(0xffffffffu, m[k], o);
+      m[k] = k < 3 ? fminf(m[k], t) : fmaxf(m[k], t);
+    }
+    if (lane == 0) part[k][wid] = m[k];
+  }
+  __syncthreads();
+  if (tid < 6) {
+    float v = part[tid][0];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) v = tid < 3 ? fminf(v, part[tid][w]) : fmaxf(v, part[tid][w]);
+    if (tid < 3) {
+      if (v < INFINITY) atomic_min_f(misc->bb + tid, v);
+    } else if (v > -INFINITY) {
+      atomic_max_f(misc->bb + tid, v);
+    }
+  }
 }
 
 __global__ __launch_bounds__(256) void k_tree_keys(const float *__restrict__ x,
                                                    const float *__restrict__ y,
                                                    const float *__restrict__ z, size_t n_max,
-                                                   const u64 *n_dev, const float *bb, u64 *keys,
-                                                   u32 *vals, u64 *bits) {
+                                                   const u64 *n_dev, const TreeMisc *misc,
+                                                   size_t n_cloud, u64 *keys, u32 *vals,
+                                                   u64 *bits) {
   __shared__ TreeFrame F;
   __shared__ unsigned short table[192];
   const size_t n = n_dev ? *n_dev : n_max;
   if (n == 0) return;
-  if (threadIdx.x == 255) tree_frame(bb, tree_key_bits(n_max), F);
+  if (threadIdx.x == 255)
+    tree_frame_fine(n_cloud, misc->bb, misc->sample, tree_key_bits(n_cloud), F);
   tree_key_table(table);
   __syncthreads();
   u64 ones = 0, zeros = 0;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
-    const u64 k = tree_key(F, table, x[i], y[i], z[i]);
+    const u64 k = tree_key<u64>(F, table, x[i], y[i], z[i]);
     keys[i] = k;
     vals[i] = (u32)i;
     ones |= k;
@@ -151,7 +210,8 @@ TreeView tree_build(rvp_context *ctx, KnnTree &w, const float *x, const float *y
   w.sort.reserve(sort_temp_bytes(n));
   w.pts.reserve(n * 16);
   w.pos.reserve(n * 4);
-  w.misc.reserve(256);
+  w.misc.reserve(sizeof(TreeMisc));
+  TreeMisc *misc = w.misc.as<TreeMisc>();
   TreeView t{};
   t.n = (u32)n;
   size_t total = 0;
@@ -170,16 +230,17 @@ TreeView tree_build(rvp_context *ctx, KnnTree &w, const float *x, const float *y
   t.pts = w.pts.as<float4>();
   t.pos_of = w.pos.as<u32>();
   t.keys = w.keys.as<u64>();
-  t.bb = w.misc.as<float>();
+  t.bb = misc->bb;
   cudaStream_t st = ctx->stream;
   const int sms = ctx->num_sms;
-  k_tree_init<<<1, 32, 0, st>>>(w.misc.as<float>());
+  k_tree_init<<<1, 32, 0, st>>>(misc);
   RVP_LAUNCH_CHECK(ctx);
-  cloud_bbox(ctx, x, y, z, n, w.misc.as<float>());
+  k_tree_box<<<grid_for(n, 256, sms * kBoxBlocks) + 1, 256, 0, st>>>(x, y, z, n, misc);
+  RVP_LAUNCH_CHECK(ctx);
   SortTemp tmp;
   sort_temp_carve(tmp, w.sort.ptr, n);
   u64 *bits = sort_key_bits(ctx, tmp, n);
-  k_tree_keys<<<grid_for(n, 256, sms * 8), 256, 0, st>>>(x, y, z, n, nullptr, t.bb,
+  k_tree_keys<<<grid_for(n, 256, sms * 8), 256, 0, st>>>(x, y, z, n, nullptr, misc, n,
                                                          w.keys.as<u64>(), w.vals.as<u32>(), bits);
   RVP_LAUNCH_CHECK(ctx);
   radix_sort_pairs(ctx, w.keys.as<u64>(), w.vals.as<u32>(), n, nullptr, tmp, bits);
@@ -217,7 +278,7 @@ TreeQueries tree_queries(rvp_context *ctx, KnnTree &w, const TreeView &t, const 
   w.qvals.reserve(nq * 4);
   w.qpts.reserve(nq * 16);
   w.sort.reserve(sort_temp_bytes(std::max<size_t>(nq, t.n)));
-  u64 *n_sort = w.misc.as<u64>() + 4;
+  u64 *n_sort = &w.misc.as<TreeMisc>()->n_sort;
   cudaStream_t st = ctx->stream;
   const unsigned gb = grid_for(nq, 256, ctx->num_sms * 8);
   k_tree_count<<<1, 1, 0, st>>>(n_sort, nq == t.n ? 0 : (u64)nq);
@@ -229,7 +290,7 @@ TreeQueries tree_queries(rvp_context *ctx, KnnTree &w, const TreeView &t, const 
   SortTemp tmp;
   sort_temp_carve(tmp, w.sort.ptr, nq);
   u64 *bits = sort_key_bits(ctx, tmp, nq);
-  k_tree_keys<<<gb, 256, 0, st>>>(qx, qy, qz, nq, n_sort, t.bb, w.qkeys.as<u64>(),
+  k_tree_keys<<<gb, 256, 0, st>>>(qx, qy, qz, nq, n_sort, w.misc.as<TreeMisc>(), t.n, w.qkeys.as<u64>(),
                                   w.qvals.as<u32>(), bits);
   RVP_LAUNCH_CHECK(ctx);
   radix_sort_pairs(ctx, w.qkeys.as<u64>(), w.qvals.as<u32>(), nq, n_sort, tmp, bits);

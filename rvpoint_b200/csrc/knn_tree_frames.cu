@@ -78,7 +78,7 @@ __global__ __launch_bounds__(256) void k_frames_keys(const float *__restrict__ x
     const int lo = s_lo, hi = s_hi;
     for (int64_t i = base + threadIdx.x; i < end; i += 256) {
       const int f = frame_of(offs, lo, hi, i);
-      const u64 k = ((u64)f << key_bits) | tree_key(F[f], table, x[i], y[i], z[i]);
+      const u64 k = ((u64)f << key_bits) | tree_key<u32>(F[f], table, x[i], y[i], z[i]);
       keys[i] = k;
       vals[i] = (u32)i;
       ones |= k;
@@ -189,7 +189,7 @@ __device__ __forceinline__ void small_frame(const float *x, const float *y, cons
   for (int r = 0; r < R; ++r) {
     const u32 i = r * 1024 + tid;
     key[r] = 0xFFFFFFFFu;
-    if ((int)i < m) key[r] = (tree_key(F, table, x[a + i], y[a + i], z[a + i]) << 11) | i;
+    if ((int)i < m) key[r] = (tree_key<u32>(F, table, x[a + i], y[a + i], z[a + i]) << 11) | i;
   }
   small_frame_sort<R>(key, s_key);
 #pragma unroll

@@ -377,3 +377,41 @@ def test_few_queries_are_one_launch(gpu_ctx):
         before = gpu_ctx.launches
         h.knn(*[a[:nq] for a in v], 16, radius)
         assert gpu_ctx.launches - before == 1
+
+
+# the codes that order the points are as long as the cloud needs: one far or
+# infinite point in a cloud of no order, or points dense in a few places, leave
+# the leaves small (with 32 bits all of the cloud was one cell: 150 times as long)
+@pytest.mark.parametrize("far", [1e6, 1e9, float("inf"), "clusters"])
+def test_far_points_do_not_spoil_the_order(gpu_ctx, far):
+    import time
+    import torch
+    from rvpoint_b200.api import SpatialHash
+    rng = np.random.default_rng(5)
+    p = (rng.uniform(-40, 40, (100_000, 3)) * [1, 1, 0.02]).astype(np.float32)
+    times, found = [], []
+    for spoilt in (False, True):
+        c = p.copy()
+        if spoilt:
+            if far == "clusters":
+                c[:50] = rng.choice([-3e6, 3e6], (50, 3))
+            else:
+                c[0] = far
+        v = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in c.T]
+        q = [a[50:] for a in v]
+        h = SpatialHash()
+        h.setInputCloud(v, 0.5)
+        h.build()
+        found.append([a.cpu().numpy() for a in h.radiusSearchBatch(*q, 0.3)])
+        t = []
+        for _ in range(5):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            h.radiusSearchBatch(*q, 0.3)
+            torch.cuda.synchronize()
+            t.append(time.perf_counter() - t0)
+        times.append(min(t))
+    near = np.diff(found[0][0])
+    lists = [[set(i[a:b][i[a:b] >= 50]) for a, b in zip(o[:500], o[1:501])] for o, i, _ in found]
+    assert lists[0] == lists[1] and near.max() > 3
+    assert times[1] < 10 * times[0]
