@@ -415,3 +415,40 @@ def test_far_points_do_not_spoil_the_order(gpu_ctx, far):
     lists = [[set(i[a:b][i[a:b] >= 50]) for a, b in zip(o[:500], o[1:501])] for o, i, _ in found]
     assert lists[0] == lists[1] and near.max() > 3
     assert times[1] < 10 * times[0]
+
+
+# many points in one place (returns that a sensor reports as 0, 0, 0), others
+# far around: their packets do not test each other's leaves
+def test_points_in_one_place(gpu_ctx, restatement):
+    import time
+    import torch
+    from rvpoint_b200 import api
+    rng = np.random.default_rng(3)
+    p = rng.normal(0, 1, (150_000, 3))
+    p = (p / np.linalg.norm(p, axis=1)[:, None] * rng.uniform(5, 6, (150_000, 1))).astype(np.float32)
+    at = rng.permutation(len(p))[:3000]
+    times = []
+    for same in (False, True):
+        if same:
+            p[at] = 0
+        v = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in p.T]
+        h = api.SpatialHash()
+        h.setInputCloud(v, 0.5)
+        h.build()
+        t = []
+        for _ in range(6):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            idx, d2, cnt = h.knn(*v, 16, 0.1)
+            torch.cuda.synchronize()
+            t.append(time.perf_counter() - t0)
+        times.append(min(t))
+    # (twice as long without the packets' early end and more)
+    assert times[1] < 1.9 * times[0]
+    first = np.sort(at)[:16]
+    assert np.array_equal(idx[at].cpu().numpy(), np.tile(first, (3000, 1)))
+    assert not d2[at].any() and bool((cnt[at] == 16).all())
+    few = D.Cloud.from_xyz(np.concatenate([p[at[:40]], p[:2500]]))
+    _, mean, keep = api.sor_rvv(few, 8, 1.0, return_stats=True)
+    _, mean2, keep2 = restatement.sor_exact(few, 8, 1.0)
+    assert np.array_equal(bits(mean), bits(mean2)) and np.array_equal(keep, keep2)
