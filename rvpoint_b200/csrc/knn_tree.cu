@@ -15,7 +15,7 @@
 // when one fills, every lane sorts its own in registers and merges them into
 // its sorted list, all lanes in step. With the K-th distance known, the leaves
 // scanned are gone over again, the points within it collected and each put at
-// its rank. Queries that do not fit this (far from their packet, equal
+// its rank. Queries that do not fit this (far from their packet, many equal
 // distances) are listed and answered one per warp by a second kernel, as are
 // few queries of their own (tree_knn_few).
 //

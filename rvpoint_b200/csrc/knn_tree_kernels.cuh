@@ -414,6 +414,26 @@ __device__ __forceinline__ void tree_normal_out(Nbr nbr, int have, const float4 
   o.nz[at] = nz;
 }
 
+// The ranks by (distance, index) of the points in a lane's column, five bits
+// each. (Not inlined: the search's own code is as long as it may be.)
+__device__ __noinline__ ulonglong2 tie_ranks(const float4 *pts, const uint2 *near, u32 *idx,
+                                             int cnt) {
+  for (int i = 0; i < cnt; ++i) idx[i * 32] = __float_as_uint(__ldg(&pts[near[i * 32].y]).w);
+  ulonglong2 ranks{0, 0};
+#pragma unroll 1
+  for (int i = 0; i < cnt; ++i) {
+    const u32 d = near[i * 32].x, own = idx[i * 32];
+    u64 r = 0;
+    for (int j = 0; j < cnt; ++j) {
+      const u32 e = near[j * 32].x;  // (distances are not negative: ordered as bits)
+      r += e < d || (e == d && idx[j * 32] < own) ? 1 : 0;
+    }
+    if (i < 12) ranks.x |= r << (5 * i);
+    else ranks.y |= r << (5 * (i - 12));
+  }
+  return ranks;
+}
+
 // One warp (block) per packet of 32 queries. The list holds the K nearest, or
 // for the cloud's own points the K - 1 nearest others (the point itself, at
 // distance 0, is the first of its row); KCAP is at least that, a power of two.
@@ -627,12 +647,12 @@ __global__ __launch_bounds__(32, KCAP > 32 ? 10 : 16) void k_knn_tree(TreeView t
   }
   if constexpr (!MEAN) {
     have = 0;
-    bool tied = false;
+    bool tied = false, twin = false;
 #pragma unroll
     for (int j = 0; j < KCAP; ++j) {
       if (j >= pad && L[j] < INFINITY) ++have;
       if (j > pad && L[j] < INFINITY && L[j] == L[j - (j > 0)]) tied = true;
-      if (drop && j == pad && L[j] == 0.0f) tied = true;  // another point in its place
+      if (drop && j == pad && L[j] == 0.0f) twin = true;  // another point in its place
     }
     // the points within the K-th distance, from the leaves scanned
     const float tau = mine ? fminf(fminf(L[KCAP - 1], bound), FLT_MAX) : -1.0f;
@@ -668,38 +688,53 @@ __global__ __launch_bounds__(32, KCAP > 32 ? 10 : 16) void k_knn_tree(TreeView t
         ++cnt;
       }
     }
-    // exactly these are within the K-th distance, no two equal (and what is
-    // missing is not there: points infinitely far would be)
-    exact = mine && cnt == have && !tied &&
-            (have == KL || bound < INFINITY || (!FRAMES && (u32)(have + (drop ? 1 : 0)) == t.n));
-    // each to its rank among the sorted distances, behind the point itself
+    // exactly these are within the K-th distance (and what is missing is not
+    // there: points infinitely far would be)
+    const bool whole =
+        have == KL || bound < INFINITY || (!FRAMES && (u32)(have + (drop ? 1 : 0)) == t.n);
+    exact = mine && cnt == have && !tied && !twin && whole;
     const int r0 = drop ? 1 : 0;
-    if (exact) {
-      if (drop) {
-        if constexpr (MODE == TREE_PAIRS) {
-          if (o.idx) o.idx[(size_t)qidx * K] = (int32_t)qidx;
-          if (o.d2) o.d2[(size_t)qidx * K] = 0.0f;
-        } else if constexpr (MODE == TREE_LIST) {
-          o.rows[(size_t)qi * K] = qi;
-        } else {
-          sorted[0][lane] = qi;
-        }
+    auto put = [&](int r, u32 p, float d) {  // the r-th neighbour
+      if constexpr (MODE == TREE_PAIRS) {
+        const size_t at = (size_t)qidx * K + r;
+        if (o.idx) o.idx[at] = (int32_t)__float_as_uint(__ldg(&t.pts[p]).w);
+        if (o.d2) o.d2[at] = d;
+      } else if constexpr (MODE == TREE_LIST) {
+        o.rows[(size_t)qi * K + r] = p;
+      } else {
+        sorted[r][lane] = p;
       }
+    };
+    // each to its rank among the sorted distances, behind the point itself
+    if (exact) {
+      if (drop) put(0, qi, 0.0f);
       for (int i = 0; i < have; ++i) {
         const uint2 b = pbuf[i][lane];
         const float d = __uint_as_float(b.x);
         int r = r0 - pad;
 #pragma unroll
         for (int j = 0; j < KCAP; ++j) r += L[j] < d ? 1 : 0;
-        if constexpr (MODE == TREE_PAIRS) {
-          const size_t at = (size_t)qidx * K + r;
-          if (o.idx) o.idx[at] = (int32_t)__float_as_uint(__ldg(&t.pts[b.y]).w);
-          if (o.d2) o.d2[at] = d;
-        } else if constexpr (MODE == TREE_LIST) {
-          o.rows[(size_t)qi * K + r] = b.y;
-        } else {
-          sorted[r][lane] = b.y;
+        put(r, b.y, d);
+      }
+    }
+    // Equal distances, and points past the list at the K-th: ranked by index as
+    // well. (In short lists: of 31 or 63 the comparisons take longer than the
+    // second kernel. Normals of a lattice of 700,000 points, k 16: 2.1 ms on the
+    // grid, 3.0 with all its queries in the second kernel, 1.2 here.)
+    if constexpr (KCAP <= 16) {
+      const bool ties =
+          mine && !twin && whole && cnt >= have && cnt <= PCAP && (tied || cnt > have);
+      if (ties) {
+        static_assert(PCAP <= kTreeNotes && PCAP <= 24, "an index, and five bits of rank, each");
+        const ulonglong2 ranks = tie_ranks(t.pts, &pbuf[0][lane], &notes[0][lane], cnt);
+        if (drop) put(0, qi, 0.0f);  // (over the notes)
+#pragma unroll 1
+        for (int i = 0; i < cnt; ++i) {
+          const int r = (int)((i < 12 ? ranks.x : ranks.y) >> (5 * (i < 12 ? i : i - 12))) & 31;
+          const uint2 b = pbuf[i][lane];
+          if (r < KL) put(r0 + r, b.y, __uint_as_float(b.x));
         }
+        exact = true;
       }
     }
     have += r0;

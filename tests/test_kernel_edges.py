@@ -452,3 +452,45 @@ def test_points_in_one_place(gpu_ctx, restatement):
     _, mean, keep = api.sor_rvv(few, 8, 1.0, return_stats=True)
     _, mean2, keep2 = restatement.sor_exact(few, 8, 1.0)
     assert np.array_equal(bits(mean), bits(mean2)) and np.array_equal(keep, keep2)
+
+
+# equal distances are ordered where a packet finds them: on a lattice, whose
+# every query has some, the second kernel is left with few
+@pytest.mark.parametrize("k", [6, 16])
+def test_lattice_stays_with_the_packets(gpu_ctx, k):
+    from rvpoint_b200.api import Pipeline
+    i = np.arange(20_000)
+    p = np.stack([i % 27, (i // 27) % 27, i // 729], 1).astype(np.float32) * 0.25 + np.float32(0.125)
+    b = D.Batch(p[:, 0].copy(), p[:, 1].copy(), p[:, 2].copy(), np.array([0, len(p)], np.int64))
+    got = []
+    for mode in (0, 1):
+        pipe = Pipeline(len(p), 1, leaf_size=0.25, sor_k=k, normal_k=k, sor_alpha=3.0,
+                        queries_per_warp=mode, ctx=gpu_ctx)
+        pipe.knn_stats(True)
+        got.append(pipe.run_host(b))
+        sor = pipe.knn_stats(False)["sor"]
+        pipe.close()
+        if mode == 0:  # (warp_ring0: the second kernel's)
+            assert sor["tile_l0"] + sor["warp_ring0"] == len(p) and sor["warp_ring0"] < len(p) / 4
+    for key in got[0]:
+        assert np.array_equal(np.asarray(got[0][key]), np.asarray(got[1][key]), equal_nan=True), key
+
+
+# and in the order of their indices, for many queries (packets) of every list
+@pytest.mark.parametrize("k", [2, 7, 9, 10, 16, 17])
+def test_packets_order_ties_by_index(gpu_ctx, k):
+    from rvpoint_b200.api import SpatialHash
+    n = 60_000
+    i = np.random.default_rng(k).permutation(n)
+    c = D.Cloud.from_xyz(np.stack([i % 41, (i // 41) % 43, i // 1763], 1) * 0.25)
+    p = c.aos()
+    h = SpatialHash()
+    h.setInputCloud(c, 0.5)
+    h.build()
+    at = np.random.default_rng(0).choice(n, 150, replace=False)
+    for q in (p, p + np.float32(0.125)):  # the cloud's own, and the middles of its cells
+        for r in (0.0, 0.5):
+            idx, d2, cnt = h.knn(*q.T, k, r)
+            idx2, dist2 = brute_knn(p, q[at], k, np.float32(r) * np.float32(r) if r else np.inf)
+            assert np.array_equal(idx[at], idx2) and np.array_equal(bits(d2[at]), bits(dist2))
+            assert np.array_equal(cnt[at], (idx2 >= 0).sum(1))
