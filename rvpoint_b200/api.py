@@ -231,6 +231,8 @@ class SpatialHash:
                 return 1
 
         st = _lib.RVP_ERR_CAPACITY
+        if capacity is None and 0 < max_nn and nq * max_nn <= 1 << 22:
+            capacity = nq * max_nn  # (the callback costs some 8 us)
         if capacity is not None:  # one call when the lists fit
             room(capacity)
             st = self.L.rvp_hash_radius_search(*args, _ptr(lists[0]), _ptr(lists[1]), capacity,

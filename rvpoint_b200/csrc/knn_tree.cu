@@ -304,11 +304,13 @@ TreeQueries tree_queries(rvp_context *ctx, KnnTree &w, const TreeView &t, const 
 
 // A packet of 32 queries takes some 200 us from end to end (with the sort that
 // makes packets of queries), however few there are; one query per warp takes
-// none of this, but five times the work. Queries among 400,000 LiDAR points, k 16, packets
-// and warps: 1000 queries 309 and 90 us, 16,000 360 and 200, 32,000 338 and 313,
-// 64,000 334 and 590; within 0.3 m 187 and 50, 257 and 74, 243 and 106, 243 and
-// 178, 128,000 292 and 311; within 3 m 32,000 305 and 221, 64,000 305 and 403.
-bool tree_knn_few(size_t nq, float radius) { return nq <= (radius > 0.0f ? 49152u : 24576u); }
+// none of this, but five times the work. Queries among 400,000 LiDAR points,
+// k 16, packets and warps: 1000 queries 309 and 90 us, 16,000 360 and 200, 32,000
+// 338 and 313, 64,000 334 and 590. Within 0.3 m of 150,000: 10,000 201 and 59,
+// 75,000 206 and 148, 110,000 228 and 203; within 1.5 m 256 and 72, 250 and 243,
+// 280 and 331; of a room's points within 0.1 m 75,000 260 and 238, 110,000 295
+// and 335.
+bool tree_knn_few(size_t nq, float radius) { return nq <= (radius > 0.0f ? 81920u : 24576u); }
 
 void tree_knn(rvp_context *ctx, const TreeView &t, const TreeQueries &q, int k, float radius,
               int mode, const TreeOut &o) {

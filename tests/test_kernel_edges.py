@@ -334,8 +334,8 @@ def test_ransac_rounds(gpu_ctx, restatement, n, iters):
     assert best2 == best and ran2 == ran
 
 
-# up to 24576 queries (49152 within a radius) go one per warp, more in packets
-@pytest.mark.parametrize("nq,radius", [(24_576, 0.0), (49_152, 0.3)])
+# up to 24576 queries (81920 within a radius) go one per warp, more in packets
+@pytest.mark.parametrize("nq,radius", [(24_576, 0.0), (81_920, 0.3)])
 @pytest.mark.parametrize("k", [1, 9, 17, 40])
 @pytest.mark.parametrize("cloud", ["room", "lattice"])
 def test_few_and_many_queries(gpu_ctx, nq, radius, k, cloud):
@@ -351,7 +351,7 @@ def test_few_and_many_queries(gpu_ctx, nq, radius, k, cloud):
     h.setInputCloud(c, 0.5)
     h.build()
     rng = np.random.default_rng(nq)
-    q = np.concatenate([p[rng.permutation(n)[:nq - 500]],
+    q = np.concatenate([p[rng.permutation(nq) % n][:nq - 500],
                         rng.uniform(-9, 9, (501, 3)).astype(np.float32)])
     few = h.knn(*q[:nq].T, k, radius)
     many = h.knn(*q.T, k, radius)
@@ -494,3 +494,37 @@ def test_packets_order_ties_by_index(gpu_ctx, k):
             idx2, dist2 = brute_knn(p, q[at], k, np.float32(r) * np.float32(r) if r else np.inf)
             assert np.array_equal(idx[at], idx2) and np.array_equal(bits(d2[at]), bits(dist2))
             assert np.array_equal(cnt[at], (idx2 >= 0).sum(1))
+
+
+# radius lists: up to 65536 queries go one per warp in their own order, more in
+# packets; lists of a few points, of hundreds and of more than 1024
+@pytest.mark.parametrize("max_nn", [0, 70])
+@pytest.mark.parametrize("mixed", [False, True])  # other queries, or the cloud itself
+def test_few_and_many_radius_queries(gpu_ctx, max_nn, mixed):
+    from rvpoint_b200 import api
+    nq = 65_536
+    rng = np.random.default_rng(1)
+    p = rng.uniform(-20, 20, (nq + 1, 3)) * [1, 1, 0.05]
+    p[rng.permutation(nq)[:1200]] = rng.normal(0, 0.05, (1200, 3))
+    p[rng.permutation(nq)[:400]] = rng.normal(3, 0.05, (400, 3))
+    p = p.astype(np.float32)
+    h = api.SpatialHash()
+    h.setInputCloud((p[:, 0], p[:, 1], p[:, 2]), 0.5)
+    h.build()
+    q = p + np.float32(0.01) if mixed else p
+    few = h.radiusSearchBatch(*q[:nq].T, 0.3, max_nn=max_nn)
+    many = h.radiusSearchBatch(*q.T, 0.3, max_nn=max_nn)
+    m = int(few[0][-1])
+    assert np.array_equal(few[0], many[0][:-1])
+    assert np.array_equal(few[1], many[1][:m]) and np.array_equal(bits(few[2]), bits(many[2][:m]))
+    if max_nn == 0:
+        n = np.diff(many[0])
+        assert n.max() > 1024 and ((n > 256) & (n < 1024)).any() and (n < 32).any()
+    at = np.concatenate([rng.choice(nq, 60, replace=False), np.argsort(np.diff(few[0]))[-3:], [nq]])
+    _, idx, d2 = brute_radius(p, q[at], 0.3)
+    o = brute_radius(p, q[at], 0.3)[0]
+    cut = max_nn or len(p)
+    for i, a in enumerate(at):
+        s = slice(many[0][a], many[0][a + 1])
+        assert np.array_equal(many[1][s], idx[o[i]:o[i + 1]][:cut])
+        assert np.array_equal(bits(many[2][s]), bits(d2[o[i]:o[i + 1]][:cut]))
