@@ -888,10 +888,11 @@ rvp_status rvp_normals_radius(rvp_hash *h, float radius, float vp_x, float vp_y,
     if (h->collision) {
       from_lists(nullptr, n);
     } else {
-      u32 *hard = static_cast<u32 *>(scratch(ctx, 15, n * 8 + 16)), *huge = hard + n;
+      u32 *hard = static_cast<u32 *>(scratch(ctx, 15, n * 12 + 16));
+      u32 *longer = hard + n, *huge = longer + n;
       rvp::tree_radius_normals(ctx, h->tree_view, radius, eigen_iters, vp_x, vp_y, vp_z, dnx, dny,
-                               dnz, hard, huge, huge + n);
-      const u32 m = read_back(ctx, huge + n + 1);
+                               dnz, hard, longer, huge, huge + n);
+      const u32 m = read_back(ctx, huge + n + 2);
       if (m) from_lists(huge, m);
     }
     out_copy(ctx, nx, dnx, n, mem);

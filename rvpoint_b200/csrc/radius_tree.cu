@@ -410,11 +410,16 @@ __global__ void k_radius_big_out(const u64 *pairs, const u32 *big, const u32 *bi
 // A packet of 32 queries per warp, each lane with its own neighbours; points
 // with more than a lane holds, and packets of points far apart (past
 // kLeafBudget leaves; one such packet kept the kernel busy for 421 us where the
-// others take 119), go one per warp. Bound by issue and, with many long lists,
+// others take 119), go one per warp. Bound by issue, and with many long lists
 // by the listed points. 87,477 points of a room, radius 0.03 (10 neighbours
-// each): 119 us and 18 for the listed ones; 100,000 and 0.05 (28 each) 165 and
-// 356 (64 neighbours a lane: 258 and 281).
+// each): 119 us and 18 for the listed ones; 100,000 and 0.05 (30 each, 28% with
+// more than 48): 161 and 100.
 constexpr int RN_CAP = 48;  // neighbours a lane holds
+// Up to so many points are all taken one per warp: packets of few points have
+// nothing to hide their latency (5000 points of a LiDAR frame 88 us, with packets
+// 114; 20,000 119 and 152, of a room 166 and 234; 40,000 156 and 162, 80,000 238
+// and 219).
+constexpr u32 kFewNormals = 32768;
 
 __global__ __launch_bounds__(32) void k_radius_normals(TreeView t, u64 minus_zero, float r2,
                                                        int iters, float vpx, float vpy, float vpz,
@@ -471,13 +476,19 @@ __global__ __launch_bounds__(32) void k_radius_normals(TreeView t, u64 minus_zer
   if (cnt >= 3) {  // normal_estimation.cpp:203
     for (int i = 0; i < cnt; ++i) {
       const uint2 e = near[i][lane];
-      int rank = 0;
+      int rank = 0, same = 0;
+#pragma unroll 8
       for (int j = 0; j < cnt; ++j) {
-        const uint2 f = near[j][lane];  // (distances are not negative: ordered as bits)
-        bool less = f.x < e.x;
-        if (f.x == e.x && j != i)
-          less = __float_as_uint(__ldg(&t.pts[f.y]).w) < __float_as_uint(__ldg(&t.pts[e.y]).w);
-        rank += less;
+        const u32 f = near[j][lane].x;  // (distances are not negative: ordered as bits)
+        rank += f < e.x;
+        same += f == e.x;
+      }
+      if (same > 1) {
+        const u32 own = __float_as_uint(__ldg(&t.pts[e.y]).w);
+        for (int j = 0; j < cnt; ++j) {
+          const uint2 f = near[j][lane];
+          if (f.x == e.x) rank += __float_as_uint(__ldg(&t.pts[f.y]).w) < own;
+        }
       }
       order[rank][lane] = (unsigned char)i;
     }
@@ -490,44 +501,80 @@ __global__ __launch_bounds__(32) void k_radius_normals(TreeView t, u64 minus_zer
 }
 
 // The points with more neighbours than a lane holds, and those of wide packets
-// (hard: places in the tree), one warp each; those past FT_CAP neighbours go on to `huge` (indices).
+// (hard: places in the tree), one warp each; those past CAP neighbours go on to
+// `more` (places, or indices where `last`). Up to 32 points per turn: a point's sums go one to a lane
+// (each in the neighbours' order, as one lane would add them), and at the end of
+// the turn every lane makes the normal of one point. With all of it by one lane
+// per point and room for 1024 in every block, 150,000 points of 60
+// neighbours each took 1.89 ms (1.13 from lists in memory), now 0.94.
+template <u32 CAP, u32 BINS>
 __global__ __launch_bounds__(32) void k_radius_normals_listed(
     TreeView t, float r2, int iters, float vpx, float vpy, float vpz, float *nx, float *ny,
-    float *nz, const u32 *hard, const u32 *hard_count, u32 *huge, u32 *huge_count) {
-  __shared__ u64 s_keys[FT_CAP];
-  __shared__ u32 s_bins[FT_BINS];
-  __shared__ float s_near[3][FT_CAP];  // in order: gathered by all lanes, summed by one
-  __shared__ unsigned short s_perm[FT_CAP];
+    float *nz, const u32 *hard, const u32 *hard_count, u32 *more, u32 *more_count, bool last) {
+  __shared__ u64 s_keys[CAP];
+  __shared__ u32 s_bins[BINS];
+  __shared__ float s_near[3][CAP];  // in order
+  __shared__ unsigned short s_perm[CAP];
   const int lane = threadIdx.x;
-  for (u32 w = blockIdx.x; w < *hard_count; w += gridDim.x) {
-    const float4 q = t.pts[hard[w]];
-    const u32 qidx = __float_as_uint(q.w);
-    u32 cnt = 0;
-    radius_walk<1>(t, q.x, q.y, q.z, r2, 0, [&](bool pass, float d, u32 idx) {
-      const unsigned b = __ballot_sync(0xffffffffu, pass);
-      const u32 at = cnt + __popc(b & ((1u << lane) - 1));
-      if (pass && at < FT_CAP) s_keys[at] = pack_nbr(d, (int)idx);
-      cnt += __popc(b);
-    });
-    __syncwarp();
-    if (cnt > FT_CAP) {
-      if (lane == 0) huge[atomicAdd(huge_count, 1u)] = qidx;
-      continue;
+  const u32 n = hard ? *hard_count : t.n, chunk = min(32u, (n + gridDim.x - 1) / gridDim.x);
+  // the products of the covariance: lane l adds up axis a times axis b
+  const int a = lane < 3 ? 0 : (lane < 5 ? 1 : 2), b = lane < 3 ? lane : (lane == 3 ? 1 : 2);
+  auto place = [&](u32 w) { return hard ? hard[w] : w; };  // (null: all points)
+  for (u32 w0 = blockIdx.x * chunk; w0 < n; w0 += gridDim.x * chunk) {
+    const u32 m = min(chunk, n - w0);
+    float C[6] = {};
+    int mine = -1;  // the lane's point's neighbours; -1: no point, or left for `more`
+    for (u32 c = 0; c < m; ++c) {
+      const float4 q = t.pts[place(w0 + c)];
+      u32 cnt = 0;
+      radius_walk<1>(t, q.x, q.y, q.z, r2, 0, [&](bool pass, float d, u32 idx) {
+        const unsigned b = __ballot_sync(0xffffffffu, pass);
+        const u32 at = cnt + __popc(b & ((1u << lane) - 1));
+        if (pass && at < CAP) s_keys[at] = pack_nbr(d, (int)idx);
+        cnt += __popc(b);
+      });
+      __syncwarp();
+      if (cnt > CAP) {
+        if (lane == 0)
+          more[atomicAdd(more_count, 1u)] = last ? __float_as_uint(q.w) : place(w0 + c);
+        continue;
+      }
+      if (lane == (int)c) mine = (int)cnt;
+      if (cnt < 3) continue;
+      order_keys<32, BINS>(s_keys, cnt, r2, s_bins, s_perm, nullptr, [&](u32 rank, u64 k) {
+        const float4 p = __ldg(&t.pts[t.pos_of[nbr_idx(k)]]);
+        s_near[0][rank] = p.x;
+        s_near[1][rank] = p.y;
+        s_near[2][rank] = p.z;
+      });
+      __syncwarp();
+      // (nd::normal_from_points: the centroid, then the six products about it)
+      float sum = 0.0f;
+      const float *axis = s_near[lane < 3 ? lane : 0];
+#pragma unroll 8
+      for (u32 j = 0; j < cnt; ++j) sum = fadd(sum, axis[j]);
+      sum = fmul(sum, fdiv(1.0f, (float)(int)cnt));
+      const float ca = __shfl_sync(0xffffffffu, sum, a), cb = __shfl_sync(0xffffffffu, sum, b);
+      float prod = 0.0f;
+      const float *pa = s_near[a], *pb = s_near[b];
+#pragma unroll 8
+      for (u32 j = 0; j < cnt; ++j) prod = fadd(prod, fmul(fsub(pa[j], ca), fsub(pb[j], cb)));
+#pragma unroll
+      for (int k = 0; k < 6; ++k) {
+        const float v = __shfl_sync(0xffffffffu, prod, k);
+        if (lane == (int)c) C[k] = v;
+      }
+      __syncwarp();
     }
-    order_keys<32, FT_BINS>(s_keys, cnt, r2, s_bins, s_perm, nullptr,
-                            [&](u32 rank, u64 k) {
-                              const float4 p = __ldg(&t.pts[t.pos_of[nbr_idx(k)]]);
-                              s_near[0][rank] = p.x;
-                              s_near[1][rank] = p.y;
-                              s_near[2][rank] = p.z;
-                            });
-    __syncwarp();
-    if (lane == 0) {
+    if (mine >= 0) {
+      const float4 q = t.pts[place(w0 + lane)];
+      const u32 qidx = __float_as_uint(q.w);
       float ax = 0.0f, ay = 0.0f, az = 0.0f;
-      if (cnt >= 3)  // normal_estimation.cpp:203
-        nd::normal_from_points(
-            [&](int j) { return make_float4(s_near[0][j], s_near[1][j], s_near[2][j], 0.0f); },
-            (int)cnt, false, iters, q.x, q.y, q.z, vpx, vpy, vpz, ax, ay, az);
+      if (mine >= 3) {  // normal_estimation.cpp:203
+        float A[3][3] = {{C[0], C[1], C[2]}, {C[1], C[3], C[4]}, {C[2], C[4], C[5]}};
+        nd::eigen_smallest_ref(A, iters, ax, ay, az);
+        nd::flip_ref(q.x, q.y, q.z, vpx, vpy, vpz, ax, ay, az);
+      }
       nx[qidx] = ax;
       ny[qidx] = ay;
       nz[qidx] = az;
@@ -605,14 +652,24 @@ void tree_radius_fill(rvp_context *ctx, const TreeView &t, const TreeQueries &q,
 
 void tree_radius_normals(rvp_context *ctx, const TreeView &t, float radius, int iters, float vpx,
                          float vpy, float vpz, float *nx, float *ny, float *nz, u32 *hard,
-                         u32 *huge, u32 *counts) {
+                         u32 *longer, u32 *huge, u32 *counts) {
   const float r2 = square_of(radius);
-  RVP_CUDA_TRY(cudaMemsetAsync(counts, 0, 8, ctx->stream));
-  k_radius_normals<<<(t.n + 31) / 32, 32, 0, ctx->stream>>>(t, kMinusZero2, r2, iters, vpx, vpy,
-                                                           vpz, nx, ny, nz, hard, counts);
+  RVP_CUDA_TRY(cudaMemsetAsync(counts, 0, 12, ctx->stream));
+  const bool few = t.n <= kFewNormals;
+  if (!few) {
+    k_radius_normals<<<(t.n + 31) / 32, 32, 0, ctx->stream>>>(
+        t, kMinusZero2, r2, iters, vpx, vpy, vpz, nx, ny, nz, hard, counts);
+    RVP_LAUNCH_CHECK(ctx);
+  }
+  // (by shared memory: 32 short lists at once on an SM, or 9 long ones)
+  k_radius_normals_listed<FT_SHORT, FT_SHORT>
+      <<<grid_for(t.n, 1, ctx->num_sms * 32), 32, 0, ctx->stream>>>(
+          t, r2, iters, vpx, vpy, vpz, nx, ny, nz, few ? nullptr : hard, counts, longer, counts + 1,
+          false);
   RVP_LAUNCH_CHECK(ctx);
-  k_radius_normals_listed<<<grid_for(t.n, 1, ctx->num_sms * 14), 32, 0, ctx->stream>>>(
-      t, r2, iters, vpx, vpy, vpz, nx, ny, nz, hard, counts, huge, counts + 1);
+  k_radius_normals_listed<FT_CAP, FT_BINS>
+      <<<grid_for(t.n, 1, ctx->num_sms * 9), 32, 0, ctx->stream>>>(
+          t, r2, iters, vpx, vpy, vpz, nx, ny, nz, longer, counts + 1, huge, counts + 2, true);
   RVP_LAUNCH_CHECK(ctx);
 }
 

@@ -528,3 +528,56 @@ def test_few_and_many_radius_queries(gpu_ctx, max_nn, mixed):
         s = slice(many[0][a], many[0][a + 1])
         assert np.array_equal(many[1][s], idx[o[i]:o[i + 1]][:cut])
         assert np.array_equal(bits(many[2][s]), bits(d2[o[i]:o[i + 1]][:cut]))
+
+
+# radius normals: up to 32768 points go one per warp, more in packets; lists of
+# a few points, past a lane's (48), past a short list's (256) and past 1024
+def test_few_and_many_radius_normals(gpu_ctx, restatement):
+    from rvpoint_b200 import api
+    n = 32_768
+    rng = np.random.default_rng(4)
+    p = rng.uniform(-20, 20, (n + 1, 3)) * [1, 1, 0.01]
+    for at, m in (((0, 0, 0), 1300), ((4, 0, 0), 500), ((8, 0, 0), 100)):
+        p[rng.permutation(n)[:m]] = rng.normal(0, 0.05, (m, 3)) * [1, 1, 0.1] + at
+    p[n] = 300
+    p = p.astype(np.float32)
+    got = []
+    for m in (n, n + 1):
+        c = D.Cloud.from_xyz(p[:m])
+        h = api.SpatialHash()
+        h.setInputCloud(c, 0.3)
+        h.build()
+        got.append(np.stack(api.normal_estimation_rvv(c, h, 10, 0.3), 1))
+    lists = np.diff(h.radiusSearchBatch(*p.T, 0.3)[0])
+    for lo, hi in ((3, 48), (49, 256), (257, 1024), (1025, n)):
+        assert ((lists >= lo) & (lists <= hi)).any()
+    assert np.array_equal(bits(got[0]), bits(got[1][:n])) and not got[1][n].any()
+    want = np.asarray(restatement.normals_radius(c, 0.3, 0.3))
+    assert np.array_equal((got[1] != 0).any(1), (want != 0).any(1))
+    # (the rotations branch on the largest entry: a few differ by more)
+    assert (np.abs(got[1] - want).max(1) < 1e-4).mean() > 0.995
+
+
+# points of some 60 neighbours each: their normals by whole warps, not by one
+# lane (less than three times a search for their lists; it was four)
+def test_radius_normals_of_longer_lists(gpu_ctx):
+    import time
+    import torch
+    from rvpoint_b200 import api
+    x = np.random.default_rng(7).uniform(-50, 50, 150_000).astype(np.float32)
+    v = [torch.from_numpy(a).cuda() for a in (x, np.zeros_like(x), np.zeros_like(x))]
+    h = api.SpatialHash()
+    h.setInputCloud(v, 0.02)
+    h.build()
+
+    def best(f):
+        t = []
+        for _ in range(6):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            f()
+            torch.cuda.synchronize()
+            t.append(time.perf_counter() - t0)
+        return min(t)
+    lists = best(lambda: h.radiusSearchBatch(*v, 0.02))
+    assert best(lambda: api.normal_estimation_rvv(v, h, 10, 0.02)) < 2.9 * lists
