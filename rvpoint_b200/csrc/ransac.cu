@@ -797,7 +797,10 @@ size_t preemptive_temp_bytes(int n_frames) {
 // Rounds: as many hypotheses as some 100M tests hold (about 15 us), 64 to
 // 1024, twice as many in each further round: a search that stops early has
 // counted at most about three times what it needed, one that goes on pays few
-// launches.
+// launches. Before the fifth round and each time their number has doubled the
+// host looks whether the search has stopped: the rounds behind that are empty
+// launches (300,000 iterations over 20,000 points, stopped in the first round:
+// 0.31 ms in one kernel, 2.9 with all rounds launched, 0.34 now).
 constexpr int kRoundMost = 1024;
 
 size_t ransac_one_bytes() { return (size_t)kRoundMost * 20; }
@@ -810,8 +813,16 @@ void ransac_one(rvp_context *ctx, const float *x, const float *y, const float *z
   const int first = (int)std::max<size_t>(64, std::min<size_t>(kRoundMost, 100000000 / n));
   const int chunks = (int)((n + CM_CHUNK - 1) / CM_CHUNK);
   const int blocks = std::min(chunks, ctx->num_sms * 8);
+  int rounds = 0, look = 4;
   for (int it0 = 0, round = first; it0 < p.max_iters; it0 += round,
            round = std::min(kRoundMost, 2 * round)) {
+    if (rounds++ == look) {
+      int stop = 0;
+      RVP_CUDA_TRY(cudaMemcpyAsync(&stop, &state->stop, 4, cudaMemcpyDeviceToHost, st));
+      RVP_CUDA_TRY(cudaStreamSynchronize(st));
+      if (stop) break;
+      look *= 2;
+    }
     round = std::min(round, p.max_iters - it0);
     k_build_models<<<(round + 127) / 128, 128, 0, st>>>(x, y, z, (u32)n, rand_dev, it0, round,
                                                        p.collinear, models, counts, state,

@@ -581,3 +581,21 @@ def test_radius_normals_of_longer_lists(gpu_ctx):
         return min(t)
     lists = best(lambda: h.radiusSearchBatch(*v, 0.02))
     assert best(lambda: api.normal_estimation_rvv(v, h, 10, 0.02)) < 2.9 * lists
+
+
+# a search that has stopped launches no further rounds
+@pytest.mark.parametrize("iters", [3000, 300_000])
+def test_ransac_stops_launching(gpu_ctx, restatement, iters):
+    from oracle import oracle as O
+    from rvpoint_b200 import api
+    rng = np.random.default_rng(1)
+    p = np.concatenate([rng.uniform(-5, 5, (18_000, 3)) * [1, 1, 0.001],
+                        rng.uniform(-5, 5, (2000, 3))]).astype(np.float32)
+    c = D.Cloud.from_xyz(p)
+    stream = O.libc_rand_stream(3 * iters)
+    best, model, _, _, ran = restatement.ransac_plane(c, 0.05, iters, stream)
+    assert ran < 1000
+    before = gpu_ctx.launches
+    got, m = api.ransac_plane_rvv(c, 0.05, iters)
+    assert gpu_ctx.launches - before <= 15  # (all rounds of 300,000: 882)
+    assert got == best and np.array_equal(bits(m), bits(np.asarray(model, np.float32)))
