@@ -183,9 +183,10 @@ __device__ __forceinline__ void insert_u64(u64 (&L)[KF], u64 key) {
 // Feature neighbourhoods among one scene's candidates: a box tree of all
 // scenes answers them; the scenes it leaves out (more than kSmallFrame
 // candidates, or coordinates that are not finite) are searched here by brute
-// force, exactly and slowly (the proposal draws far fewer). 512 scenes of 1024
-// candidates: a grid in shared memory per scene 762 us, the tree 41 to build and
-// 460 to search.
+// force, exactly and slowly (the proposal draws far fewer), each by as many
+// blocks as the device has for it (one scene of 6000 by one block 14.5 ms, by
+// two 8.0, by 64 0.7). 512 scenes of 1024 candidates: a grid in shared memory
+// per scene 762 us, the tree 41 to build and 460 to search.
 constexpr int CB_TH = 256;
 __global__ __launch_bounds__(CB_TH) void k_cand_brute(const float *__restrict__ x,
                                                       const float *__restrict__ y,
@@ -193,11 +194,11 @@ __global__ __launch_bounds__(CB_TH) void k_cand_brute(const float *__restrict__ 
                                                       const int64_t *offs, int n_frames,
                                                       const int32_t *skipped, int32_t *idx,
                                                       int32_t *counts) {
-  for (int f = blockIdx.x; f < n_frames; f += gridDim.x) {
+  for (int f = blockIdx.y; f < n_frames; f += gridDim.y) {
     if (!skipped[f]) continue;
     const int64_t a = offs[f];
     const int m = (int)(offs[f + 1] - a);
-    for (int i = threadIdx.x; i < m; i += CB_TH) {
+    for (int i = blockIdx.x * CB_TH + threadIdx.x; i < m; i += gridDim.x * CB_TH) {
       const float qx = x[a + i], qy = y[a + i], qz = z[a + i];
       u64 L[KF];
 #pragma unroll
@@ -1024,7 +1025,9 @@ rvp_status rvp_scorer_features(rvp_scorer *s, const float *x, const float *y, co
           skipped + f0);
       rvp::tree_knn_frames(ctx, s->tree, t, nullptr, nullptr, rvp::KF, rvp::TREE_PAIRS, o);
     }
-    rvp::k_cand_brute<<<(unsigned)std::min(n_frames, ctx->num_sms * 8), rvp::CB_TH, 0, st>>>(
+    const int rows = std::min(n_frames, ctx->num_sms * 8);
+    const dim3 brute((unsigned)std::max(2, std::min(64, ctx->num_sms * 8 / rows)), (unsigned)rows);
+    rvp::k_cand_brute<<<brute, rvp::CB_TH, 0, st>>>(
         gx, gy, gz, cand_offsets_dev, n_frames, skipped, idx, counts);
     RVP_LAUNCH_CHECK(ctx);
     rvp::k_features<<<rvp::grid_for(n_cand, 256, ctx->num_sms * 16), 256, 0, st>>>(

@@ -599,3 +599,31 @@ def test_ransac_stops_launching(gpu_ctx, restatement, iters):
     got, m = api.ransac_plane_rvv(c, 0.05, iters)
     assert gpu_ctx.launches - before <= 15  # (all rounds of 300,000: 882)
     assert got == best and np.array_equal(bits(m), bits(np.asarray(model, np.float32)))
+
+
+# a scene of more candidates than a tree takes has the whole device: one of 6000
+# is an eighth of the work of 32 of 3000 (and took three times as long)
+def test_large_candidate_scene_uses_the_device(gpu_ctx):
+    import time
+    import torch
+    from rvpoint_b200.learned import DeviceBatch, PlaneScorer
+    rng = np.random.default_rng(0)
+    times = []
+    for scenes, m in ((1, 6000), (32, 3000)):
+        n = scenes * m
+        p = rng.uniform(-5, 5, (n, 3)).astype(np.float32)
+        offs = np.arange(scenes + 1, dtype=np.int64) * m
+        b = DeviceBatch.from_host(D.Batch(p[:, 0].copy(), p[:, 1].copy(), p[:, 2].copy(), offs))
+        s = PlaneScorer(n, scenes, ctx=gpu_ctx)
+        cand = torch.arange(n, dtype=torch.int32, device="cuda")
+        coffs = torch.from_numpy(offs).cuda()
+        t = []
+        for _ in range(4):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            s.features(b, 1.0, cand, coffs, among_candidates=True)
+            torch.cuda.synchronize()
+            t.append(time.perf_counter() - t0)
+        times.append(min(t))
+        s.close()
+    assert times[0] < times[1]
