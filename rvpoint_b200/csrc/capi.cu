@@ -145,6 +145,13 @@ void out_copy(rvp_context *ctx, T *user, const T *dev, size_t n, int mem) {
   RVP_CUDA_TRY(cudaMemcpyAsync(user, dev, n * sizeof(T), cudaMemcpyDeviceToHost, ctx->stream));
 }
 
+// memory of the context's own GPU
+bool on_device(rvp_context *ctx, const void *p) {
+  cudaPointerAttributes a{};
+  RVP_CUDA_TRY(cudaPointerGetAttributes(&a, p));
+  return a.type == cudaMemoryTypeDevice && a.device == ctx->device;
+}
+
 void sync(rvp_context *ctx) { RVP_CUDA_TRY(cudaStreamSynchronize(ctx->stream)); }
 
 template <class T>
@@ -433,14 +440,17 @@ rvp_status rvp_hash_set_input_cloud(rvp_hash *h, const float *x, const float *y,
     h->tree_built = false;
     h->n = 0;
     h->x.reserve(n * 4 + 16); h->y.reserve(n * 4 + 16); h->z.reserve(n * 4 + 16);
-    if (n && mem == RVP_MEM_DEVICE) {
+    if (n && mem == RVP_MEM_DEVICE && on_device(ctx, x) && on_device(ctx, y) &&
+        on_device(ctx, z)) {
       k_copy3<<<rvp::grid_for(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(
           x, y, z, n, h->x.as<float>(), h->y.as<float>(), h->z.as<float>());
       RVP_LAUNCH_CHECK(ctx);
-    } else if (n) {
-      RVP_CUDA_TRY(cudaMemcpyAsync(h->x.ptr, x, n * 4, cudaMemcpyHostToDevice, ctx->stream));
-      RVP_CUDA_TRY(cudaMemcpyAsync(h->y.ptr, y, n * 4, cudaMemcpyHostToDevice, ctx->stream));
-      RVP_CUDA_TRY(cudaMemcpyAsync(h->z.ptr, z, n * 4, cudaMemcpyHostToDevice, ctx->stream));
+    } else if (n) {  // (another GPU's memory: a kernel here may not read it)
+      const cudaMemcpyKind k =
+          mem == RVP_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+      RVP_CUDA_TRY(cudaMemcpyAsync(h->x.ptr, x, n * 4, k, ctx->stream));
+      RVP_CUDA_TRY(cudaMemcpyAsync(h->y.ptr, y, n * 4, k, ctx->stream));
+      RVP_CUDA_TRY(cudaMemcpyAsync(h->z.ptr, z, n * 4, k, ctx->stream));
     }
     sync(ctx);
     h->n = n;

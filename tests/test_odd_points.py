@@ -130,3 +130,21 @@ def test_radius_search_of_a_billion_queries(gpu_ctx, max_nn):
     assert torch.equal(idx, i2) and torch.equal(d2, e2)
     h.close()
     ctx.close()
+
+
+# a hash copies its cloud, from another GPU's memory as well
+def test_cloud_of_another_gpu(gpu_ctx):
+    import torch
+    from rvpoint_b200 import api
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two GPUs")
+    c = D.room_cloud(n=3000, seed=1)
+    found = []
+    for dev in ("cuda:0", "cuda:1"):
+        h = api.SpatialHash()
+        h.setInputCloud(tuple(torch.from_numpy(np.array(a)).to(dev) for a in (c.x, c.y, c.z)), 0.2)
+        torch.cuda.synchronize(dev)
+        h.build()
+        found.append(h.knn(c.x, c.y, c.z, 8))
+        h.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*found))
