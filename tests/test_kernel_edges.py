@@ -627,3 +627,63 @@ def test_large_candidate_scene_uses_the_device(gpu_ctx):
         times.append(min(t))
         s.close()
     assert times[0] < times[1]
+
+
+# neighbours at indices from all over clouds that fill two (32,769 points on),
+# three and four levels of nodes (1,048,577 on): SOR's means, and normals in
+# high precision against eigenvectors over brute-force neighbours
+@pytest.mark.parametrize("n", [32_769, 70_001, 1_100_000])
+def test_neighbours_through_all_levels(gpu_ctx, n):
+    from rvpoint_b200 import api
+    k = 9
+    c = D.room_cloud(n=n, seed=n)
+    p = c.aos()
+    at = np.sort(np.random.default_rng(n).choice(n, 120, replace=False))
+    idx, d2 = brute_knn(p, p[at], k + 1)
+    want = np.zeros(len(at), np.float32)
+    for j in range(1, k + 1):
+        want += np.sqrt(d2[:, j])
+    mean = api.sor_rvv(c, k, 1.0, return_stats=True)[1]
+    assert np.array_equal(bits(mean[at]), bits(want / np.float32(k)))
+    nrm, _, _ = api.normal_estimation_precise(c, k)
+    q = p.astype(np.float64)[idx]
+    q -= q.mean(1, keepdims=True)
+    w, v = np.linalg.eigh(np.einsum("nki,nkj->nij", q, q))
+    clear = w[:, 0] < 0.5 * w[:, 1]  # a normal that is well defined
+    assert clear.mean() > 0.8 and (1 - np.abs((nrm[at] * v[:, :, 0]).sum(1))[clear] < 1e-5).all()
+
+
+# the reference's own normals, point by point, past one level of nodes
+def test_normals_past_one_level(gpu_ctx, restatement):
+    from rvpoint_b200 import api
+    c = D.room_cloud(n=33_000, seed=8)
+    got = np.stack(api.normal_estimation_sc(c, 9), 1)
+    want = restatement.normals_knn(c, 9)
+    # (the rotations branch on the largest entry: a few differ by more)
+    assert (np.abs(got - want).max(1) < 1e-4).mean() > 0.995
+
+
+# SOR's sums go by chunks of 4096 values, runs of 8, after eight segments of 256
+# that were not foreseen: sizes about a chunk's edge behind those, with equal
+# distances (ties) and a binade left on the way
+@pytest.mark.parametrize("n", [2048, 2049, 6143, 6144, 6145, 6152, 10_239, 10_241, 30_001])
+def test_sor_statistics_chunks(gpu_ctx, n):
+    from rvpoint_b200.api import sor_rvv
+    far = 2**20 - int(0.125 * n / 2)
+    i = np.arange(n)
+    p = np.stack([i % 31, (i // 31) % 37, i // 1147], 1).astype(np.float32) * np.float32(0.1)
+    p[0] = [-far, 0, 0]
+    c = D.Cloud.from_xyz(p)
+    _, mean, _ = sor_rvv(c, 3, 0.5, return_stats=True)
+    f = np.float32
+    mu = np.add.accumulate(mean)[-1] / f(n)  # in order, in float
+    sd = np.sqrt(np.add.accumulate((mean - mu) * (mean - mu))[-1] / f(n))
+    target = np.sort(mean)[-2]
+    alpha = f((target - mu) / sd)
+    for _ in range(64):
+        t = mu + alpha * sd
+        if t == target:
+            break
+        alpha = np.nextafter(alpha, f(np.inf) if t < target else f(-np.inf))
+    _, _, keep = sor_rvv(c, 3, float(alpha), return_stats=True)
+    assert np.array_equal(keep.astype(bool), mean <= mu + alpha * sd)
