@@ -633,7 +633,9 @@ __global__ __launch_bounds__(32, KCAP > 32 ? 10 : 16) void k_knn_tree(TreeView t
   int have = 0;  // distances in the list
   float sum = 0.0f;
   if constexpr (MEAN || MODE == TREE_LIST) {
-    // (without a radius they are all there, some infinitely far perhaps)
+    // (without a bound, a list that is not full is of a frame of few points, or
+    // some are infinitely far: the second kernel tells)
+    if (MEAN) exact = exact && (bound < INFINITY || L[KCAP - 1] < INFINITY);
     bool first = !drop;  // the nearest of all does not count
 #pragma unroll
     for (int j = 0; j < KCAP; ++j) {

@@ -687,3 +687,26 @@ def test_sor_statistics_chunks(gpu_ctx, n):
         alpha = np.nextafter(alpha, f(np.inf) if t < target else f(-np.inf))
     _, _, keep = sor_rvv(c, 3, float(alpha), return_stats=True)
     assert np.array_equal(keep.astype(bool), mean <= mu + alpha * sd)
+
+
+# frames of fewer than k + 1 points, where the search keeps means only (the
+# normals' lists are longer): a mean is over the points there are
+@pytest.mark.parametrize("sor_k,normal_k", [(1, 28), (8, 9), (16, 17), (30, 40)])
+def test_frames_of_few_points(gpu_ctx, sor_k, normal_k):
+    from rvpoint_b200.api import Pipeline
+    rng = np.random.default_rng(sor_k)
+    sizes = (1, 2, 0, 5, 9, 16, 17, 30, 33, 70, 1)
+    n = sum(sizes)
+    i = rng.permutation(40 * 40)[:n]
+    p = (np.stack([i % 40, i // 40, i % 3], 1) * 0.1 + rng.uniform(0.02, 0.08, (n, 3))).astype(np.float32)
+    offs = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    b = D.Batch(p[:, 0].copy(), p[:, 1].copy(), p[:, 2].copy(), offs)
+    got = []
+    for mode in (0, 3, 1):
+        pipe = Pipeline(n, len(sizes), leaf_size=0.1, sor_k=sor_k, normal_k=normal_k, sor_alpha=2.0,
+                        ransac_iters=20, queries_per_warp=mode, ctx=gpu_ctx)
+        got.append(pipe.run_host(b))
+        pipe.close()
+    for g in got[:2]:
+        for key in g:
+            assert np.array_equal(np.asarray(g[key]), np.asarray(got[2][key]), equal_nan=True), key
