@@ -166,12 +166,15 @@ __device__ __forceinline__ u64 mix64(u64 k) {  // splitmix64 finaliser
   return k;
 }
 
-// float atomics on ordered int images (valid for non-NaN values)
+// float atomics on ordered int images (valid for non-NaN values; -0, which is
+// the least of the integers, goes as 0)
 __device__ __forceinline__ void atomic_min_f(float *a, float v) {
+  v = fadd(v, 0.0f);
   if (v >= 0.0f) atomicMin((int *)a, __float_as_int(v));
   else atomicMax((unsigned *)a, __float_as_uint(v));
 }
 __device__ __forceinline__ void atomic_max_f(float *a, float v) {
+  v = fadd(v, 0.0f);
   if (v >= 0.0f) atomicMax((int *)a, __float_as_int(v));
   else atomicMin((unsigned *)a, __float_as_uint(v));
 }

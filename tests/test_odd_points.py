@@ -148,3 +148,40 @@ def test_cloud_of_another_gpu(gpu_ctx):
         found.append(h.knn(c.x, c.y, c.z, 8))
         h.close()
     assert all(np.array_equal(a, b) for a, b in zip(*found))
+
+
+# a frame, or a whole cloud, whose largest (or smallest) coordinate is -0: its
+# box takes it in
+@pytest.mark.parametrize("sign", [-1, 1])
+def test_coordinates_of_minus_zero(gpu_ctx, restatement, sign):
+    import torch
+    from rvpoint_b200 import api
+    from rvpoint_b200.learned import DeviceBatch, PlaneScorer
+    rng = np.random.default_rng(3)
+    sizes = (17, 8, 40, 1, 300)
+    n = sum(sizes)
+    offs = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    p = (rng.uniform(0.05, 2.0, (n, 3)) * sign).astype(np.float32)
+    for a, b in zip(offs, offs[1:]):  # each axis of each frame
+        for axis in range(3):
+            p[rng.integers(a, b), axis] = -0.0
+    assert (p * sign).min() == 0
+    b = DeviceBatch.from_host(D.Batch(p[:, 0].copy(), p[:, 1].copy(), p[:, 2].copy(), offs))
+    s = PlaneScorer(n, len(sizes), ctx=gpu_ctx)
+    cand = torch.arange(n, dtype=torch.int32, device="cuda")
+    coffs = torch.from_numpy(offs).cuda()
+    every = s.features(b, 1.0).cpu().numpy()
+    among = s.features(b, 1.0, cand, coffs, among_candidates=True).cpu().numpy()
+    s.close()
+    assert np.array_equal(bits(every), bits(among))
+    c = D.Cloud.from_xyz(p)
+    got = api.euclidean_clusters(c, 0.3)
+    want = restatement.euclidean_clusters(c, 0.3)
+    assert len(got) == len(want) and all(np.array_equal(g, w) for g, w in zip(got, want))
+    h = api.SpatialHash()
+    h.setHashPrimes(1, 1)  # (the reference's buckets)
+    h.setInputCloud(c, 0.5)
+    h.build()
+    o, i, _ = h.radiusSearchBatch(c.x, c.y, c.z, 0.3)
+    o2, i2, _ = restatement.radius_search(c, 0.5, 0.3, p1=1, p2=1)
+    assert np.array_equal(o, o2) and np.array_equal(i, i2)
