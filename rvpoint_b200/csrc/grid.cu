@@ -625,22 +625,26 @@ __global__ __launch_bounds__(1024) void k_sort_big(const u64 *offsets, u64 *pair
       for (u64 i = threadIdx.x; i < cnt; i += blockDim.x) a[i] = sb[i];
       __syncthreads();
     } else {
-      // virtual padding: indices >= cnt hold +inf and never move
-      for (u64 k = 2; k <= P; k <<= 1)
-        for (u64 j = k >> 1; j > 0; j >>= 1) {
-          for (u64 i = threadIdx.x; i < P; i += blockDim.x) {
-            const u64 l = i ^ j;
-            if (l > i) {
-              const u64 x = i < cnt ? a[i] : ~0ull;
-              const u64 y = l < cnt ? a[l] : ~0ull;
-              if ((x > y) == ((i & k) == 0)) {
-                if (i < cnt) a[i] = y;
-                if (l < cnt) a[l] = x;
-              }
+      // every comparison puts the smaller key at the lower place (each merge
+      // starts with mirrored places), so that the places past cnt, which would
+      // hold +inf, need not be there
+      auto step = [&](u64 mask) {
+        for (u64 i = threadIdx.x; i < cnt; i += blockDim.x) {
+          const u64 l = i ^ mask;
+          if (l > i && l < cnt) {
+            const u64 x = a[i], y = a[l];
+            if (x > y) {
+              a[i] = y;
+              a[l] = x;
             }
           }
-          __syncthreads();
         }
+        __syncthreads();
+      };
+      for (u64 k = 2; k <= P; k <<= 1) {
+        step(k - 1);
+        for (u64 j = k >> 2; j > 0; j >>= 1) step(j);
+      }
     }
   }
 }

@@ -710,3 +710,26 @@ def test_frames_of_few_points(gpu_ctx, sor_k, normal_k):
     for g in got[:2]:
         for key in g:
             assert np.array_equal(np.asarray(g[key]), np.asarray(got[2][key]), equal_nan=True), key
+
+
+# lists past the 8192 pairs that a block sorts in shared memory
+@pytest.mark.parametrize("n", [8192, 8193, 9729, 20_000])
+@pytest.mark.parametrize("same", [False, True])  # all points in one place
+def test_very_long_lists(gpu_ctx, restatement, n, same):
+    from rvpoint_b200 import api
+    rng = np.random.default_rng(n)
+    p = np.zeros((n, 3)) if same else rng.normal(0, 0.1, (n, 3))
+    p = p.astype(np.float32)
+    h = api.SpatialHash()
+    h.setInputCloud((p[:, 0], p[:, 1], p[:, 2]), 0.5)
+    h.build()
+    q = np.concatenate([p[:20], p[:5] + np.float32(0.3)])
+    offs, idx, d2 = h.radiusSearchBatch(*q.T, 1.5)
+    o2, i2, e2 = brute_radius(p, q, 1.5)
+    assert np.array_equal(offs, o2) and np.diff(offs).max() == n
+    assert np.array_equal(idx, i2) and np.array_equal(bits(d2), bits(e2))
+    if n < 10_000 and not same:
+        c = D.Cloud.from_xyz(p)
+        got = np.stack(api.normal_estimation_rvv(c, h, 10, 1.5), 1)
+        want = np.asarray(restatement.normals_radius(c, 0.5, 1.5))
+        assert (np.abs(got - want).max(1) < 1e-4).mean() > 0.995
