@@ -900,10 +900,15 @@ rvp_status rvp_normals_radius(rvp_hash *h, float radius, float vp_x, float vp_y,
     } else {
       u32 *hard = static_cast<u32 *>(scratch(ctx, 15, n * 12 + 16));
       u32 *longer = hard + n, *huge = longer + n;
+      u32 *counts = huge + n;
       rvp::tree_radius_normals(ctx, h->tree_view, radius, eigen_iters, vp_x, vp_y, vp_z, dnx, dny,
-                               dnz, hard, longer, huge, huge + n);
-      const u32 m = read_back(ctx, huge + n + 2);
-      if (m) from_lists(huge, m);
+                               dnz, hard, longer, counts);
+      if (read_back(ctx, counts + 1)) {  // (seldom)
+        rvp::tree_radius_normals_longer(ctx, h->tree_view, radius, eigen_iters, vp_x, vp_y, vp_z,
+                                        dnx, dny, dnz, longer, huge, counts);
+        const u32 m = read_back(ctx, counts + 2);
+        if (m) from_lists(huge, m);
+      }
     }
     out_copy(ctx, nx, dnx, n, mem);
     out_copy(ctx, ny, dny, n, mem);

@@ -523,11 +523,15 @@ void tree_radius_fill(rvp_context *ctx, const TreeView &t, const TreeQueries &q,
                       const float *qy, const float *qz, float radius, const u64 *full,
                       const u64 *offsets, u32 cut, u32 n_long, int32_t *idx, float *d2,
                       u64 *big_pairs, u32 *big, u32 *big_count);
-// normals of the cloud's own points; the counts[2] points past
-// tree_radius_cap() neighbours are left, listed in huge (hard, longer: room for n)
+// normals of the cloud's own points; the counts[1] points with lists too long
+// for a short block are left, listed in longer (hard, longer: room for n), and of
+// these by the second call the counts[2] past tree_radius_cap(), listed in huge
 void tree_radius_normals(rvp_context *ctx, const TreeView &t, float radius, int iters, float vpx,
                          float vpy, float vpz, float *nx, float *ny, float *nz, u32 *hard,
-                         u32 *longer, u32 *huge, u32 *counts);
+                         u32 *longer, u32 *counts);
+void tree_radius_normals_longer(rvp_context *ctx, const TreeView &t, float radius, int iters,
+                                float vpx, float vpy, float vpz, float *nx, float *ny, float *nz,
+                                const u32 *longer, u32 *huge, u32 *counts);
 void gather_queries(rvp_context *ctx, const float *x, const float *y, const float *z,
                     const u32 *list, size_t n, float *qx, float *qy, float *qz);
 

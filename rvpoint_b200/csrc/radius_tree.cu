@@ -652,7 +652,7 @@ void tree_radius_fill(rvp_context *ctx, const TreeView &t, const TreeQueries &q,
 
 void tree_radius_normals(rvp_context *ctx, const TreeView &t, float radius, int iters, float vpx,
                          float vpy, float vpz, float *nx, float *ny, float *nz, u32 *hard,
-                         u32 *longer, u32 *huge, u32 *counts) {
+                         u32 *longer, u32 *counts) {
   const float r2 = square_of(radius);
   RVP_CUDA_TRY(cudaMemsetAsync(counts, 0, 12, ctx->stream));
   const bool few = t.n <= kFewNormals;
@@ -667,6 +667,12 @@ void tree_radius_normals(rvp_context *ctx, const TreeView &t, float radius, int 
           t, r2, iters, vpx, vpy, vpz, nx, ny, nz, few ? nullptr : hard, counts, longer, counts + 1,
           false);
   RVP_LAUNCH_CHECK(ctx);
+}
+
+void tree_radius_normals_longer(rvp_context *ctx, const TreeView &t, float radius, int iters,
+                                float vpx, float vpy, float vpz, float *nx, float *ny, float *nz,
+                                const u32 *longer, u32 *huge, u32 *counts) {
+  const float r2 = square_of(radius);
   k_radius_normals_listed<FT_CAP, FT_BINS>
       <<<grid_for(t.n, 1, ctx->num_sms * 9), 32, 0, ctx->stream>>>(
           t, r2, iters, vpx, vpy, vpz, nx, ny, nz, longer, counts + 1, huge, counts + 2, true);
